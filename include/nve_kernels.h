@@ -220,8 +220,8 @@ NVE_API int nve_b200_silu_mul(void* gate, const void* up, int n, int dtype, nve_
  *   caches (which already hold the block); out has q's layout.  Replaces the unfused masked SDPA of
  *   src/gpu_layer.rs:846-885.  Blocks of fewer than 64 (row, KV head) pairs run the decode kernel with the row as
  *   second grid dimension: every row equals a nve_flash_decode_f16 call of length start_pos + r + 1 bit for bit.
- *   Larger blocks run a tensor-core kernel (one CTA per row and KV head; f16 probabilities, another summation
- *   order): equal to those calls within 5e-3 of the largest output.  head_dim 64 or 128; q and caches 16-byte
+ *   Larger blocks run a tiled tensor-core kernel (128 query rows share the K/V they read; f16 probabilities, another
+ *   summation order): equal to those calls within 5e-3 of the largest output.  head_dim 64 or 128; q and caches 16-byte
  *   aligned. */
 NVE_API int nve_b200_rms_norm_rows(const void* x, const void* weight, void* out, int rows, int n, float eps, int dtype,
                                    nve_stream_t stream);
@@ -330,7 +330,7 @@ NVE_API int nve_b200_quantize_matvec_w4a8_allreduce(const void* x, int x_dtype, 
  * flash-decode and quantise launches of this library.
  * Two attention kernels exist and nve_flash_decode_f16 / _dyn, nve_b200_attn_prefill_causal (small blocks) and this
  * entry point always run the same one: by default a tensor-core kernel (a cluster of 8 CTAs per KV head, all its
- * query heads as rows of mma.sync, f16 probabilities) when there are 1, 2, 4 or 8 query heads per KV head and the
+ * query heads as rows of mma.sync, f16 probabilities) when there are up to 8 query heads per KV head and the
  * pointers are 16-byte aligned; nve_b200_set_attn_decode_kernel(1) selects the CUDA-core kernel for all of them
  * (also used for other shapes; it is the arithmetic of the persistent one-kernel step), 0 restores the default.  The
  * two kernels agree within 5e-3 of the largest output.  The setting is process-wide, a captured graph keeps the
@@ -347,7 +347,7 @@ NVE_API int nve_b200_set_attn_decode_kernel(int mode);
  * The cache row written is bit-identical to a single-sequence call.  Up to 63 (sequence, KV head) units the clustered
  * decode kernel that nve_b200_attn_decode_fused would launch (see nve_b200_set_attn_decode_kernel) runs with the
  * sequence as second grid dimension and row b of out [batch, nh*hd] is bit-identical too;
- * from 64 units on (and 1, 2, 4 or 8 query heads per KV head) one CTA per unit streams all positions and computes
+ * from 64 units on (and up to 8 query heads per KV head) one CTA per unit streams all positions and computes
  * q.K^T and p.V with mma.sync (probabilities rounded to f16): rows then agree with the single-sequence call to about
  * 1e-3 of their RMS.  q / k_new / v_new and the caches 16-byte aligned. */
 NVE_API int nve_b200_attn_decode_fused_batch(const uint16_t* q, const uint16_t* k_new, const uint16_t* v_new,

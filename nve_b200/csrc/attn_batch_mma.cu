@@ -26,26 +26,21 @@
 
 namespace nve {
 
-template <int HD, int G, bool FUSED>
+template <int HD, int G>
 __global__ void __launch_bounds__(kAmThreads, 2) attn_batch_mma_kernel(const AttnParams pin) {
     constexpr int DC = HD / 8;        // 16-byte chunks per row
     constexpr int NT = HD / 8;        // output dim tiles = dims of a V row per lane
     static_assert((HD == 64 || HD == 128) && G >= 1 && G <= 8, "head_dim 64 or 128, up to 8 query heads per KV head");
     AttnParams p = pin;
-    if constexpr (FUSED) {
-        const long long b = blockIdx.y;
-        p.q += b * (static_cast<long long>(p.num_heads) * HD);
-        p.out += b * (static_cast<long long>(p.num_heads) * HD);
-        p.k_new += b * (static_cast<long long>(p.num_kv_heads) * HD);
-        p.v_new += b * (static_cast<long long>(p.num_kv_heads) * HD);
-        p.k_cache += b * p.cache_stride;
-        p.v_cache += b * p.cache_stride;
-        p.d_pos += b;
-        p.d_seq_len += b;
-    } else {  // causal block: row blockIdx.y of q attends to seq_len + row positions of the one cache
-        p.q += static_cast<long long>(blockIdx.y) * p.row_stride;
-        p.out += static_cast<long long>(blockIdx.y) * p.row_stride;
-    }
+    const long long b = blockIdx.y;
+    p.q += b * (static_cast<long long>(p.num_heads) * HD);
+    p.out += b * (static_cast<long long>(p.num_heads) * HD);
+    p.k_new += b * (static_cast<long long>(p.num_kv_heads) * HD);
+    p.v_new += b * (static_cast<long long>(p.num_kv_heads) * HD);
+    p.k_cache += b * p.cache_stride;
+    p.v_cache += b * p.cache_stride;
+    p.d_pos += b;
+    p.d_seq_len += b;
     __shared__ AmShared<HD, G> sh;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
@@ -55,25 +50,18 @@ __global__ void __launch_bounds__(kAmThreads, 2) attn_batch_mma_kernel(const Att
     uint16_t* vh = p.v_cache + static_cast<long long>(kvh) * p.kv_stride * HD;
 
     pdl_wait();
-    int seq_len;
-    if constexpr (FUSED) {
-        seq_len = max(0, min(*p.d_seq_len, p.kv_stride));
-        const int pos = *p.d_pos;
-        const bool pos_ok = pos >= 0 && pos < p.kv_stride;
-        attn_stage_q<HD, G, true>(sh, tid, p.q, p.k_new, p.v_new, p.cos_tab, p.sin_tab, h0, kvh, pos, pos_ok);
-        __syncthreads();
-        pdl_launch_dependents();
-        // the new row goes to the cache first and is read back from there like every other row (same CTA: the barrier
-        // orders the store before the loads, which are ordinary coherent loads)
-        if (pos_ok && tid < 2 * DC) {
-            const int which = tid / DC, d = tid % DC;
-            uint16_t* dst = (which == 0 ? kh : vh) + static_cast<long long>(pos) * HD;
-            reinterpret_cast<uint4*>(dst)[d] = reinterpret_cast<const uint4*>(which == 0 ? sh.knew_s : sh.vnew_s)[d];
-        }
-    } else {
-        seq_len = max(0, min(p.seq_len + static_cast<int>(blockIdx.y), p.kv_stride));
-        attn_stage_q<HD, G, false>(sh, tid, p.q, nullptr, nullptr, nullptr, nullptr, h0, kvh, 0, false);
-        pdl_launch_dependents();
+    const int seq_len = max(0, min(*p.d_seq_len, p.kv_stride));
+    const int pos = *p.d_pos;
+    const bool pos_ok = pos >= 0 && pos < p.kv_stride;
+    attn_stage_q<HD, G, true>(sh, tid, p.q, p.k_new, p.v_new, p.cos_tab, p.sin_tab, h0, kvh, pos, pos_ok);
+    __syncthreads();
+    pdl_launch_dependents();
+    // the new row goes to the cache first and is read back from there like every other row (same CTA: the barrier
+    // orders the store before the loads, which are ordinary coherent loads)
+    if (pos_ok && tid < 2 * DC) {
+        const int which = tid / DC, d = tid % DC;
+        uint16_t* dst = (which == 0 ? kh : vh) + static_cast<long long>(pos) * HD;
+        reinterpret_cast<uint4*>(dst)[d] = reinterpret_cast<const uint4*>(which == 0 ? sh.knew_s : sh.vnew_s)[d];
     }
     __syncthreads();
 
@@ -103,7 +91,7 @@ __global__ void __launch_bounds__(kAmThreads, 2) attn_batch_mma_kernel(const Att
     }
 }
 
-template <int HD, int G> static cudaError_t launch_am(const AttnParams& p, cudaStream_t st, bool fused) {
+template <int HD, int G> static cudaError_t launch_am(const AttnParams& p, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p.num_kv_heads, p.rows);
     cfg.blockDim = dim3(kAmThreads);
@@ -115,30 +103,26 @@ template <int HD, int G> static cudaError_t launch_am(const AttnParams& p, cudaS
         cfg.attrs = attr;
         cfg.numAttrs = 1;
     }
-    return fused ? cudaLaunchKernelEx(&cfg, attn_batch_mma_kernel<HD, G, true>, p)
-                 : cudaLaunchKernelEx(&cfg, attn_batch_mma_kernel<HD, G, false>, p);
+    return cudaLaunchKernelEx(&cfg, attn_batch_mma_kernel<HD, G>, p);
 }
 
-bool attn_batch_mma_try(const AttnParams& p, int head_dim, cudaStream_t st, cudaError_t& err, bool fused) {
-    const int groups = p.num_heads / p.num_kv_heads;
-    if (head_dim == 128) {
-        switch (groups) {
-            case 1: err = launch_am<128, 1>(p, st, fused); return true;
-            case 2: err = launch_am<128, 2>(p, st, fused); return true;
-            case 4: err = launch_am<128, 4>(p, st, fused); return true;
-            case 8: err = launch_am<128, 8>(p, st, fused); return true;
-            default: return false;
-        }
+template <int HD> static bool launch_am_groups(const AttnParams& p, cudaStream_t st, cudaError_t& err) {
+    switch (p.num_heads / p.num_kv_heads) {
+        case 1: err = launch_am<HD, 1>(p, st); return true;
+        case 2: err = launch_am<HD, 2>(p, st); return true;
+        case 3: err = launch_am<HD, 3>(p, st); return true;
+        case 4: err = launch_am<HD, 4>(p, st); return true;
+        case 5: err = launch_am<HD, 5>(p, st); return true;
+        case 6: err = launch_am<HD, 6>(p, st); return true;
+        case 7: err = launch_am<HD, 7>(p, st); return true;
+        case 8: err = launch_am<HD, 8>(p, st); return true;
+        default: return false;
     }
-    if (head_dim == 64) {
-        switch (groups) {
-            case 1: err = launch_am<64, 1>(p, st, fused); return true;
-            case 2: err = launch_am<64, 2>(p, st, fused); return true;
-            case 4: err = launch_am<64, 4>(p, st, fused); return true;
-            case 8: err = launch_am<64, 8>(p, st, fused); return true;
-            default: return false;
-        }
-    }
+}
+
+bool attn_batch_mma_try(const AttnParams& p, int head_dim, cudaStream_t st, cudaError_t& err) {
+    if (head_dim == 128) return launch_am_groups<128>(p, st, err);
+    if (head_dim == 64) return launch_am_groups<64>(p, st, err);
     return false;
 }
 

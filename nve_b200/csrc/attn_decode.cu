@@ -269,7 +269,7 @@ extern "C" int nve_b200_attn_decode_fused(const uint16_t* q, const uint16_t* k_n
 }
 
 /* Which kernel nve_b200_attn_decode_fused launches: 0 (default) = the tensor-core kernel where it covers the shape
- * (head_dim 64 / 128, 1, 2, 4 or 8 query heads per KV head), 1 = always the CUDA-core kernel, whose output equals the
+ * (head_dim 64 / 128, up to 8 query heads per KV head), 1 = always the CUDA-core kernel, whose output equals the
  * un-fused sequence RoPE -> K/V write -> nve_flash_decode_f16 bit for bit.  Process-wide; a captured graph keeps the
  * kernel it was recorded with.  Returns the previous setting. */
 extern "C" int nve_b200_set_attn_decode_kernel(int mode) {
@@ -279,8 +279,8 @@ extern "C" int nve_b200_set_attn_decode_kernel(int mode) {
 /* Causal attention of a block of S new positions against the cache (which already holds them): row r of q
  * [S, num_heads * head_dim] attends to positions [0, start_pos + r]; out has q's layout.  One launch.  Small blocks
  * (fewer than 64 (row, KV head) pairs) run the decode kernel with the row as second grid dimension, so every row
- * equals a nve_flash_decode_f16 call of that length bit for bit; larger ones run the tensor-core kernel of
- * attn_batch_mma.cu (one CTA per row and KV head, scores and outputs on mma.sync), equal to it within rounding. */
+ * equals a nve_flash_decode_f16 call of that length bit for bit; larger ones run the tiled kernel of
+ * attn_prefill_mma.cu (128 query rows share the K/V they read), equal to it within rounding. */
 extern "C" int nve_b200_attn_prefill_causal(const uint16_t* q, const uint16_t* k_cache, const uint16_t* v_cache, uint16_t* out,
                                             int rows, int start_pos, int num_heads, int num_kv_heads, int head_dim,
                                             int max_seq_len, float scale, nve_stream_t stream) {
@@ -300,7 +300,9 @@ extern "C" int nve_b200_attn_prefill_causal(const uint16_t* q, const uint16_t* k
     p.rows = rows;
     p.row_stride = num_heads * head_dim;
     cudaError_t e = cudaSuccess;
-    if (static_cast<long long>(rows) * num_kv_heads >= 64 && attn_batch_mma_try(p, head_dim, static_cast<cudaStream_t>(stream), e, false)) {
+    // a masked score times the scale has to stay -inf, hence scale > 0; whole tiles are stored in 16-byte pieces
+    if (static_cast<long long>(rows) * num_kv_heads >= 64 && scale > 0.0f && aligned(out, 16) &&
+        attn_prefill_mma_try(p, head_dim, static_cast<cudaStream_t>(stream), e)) {
         count_launch();
         return set_cuda_status(e);
     }

@@ -333,28 +333,25 @@ template <int HD, int G> static cudaError_t launch_adm(const AttnParams& p, cuda
     return fused ? launch_adm_f<HD, G, true>(p, st) : launch_adm_f<HD, G, false>(p, st);
 }
 
-// Fused decode attention of one sequence; false when the shape is not covered (query heads per KV head other than
-// 1, 2, 4 or 8, other head sizes): the caller then uses the CUDA-core kernel.
+template <int HD> static bool launch_adm_groups(const AttnParams& p, cudaStream_t st, cudaError_t& err, bool fused) {
+    switch (p.num_heads / p.num_kv_heads) {
+        case 1: err = launch_adm<HD, 1>(p, st, fused); return true;
+        case 2: err = launch_adm<HD, 2>(p, st, fused); return true;
+        case 3: err = launch_adm<HD, 3>(p, st, fused); return true;
+        case 4: err = launch_adm<HD, 4>(p, st, fused); return true;
+        case 5: err = launch_adm<HD, 5>(p, st, fused); return true;
+        case 6: err = launch_adm<HD, 6>(p, st, fused); return true;
+        case 7: err = launch_adm<HD, 7>(p, st, fused); return true;
+        case 8: err = launch_adm<HD, 8>(p, st, fused); return true;
+        default: return false;
+    }
+}
+
+// Decode attention of one or a few sequences; false when the shape is not covered (more than 8 query heads per KV head,
+// other head sizes): the caller then uses the CUDA-core kernel.
 bool attn_decode_mma_try(const AttnParams& p, int head_dim, cudaStream_t st, cudaError_t& err, bool fused) {
-    const int groups = p.num_heads / p.num_kv_heads;
-    if (head_dim == 128) {
-        switch (groups) {
-            case 1: err = launch_adm<128, 1>(p, st, fused); return true;
-            case 2: err = launch_adm<128, 2>(p, st, fused); return true;
-            case 4: err = launch_adm<128, 4>(p, st, fused); return true;
-            case 8: err = launch_adm<128, 8>(p, st, fused); return true;
-            default: return false;
-        }
-    }
-    if (head_dim == 64) {
-        switch (groups) {
-            case 1: err = launch_adm<64, 1>(p, st, fused); return true;
-            case 2: err = launch_adm<64, 2>(p, st, fused); return true;
-            case 4: err = launch_adm<64, 4>(p, st, fused); return true;
-            case 8: err = launch_adm<64, 8>(p, st, fused); return true;
-            default: return false;
-        }
-    }
+    if (head_dim == 128) return launch_adm_groups<128>(p, st, err, fused);
+    if (head_dim == 64) return launch_adm_groups<64>(p, st, err, fused);
     return false;
 }
 

@@ -27,9 +27,12 @@ struct AttnParams {
     long long cache_stride;
 };
 
-// attn_batch_mma.cu: false when the shape is not covered (the caller then uses another kernel).  fused: `rows`
-// independent sequences with RoPE and the K/V write inside; else the un-fused causal block described above.
-bool attn_batch_mma_try(const AttnParams& p, int head_dim, cudaStream_t st, cudaError_t& err, bool fused = true);
+// attn_batch_mma.cu: `rows` independent sequences with RoPE and the K/V write inside; false when the shape is not
+// covered (the caller then uses another kernel).
+bool attn_batch_mma_try(const AttnParams& p, int head_dim, cudaStream_t st, cudaError_t& err);
+
+// attn_prefill_mma.cu: the causal block described above, in tiles of query rows; false when the shape is not covered.
+bool attn_prefill_mma_try(const AttnParams& p, int head_dim, cudaStream_t st, cudaError_t& err);
 
 // attn_decode_mma.cu: the fused decode attention of one sequence on the tensor cores; false when the shape is not
 // covered.

@@ -1,0 +1,335 @@
+// Causal attention of a block of new positions (prefill) on the tensor cores: tiles of 128 query rows against tiles
+// of 64 cached positions, online softmax, K/V staged in shared memory once per tile and used by all its rows.
+//
+// What bounds it: with one CTA per (row, KV head) every row read the whole K/V prefix through L2 by itself (1777 rows
+// of an 8B model: 1.58 M (row, position) pairs x 512 bytes x 8 KV heads = 6.5 GB per layer); a tile of 128 rows reads
+// it 128 / G times less often and the kernel is bound by the mma.sync rate instead.  Whole prefill passes before / after:
+// 8B, 1777 positions 57.4 -> 31.8 ms; 3B (3 query heads per KV head), 300 positions at 700 20.7 -> 7.6 ms.
+//
+// A query row of a tile is a (position, head) pair of ONE KV head: row r of a tile is position t * PT + r / G, head
+// h0 + r % G with PT = 128 / G positions per tile.  All G heads of the group share the staged K/V, and a short block
+// (61 rows x 4 heads) fills its tiles; any group size works.  Four warps take 32 rows each (two m16 row blocks, so that
+// every K / V fragment that is read from shared memory feeds two MMAs).
+//
+// Few tiles (a short block behind a long prefix) would leave most SMs idle: a cluster of 2, 4 or 8 CTAs then splits
+// the positions of one tile, leaves unnormalised partials in shared memory and every CTA merges 128 / C of the rows
+// through distributed shared memory.
+#include <cooperative_groups.h>
+
+#include "attn_mma.cuh"
+#include "attn_params.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace nve {
+
+constexpr int kApRows = 128;     // query rows per tile
+constexpr int kApKeys = 64;      // cached positions per step
+constexpr int kApThreads = 128;  // four warps of 32 rows
+
+__device__ __forceinline__ uint32_t ap_smem(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ void ap_cp16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void ap_ldm4(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr)
+                 : "memory");
+}
+__device__ __forceinline__ void ap_ldm4t(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr)
+                 : "memory");
+}
+__device__ __forceinline__ float ap_exp2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// byte offset of 16-byte chunk c of row r in a tile of HD f16 per row; chunks XORed with the row so that the eight
+// rows of an 8x8 matrix lie in eight different bank groups
+template <int HD> __device__ __forceinline__ uint32_t ap_off(int r, int c) {
+    return static_cast<uint32_t>(r * (HD * 2) + ((c ^ (r & 7)) << 4));
+}
+
+template <int HD> constexpr int ap_smem_bytes() {
+    constexpr int stage = kApRows * HD * 2 + 4 * kApKeys * HD * 2;  // Q, two K and two V tiles
+    constexpr int part = kApRows * (HD + 4) * 4 + kApRows * 8;      // f32 partials of a split tile + their m, l
+    return stage > part ? stage : part;
+}
+
+template <int HD>
+__global__ void __launch_bounds__(kApThreads, 2) attn_prefill_mma_kernel(const AttnParams p, int groups, int tiles) {
+    extern __shared__ __align__(128) unsigned char ap_raw[];
+    constexpr int CH = HD / 8;  // 16-byte chunks per row
+    constexpr int KVB = kApKeys * HD * 2;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int csize = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
+    const int tile = tiles - 1 - static_cast<int>(blockIdx.x) / csize;  // the tiles with the longest prefix first
+    const int kvh = blockIdx.y;
+    const int h0 = kvh * groups;
+    const int PT = kApRows / groups;
+    const int pos0 = tile * PT;                    // first block row of the tile
+    const int npos = min(PT, p.rows - pos0);
+    const int nrows = npos * groups;               // valid query rows
+    const int start = p.seq_len - 1;               // position of block row 0
+    const uint16_t* kh = p.k_cache + static_cast<long long>(kvh) * p.kv_stride * HD;
+    const uint16_t* vh = p.v_cache + static_cast<long long>(kvh) * p.kv_stride * HD;
+    const uint32_t sq = ap_smem(ap_raw), sk = sq + kApRows * HD * 2, sv = sk + 2 * KVB;
+
+    const int kend = start + pos0 + npos;          // positions that the last row of the tile sees
+    const int nkt = (kend + kApKeys - 1) / kApKeys;
+    const int per = (nkt + csize - 1) / csize;
+    const int kt0 = rank * per, kt1 = min(nkt, kt0 + per);
+
+    pdl_wait();
+    pdl_launch_dependents();
+    auto load_kv = [&](int kt, int buf) {
+#pragma unroll
+        for (int i = 0; i < kApKeys * CH / kApThreads; i++) {
+            const int id = tid + i * kApThreads;
+            const int r = id / CH, c = id % CH;
+            // rows past the end repeat the last one: finite values, masked below
+            const long long src = static_cast<long long>(min(kt * kApKeys + r, kend - 1)) * HD + c * 8;
+            ap_cp16(sk + buf * KVB + ap_off<HD>(r, c), kh + src);
+            ap_cp16(sv + buf * KVB + ap_off<HD>(r, c), vh + src);
+        }
+    };
+    for (int id = tid; id < kApRows * CH; id += kApThreads) {
+        const int r = min(id / CH, nrows - 1), c = id % CH;
+        const int pr = r / groups, h = r - pr * groups;
+        ap_cp16(sq + ap_off<HD>(id / CH, c), p.q + static_cast<long long>(pos0 + pr) * p.row_stride + (h0 + h) * HD + c * 8);
+    }
+    if (kt0 < kt1) load_kv(kt0, 0);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+
+    // this thread's four query rows: row block mt (16 rows), rows g and g + 8 of it; lim = positions the row may see
+    int lim[2][2];
+#pragma unroll
+    for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+        for (int hh = 0; hh < 2; hh++) {
+            const int r = warp * 32 + mt * 16 + hh * 8 + g;
+            lim[mt][hh] = start + pos0 + min(r, nrows - 1) / groups + 1;
+        }
+    const int lim_min = start + pos0 + 1;
+    const float sl2 = p.scale * 1.4426950408889634f;  // exponentials in base 2
+    float m[2][2], l[2][2];
+    float o[2][CH][4];
+#pragma unroll
+    for (int mt = 0; mt < 2; mt++) {
+        m[mt][0] = m[mt][1] = -1e30f;
+        l[mt][0] = l[mt][1] = 0.0f;
+#pragma unroll
+        for (int j = 0; j < CH; j++) o[mt][j][0] = o[mt][j][1] = o[mt][j][2] = o[mt][j][3] = 0.0f;
+    }
+
+    for (int kt = kt0; kt < kt1; kt++) {
+        const int buf = (kt - kt0) & 1;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();  // the tile is there, and everyone is done with the other buffer
+        if (kt + 1 < kt1) load_kv(kt + 1, buf ^ 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+
+        float s[2][8][4];
+#pragma unroll
+        for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+            for (int n = 0; n < 8; n++) s[mt][n][0] = s[mt][n][1] = s[mt][n][2] = s[mt][n][3] = 0.0f;
+        const uint32_t kb = sk + buf * KVB, vb = sv + buf * KVB;
+#pragma unroll
+        for (int kk = 0; kk < HD / 16; kk++) {
+            uint32_t qa[2][4];
+#pragma unroll
+            for (int mt = 0; mt < 2; mt++)
+                ap_ldm4(sq + ap_off<HD>(warp * 32 + mt * 16 + (lane & 15), 2 * kk + (lane >> 4)), qa[mt]);
+#pragma unroll
+            for (int np = 0; np < 4; np++) {
+                uint32_t b[4];  // positions np*16 .. +7 (b0, b1) and +8 .. +15 (b2, b3)
+                ap_ldm4(kb + ap_off<HD>(np * 16 + (lane & 7) + ((lane >> 4) << 3), 2 * kk + ((lane >> 3) & 1)), b);
+#pragma unroll
+                for (int mt = 0; mt < 2; mt++) {
+                    mma_f16_16816(s[mt][2 * np], qa[mt], b[0], b[1]);
+                    mma_f16_16816(s[mt][2 * np + 1], qa[mt], b[2], b[3]);
+                }
+            }
+        }
+        if ((kt + 1) * kApKeys > lim_min) {  // some row does not see the whole tile
+#pragma unroll
+            for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+                for (int n = 0; n < 8; n++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++)
+                        if (kt * kApKeys + n * 8 + 2 * t + (e & 1) >= lim[mt][e >> 1]) s[mt][n][e] = -INFINITY;
+        }
+        uint32_t pa[2][4][4];
+#pragma unroll
+        for (int mt = 0; mt < 2; mt++) {
+#pragma unroll
+            for (int hh = 0; hh < 2; hh++) {
+                float mx = s[mt][0][2 * hh];
+#pragma unroll
+                for (int n = 0; n < 8; n++) mx = fmaxf(mx, fmaxf(s[mt][n][2 * hh], s[mt][n][2 * hh + 1]));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+                const float mn = fmaxf(m[mt][hh], mx * sl2);  // stays finite: the masked value is below -1e30
+                const float corr = ap_exp2(m[mt][hh] - mn);
+                m[mt][hh] = mn;
+                float sum = 0.0f;
+#pragma unroll
+                for (int n = 0; n < 8; n++) {
+                    s[mt][n][2 * hh] = ap_exp2(fmaf(s[mt][n][2 * hh], sl2, -mn));
+                    s[mt][n][2 * hh + 1] = ap_exp2(fmaf(s[mt][n][2 * hh + 1], sl2, -mn));
+                    sum += s[mt][n][2 * hh] + s[mt][n][2 * hh + 1];
+                }
+                l[mt][hh] = l[mt][hh] * corr + sum;
+#pragma unroll
+                for (int j = 0; j < CH; j++) {
+                    o[mt][j][2 * hh] *= corr;
+                    o[mt][j][2 * hh + 1] *= corr;
+                }
+            }
+#pragma unroll
+            for (int kp = 0; kp < 4; kp++) {  // probabilities of 16 positions as the A operand of the second product
+                pa[mt][kp][0] = pack_f16x2(s[mt][2 * kp][0], s[mt][2 * kp][1]);
+                pa[mt][kp][1] = pack_f16x2(s[mt][2 * kp][2], s[mt][2 * kp][3]);
+                pa[mt][kp][2] = pack_f16x2(s[mt][2 * kp + 1][0], s[mt][2 * kp + 1][1]);
+                pa[mt][kp][3] = pack_f16x2(s[mt][2 * kp + 1][2], s[mt][2 * kp + 1][3]);
+            }
+        }
+#pragma unroll
+        for (int kp = 0; kp < 4; kp++)
+#pragma unroll
+            for (int dp = 0; dp < HD / 16; dp++) {
+                uint32_t b[4];  // dims dp*16 .. +7 (b0, b1) and +8 .. +15 (b2, b3) of positions kp*16 .. +15
+                ap_ldm4t(vb + ap_off<HD>(kp * 16 + (lane & 15), 2 * dp + (lane >> 4)), b);
+#pragma unroll
+                for (int mt = 0; mt < 2; mt++) {
+                    mma_f16_16816(o[mt][2 * dp], pa[mt][kp], b[0], b[1]);
+                    mma_f16_16816(o[mt][2 * dp + 1], pa[mt][kp], b[2], b[3]);
+                }
+            }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+    for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+        for (int hh = 0; hh < 2; hh++) {
+            l[mt][hh] += __shfl_xor_sync(0xffffffffu, l[mt][hh], 1);
+            l[mt][hh] += __shfl_xor_sync(0xffffffffu, l[mt][hh], 2);
+        }
+    __syncthreads();  // the staged tiles are no longer read: the buffers are free
+
+    if (csize == 1) {
+        // rows through shared memory (each warp its own 32) so that they leave in 16-byte pieces
+#pragma unroll
+        for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+            for (int hh = 0; hh < 2; hh++) {
+                const int r = warp * 32 + mt * 16 + hh * 8 + g;
+                const float inv = l[mt][hh] > 0.0f ? 1.0f / l[mt][hh] : 0.0f;
+#pragma unroll
+                for (int j = 0; j < CH; j++)
+                    *reinterpret_cast<uint32_t*>(ap_raw + ap_off<HD>(r, j) + 4 * t) =
+                        pack_f16x2(o[mt][j][2 * hh] * inv, o[mt][j][2 * hh + 1] * inv);
+            }
+        __syncwarp();
+        for (int id = lane; id < 32 * CH; id += 32) {
+            const int r = warp * 32 + id / CH, c = id % CH;
+            if (r < nrows) {
+                const int pr = r / groups, h = r - pr * groups;
+                *reinterpret_cast<uint4*>(p.out + static_cast<long long>(pos0 + pr) * p.row_stride + (h0 + h) * HD + c * 8) =
+                    *reinterpret_cast<const uint4*>(ap_raw + ap_off<HD>(r, c));
+            }
+        }
+        return;
+    }
+    // ---- split tile: unnormalised partials in shared memory, merged across the cluster
+    constexpr int PR = HD + 4;  // floats per partial row
+    float* part = reinterpret_cast<float*>(ap_raw);
+    float* pm = part + kApRows * PR;
+    float* pl = pm + kApRows;
+#pragma unroll
+    for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+        for (int hh = 0; hh < 2; hh++) {
+            const int r = warp * 32 + mt * 16 + hh * 8 + g;
+            if (t == 0) {
+                pm[r] = m[mt][hh];
+                pl[r] = l[mt][hh];
+            }
+#pragma unroll
+            for (int j = 0; j < CH; j++)
+                *reinterpret_cast<float2*>(part + r * PR + j * 8 + 2 * t) = make_float2(o[mt][j][2 * hh], o[mt][j][2 * hh + 1]);
+        }
+    cluster.sync();
+    const int rows_per = kApRows / csize;
+    for (int id = tid; id < rows_per * (HD / 4); id += kApThreads) {
+        const int r = rank * rows_per + id / (HD / 4), c = id % (HD / 4);
+        if (r >= nrows) continue;
+        float mm = -1e30f;
+        for (int k = 0; k < csize; k++) mm = fmaxf(mm, cluster.map_shared_rank(pm, k)[r]);
+        float ss = 0.0f;
+        float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int k = 0; k < csize; k++) {  // ranks in ascending order
+            const float w = ap_exp2(cluster.map_shared_rank(pm, k)[r] - mm);
+            ss = fmaf(cluster.map_shared_rank(pl, k)[r], w, ss);
+            const float4 v = *reinterpret_cast<const float4*>(cluster.map_shared_rank(part, k) + r * PR + c * 4);
+            a.x = fmaf(v.x, w, a.x);
+            a.y = fmaf(v.y, w, a.y);
+            a.z = fmaf(v.z, w, a.z);
+            a.w = fmaf(v.w, w, a.w);
+        }
+        const float inv = ss > 0.0f ? 1.0f / ss : 0.0f;
+        const int pr = r / groups, h = r - pr * groups;
+        *reinterpret_cast<uint2*>(p.out + static_cast<long long>(pos0 + pr) * p.row_stride + (h0 + h) * HD + c * 4) =
+            make_uint2(pack_f16x2(a.x * inv, a.y * inv), pack_f16x2(a.z * inv, a.w * inv));
+    }
+    cluster.sync();  // nobody leaves while its shared memory is read
+}
+
+template <int HD> static cudaError_t launch_ap(const AttnParams& p, cudaStream_t st) {
+    constexpr int smem = ap_smem_bytes<HD>();
+    if (ensure_dynamic_smem(reinterpret_cast<const void*>(attn_prefill_mma_kernel<HD>), smem) != NVE_OK) return cudaErrorInvalidValue;
+    const int groups = p.num_heads / p.num_kv_heads;
+    const int PT = kApRows / groups;
+    const int tiles = (p.rows + PT - 1) / PT;
+    const int nkt = (p.seq_len - 1 + p.rows + kApKeys - 1) / kApKeys;
+    // Split the positions of a tile while the larger grid still fits two CTAs per SM (what shared memory allows) and
+    // every CTA keeps two steps: more CTAs than that only add merging.
+    int csize = 1;
+    while (csize < 8 && static_cast<long long>(tiles) * p.num_kv_heads * csize * 2 <= 2 * sm_count() && nkt >= 4 * csize) csize *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.dynamicSmemBytes = smem;
+    cfg.gridDim = dim3(tiles * csize, p.num_kv_heads);
+    cfg.blockDim = dim3(kApThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = csize;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (pdl_enabled()) {
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.numAttrs = 2;
+    }
+    return cudaLaunchKernelEx(&cfg, attn_prefill_mma_kernel<HD>, p, groups, tiles);
+}
+
+bool attn_prefill_mma_try(const AttnParams& p, int head_dim, cudaStream_t st, cudaError_t& err) {
+    if (p.num_heads / p.num_kv_heads > kApRows || p.num_kv_heads > 65535) return false;
+    if (head_dim == 128) err = launch_ap<128>(p, st);
+    else if (head_dim == 64) err = launch_ap<64>(p, st);
+    else return false;
+    return true;
+}
+
+}  // namespace nve

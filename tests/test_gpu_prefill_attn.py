@@ -1,0 +1,40 @@
+"""GPU: the tiled causal attention of a block of new positions against an f64 softmax over the same 16-bit inputs, at
+the edges of its tiles (128 query rows, 64 positions per step) and with the positions of a tile split over a cluster."""
+import pytest
+
+from helpers import dev
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nh,nkv,hd,S,start", [
+    (32, 8, 128, 32, 32),    # one full tile of 32 positions x 4 heads per KV head, 64 positions in all: one step
+    (32, 8, 128, 33, 31),    # one row more than a tile
+    (24, 8, 128, 43, 0),     # 3 heads per KV head: 42 positions (126 rows) per tile, one position in the second
+    (24, 8, 128, 8, 1013),   # few rows behind a long prefix: eight CTAs share the positions, the last one has fewer
+    (8, 8, 64, 129, 64),     # one head per KV head, a tile of a single row
+    (5, 1, 64, 70, 250),     # odd group
+    (16, 1, 128, 64, 5),     # more heads per KV head than the decode kernels take
+    (64, 2, 128, 300, 700),  # several tiles, split in two or four
+])
+def test_tiled_causal_attention(cuda, orc, nh, nkv, hd, S, start):
+    from nve_b200 import cuda_kernels as ck
+
+    torch = cuda
+    max_seq, G = start + S + 3, nh // nkv
+    q = dev(orc.to_act16(orc.fill_normal(S * nh * hd, 881, 1)), torch.float16).view(S, nh * hd)
+    kc = dev(orc.to_act16(orc.fill_normal(nkv * max_seq * hd, 881, 2)), torch.float16).view(nkv, max_seq, hd)
+    vc = dev(orc.to_act16(orc.fill_normal(nkv * max_seq * hd, 881, 3)), torch.float16).view(nkv, max_seq, hd)
+    kc[:, start + S:] = float("nan")  # positions behind the block must not be touched
+    vc[:, start + S:] = float("nan")
+    got = ck.attn_prefill_causal(q, kc, vc, start, nh, nkv, hd, max_seq, hd ** -0.5)
+    L = start + S
+    qd = q.double().view(S, nkv, G, hd)
+    s = torch.einsum("skgd,kld->skgl", qd, kc[:, :L].double()) * hd ** -0.5
+    seen = torch.arange(L, device="cuda")[None, :] <= torch.arange(start, L, device="cuda")[:, None]
+    s = s.masked_fill(~seen[:, None, None, :], float("-inf"))
+    want = torch.einsum("skgl,kld->skgd", s.softmax(-1), vc[:, :L].double()).reshape(S, nh * hd)
+    # f16 probabilities (2^-11 relative each, so 2^-11 of the largest |v| at most) and one f16 rounding of the result,
+    # plus f32 scores and sums (2^-16 of a score of at most ~60 in the exponent)
+    bound = (2.0 ** -10 + 2.0 ** -11) * vc[:, :L].double().abs().max().item()
+    assert (got.double() - want).abs().max().item() < bound
