@@ -384,20 +384,17 @@ NVE_API int nve_b200_fill_normal_16(void* out, long long n, unsigned long long s
 
 /* Batched W4A16 GEMM for decode batches 1 < M <= 64 on the tensor cores: Y[M,N] = X[M,K] . W^T with the packed
  * weights read once and dequantised on the fly (replaces nve_dequant_w4a16 + dense GEMM,
- * src/gpu_layer.rs:220-239).  Above 8 rows the weights go to tensor memory and tcgen05.mma; up to 8 rows a kernel
- * that keeps them in registers and issues mma.sync is faster and is used instead (same arguments, same work split
- * and workspace, results equal up to the order of the f32 additions).  The environment variable
- * NVE_B200_GEMM_KERNEL = tc | mma, read at the first call, forces one kernel (mma: M <= 32 only).
+ * src/gpu_layer.rs:220-239): they go to tensor memory and pairs of SMs multiply them with tcgen05.mma.
  * X and Y are row-major; x_dtype f16 or bf16, y_dtype = x_dtype or f32; K % 64 == 0; X and nibbles 16-byte aligned,
  * scales 8-byte aligned.  Weights are rounded to f16 as (q-8)*scale like the reference's dequantisation;
  * accumulation is f32.
  * `scratch` (may be NULL for f16 activations) holds, in this order, an f16 copy of bf16 activations (exact up to
  * +-65504, saturating beyond) and f32 partial tiles: with a workspace the (tile, 256-weight K slice) units are dealt
- * to the SMs in equal contiguous runs, so that few tiles still fill all SMs and a tile count that is not a multiple
- * of the SM count is balanced; tiles that several CTAs share are summed in ascending K order by a second kernel
+ * to the pairs of SMs in equal contiguous runs, so that few tiles still fill all SMs and a tile count that is not a multiple
+ * of the SM count is balanced; tiles that several pairs share are summed in ascending K order by a second kernel
  * (reproducible for a given SM count).  Its size comes from nve_b200_gemm_w4a16_scratch_bytes.  bf16 activations
  * without enough scratch for their copy are refused with NVE_ERR_TOO_LARGE; a scratch too small for the partial
- * tiles only lengthens the runs (fewer CTAs), down to one whole tile per CTA, which needs none.
+ * tiles only lengthens the runs (fewer CTAs), down to one whole tile per pair, which needs none.
  * nve_b200_gemm_error returns the code latched by an expired bounded wait. */
 NVE_API size_t nve_b200_gemm_w4a16_scratch_bytes(int M, int N, int K);
 NVE_API int nve_b200_gemm_w4a16(const void* X, int x_dtype, const uint8_t* nibbles, const float* scales, void* Y,
@@ -410,6 +407,9 @@ NVE_API size_t nve_b200_gemm_w4a16_multi_scratch_bytes(int M, const int* Ns, int
 NVE_API int nve_b200_gemm_w4a16_multi(const void* X, int x_dtype, const nve_b200_w4_matrix* mats, int num_mats,
                                       int y_dtype, int M, int K, void* scratch, size_t scratch_bytes,
                                       nve_stream_t stream);
+/* nve_b200_gemm_w4a16_multi for any number of rows of X (prompt blocks): the same arguments, M >= 1. */
+NVE_API int nve_b200_gemm_w4a16_wide(const void* X, int x_dtype, const nve_b200_w4_matrix* mats, int num_mats,
+                                     int y_dtype, int M, int K, void* scratch, size_t scratch_bytes, nve_stream_t stream);
 NVE_API int nve_b200_gemm_error(int reset);
 
 /* Allocation-free form of nve_b200_gemm_w4a16.  No counterpart in the reference: it exists for callers that have

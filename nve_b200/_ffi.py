@@ -153,6 +153,7 @@ SIGNATURES = {
     "nve_b200_gemm_w4a16": (_I, [_P, _I, _P, _P, _P, _I, _I, _I, _I, _P, _S, _P]),
     "nve_b200_gemm_w4a16_multi_scratch_bytes": (_S, [_I, _P, _I, _I]),
     "nve_b200_gemm_w4a16_multi": (_I, [_P, _I, C.POINTER(W4Matrix), _I, _I, _I, _I, _P, _S, _P]),
+    "nve_b200_gemm_w4a16_wide": (_I, [_P, _I, C.POINTER(W4Matrix), _I, _I, _I, _I, _P, _S, _P]),
     "nve_b200_gemm_error": (_I, [_I]),
     "nve_b200_gemm_w4a16_noalloc": (_I, [_P, _I, _P, _P, _P, _I, _I, _I, _I, _P]),
     "nve_b200_decode_step_workspace_bytes": (_S, [C.POINTER(DecodeModel)]),

@@ -1,57 +1,12 @@
-// Shared by the two batched W4A16 GEMM kernels (tcgen05 for wide batches, mma.sync for narrow ones): the launch
-// parameters, the work split over (tile, super-block) units, the nibble dequantisation and the cp.async helpers.
+// The batched W4A16 GEMM: nibble dequantisation and the interface between its entry points (gemm_w4a16.cu) and its
+// kernel (gemm_w4a16_pair.cu).
 #pragma once
 
 #include "common.cuh"
 
 namespace nve {
 
-constexpr int kTileN = 128;      // weight rows per tile
-constexpr int kKBlock = 64;      // K elements per pipeline stage of the tcgen05 kernel (128 bytes of 16-bit)
-constexpr int kSuper = 4;        // K blocks per super-block: 256 elements = 128 contiguous nibble bytes per row
-
-struct GemmParams {
-    const uint16_t* X;     // [M, K] f16
-    const uint8_t* nib[3]; // per matrix [N_i, K/2]
-    const float* sc[3];    // per matrix [N_i, K/32]
-    void* Y[3];            // per matrix [M, N_i]
-    int Nm[3];             // rows of each matrix
-    int tile_end[3];       // cumulative 128-row tiles
-    int col0[3];           // first column of each matrix in the concatenated [M, N] view
-    float* partial;        // [2 * grid][M][128] f32: slot 2c = first, slot 2c + 1 = last partial tile of CTA c
-    int M, N, K;           // N = sum of Nm
-    int nb;                // K / 32
-    int kblocks;           // K / 64
-    int sb_per_tile;       // super-blocks (4 K blocks) per tile
-    int units_per_cta;     // super-blocks in a CTA's contiguous run of the (tile, super-block) sequence
-    int total_units;       // tiles * sb_per_tile
-};
-
-// matrix and first row (inside that matrix) of a 128-row tile of the side-by-side tile sequence
-__device__ __forceinline__ void tile_locate(const GemmParams& p, int tile, int& mi, int& n0) {
-    mi = tile < p.tile_end[0] ? 0 : (tile < p.tile_end[1] ? 1 : 2);
-    n0 = (tile - (mi == 0 ? 0 : p.tile_end[mi - 1])) * kTileN;
-}
-
 __device__ __forceinline__ uint32_t s_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-
-__device__ __forceinline__ void cp_async_16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s_addr(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_16s(uint32_t dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_8s(uint32_t dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_8(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(s_addr(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_4(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(s_addr(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // Dequantisation of two nibbles.  0x6400 is 1024.0 in f16 with one ulp = 1, so OR-ing a nibble into mantissa bits
 // 0-3 gives 1024 + q exactly; 0x5400 is 64.0 with one ulp = 1/16, so a nibble left in place at bits 4-7 gives
@@ -105,8 +60,20 @@ __device__ __forceinline__ void dequant_word(uint32_t w, const DequantScale& d, 
     hi1 = dequant_pair<true>(t, d, c);   // b2 high, b3 high
 }
 
-// The narrow-batch kernel (gemm_w4a16_mma.cu): same parameters, same partial-tile layout, same reduce kernel.
-// Returns false when it has no instantiation for this batch, else true with the launch status in `status`.
-bool gemm_mma_try(const GemmParams& p, int y_dtype, cudaStream_t st, int& status);
+// The two-SM tcgen05 kernel (gemm_w4a16_pair.cu): any number of rows of X (f16), up to three matrices side by side.
+struct PairMat {
+    const uint8_t* nib;
+    const float* sc;
+    void* Y;
+    int N;
+};
+struct PairPlan {
+    int NB, XT, SB;        // rows of X per tile, X tiles, units (256 elements of K) per tile
+    long long tiles, U, grid_pairs;
+    size_t partial_bytes;  // workspace for partial tiles, 0 when every run consists of whole tiles
+};
+PairPlan pair_plan(const int* Ns, int num_mats, int M, int K, bool have_scratch, size_t avail);
+int gemm_pair(const uint16_t* X, const PairMat* mats, int num_mats, int y_dtype, int M, int K, void* partial, size_t avail, cudaStream_t st);
+int gemm_pair_error(bool reset);
 
 }  // namespace nve

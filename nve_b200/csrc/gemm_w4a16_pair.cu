@@ -1,0 +1,755 @@
+// W4A16 GEMM on the 5th-generation tensor cores, two SMs per tile:  Y[M,N] = X[M,K] . W^T.
+//
+// A pair of CTAs (cluster of two, tcgen05 cta_group::2) computes tiles of 256 weight rows x NB rows of X.  The packed
+// weights are read once per X tile, dequantised to f16 in registers, written into tensor memory and consumed from
+// there (A operand); the rows of X come by TMA into shared memory (B operand), HALF of them into each CTA: what one SM
+// loads per 128 x 128 weights is 10 KB of weights and NB / 2 x 256 bytes of X, so that neither L2 nor shared memory
+// is the limit at NB = 64, and at NB = 256 the tensor pipe is.
+//
+//   step  = 128 elements of K: A slot of 64 TMEM columns, X slot of NB / 2 rows x 256 bytes, one phase of the "full"
+//           (A), "xfull" (X) and "empty" barriers, eight tcgen05.mma (M = 256, N = NB, K = 16).  The X ring is deeper than
+//           the A ring: a slot that waits for a TMA load from L2 (about a microsecond) would set the pace otherwise.
+//   unit  = 2 steps = 256 elements of K: one raw stage (128 rows x 128 nibble bytes by TMA, 128 rows x 8 scales)
+//   tile  = SB units;  the sequence of all (tile, unit) is dealt out in equal contiguous runs, one per pair
+//
+// Roles (768 threads per CTA):
+//   warps 0-2    issue the MMAs (leader, cluster rank 0, only): warp w < W the steps w, w + W, ... of a segment into
+//                accumulator set w
+//   warp 3       X loader: TMA of this CTA's half of the X rows, bytes counted on the leader's full barrier
+//   warps 4-7    raw loaders: run ahead by the depth of the raw ring; start before the grid dependency resolves
+//   warps 8-23   dequantisers: four groups of four warps (thread = weight row = TMEM lane), group s % 4 takes step s.
+//                Waits for the raw stage and for the A slot, 4 blocks of 32 weights per thread: LDS, (q - 8) * scale,
+//                tcgen05.st; one arrival per warp on the LEADER's full barrier.  The same warps are the epilogue.
+// TMEM: W accumulator sets of NB columns, then the A slots.  X is loaded without multicast.
+//
+// Ring discipline: a parity wait is only meaningful when the waiter knows the barrier's previous phase to be complete.
+// full / empty barriers are indexed by the step modulo kBarRing = 12 (a multiple of the number of dequantiser groups
+// and of issuing warps), raw barriers by the unit modulo an even ring: consecutive phases of a barrier are always
+// awaited by the same threads, in order.  Every wait is bounded in time; an expired one latches an error code
+// (nve_b200_gemm_error) and both CTAs leave through the normal path.
+#include <cuda.h>
+
+#include "common.cuh"
+#include "gemm_w4a16.cuh"
+
+namespace nve {
+
+constexpr int kPairRows = 128;           // weight rows per CTA
+constexpr int kPairTile = 256;           // per pair
+constexpr int kPairStepCols = 64;        // TMEM columns of an A slot (128 f16 per row)
+constexpr int kPairIssueWarp = 0;        // first of up to three issuing warps
+constexpr int kPairRawWarp = 4, kPairRawWarps = 4;
+constexpr int kPairDeqWarp = 8, kPairDeqWarps = 16;
+constexpr int kPairXWarp = 3;
+constexpr int kPairThreads = 24 * 32;
+constexpr int kBarRing = 24;
+constexpr int kMaxRaw = 8;
+constexpr int kRawNib = kPairRows * 128, kRawSc = kPairRows * 32, kRawBytes = kRawNib + kRawSc;
+constexpr int kPairSmemMax = 226 * 1024;  // dynamic; the barriers take the first (static) kilobyte
+constexpr unsigned long long kPairWaitLimitNs = 50ull * 1000 * 1000;  // a legitimate wait lasts microseconds
+
+struct PairParams {
+    const uint8_t* nib[3];
+    const float* sc[3];
+    void* Y[3];
+    int Nm[3];
+    int wt_end[3];   // cumulative 256-row tiles of the matrices
+    float* partial;  // [2 * pairs][part_rows][256] f32: slot 2c = first, 2c + 1 = last cut segment of pair c
+    int M, K, nb;
+    int part_rows;   // rows of X that a partial tile holds: min(M, NB)
+    int NB;          // rows of X per tile (multiple of 32, <= 256)
+    int XT;          // X tiles
+    int W;           // accumulator sets = issuing warps
+    int slots;       // A slots (TMEM)
+    int xslots;      // X slots (shared memory), at most kBarRing
+    int raw;         // raw stages (even)
+    int SB;          // units per tile
+    int U;           // units per pair
+    int total;       // units
+    int sc16;        // 1: rows of scales are 16-byte aligned
+};
+
+// ---- mbarrier / TMA / tcgen05 wrappers
+__device__ __forceinline__ void pg_init(uint32_t bar, unsigned count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+}
+__device__ __forceinline__ void pg_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void pg_arrive_cluster(uint32_t cluster_bar) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ void pg_expect(uint32_t bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ uint32_t pg_map(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ bool pg_try(uint32_t bar, unsigned parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+// Wait of a whole, converged warp; the answer is the same for all its lanes (the tcgen05 instructions that follow need
+// the whole warp).
+__device__ __noinline__ bool pg_wait_slow(uint32_t bar, unsigned parity) {
+    unsigned long long t0, t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+    bool late;
+    do {
+        for (int i = 0; i < 64; i++)
+            if (__all_sync(0xffffffffu, pg_try(bar, parity))) return true;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+        late = __any_sync(0xffffffffu, t - t0 >= kPairWaitLimitNs);
+    } while (!late);
+    return false;
+}
+__device__ __forceinline__ bool pg_wait(uint32_t bar, unsigned parity) {
+    if (__all_sync(0xffffffffu, pg_try(bar, parity))) return true;
+    return pg_wait_slow(bar, parity);
+}
+// tile load into this CTA's shared memory, bytes counted on a barrier of either CTA of the pair
+__device__ __forceinline__ void pg_tma_pair(uint32_t dst, const CUtensorMap* map, int row, int kblock, uint32_t cluster_bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+        ::"r"(dst), "l"(map), "r"(0), "r"(row), "r"(kblock), "r"(cluster_bar)
+        : "memory");
+}
+__device__ __forceinline__ bool pg_elect() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
+}
+__device__ __forceinline__ void pg_mma(bool issuer, uint32_t d, uint32_t a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d), "r"(a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(static_cast<uint32_t>(issuer))
+        : "memory");
+}
+// arrives on the barrier at this offset in both CTAs when the thread's MMAs so far are complete
+__device__ __forceinline__ void pg_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+                 "h"(static_cast<uint16_t>(3))
+                 : "memory");
+}
+__device__ __forceinline__ void pg_tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
+          "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+        : "memory");
+}
+__device__ __forceinline__ void pg_tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+          "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void pg_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void pg_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// K-major SWIZZLE_128B descriptor: 1024 bytes between 8-row groups, descriptor version 1, layout type 2
+__device__ __forceinline__ uint64_t pg_desc(uint32_t smem_addr) {
+    uint64_t d = static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);
+    d |= static_cast<uint64_t>(1) << 16;
+    d |= static_cast<uint64_t>(1024 >> 4) << 32;
+    d |= static_cast<uint64_t>(1) << 46;
+    d |= static_cast<uint64_t>(2) << 61;
+    return d;
+}
+
+static __device__ int g_pair_error = 0;
+
+struct PairTile {
+    int mi, n0, xt;  // matrix, first weight row of the pair's tile inside it, X tile
+};
+__device__ __forceinline__ PairTile pair_locate(const PairParams& p, int tile) {
+    PairTile t;
+    const int wt = tile / p.XT;
+    t.xt = tile - wt * p.XT;
+    t.mi = wt < p.wt_end[0] ? 0 : (wt < p.wt_end[1] ? 1 : 2);
+    t.n0 = (wt - (t.mi == 0 ? 0 : p.wt_end[t.mi - 1])) * kPairTile;
+    return t;
+}
+
+// Sixteen rows of X (rows m, m + 1, ... of Y) x this lane's feature n.  16-bit types: lanes 2i and 2i + 1 exchange values
+// so that every lane stores two neighbouring features of every second row in one 4-byte store.
+template <int ODT> __device__ __forceinline__ void pair_store(void* Y, int Nloc, int n, int lane, int m, int rows, const float (&y)[16]) {
+    if (ODT == NVE_DT_F32 || (Nloc & 1)) {
+#pragma unroll
+        for (int e = 0; e < 16; e++)
+            if (e < rows && n < Nloc) store_out<ODT>(Y, static_cast<long long>(m + e) * Nloc + n, y[e]);
+    } else {
+        const int odd = lane & 1;
+        uint16_t* dst = static_cast<uint16_t*>(Y) + static_cast<long long>(m + odd) * Nloc + (n - odd);
+#pragma unroll
+        for (int e = 0; e < 16; e += 2) {
+            constexpr int DT16 = ODT == NVE_DT_BF16 ? NVE_DT_BF16 : NVE_DT_F16;
+            const uint32_t own = static_cast<uint32_t>(Act16<DT16>::from_f32(y[e])) | (static_cast<uint32_t>(Act16<DT16>::from_f32(y[e + 1])) << 16);
+            const uint32_t other = __shfl_xor_sync(0xffffffffu, own, 1);
+            // even lane: row e of (n, n + 1); odd lane: row e + 1 of (n - 1, n)
+            const uint32_t v = odd ? __byte_perm(other, own, 0x7632) : __byte_perm(own, other, 0x5410);
+            if (e + odd < rows && n < Nloc) *reinterpret_cast<uint32_t*>(dst) = v;
+            dst += 2 * static_cast<long long>(Nloc);
+        }
+    }
+}
+
+template <int ODT>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
+    gemm_w4a16_pair_kernel(const PairParams p, const __grid_constant__ CUtensorMap xmap) {
+    extern __shared__ __align__(1024) unsigned char pg_raw[];
+    __shared__ __align__(8) uint64_t bars[2 * kBarRing + 2 * kMaxRaw + 2];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int abort_flag;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t smem = (s_addr(pg_raw) + 1023u) & ~1023u;
+    const uint32_t bslot_bytes = static_cast<uint32_t>(p.NB) * 128;  // NB / 2 rows x 256 bytes
+    const uint32_t sB = smem, sRaw = smem + p.xslots * bslot_bytes;
+    const uint32_t full = s_addr(bars), empty = full + 8 * kBarRing, rawf = empty + 8 * kBarRing, rawe = rawf + 8 * kMaxRaw;
+    const uint32_t accum = rawe + 8 * kMaxRaw, accfree = accum + 8;
+    uint32_t rank;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const int pair = blockIdx.x >> 1;
+    const int u0 = pair * p.U;
+    const int n_units = min(p.U, p.total - u0);
+    const int n_steps = 2 * n_units;
+
+    if (tid < kBarRing) {
+        pg_init(full + 8 * tid, 9);   // leader: four dequantiser warps of each CTA + expect_tx of both halves of the X rows
+        pg_init(empty + 8 * tid, 1);  // tcgen05.commit
+        if (tid < p.raw) {
+            pg_init(rawf + 8 * tid, 32 * kPairRawWarps);  // the copies of every loader lane
+            pg_init(rawe + 8 * tid, 8);                   // the eight warps that read the stage
+        }
+        if (tid == 0) {
+            pg_init(accum, p.W);
+            pg_init(accfree, 2 * kPairDeqWarps);  // leader: every dequantiser (= epilogue) warp of both CTAs
+            abort_flag = 0;
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    pg_cluster_arrive();  // matched below: nothing reaches into the other CTA before its barriers are set up
+    bool ok = true;
+    auto fail = [&](int code) {
+        atomicCAS(&g_pair_error, 0, code);
+        *reinterpret_cast<volatile int*>(&abort_flag) = 1;
+        ok = false;
+    };
+
+    if (warp >= kPairRawWarp && warp < kPairRawWarp + kPairRawWarps) {
+        // ------------------------------------------------------------------ raw loaders (weights: no dependency wait)
+        // Plain asynchronous copies, not TMA: the TMA unit needs about four cycles per 128-byte row, and 256 rows of
+        // nibbles and scales per unit next to the rows of X made it the slowest part of the kernel.
+        const int lw = warp - kPairRawWarp;
+        const int nr = lw * 32 + (lane >> 3), nc = lane & 7;  // nibbles: rows nr, nr + 4, ..., nr + 28, 16-byte chunk nc
+        const int half_k = p.K / 2;
+        int tile = u0 / p.SB, sbi = u0 - (u0 / p.SB) * p.SB;
+        PairTile tl = pair_locate(p, tile);
+        int st = 0;
+        unsigned par = 1;
+        for (int j = 0; j < n_units; j++) {
+            if (j >= p.raw) {
+                if (!pg_wait(rawe + 8 * st, par)) {
+                    fail(3);
+                    break;
+                }
+            }
+            const int row0 = tl.n0 + static_cast<int>(rank) * kPairRows, nlast = p.Nm[tl.mi] - 1;
+            const uint32_t dst = sRaw + st * kRawBytes;
+            {
+                // chunks past the end of K read as zero, rows past the end repeat the last one
+                const int kb = sbi * 128 + nc * 16;
+                const uint8_t* src = p.nib[tl.mi] + (kb < half_k ? kb : 0);
+                const int have = kb < half_k ? 16 : 0;
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const int r = nr + 4 * i;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + r * 128 + ((nc ^ (r & 7)) << 4)),
+                                 "l"(src + static_cast<long long>(min(row0 + r, nlast)) * half_k), "r"(have)
+                                 : "memory");
+                }
+            }
+            const float* sc = p.sc[tl.mi];
+            const int b0 = sbi * 8;
+            if (p.sc16) {
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    const int r = lw * 32 + (lane >> 1) + 16 * i, c = lane & 1;
+                    const int have = min(16, max(0, (p.nb - b0 - 4 * c) * 4));
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + kRawNib + r * 32 + c * 16),
+                                 "l"(sc + static_cast<long long>(min(row0 + r, nlast)) * p.nb + (have > 0 ? b0 + 4 * c : 0)), "r"(have)
+                                 : "memory");
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int r = lw * 32 + (lane >> 2) + 8 * i, c = lane & 3;
+                    const int have = min(8, max(0, (p.nb - b0 - 2 * c) * 4));
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst + kRawNib + r * 32 + c * 8),
+                                 "l"(sc + static_cast<long long>(min(row0 + r, nlast)) * p.nb + (have > 0 ? b0 + 2 * c : 0)), "r"(have)
+                                 : "memory");
+                }
+            }
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(rawf + 8 * st) : "memory");
+            if (++st == p.raw) {
+                st = 0;
+                par ^= 1;
+            }
+            if (++sbi == p.SB) {
+                sbi = 0;
+                tile++;
+                if (j + 1 < n_units) tl = pair_locate(p, tile);
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        pdl_launch_dependents();
+        pg_cluster_wait();
+    } else {
+        if (warp == kPairIssueWarp) {  // TMEM allocation is warp-wide, one warp of each CTA of the pair
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_addr(&tmem_slot)), "r"(512) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"(kPairThreads - 32 * kPairRawWarps) : "memory");  // everyone but the raw loaders
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        pg_cluster_wait();
+        const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&tmem_slot);
+        const uint32_t acols = p.W * p.NB;
+
+        if (warp >= kPairDeqWarp && warp < kPairDeqWarp + kPairDeqWarps) {
+            // -------------------------------------------------------------- dequantisers
+            const int grp = (warp - kPairDeqWarp) >> 2;                       // takes steps grp, grp + 4, ...
+            const int r = (warp & 3) * 32 + lane;            // weight row of the CTA = TMEM lane
+            const uint32_t tmem_lane = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + acols;
+            const uint32_t lfull = pg_map(full, 0);
+            uint32_t roff[4];  // chunk (4 * half + q) of the 128-byte swizzled row
+#pragma unroll
+            for (int q = 0; q < 4; q++) roff[q] = r * 128 + (((4 * (grp & 1) + q) ^ (r & 7)) << 4);
+            const uint32_t soff = kRawNib + r * 32 + (grp & 1) * 16;
+            const DequantConsts dc = make_dequant_consts();
+            // The epilogue of a segment is shared by all sixteen warps: a quarter of the columns per group.  A group runs
+            // on into the next segment first and comes back here before it would wait for one of that segment's MMAs, which
+            // in turn wait for the accumulators: the operand slots are full again when the epilogue ends.
+            const uint32_t lfree = pg_map(accfree, 0);
+            int ej = 0, eseg = 0, etile = u0 / p.SB, esbi = u0 - (u0 / p.SB) * p.SB;  // first segment without its epilogue
+            int eunits = min(p.SB - esbi, n_units);
+            int lim = min(n_steps, 2 * eunits + p.slots);  // the group's steps from here on need a slot of the next segment
+            auto epilogue = [&]() -> bool {
+                if (eseg == 0) pdl_wait();  // the stores below must not overtake the previous kernel's reads
+                if (!pg_wait(accum, static_cast<unsigned>(eseg) & 1u)) {
+                    fail(5);
+                    return false;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const PairTile tl = pair_locate(p, etile);
+                const int Nloc = p.Nm[tl.mi];
+                const bool whole = eunits == p.SB;
+                const int col = static_cast<int>(rank) * kPairRows + r;
+                const int n = tl.n0 + col;  // this thread's output feature
+                const int m0 = tl.xt * p.NB;
+                const uint32_t taddr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+                float* part = p.partial + static_cast<long long>(2 * pair + (eseg > 0 ? 1 : 0)) * p.part_rows * kPairTile + col;
+                const int mrows = min(p.NB, p.M - m0);
+                for (int cb = 16 * grp; cb < mrows; cb += 64) {
+                    float y[16];
+                    uint32_t v[16];
+                    pg_tmem_ld16(taddr + cb, v);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int e = 0; e < 16; e++) y[e] = __uint_as_float(v[e]);
+                    for (int a = 1; a < min(p.W, 2 * eunits); a++) {
+                        pg_tmem_ld16(taddr + a * p.NB + cb, v);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                        for (int e = 0; e < 16; e++) y[e] = __fadd_rn(y[e], __uint_as_float(v[e]));
+                    }
+                    if (!whole) {
+#pragma unroll
+                        for (int e = 0; e < 16; e++)
+                            if (cb + e < mrows) part[(cb + e) * kPairTile] = y[e];
+                    } else {
+                        pair_store<ODT>(p.Y[tl.mi], Nloc, n, lane, m0 + cb, min(16, mrows - cb), y);
+                    }
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) pg_arrive_cluster(lfree);
+                ej += eunits;
+                esbi += eunits;
+                if (esbi == p.SB) {
+                    esbi = 0;
+                    etile++;
+                }
+                eunits = min(p.SB - esbi, n_units - ej);
+                eseg++;
+                lim = min(n_steps, 2 * (ej + eunits) + p.slots);
+                return true;
+            };
+            const uint32_t col_end = tmem_lane + p.slots * kPairStepCols;
+            uint32_t col = tmem_lane + grp * kPairStepCols;                            // A slot (there are at least four)
+            uint32_t rsrc = sRaw + (grp >> 1) * kRawBytes, rbar = 8 * (grp >> 1);      // raw stage
+            unsigned rpar = 0, epar = 1;
+            int fb = 8 * grp;                                                          // full barrier of the step
+            int eb = 8 * (grp - p.slots + kBarRing);                                   // empty barrier of the step p.slots before
+            for (int s = grp;;) {
+                if (s >= lim) {
+                    if (ej == n_units) break;
+                    if (!epilogue()) break;
+                    continue;
+                }
+                if (!pg_wait(rawf + rbar, rpar)) {
+                    fail(1);
+                    break;
+                }
+                uint4 raw[4];
+                float4 scv;
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                                 : "=r"(raw[q].x), "=r"(raw[q].y), "=r"(raw[q].z), "=r"(raw[q].w)
+                                 : "r"(rsrc + roff[q])
+                                 : "memory");
+                asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];"
+                             : "=f"(scv.x), "=f"(scv.y), "=f"(scv.z), "=f"(scv.w)
+                             : "r"(rsrc + soff)
+                             : "memory");
+                if (s >= p.slots) {  // the step that used this slot last has been multiplied
+                    if (!pg_wait(empty + eb, epar)) {
+                        fail(1);
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                }
+                const float scq[4] = {scv.x, scv.y, scv.z, scv.w};
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const DequantScale ds = make_dequant_scale(scq[q]);
+                    uint32_t v[16];  // v[c] = elements (2c, 2c+1) of the block
+                    dequant_word(raw[q].x, ds, dc, v[0], v[1], v[8], v[9]);
+                    dequant_word(raw[q].y, ds, dc, v[2], v[3], v[10], v[11]);
+                    dequant_word(raw[q].z, ds, dc, v[4], v[5], v[12], v[13]);
+                    dequant_word(raw[q].w, ds, dc, v[6], v[7], v[14], v[15]);
+                    pg_tmem_st16(col + 16 * q, v);
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) {
+                    pg_arrive_cluster(lfull + fb);
+                    pg_arrive(rawe + rbar);
+                }
+                s += 4;
+                col += 4 * kPairStepCols;
+                if (col >= col_end) col -= p.slots * kPairStepCols;
+                rsrc += 2 * kRawBytes;
+                rbar += 16;
+                if (rbar >= static_cast<uint32_t>(8 * p.raw)) {
+                    rbar -= 8 * p.raw;
+                    rsrc -= p.raw * kRawBytes;
+                    rpar ^= 1u;
+                }
+                fb += 32;
+                if (fb >= 8 * kBarRing) fb -= 8 * kBarRing;
+                eb += 32;
+                if (eb >= 8 * kBarRing) {
+                    eb -= 8 * kBarRing;
+                    epar ^= 1u;
+                }
+            }
+        } else if (warp == kPairXWarp) {
+            // -------------------------------------------------------------- X loader
+            // the whole warp runs the loop, one lane issues (operands in uniform registers)
+            const bool issuer = pg_elect();
+            pdl_wait();  // activations come from the previous kernel
+            const uint32_t lfull = pg_map(full, 0);
+            int tile = u0 / p.SB, ts = 2 * (u0 - (u0 / p.SB) * p.SB);
+            int xrow = (tile % p.XT) * p.NB + static_cast<int>(rank) * (p.NB / 2);
+            int slot = 0, bi = 0, eb = 0;  // X slot; full barrier of the step; empty barrier of the step that used the slot last
+            unsigned epar = 0;
+            for (int s = 0; s < n_steps; s++) {
+                if (s >= p.xslots) {
+                    if (!pg_wait(empty + 8 * eb, epar)) {
+                        fail(4);
+                        break;
+                    }
+                    if (++eb == kBarRing) {
+                        eb = 0;
+                        epar ^= 1u;
+                    }
+                }
+                if (issuer) {
+                    if (rank == 0) pg_expect(full + 8 * bi, 2 * bslot_bytes);
+                    pg_tma_pair(sB + slot * bslot_bytes, &xmap, xrow, 2 * ts, lfull + 8 * bi);
+                }
+                __syncwarp();
+                if (++slot == p.xslots) slot = 0;
+                if (++bi == kBarRing) bi = 0;
+                if (++ts == 2 * p.SB) {
+                    ts = 0;
+                    tile++;
+                    xrow = (tile % p.XT) * p.NB + static_cast<int>(rank) * (p.NB / 2);
+                }
+            }
+        } else if (rank == 0 && warp < kPairIssueWarp + p.W) {
+            // -------------------------------------------------------------- MMA issue
+            // The whole warp runs this loop and one lane of it issues: operands then live in uniform registers.  Warp w
+            // takes the steps w, w + W, ... of a segment into accumulator set w.
+            const int w = warp - kPairIssueWarp;
+            const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(p.NB >> 3) << 17) | (static_cast<uint32_t>(kPairTile >> 4) << 24);
+            const bool issuer = pg_elect();
+            int j = 0, seg = 0;
+            int tile = u0 / p.SB, sbi = u0 - (u0 / p.SB) * p.SB;
+            while (j < n_units) {
+                const int seg_units = min(p.SB - sbi, n_units - j);
+                const int seg_steps = 2 * seg_units;
+                if (seg > 0 && !pg_wait(accfree, static_cast<unsigned>(seg - 1) & 1u)) fail(2);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                int s = 2 * j + w;
+                int bi = s % kBarRing, slot = s % p.slots, xslot = s % p.xslots;
+                unsigned par = static_cast<unsigned>(s / kBarRing) & 1u;
+                uint32_t acc = 0;
+                for (int q = w; q < seg_steps; q += p.W) {
+                    if (!pg_wait(full + 8 * bi, par)) {
+                        fail(2);
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t a = tmem + acols + slot * kPairStepCols;
+                    const uint32_t xs = sB + xslot * bslot_bytes;
+                    const uint64_t bd0 = pg_desc(xs), bd1 = pg_desc(xs + bslot_bytes / 2);
+                    pg_mma(issuer, tmem + w * p.NB, a, bd0, idesc, acc);
+#pragma unroll
+                    for (int kk = 1; kk < 8; kk++)  // 16 elements along K: 8 TMEM columns of A, 32 bytes of B
+                        pg_mma(issuer, tmem + w * p.NB, a + 8 * kk, (kk < 4 ? bd0 : bd1) + 2 * (kk & 3), idesc, 1u);
+                    acc = 1;
+                    if (issuer) pg_commit(empty + 8 * bi);
+                    __syncwarp();
+                    bi += p.W;
+                    if (bi >= kBarRing) {
+                        bi -= kBarRing;
+                        par ^= 1u;
+                    }
+                    slot += p.W;
+                    if (slot >= p.slots) slot -= p.slots;
+                    xslot += p.W;
+                    if (xslot >= p.xslots) xslot -= p.xslots;
+                }
+                if (!ok) break;
+                if (issuer) pg_commit(accum);  // a warp without a step in the segment arrives at once
+                __syncwarp();
+                j += seg_units;
+                sbi += seg_units;
+                if (sbi == p.SB) {
+                    sbi = 0;
+                    tile++;
+                }
+                seg++;
+            }
+        }
+    }
+    // ---- teardown.  After an expired wait copies may still be in flight into this CTA: give them time to land.
+    if (*reinterpret_cast<volatile int*>(&abort_flag)) {
+        for (int i = 0; i < 100; i++) __nanosleep(10000);
+    }
+    __syncwarp();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    pg_cluster_arrive();
+    pg_cluster_wait();  // neither CTA leaves, or frees its TMEM, while the other may still reach into it
+    if (warp == kPairIssueWarp) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&tmem_slot);
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    }
+}
+
+// Tiles that more than one pair worked on: sum their partial tiles in ascending K order, convert and store.  One block
+// per (tile, four rows of X), a thread takes four consecutive features.
+template <int ODT> __global__ void __launch_bounds__(256) gemm_pair_reduce_kernel(const PairParams p) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int tile = blockIdx.x;
+    const int first = (tile * p.SB) / p.U, last = ((tile + 1) * p.SB - 1) / p.U;
+    if (first == last) return;
+    const PairTile tl = pair_locate(p, tile);
+    const int Nloc = p.Nm[tl.mi];
+    const int c4 = static_cast<int>(threadIdx.x) * 4, n = tl.n0 + c4;
+    const int mm = static_cast<int>(blockIdx.y * blockDim.y + threadIdx.y), m = tl.xt * p.NB + mm;
+    if (n >= Nloc || mm >= p.NB || m >= p.M) return;
+    auto part = [&](int c) {
+        const int slot = 2 * c + (c * p.U >= tile * p.SB ? 0 : 1);  // the pair's first segment when its run starts inside this tile
+        return __ldcg(reinterpret_cast<const float4*>(p.partial + (static_cast<long long>(slot) * p.part_rows + mm) * kPairTile + c4));
+    };
+    float4 y = part(first);
+    for (int c = first + 1; c <= last; c++) {
+        const float4 v = part(c);
+        y.x = __fadd_rn(y.x, v.x);
+        y.y = __fadd_rn(y.y, v.y);
+        y.z = __fadd_rn(y.z, v.z);
+        y.w = __fadd_rn(y.w, v.w);
+    }
+    const long long o = static_cast<long long>(m) * Nloc + n;
+    const float yy[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+        if (n + e < Nloc) store_out<ODT>(p.Y[tl.mi], o + e, yy[e]);
+}
+
+using PairEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+// cuTensorMapEncodeTiled through the runtime's driver entry point lookup (a pure host-side encoder, legal in capture)
+static PairEncodeFn pair_encode_fn() {
+    static PairEncodeFn fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return reinterpret_cast<PairEncodeFn>(f);
+    }();
+    return fn;
+}
+// X [M, K] f16 seen as [K / 64][M][64]: one box = two K blocks x box_rows rows x 64 elements (128 bytes, 128-byte
+// swizzle), i.e. all X rows of a step in one instruction; zeros outside.
+static bool pair_x_map(CUtensorMap* map, const uint16_t* X, int K, int M, int box_rows) {
+    PairEncodeFn fn = pair_encode_fn();
+    if (fn == nullptr) return false;
+    const cuuint64_t dims[3] = {64, static_cast<cuuint64_t>(M), static_cast<cuuint64_t>(K / 64)};
+    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(K) * 2, 128};
+    const cuuint32_t box[3] = {64, static_cast<cuuint32_t>(box_rows), 2};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<uint16_t*>(X), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// How the (tile, unit) sequence is cut into one contiguous run per pair.  With a workspace the runs are equal (total /
+// pairs, rounded up; at least two units = 512 weights per row): few tiles are split over K so that every SM works, and
+// a tile count that is not a multiple of the pair count costs total / pairs instead of a whole extra wave.  Without a
+// workspace a pair takes exactly one tile.
+PairPlan pair_plan(const int* Ns, int num_mats, int M, int K, bool have_scratch, size_t avail) {
+    PairPlan g;
+    g.XT = (M + 255) / 256;
+    g.NB = ((M + g.XT - 1) / g.XT + 31) / 32 * 32;
+    g.XT = (M + g.NB - 1) / g.NB;
+    g.SB = (K + 255) / 256;
+    long long wt = 0;
+    for (int i = 0; i < num_mats; i++) wt += (Ns[i] + kPairTile - 1) / kPairTile;
+    g.tiles = wt * g.XT;
+    const long long total = g.tiles * g.SB;
+    const int pairs = max(1, sm_count() / 2);
+    const long long rows = M < g.NB ? M : g.NB;
+    long long U = g.SB;
+    auto bytes = [&](long long u) -> size_t {
+        return u % g.SB == 0 ? 0 : static_cast<size_t>(2 * ((total + u - 1) / u) * rows * kPairTile) * sizeof(float);
+    };
+    if (have_scratch) {
+        U = (total + pairs - 1) / pairs;
+        if (U < 2) U = g.SB < 2 ? g.SB : 2;
+        while (bytes(U) > avail) U++;  // a workspace too small for the partial tiles: longer runs; whole tiles need none
+    }
+    g.U = U;
+    g.grid_pairs = (total + U - 1) / U;
+    g.partial_bytes = bytes(U);
+    return g;
+}
+
+template <int ODT> static int launch_pair(const PairParams& p, long long pairs, long long tiles, const CUtensorMap& xmap, int smem, cudaStream_t st) {
+    auto kern = gemm_w4a16_pair_kernel<ODT>;
+    if (int s = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kPairSmemMax); s != NVE_OK) return s;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(2 * pairs));
+    cfg.blockDim = dim3(kPairThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    if (pdl_enabled()) {
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p, xmap);
+    count_launch();
+    if (e != cudaSuccess) return set_cuda_status(e);
+    if (p.U % p.SB != 0) {
+        cfg.gridDim = dim3(static_cast<unsigned>(tiles), static_cast<unsigned>((p.part_rows + 3) / 4));
+        cfg.blockDim = dim3(kPairTile / 4, 4);
+        cfg.dynamicSmemBytes = 0;
+        e = cudaLaunchKernelEx(&cfg, gemm_pair_reduce_kernel<ODT>, p);
+        count_launch();
+    }
+    return set_cuda_status(e);
+}
+
+int gemm_pair(const uint16_t* X, const PairMat* mats, int num_mats, int y_dtype, int M, int K, void* partial, size_t avail, cudaStream_t st) {
+    PairParams p = {};
+    int Ns[3] = {0, 0, 0};
+    for (int i = 0; i < num_mats; i++) Ns[i] = mats[i].N;
+    const PairPlan g = pair_plan(Ns, num_mats, M, K, partial != nullptr, avail);
+    if (g.tiles * g.SB > 0x3FFFFFFFll) return set_status(NVE_ERR_BAD_SHAPE);
+    CUtensorMap xmap;
+    if (!pair_x_map(&xmap, X, K, M, g.NB / 2)) return set_status(NVE_ERR_CUDA);
+    int wt = 0;
+    p.sc16 = (K % 128) == 0;
+    for (int i = 0; i < 3; i++) {
+        const PairMat& m = mats[i < num_mats ? i : 0];
+        p.nib[i] = m.nib;
+        p.sc[i] = m.sc;
+        p.Y[i] = m.Y;
+        p.Nm[i] = i < num_mats ? m.N : 0;
+        if (i < num_mats) wt += (m.N + kPairTile - 1) / kPairTile;
+        p.wt_end[i] = wt;
+        if (!aligned(m.sc, 16)) p.sc16 = 0;
+    }
+    p.partial = static_cast<float*>(partial);
+    p.M = M;
+    p.K = K;
+    p.nb = K / 32;
+    p.NB = g.NB;
+    p.part_rows = M < g.NB ? M : g.NB;
+    p.XT = g.XT;
+    p.SB = g.SB;
+    p.U = static_cast<int>(g.U);
+    p.total = static_cast<int>(g.tiles * g.SB);
+    // Accumulator sets = issuing warps: a step costs an issuing warp about a thousand cycles of waiting and issuing, the
+    // MMAs themselves 8 * NB / 2.  The sets of a step follow its index in the segment.
+    p.W = g.NB <= 64 ? 3 : (g.NB <= 128 ? 2 : 1);
+    p.slots = min(7, (512 - p.W * p.NB) / kPairStepCols);
+    // shared memory: the X rows of a step take NB * 128 bytes per CTA; at 256 rows five of them and two raw units
+    // (four steps), for narrow tiles up to twelve steps of X and eight raw units, which is what hides HBM latency
+    p.raw = g.NB > 192 ? 2 : (g.NB > 96 ? 4 : (g.NB > 32 ? 6 : 8));
+    p.xslots = min(12, (kPairSmemMax - 1024 - p.raw * kRawBytes) / (p.NB * 128));
+    const int smem = 1024 + p.xslots * p.NB * 128 + p.raw * kRawBytes;
+    if (y_dtype == NVE_DT_F32) return launch_pair<NVE_DT_F32>(p, g.grid_pairs, g.tiles, xmap, smem, st);
+    return y_dtype == NVE_DT_F16 ? launch_pair<NVE_DT_F16>(p, g.grid_pairs, g.tiles, xmap, smem, st)
+                                 : launch_pair<NVE_DT_BF16>(p, g.grid_pairs, g.tiles, xmap, smem, st);
+}
+
+int gemm_pair_error(bool reset) {
+    int v = 0;
+    if (cudaError_t e = cudaMemcpyFromSymbol(&v, g_pair_error, sizeof(int)); e != cudaSuccess) {
+        set_cuda_status(e);
+        return -1;
+    }
+    if (reset && v != 0) {
+        const int zero = 0;
+        cudaMemcpyToSymbol(g_pair_error, &zero, sizeof(int));
+    }
+    return v;
+}
+
+}  // namespace nve

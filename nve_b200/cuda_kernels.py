@@ -753,6 +753,18 @@ def gemm_w4a16_multi(x: Tensor, weights: Sequence, k: int, out_dtype=None, outs:
     return list(outs)
 
 
+def gemm_w4a16_wide(x: Tensor, weights: Sequence, k: int, outs: Sequence[Tensor], scratch: Optional[Tensor] = None):
+    """gemm_w4a16_multi for any number of rows of x, into `outs`.  Without `scratch` the workspace is allocated here."""
+    m = x.shape[0]
+    if scratch is None:
+        scratch = torch.empty(max(16, gemm_w4a16_multi_scratch_bytes(m, [w[2] for w in weights], k)), dtype=torch.uint8, device=x.device)
+    arr = _mats(weights, outs, None, x.dtype)
+    _ffi.check("nve_b200_gemm_w4a16_wide",
+               _lib().nve_b200_gemm_w4a16_wide(_ptr(x, (torch.float16, torch.bfloat16), "x"), _dt(x), arr, len(weights), _dt(x), m, k,
+                                               _ptr(scratch), scratch.numel() * scratch.element_size(), stream()))
+    return list(outs)
+
+
 def gemm_w4a16_noalloc(x: Tensor, nibbles: Tensor, scales: Tensor, n: int, k: int, out: Tensor) -> Tensor:
     """Batched W4A16 GEMM for callers that cannot allocate: the caller passes input and output tensors only, the
     workspace for partial tiles is a fixed 4 MiB array inside the library (shapes needing more raise NVE_ERR_TOO_LARGE).
