@@ -410,6 +410,39 @@ NVE_API int nve_b200_gemm_w4a16_multi(const void* X, int x_dtype, const nve_b200
 /* nve_b200_gemm_w4a16_multi for any number of rows of X (prompt blocks): the same arguments, M >= 1. */
 NVE_API int nve_b200_gemm_w4a16_wide(const void* X, int x_dtype, const nve_b200_w4_matrix* mats, int num_mats,
                                      int y_dtype, int M, int K, void* scratch, size_t scratch_bytes, nve_stream_t stream);
+/* The GEMM with what a layer does to its product next, f16 throughout (scratch as above; finished inside the GEMM's
+ * epilogue or in the kernel that sums partial tiles; bits of the separate calls):
+ *   _add_rmsnorm: Y = residual + X . W^T and normed = RMSNorm(Y) (N % 8 == 0, N <= 8192; Y, residual, norm_weight and
+ *                 normed 16-byte aligned; residual may not alias Y);
+ *   _gateup_silu: mid = silu(X . gate^T) * (X . up^T), both matrices with N rows. */
+NVE_API int nve_b200_gemm_w4a16_add_rmsnorm(const uint16_t* X, const uint8_t* nibbles, const float* scales,
+                                            const uint16_t* residual, uint16_t* Y, const uint16_t* norm_weight,
+                                            uint16_t* normed, float eps, int M, int N, int K, void* scratch,
+                                            size_t scratch_bytes, nve_stream_t stream);
+NVE_API int nve_b200_gemm_w4a16_gateup_silu(const uint16_t* X, const nve_b200_w4_matrix* gate,
+                                            const nve_b200_w4_matrix* up, uint16_t* mid, int M, int K, void* scratch,
+                                            size_t scratch_bytes, nve_stream_t stream);
+
+/* One Llama-style layer over a block of prompt positions (src/gpu_layer.rs:1086-1160 with :777-890 and :977-996), all
+ * its launches from one call: hidden [rows, hidden] f16 -> out (no alias), K/V rows start_pos .. start_pos + rows - 1 of
+ * the caches are written.  16-bit activations on every projection.  Matrices in the order q, k, v, o, gate, up, down;
+ * hidden % 64 == 0, hidden <= 8192, ffn % 64 == 0, head_dim 64 or 128; pointers 16-byte aligned (scales 8), the
+ * workspace 256-byte aligned and of at least nve_b200_prefill_layer_workspace_bytes (0: the shape is not covered). */
+typedef struct {
+    const uint8_t* nibbles[7];
+    const float* scales[7];
+    const void* input_norm;     /* [hidden] f16 */
+    const void* post_attn_norm; /* [hidden] f16 */
+    uint16_t* k_cache;          /* [num_kv_heads, max_seq, head_dim] f16 */
+    uint16_t* v_cache;
+    const uint16_t* rope_cos;   /* [max_seq, head_dim/2] f16 */
+    const uint16_t* rope_sin;
+    int hidden, ffn, num_heads, num_kv_heads, head_dim, max_seq;
+    float norm_eps, attn_scale;
+} nve_b200_rows_layer;
+NVE_API size_t nve_b200_prefill_layer_workspace_bytes(const nve_b200_rows_layer* layer, int rows);
+NVE_API int nve_b200_prefill_layer(const nve_b200_rows_layer* layer, const uint16_t* hidden, uint16_t* out, int rows,
+                                   int start_pos, void* workspace, size_t workspace_bytes, nve_stream_t stream);
 NVE_API int nve_b200_gemm_error(int reset);
 
 /* Allocation-free form of nve_b200_gemm_w4a16.  No counterpart in the reference: it exists for callers that have

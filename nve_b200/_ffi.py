@@ -78,6 +78,18 @@ class DecodeModel(C.Structure):
     ]
 
 
+class RowsLayer(C.Structure):
+    """nve_b200_rows_layer."""
+
+    _fields_ = [
+        ("nibbles", C.c_void_p * 7), ("scales", C.c_void_p * 7),
+        ("input_norm", C.c_void_p), ("post_attn_norm", C.c_void_p), ("k_cache", C.c_void_p), ("v_cache", C.c_void_p),
+        ("rope_cos", C.c_void_p), ("rope_sin", C.c_void_p),
+        ("hidden", C.c_int), ("ffn", C.c_int), ("num_heads", C.c_int), ("num_kv_heads", C.c_int),
+        ("head_dim", C.c_int), ("max_seq", C.c_int), ("norm_eps", C.c_float), ("attn_scale", C.c_float),
+    ]
+
+
 _P, _I, _F, _S = C.c_void_p, C.c_int, C.c_float, C.c_size_t
 _LL, _ULL = C.c_longlong, C.c_ulonglong
 
@@ -153,6 +165,10 @@ SIGNATURES = {
     "nve_b200_gemm_w4a16": (_I, [_P, _I, _P, _P, _P, _I, _I, _I, _I, _P, _S, _P]),
     "nve_b200_gemm_w4a16_multi_scratch_bytes": (_S, [_I, _P, _I, _I]),
     "nve_b200_gemm_w4a16_multi": (_I, [_P, _I, C.POINTER(W4Matrix), _I, _I, _I, _I, _P, _S, _P]),
+    "nve_b200_gemm_w4a16_add_rmsnorm": (_I, [_P, _P, _P, _P, _P, _P, _P, _F, _I, _I, _I, _P, _S, _P]),
+    "nve_b200_gemm_w4a16_gateup_silu": (_I, [_P, C.POINTER(W4Matrix), C.POINTER(W4Matrix), _P, _I, _I, _P, _S, _P]),
+    "nve_b200_prefill_layer_workspace_bytes": (_S, [C.POINTER(RowsLayer), _I]),
+    "nve_b200_prefill_layer": (_I, [C.POINTER(RowsLayer), _P, _P, _I, _I, _P, _S, _P]),
     "nve_b200_gemm_w4a16_wide": (_I, [_P, _I, C.POINTER(W4Matrix), _I, _I, _I, _I, _P, _S, _P]),
     "nve_b200_gemm_error": (_I, [_I]),
     "nve_b200_gemm_w4a16_noalloc": (_I, [_P, _I, _P, _P, _P, _I, _I, _I, _I, _P]),

@@ -40,6 +40,7 @@ template <int DT> __global__ void __launch_bounds__(kActThreads) quantize_q8_ker
                                                                                      float* scales, int K,
                                                                                      const float* awq_inv) {
     pdl_wait();
+    pdl_launch_dependents();
     const long long chunk = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     const bool active = chunk * 8 < K;
     float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -53,7 +54,6 @@ template <int DT> __global__ void __launch_bounds__(kActThreads) quantize_q8_ker
             for (int e = 0; e < 8; e++) v[e] = __fmul_rn(v[e], awq_inv[chunk * 8 + e]);
         }
     }
-    pdl_launch_dependents();
     quantize_quad(v, xq, scales, chunk, active);
 }
 
@@ -100,28 +100,54 @@ template <int DT, bool VEC> __device__ __forceinline__ float sum_squares(const u
     return total;
 }
 
-// RMSNorm, optionally followed by the int8 quantisation of the rounded result.  Single CTA.
+// A row of up to kRegChunks * 256 chunks stays in registers between the sum of squares and the normalisation: one round
+// trip to memory instead of two, all loads in flight together.  The norm weights, which no kernel writes, are requested
+// before the grid dependency resolves.  Same order of additions as sum_squares.
+constexpr int kRegChunks = 4;
+template <int DT> __device__ __forceinline__ float sum_squares_reg(const uint4 (&x)[kRegChunks], int chunks) {
+    __shared__ float warp_part[kActThreads / 32];
+    float acc = 0.0f;
+#pragma unroll
+    for (int j = 0; j < kRegChunks; j++)
+        if (j * kActThreads + static_cast<int>(threadIdx.x) < chunks) {
+            uint16_t h[8];
+            unpack8(x[j], h);
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+                const float v = Act16<DT>::to_f32(h[e]);
+                acc = __fmaf_rn(v, v, acc);
+            }
+        }
+    acc = warp_sum(acc);
+    if ((threadIdx.x & 31) == 0) warp_part[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    float total = warp_part[0];
+#pragma unroll
+    for (int w = 1; w < kActThreads / 32; w++) total = __fadd_rn(total, warp_part[w]);
+    return total;
+}
+__device__ __forceinline__ void load_row_reg(const uint16_t* p, int chunks, uint4 (&r)[kRegChunks]) {
+#pragma unroll
+    for (int j = 0; j < kRegChunks; j++) {
+        const int c = j * kActThreads + static_cast<int>(threadIdx.x);
+        r[j] = c < chunks ? reinterpret_cast<const uint4*>(p)[c] : make_uint4(0, 0, 0, 0);
+    }
+}
+
+// RMSNorm, optionally followed by the int8 quantisation of the rounded result.
 template <int DT, bool VEC, bool QUANT>
 __global__ void __launch_bounds__(kActThreads) rmsnorm_kernel(const uint16_t* x, const uint16_t* w, uint16_t* out,
                                                               int8_t* xq, float* scales, int n, float eps) {
     // one CTA per row of n values (a single row in every form but nve_b200_rms_norm_rows)
     x += static_cast<long long>(blockIdx.x) * n;
     if (out != nullptr) out += static_cast<long long>(blockIdx.x) * n;
-    pdl_wait();
-    const float total = sum_squares<DT, VEC>(x, n);
-    const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(n)), eps)));
-    pdl_launch_dependents();
     const int chunks = (n + 7) / 8;
     // all threads of a quad iterate together so that the group maximum can use shuffles
     const int iters = (chunks + kActThreads - 1) / kActThreads;
-    for (int it = 0; it < iters; it++) {
-        const int c = it * kActThreads + threadIdx.x;
-        const bool active = c < chunks;
+    auto finish = [&](int c, bool active, const uint16_t (&hx)[8], const uint16_t (&hw)[8], float r) {
         float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         if (active) {
-            uint16_t hx[8], hw[8], ho[8];
-            load_chunk<VEC>(x, c, n, hx);
-            load_chunk<VEC>(w, c, n, hw);
+            uint16_t ho[8];
 #pragma unroll
             for (int e = 0; e < 8; e++) {
                 const float o = __fmul_rn(__fmul_rn(Act16<DT>::to_f32(hx[e]), r), Act16<DT>::to_f32(hw[e]));
@@ -131,39 +157,107 @@ __global__ void __launch_bounds__(kActThreads) rmsnorm_kernel(const uint16_t* x,
             if (out != nullptr) store_chunk<VEC>(out, c, n, ho);
         }
         if constexpr (QUANT) quantize_quad(v, xq, scales, c, active);
+    };
+    if (VEC && chunks <= kRegChunks * kActThreads) {
+        uint4 xr[kRegChunks], wr[kRegChunks];
+        load_row_reg(w, chunks, wr);
+        pdl_wait();
+        pdl_launch_dependents();
+        load_row_reg(x, chunks, xr);
+        const float total = sum_squares_reg<DT>(xr, chunks);
+        const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(n)), eps)));
+#pragma unroll
+        for (int j = 0; j < kRegChunks; j++)
+            if (j < iters) {
+                const int c = j * kActThreads + threadIdx.x;
+                uint16_t hx[8], hw[8];
+                unpack8(xr[j], hx);
+                unpack8(wr[j], hw);
+                finish(c, c < chunks, hx, hw, r);
+            }
+        return;
+    }
+    pdl_wait();
+    pdl_launch_dependents();
+    const float total = sum_squares<DT, VEC>(x, n);
+    const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(n)), eps)));
+    for (int it = 0; it < iters; it++) {
+        const int c = it * kActThreads + threadIdx.x;
+        uint16_t hx[8] = {0, 0, 0, 0, 0, 0, 0, 0}, hw[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        if (c < chunks) {
+            load_chunk<VEC>(x, c, n, hx);
+            load_chunk<VEC>(w, c, n, hw);
+        }
+        finish(c, c < chunks, hx, hw, r);
     }
 }
 
 // x[row] += delta[row] (the residual add, stored in place with add_inplace_kernel's arithmetic) followed by the RMSNorm
-// of the updated row into out: one launch for the pair of launches between two projections of a batched layer.  The
-// CTA reads back what it stored (ordered by the CTA barrier), so the bits are those of the two separate kernels.
+// of the updated row into out: one launch for the pair of launches between two projections of a batched layer, same bits
+// as the two separate kernels.
 template <int DT> __global__ void __launch_bounds__(kActThreads) add_rmsnorm_rows_kernel(uint16_t* x, const uint16_t* delta,
                                                                                          const uint16_t* w, uint16_t* out, int n,
                                                                                          float eps) {
     x += static_cast<long long>(blockIdx.x) * n;
     delta += static_cast<long long>(blockIdx.x) * n;
     out += static_cast<long long>(blockIdx.x) * n;
-    pdl_wait();
     const int chunks = n / 8;
+    auto add8 = [](uint16_t (&hd)[8], const uint16_t (&hs)[8]) {
+#pragma unroll
+        for (int e = 0; e < 8; e++) hd[e] = Act16<DT>::from_f32(__fadd_rn(Act16<DT>::to_f32(hd[e]), Act16<DT>::to_f32(hs[e])));
+    };
+    auto norm8 = [](const uint16_t (&hx)[8], const uint16_t (&hw)[8], float r, uint16_t (&ho)[8]) {
+#pragma unroll
+        for (int e = 0; e < 8; e++)
+            ho[e] = Act16<DT>::from_f32(__fmul_rn(__fmul_rn(Act16<DT>::to_f32(hx[e]), r), Act16<DT>::to_f32(hw[e])));
+    };
+    if (chunks <= kRegChunks * kActThreads) {
+        uint4 xr[kRegChunks], dr[kRegChunks], wr[kRegChunks];
+        load_row_reg(w, chunks, wr);
+        pdl_wait();
+        pdl_launch_dependents();
+        load_row_reg(x, chunks, xr);
+        load_row_reg(delta, chunks, dr);
+#pragma unroll
+        for (int j = 0; j < kRegChunks; j++) {
+            const int c = j * kActThreads + threadIdx.x;
+            uint16_t hd[8], hs[8];
+            unpack8(xr[j], hd);
+            unpack8(dr[j], hs);
+            add8(hd, hs);
+            xr[j] = pack8(hd);
+            if (c < chunks) store_chunk<true>(x, c, n, hd);
+        }
+        const float total = sum_squares_reg<DT>(xr, chunks);
+        const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(n)), eps)));
+#pragma unroll
+        for (int j = 0; j < kRegChunks; j++) {
+            const int c = j * kActThreads + threadIdx.x;
+            uint16_t hx[8], hw[8], ho[8];
+            unpack8(xr[j], hx);
+            unpack8(wr[j], hw);
+            norm8(hx, hw, r, ho);
+            if (c < chunks) store_chunk<true>(out, c, n, ho);
+        }
+        return;
+    }
+    pdl_wait();
+    pdl_launch_dependents();
     for (int c = threadIdx.x; c < chunks; c += kActThreads) {
         uint16_t hd[8], hs[8];
         load_chunk<true>(x, c, n, hd);
         load_chunk<true>(delta, c, n, hs);
-#pragma unroll
-        for (int e = 0; e < 8; e++) hd[e] = Act16<DT>::from_f32(__fadd_rn(Act16<DT>::to_f32(hd[e]), Act16<DT>::to_f32(hs[e])));
+        add8(hd, hs);
         store_chunk<true>(x, c, n, hd);
     }
-    __syncthreads();
+    __syncthreads();  // the CTA reads back what it stored
     const float total = sum_squares<DT, true>(x, n);
     const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(n)), eps)));
-    pdl_launch_dependents();
     for (int c = threadIdx.x; c < chunks; c += kActThreads) {
         uint16_t hx[8], hw[8], ho[8];
         load_chunk<true>(x, c, n, hx);
         load_chunk<true>(w, c, n, hw);
-#pragma unroll
-        for (int e = 0; e < 8; e++)
-            ho[e] = Act16<DT>::from_f32(__fmul_rn(__fmul_rn(Act16<DT>::to_f32(hx[e]), r), Act16<DT>::to_f32(hw[e])));
+        norm8(hx, hw, r, ho);
         store_chunk<true>(out, c, n, ho);
     }
 }
@@ -175,6 +269,7 @@ __global__ void __launch_bounds__(kActThreads) silu_mul_kernel(const uint16_t* g
                                                                int8_t* xq, float* scales, int n, uint8_t* xlo,
                                                                const float* awq) {
     pdl_wait();
+    pdl_launch_dependents();
     const long long c = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     const bool active = c * 8 < n;
     float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -189,7 +284,6 @@ __global__ void __launch_bounds__(kActThreads) silu_mul_kernel(const uint16_t* g
         }
         if (out != nullptr) store_chunk<true>(out, c, n, ho);
     }
-    pdl_launch_dependents();
     if constexpr (QUANT == 1) quantize_quad(v, xq, scales, c, active);
     if constexpr (QUANT == 2) {
         if (active && awq != nullptr) {
@@ -208,6 +302,7 @@ template <int DT> __global__ void silu_mul_scalar_kernel(uint16_t* gate, const u
 template <int DT, bool VEC> __global__ void __launch_bounds__(kActThreads) add_inplace_kernel(uint16_t* dst, const uint16_t* src,
                                                                                              int n) {
     pdl_wait();
+    pdl_launch_dependents();
     const long long c = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (c * 8 >= n) return;
     uint16_t hd[8], hs[8];

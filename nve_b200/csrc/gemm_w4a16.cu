@@ -122,6 +122,36 @@ extern "C" int nve_b200_gemm_w4a16(const void* X, int x_dtype, const uint8_t* ni
     return nve_b200_gemm_w4a16_multi(X, x_dtype, &one, 1, y_dtype, M, K, scratch, scratch_bytes, stream);
 }
 
+extern "C" int nve_b200_gemm_w4a16_add_rmsnorm(const uint16_t* X, const uint8_t* nibbles, const float* scales, const uint16_t* residual,
+                                               uint16_t* Y, const uint16_t* norm_weight, uint16_t* normed, float eps, int M, int N, int K,
+                                               void* scratch, size_t scratch_bytes, nve_stream_t stream) {
+    const nve_b200_w4_matrix one = {nibbles, scales, Y, nullptr, N};
+    PairMat g[3];
+    if (!residual || !norm_weight || !normed) return set_status(NVE_ERR_BAD_POINTER);
+    if (int s = check_gemm_multi(X, NVE_DT_F16, &one, 1, NVE_DT_F16, K, g); s != NVE_OK) return s;
+    if (M < 1 || !pair_norm_fits(N)) return set_status(NVE_ERR_BAD_SHAPE);
+    if (!aligned(residual, 16) || !aligned(Y, 16) || !aligned(norm_weight, 16) || !aligned(normed, 16)) return set_status(NVE_ERR_BAD_ALIGNMENT);
+    PairFinish fin;
+    fin.res = residual;
+    fin.norm_w = norm_weight;
+    fin.normed = normed;
+    fin.eps = eps;
+    return gemm_pair(X, g, 1, NVE_DT_F16, M, K, scratch, scratch != nullptr ? scratch_bytes : 0, static_cast<cudaStream_t>(stream), fin);
+}
+
+extern "C" int nve_b200_gemm_w4a16_gateup_silu(const uint16_t* X, const nve_b200_w4_matrix* gate, const nve_b200_w4_matrix* up, uint16_t* mid,
+                                               int M, int K, void* scratch, size_t scratch_bytes, nve_stream_t stream) {
+    if (!gate || !up || !mid) return set_status(NVE_ERR_BAD_POINTER);
+    nve_b200_w4_matrix mats[2] = {*gate, *up};
+    mats[0].out = mats[1].out = mid;
+    PairMat g[3];
+    if (int s = check_gemm_multi(X, NVE_DT_F16, mats, 2, NVE_DT_F16, K, g); s != NVE_OK) return s;
+    if (M < 1 || gate->N != up->N) return set_status(NVE_ERR_BAD_SHAPE);
+    PairFinish fin;
+    fin.silu = true;
+    return gemm_pair(X, g, 2, NVE_DT_F16, M, K, scratch, scratch != nullptr ? scratch_bytes : 0, static_cast<cudaStream_t>(stream), fin);
+}
+
 extern "C" int nve_b200_gemm_error(int reset) { return gemm_pair_error(reset != 0); }
 
 // ---------------------------------------------------------------------------------------------------------

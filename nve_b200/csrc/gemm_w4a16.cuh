@@ -72,8 +72,18 @@ struct PairPlan {
     long long tiles, U, grid_pairs;
     size_t partial_bytes;  // workspace for partial tiles, 0 when every run consists of whole tiles
 };
-PairPlan pair_plan(const int* Ns, int num_mats, int M, int K, bool have_scratch, size_t avail);
-int gemm_pair(const uint16_t* X, const PairMat* mats, int num_mats, int y_dtype, int M, int K, void* partial, size_t avail, cudaStream_t st);
+// What becomes of the product (f16 outputs only; nothing set: Y = X . W^T)
+struct PairFinish {
+    const uint16_t* res = nullptr;     // one matrix: Y = res + round16(product)
+    const uint16_t* norm_w = nullptr;  // with res: also normed = RMSNorm(Y) with this weight (pair_norm_fits)
+    uint16_t* normed = nullptr;
+    float eps = 0.0f;
+    bool silu = false;                 // two matrices of the same N: Y of the first = silu(first product) * second product
+};
+PairPlan pair_plan(const int* Ns, int num_mats, int M, int K, bool have_scratch, size_t avail, bool silu = false);
+int gemm_pair(const uint16_t* X, const PairMat* mats, int num_mats, int y_dtype, int M, int K, void* partial, size_t avail, cudaStream_t st,
+              const PairFinish& fin = PairFinish());
+bool pair_norm_fits(int N);
 int gemm_pair_error(bool reset);
 
 }  // namespace nve

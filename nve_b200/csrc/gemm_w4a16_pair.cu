@@ -29,7 +29,7 @@
 // (nve_b200_gemm_error) and both CTAs leave through the normal path.
 #include <cuda.h>
 
-#include "common.cuh"
+#include "act_ops.cuh"
 #include "gemm_w4a16.cuh"
 
 namespace nve {
@@ -45,6 +45,7 @@ constexpr int kPairThreads = 24 * 32;
 constexpr int kBarRing = 24;
 constexpr int kMaxRaw = 8;
 constexpr int kRawNib = kPairRows * 128, kRawSc = kPairRows * 32, kRawBytes = kRawNib + kRawSc;
+constexpr int kPairSiluBytes = 4 * 2 * 64 * 32;
 constexpr int kPairSmemMax = 226 * 1024;  // dynamic; the barriers take the first (static) kilobyte
 constexpr unsigned long long kPairWaitLimitNs = 50ull * 1000 * 1000;  // a legitimate wait lasts microseconds
 
@@ -67,7 +68,14 @@ struct PairParams {
     int U;           // units per pair
     int total;       // units
     int sc16;        // 1: rows of scales are 16-byte aligned
+    int y2;          // 1: an output is not 4-byte aligned
+    const uint16_t* res;  // kPairAdd: [M, N] f16, added to the rounded product
 };
+// What happens to the product on its way out
+constexpr int kPairPlain = 0;  // Y = X . W^T
+constexpr int kPairAdd = 1;    // Y = res + round16(X . W^T), f16, one matrix
+constexpr int kPairSilu = 2;   // Y = silu(round16(X . G^T)) * round16(X . U^T), f16: a tile is 128 rows of G and the 128 rows of U
+                               // of the same indices, each CTA has 64 of both (TMEM lanes 0-63 and 64-127)
 
 // ---- mbarrier / TMA / tcgen05 wrappers
 __device__ __forceinline__ void pg_init(uint32_t bar, unsigned count) {
@@ -174,39 +182,55 @@ static __device__ int g_pair_error = 0;
 struct PairTile {
     int mi, n0, xt;  // matrix, first weight row of the pair's tile inside it, X tile
 };
-__device__ __forceinline__ PairTile pair_locate(const PairParams& p, int tile) {
+template <int MODE> __device__ __forceinline__ PairTile pair_locate(const PairParams& p, int tile) {
     PairTile t;
     const int wt = tile / p.XT;
     t.xt = tile - wt * p.XT;
     t.mi = wt < p.wt_end[0] ? 0 : (wt < p.wt_end[1] ? 1 : 2);
-    t.n0 = (wt - (t.mi == 0 ? 0 : p.wt_end[t.mi - 1])) * kPairTile;
+    t.n0 = (wt - (t.mi == 0 ? 0 : p.wt_end[t.mi - 1])) * (MODE == kPairSilu ? kPairTile / 2 : kPairTile);
     return t;
 }
 
 // Sixteen rows of X (rows m, m + 1, ... of Y) x this lane's feature n.  16-bit types: lanes 2i and 2i + 1 exchange values
 // so that every lane stores two neighbouring features of every second row in one 4-byte store.
-template <int ODT> __device__ __forceinline__ void pair_store(void* Y, int Nloc, int n, int lane, int m, int rows, const float (&y)[16]) {
-    if (ODT == NVE_DT_F32 || (Nloc & 1)) {
+template <int ODT, int MODE>
+__device__ __forceinline__ void pair_store(void* Y, const uint16_t* res, bool narrow, int Nloc, int n, int lane, int m, int rows, const float (&y)[16]) {
+    constexpr int DT16 = ODT == NVE_DT_BF16 ? NVE_DT_BF16 : NVE_DT_F16;
+    auto add = [](uint16_t a, uint16_t b) { return Act16<DT16>::from_f32(__fadd_rn(Act16<DT16>::to_f32(a), Act16<DT16>::to_f32(b))); };
+    if (ODT == NVE_DT_F32 || narrow || (Nloc & 1)) {
 #pragma unroll
         for (int e = 0; e < 16; e++)
-            if (e < rows && n < Nloc) store_out<ODT>(Y, static_cast<long long>(m + e) * Nloc + n, y[e]);
+            if (e < rows && n < Nloc) {
+                const long long o = static_cast<long long>(m + e) * Nloc + n;
+                if (MODE == kPairAdd) static_cast<uint16_t*>(Y)[o] = add(Act16<DT16>::from_f32(y[e]), res[o]);
+                else store_out<ODT>(Y, o, y[e]);
+            }
     } else {
         const int odd = lane & 1;
-        uint16_t* dst = static_cast<uint16_t*>(Y) + static_cast<long long>(m + odd) * Nloc + (n - odd);
+        const long long o = static_cast<long long>(m + odd) * Nloc + (n - odd);
+        uint16_t* dst = static_cast<uint16_t*>(Y) + o;
+        const uint16_t* src = MODE == kPairAdd ? res + o : nullptr;
 #pragma unroll
         for (int e = 0; e < 16; e += 2) {
-            constexpr int DT16 = ODT == NVE_DT_BF16 ? NVE_DT_BF16 : NVE_DT_F16;
             const uint32_t own = static_cast<uint32_t>(Act16<DT16>::from_f32(y[e])) | (static_cast<uint32_t>(Act16<DT16>::from_f32(y[e + 1])) << 16);
             const uint32_t other = __shfl_xor_sync(0xffffffffu, own, 1);
             // even lane: row e of (n, n + 1); odd lane: row e + 1 of (n - 1, n)
-            const uint32_t v = odd ? __byte_perm(other, own, 0x7632) : __byte_perm(own, other, 0x5410);
-            if (e + odd < rows && n < Nloc) *reinterpret_cast<uint32_t*>(dst) = v;
+            uint32_t v = odd ? __byte_perm(other, own, 0x7632) : __byte_perm(own, other, 0x5410);
+            if (e + odd < rows && n < Nloc) {
+                if (MODE == kPairAdd) {
+                    const uint32_t r = *reinterpret_cast<const uint32_t*>(src);
+                    v = static_cast<uint32_t>(add(static_cast<uint16_t>(v), static_cast<uint16_t>(r))) |
+                        (static_cast<uint32_t>(add(static_cast<uint16_t>(v >> 16), static_cast<uint16_t>(r >> 16))) << 16);
+                }
+                *reinterpret_cast<uint32_t*>(dst) = v;
+            }
             dst += 2 * static_cast<long long>(Nloc);
+            if (MODE == kPairAdd) src += 2 * static_cast<long long>(Nloc);
         }
     }
 }
 
-template <int ODT>
+template <int ODT, int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     gemm_w4a16_pair_kernel(const PairParams p, const __grid_constant__ CUtensorMap xmap) {
     extern __shared__ __align__(1024) unsigned char pg_raw[];
@@ -217,6 +241,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     const uint32_t smem = (s_addr(pg_raw) + 1023u) & ~1023u;
     const uint32_t bslot_bytes = static_cast<uint32_t>(p.NB) * 128;  // NB / 2 rows x 256 bytes
     const uint32_t sB = smem, sRaw = smem + p.xslots * bslot_bytes;
+    const uint32_t sX = sRaw + p.raw * kRawBytes;  // kPairSilu: exchange between the halves of a tile, [4 groups][2][64 lanes][32 B]
     const uint32_t full = s_addr(bars), empty = full + 8 * kBarRing, rawf = empty + 8 * kBarRing, rawe = rawf + 8 * kMaxRaw;
     const uint32_t accum = rawe + 8 * kMaxRaw, accfree = accum + 8;
     uint32_t rank;
@@ -257,7 +282,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
         const int nr = lw * 32 + (lane >> 3), nc = lane & 7;  // nibbles: rows nr, nr + 4, ..., nr + 28, 16-byte chunk nc
         const int half_k = p.K / 2;
         int tile = u0 / p.SB, sbi = u0 - (u0 / p.SB) * p.SB;
-        PairTile tl = pair_locate(p, tile);
+        PairTile tl = pair_locate<MODE>(p, tile);
         int st = 0;
         unsigned par = 1;
         for (int j = 0; j < n_units; j++) {
@@ -267,12 +292,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
                     break;
                 }
             }
-            const int row0 = tl.n0 + static_cast<int>(rank) * kPairRows, nlast = p.Nm[tl.mi] - 1;
+            // row 0 of the warp's 32: rows of one matrix, or (gate / up) rows 0-63 of the one and 64-127 of the other
+            const int mi = MODE == kPairSilu ? lw >> 1 : tl.mi;
+            const int row0 = MODE == kPairSilu ? tl.n0 + static_cast<int>(rank) * 64 - (lw >> 1) * 64 : tl.n0 + static_cast<int>(rank) * kPairRows;
+            const int nlast = p.Nm[mi] - 1;
             const uint32_t dst = sRaw + st * kRawBytes;
             {
                 // chunks past the end of K read as zero, rows past the end repeat the last one
                 const int kb = sbi * 128 + nc * 16;
-                const uint8_t* src = p.nib[tl.mi] + (kb < half_k ? kb : 0);
+                const uint8_t* src = p.nib[mi] + (kb < half_k ? kb : 0);
                 const int have = kb < half_k ? 16 : 0;
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
@@ -282,7 +310,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
                                  : "memory");
                 }
             }
-            const float* sc = p.sc[tl.mi];
+            const float* sc = p.sc[mi];
             const int b0 = sbi * 8;
             if (p.sc16) {
 #pragma unroll
@@ -311,7 +339,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
             if (++sbi == p.SB) {
                 sbi = 0;
                 tile++;
-                if (j + 1 < n_units) tl = pair_locate(p, tile);
+                if (j + 1 < n_units) tl = pair_locate<MODE>(p, tile);
             }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
@@ -354,11 +382,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
                     return false;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const PairTile tl = pair_locate(p, etile);
+                const PairTile tl = pair_locate<MODE>(p, etile);
                 const int Nloc = p.Nm[tl.mi];
                 const bool whole = eunits == p.SB;
                 const int col = static_cast<int>(rank) * kPairRows + r;
-                const int n = tl.n0 + col;  // this thread's output feature
+                // this thread's output feature (kPairSilu: lanes 64 and up hold the second factor of the same features)
+                const int n = MODE == kPairSilu ? tl.n0 + static_cast<int>(rank) * 64 + (r & 63) : tl.n0 + col;
+                int xb = 0;  // kPairSilu: half of the exchange buffer
                 const int m0 = tl.xt * p.NB;
                 const uint32_t taddr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
                 float* part = p.partial + static_cast<long long>(2 * pair + (eseg > 0 ? 1 : 0)) * p.part_rows * kPairTile + col;
@@ -381,7 +411,35 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
                         for (int e = 0; e < 16; e++)
                             if (cb + e < mrows) part[(cb + e) * kPairTile] = y[e];
                     } else {
-                        pair_store<ODT>(p.Y[tl.mi], Nloc, n, lane, m0 + cb, min(16, mrows - cb), y);
+                        if constexpr (MODE == kPairSilu) {
+                            // the upper warps hand their sixteen values over, rounded to f16 like a stored product
+                            const uint32_t buf = sX + static_cast<uint32_t>(((grp * 2 + xb) * 64 + (r & 63)) * 32);
+                            xb ^= 1;  // the other half next time: one barrier per exchange is enough
+                            if (r >= 64) {
+                                uint32_t h[8];
+#pragma unroll
+                                for (int e = 0; e < 8; e++) {
+                                    const __half2 v2 = __floats2half2_rn(y[2 * e], y[2 * e + 1]);
+                                    h[e] = *reinterpret_cast<const uint32_t*>(&v2);
+                                }
+                                asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(buf), "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3]) : "memory");
+                                asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(buf + 16), "r"(h[4]), "r"(h[5]), "r"(h[6]), "r"(h[7]) : "memory");
+                            }
+                            asm volatile("bar.sync %0, 128;" ::"r"(2 + grp) : "memory");
+                            if (r < 64) {
+                                uint32_t h[8];
+                                asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(h[0]), "=r"(h[1]), "=r"(h[2]), "=r"(h[3]) : "r"(buf) : "memory");
+                                asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(h[4]), "=r"(h[5]), "=r"(h[6]), "=r"(h[7]) : "r"(buf + 16) : "memory");
+#pragma unroll
+                                for (int e = 0; e < 16; e++) {
+                                    const float g = Act16<NVE_DT_F16>::to_f32(Act16<NVE_DT_F16>::from_f32(y[e]));
+                                    y[e] = silu_mul_f32(g, Act16<NVE_DT_F16>::to_f32(static_cast<uint16_t>(h[e >> 1] >> (16 * (e & 1)))));
+                                }
+                                pair_store<ODT, MODE>(p.Y[0], nullptr, p.y2 != 0, Nloc, n, lane, m0 + cb, min(16, mrows - cb), y);
+                            }
+                        } else {
+                            pair_store<ODT, MODE>(p.Y[tl.mi], p.res, p.y2 != 0, Nloc, n, lane, m0 + cb, min(16, mrows - cb), y);
+                        }
                     }
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -576,22 +634,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     }
 }
 
-// Tiles that more than one pair worked on: sum their partial tiles in ascending K order, convert and store.  One block
-// per (tile, four rows of X), a thread takes four consecutive features.
-template <int ODT> __global__ void __launch_bounds__(256) gemm_pair_reduce_kernel(const PairParams p) {
-    pdl_wait();
-    pdl_launch_dependents();
-    const int tile = blockIdx.x;
-    const int first = (tile * p.SB) / p.U, last = ((tile + 1) * p.SB - 1) / p.U;
-    if (first == last) return;
-    const PairTile tl = pair_locate(p, tile);
-    const int Nloc = p.Nm[tl.mi];
-    const int c4 = static_cast<int>(threadIdx.x) * 4, n = tl.n0 + c4;
-    const int mm = static_cast<int>(blockIdx.y * blockDim.y + threadIdx.y), m = tl.xt * p.NB + mm;
-    if (n >= Nloc || mm >= p.NB || m >= p.M) return;
+// Sum of four consecutive columns of row mm of a tile over the pairs that worked on it, in ascending K order.
+__device__ __forceinline__ float4 pair_sum4(const PairParams& p, int tile, int first, int last, int mm, int col) {
     auto part = [&](int c) {
         const int slot = 2 * c + (c * p.U >= tile * p.SB ? 0 : 1);  // the pair's first segment when its run starts inside this tile
-        return __ldcg(reinterpret_cast<const float4*>(p.partial + (static_cast<long long>(slot) * p.part_rows + mm) * kPairTile + c4));
+        return __ldcg(reinterpret_cast<const float4*>(p.partial + (static_cast<long long>(slot) * p.part_rows + mm) * kPairTile + col));
     };
     float4 y = part(first);
     for (int c = first + 1; c <= last; c++) {
@@ -601,11 +648,115 @@ template <int ODT> __global__ void __launch_bounds__(256) gemm_pair_reduce_kerne
         y.z = __fadd_rn(y.z, v.z);
         y.w = __fadd_rn(y.w, v.w);
     }
+    return y;
+}
+
+// Tiles that more than one pair worked on: sum their partial tiles, finish as the epilogue would and store.  One block
+// per (tile, four rows of X), a thread takes four consecutive features.
+template <int ODT, int MODE> __global__ void __launch_bounds__(256) gemm_pair_reduce_kernel(const PairParams p) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int tile = blockIdx.x;
+    const int first = (tile * p.SB) / p.U, last = ((tile + 1) * p.SB - 1) / p.U;
+    if (first == last) return;
+    const PairTile tl = pair_locate<MODE>(p, tile);
+    const int Nloc = p.Nm[tl.mi];
+    const int c4 = static_cast<int>(threadIdx.x) * 4, n = tl.n0 + c4;
+    const int mm = static_cast<int>(blockIdx.y * blockDim.y + threadIdx.y), m = tl.xt * p.NB + mm;
+    if (n >= Nloc || mm >= p.NB || m >= p.M) return;
     const long long o = static_cast<long long>(m) * Nloc + n;
-    const float yy[4] = {y.x, y.y, y.z, y.w};
+    // kPairSilu: feature c4 of the tile is column (c4 & 63) of CTA c4 / 64, its second factor 64 columns further
+    const int col = MODE == kPairSilu ? (c4 >> 6) * kPairRows + (c4 & 63) : c4;
+    const float4 y = pair_sum4(p, tile, first, last, mm, col);
+    float yy[4] = {y.x, y.y, y.z, y.w};
+    if constexpr (MODE == kPairSilu) {
+        const float4 u = pair_sum4(p, tile, first, last, mm, col + 64);
+        const float uu[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            yy[e] = silu_mul_f32(Act16<NVE_DT_F16>::to_f32(Act16<NVE_DT_F16>::from_f32(yy[e])), Act16<NVE_DT_F16>::to_f32(Act16<NVE_DT_F16>::from_f32(uu[e])));
+    }
+    if constexpr (MODE == kPairAdd) {
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            if (n + e < Nloc)
+                yy[e] = __fadd_rn(Act16<NVE_DT_F16>::to_f32(Act16<NVE_DT_F16>::from_f32(yy[e])), Act16<NVE_DT_F16>::to_f32(p.res[o + e]));
+    }
 #pragma unroll
     for (int e = 0; e < 4; e++)
         if (n + e < Nloc) store_out<ODT>(p.Y[tl.mi], o + e, yy[e]);
+}
+
+// The same for one matrix whose product goes through the residual add and an RMSNorm: one block per row of X finishes
+// the row -- Y = res + round16(product), normed = RMSNorm(Y) -- with the arithmetic and the summation order of the separate
+// kernels (thread t takes the 8-element chunks t, t + 256, ...).  Tiles that one pair covered are in Y already.
+constexpr int kPairNormChunks = 4;  // 8-element chunks per thread: N <= 8192
+__global__ void __launch_bounds__(256) gemm_pair_reduce_norm_kernel(const PairParams p, const uint16_t* norm_w, uint16_t* normed, float eps) {
+    __shared__ float warp_part[8];
+    const int m = blockIdx.x, N = p.Nm[0], chunks = N >> 3;
+    const int xt = m / p.NB, mm = m - xt * p.NB;
+    const long long row = static_cast<long long>(m) * N;
+    uint4 w[kPairNormChunks], rs[kPairNormChunks], h[kPairNormChunks];
+#pragma unroll
+    for (int j = 0; j < kPairNormChunks; j++) {
+        const int c = j * 256 + static_cast<int>(threadIdx.x);
+        if (c < chunks) w[j] = reinterpret_cast<const uint4*>(norm_w)[c];  // static, unlike what follows
+    }
+    pdl_wait();
+    pdl_launch_dependents();
+    uint16_t* y16 = static_cast<uint16_t*>(p.Y[0]);
+#pragma unroll
+    for (int j = 0; j < kPairNormChunks; j++) {
+        const int c = j * 256 + static_cast<int>(threadIdx.x);
+        if (c < chunks) rs[j] = reinterpret_cast<const uint4*>(p.res + row)[c];
+    }
+    float acc = 0.0f;
+#pragma unroll
+    for (int j = 0; j < kPairNormChunks; j++) {
+        const int c = j * 256 + static_cast<int>(threadIdx.x);
+        if (c < chunks) {
+            const int wt = c >> 5, col = (c & 31) * 8, tile = wt * p.XT + xt;
+            const int first = (tile * p.SB) / p.U, last = ((tile + 1) * p.SB - 1) / p.U;
+            uint16_t a[8], b[8];
+            if (first == last) {
+                unpack8(__ldcg(reinterpret_cast<const uint4*>(y16 + row) + c), a);
+            } else {
+                const float4 lo = pair_sum4(p, tile, first, last, mm, col), hi = pair_sum4(p, tile, first, last, mm, col + 4);
+                const float f[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+                for (int e = 0; e < 8; e++) a[e] = Act16<NVE_DT_F16>::from_f32(f[e]);
+            }
+            unpack8(rs[j], b);
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+                a[e] = Act16<NVE_DT_F16>::from_f32(__fadd_rn(Act16<NVE_DT_F16>::to_f32(a[e]), Act16<NVE_DT_F16>::to_f32(b[e])));
+                const float v = Act16<NVE_DT_F16>::to_f32(a[e]);
+                acc = __fmaf_rn(v, v, acc);
+            }
+            h[j] = pack8(a);
+            reinterpret_cast<uint4*>(y16 + row)[c] = h[j];
+        }
+    }
+    acc = warp_sum(acc);
+    if ((threadIdx.x & 31) == 0) warp_part[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    float total = warp_part[0];
+#pragma unroll
+    for (int i = 1; i < 8; i++) total = __fadd_rn(total, warp_part[i]);
+    const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(N)), eps)));
+#pragma unroll
+    for (int j = 0; j < kPairNormChunks; j++) {
+        const int c = j * 256 + static_cast<int>(threadIdx.x);
+        if (c < chunks) {
+            uint16_t a[8], b[8];
+            unpack8(h[j], a);
+            unpack8(w[j], b);
+#pragma unroll
+            for (int e = 0; e < 8; e++)
+                a[e] = Act16<NVE_DT_F16>::from_f32(__fmul_rn(__fmul_rn(Act16<NVE_DT_F16>::to_f32(a[e]), r), Act16<NVE_DT_F16>::to_f32(b[e])));
+            reinterpret_cast<uint4*>(normed + row)[c] = pack8(a);
+        }
+    }
 }
 
 using PairEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -640,14 +791,16 @@ static bool pair_x_map(CUtensorMap* map, const uint16_t* X, int K, int M, int bo
 // pairs, rounded up; at least two units = 512 weights per row): few tiles are split over K so that every SM works, and
 // a tile count that is not a multiple of the pair count costs total / pairs instead of a whole extra wave.  Without a
 // workspace a pair takes exactly one tile.
-PairPlan pair_plan(const int* Ns, int num_mats, int M, int K, bool have_scratch, size_t avail) {
+PairPlan pair_plan(const int* Ns, int num_mats, int M, int K, bool have_scratch, size_t avail, bool silu) {
     PairPlan g;
     g.XT = (M + 255) / 256;
     g.NB = ((M + g.XT - 1) / g.XT + 31) / 32 * 32;
     g.XT = (M + g.NB - 1) / g.NB;
     g.SB = (K + 255) / 256;
     long long wt = 0;
-    for (int i = 0; i < num_mats; i++) wt += (Ns[i] + kPairTile - 1) / kPairTile;
+    if (silu) wt = (Ns[0] + kPairTile / 2 - 1) / (kPairTile / 2);
+    else
+        for (int i = 0; i < num_mats; i++) wt += (Ns[i] + kPairTile - 1) / kPairTile;
     g.tiles = wt * g.XT;
     const long long total = g.tiles * g.SB;
     const int pairs = max(1, sm_count() / 2);
@@ -667,11 +820,12 @@ PairPlan pair_plan(const int* Ns, int num_mats, int M, int K, bool have_scratch,
     return g;
 }
 
-template <int ODT> static int launch_pair(const PairParams& p, long long pairs, long long tiles, const CUtensorMap& xmap, int smem, cudaStream_t st) {
-    auto kern = gemm_w4a16_pair_kernel<ODT>;
+template <int ODT, int MODE>
+static int launch_pair(const PairParams& p, const PairPlan& g, const CUtensorMap& xmap, int smem, const PairFinish& fin, cudaStream_t st) {
+    auto kern = gemm_w4a16_pair_kernel<ODT, MODE>;
     if (int s = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kPairSmemMax); s != NVE_OK) return s;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(2 * pairs));
+    cfg.gridDim = dim3(static_cast<unsigned>(2 * g.grid_pairs));
     cfg.blockDim = dim3(kPairThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -685,36 +839,47 @@ template <int ODT> static int launch_pair(const PairParams& p, long long pairs, 
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p, xmap);
     count_launch();
     if (e != cudaSuccess) return set_cuda_status(e);
-    if (p.U % p.SB != 0) {
-        cfg.gridDim = dim3(static_cast<unsigned>(tiles), static_cast<unsigned>((p.part_rows + 3) / 4));
-        cfg.blockDim = dim3(kPairTile / 4, 4);
-        cfg.dynamicSmemBytes = 0;
-        e = cudaLaunchKernelEx(&cfg, gemm_pair_reduce_kernel<ODT>, p);
+    cfg.dynamicSmemBytes = 0;
+    if (fin.norm_w != nullptr) {
+        cfg.gridDim = dim3(static_cast<unsigned>(p.M));
+        cfg.blockDim = dim3(256);
+        e = cudaLaunchKernelEx(&cfg, gemm_pair_reduce_norm_kernel, p, fin.norm_w, fin.normed, fin.eps);
+        count_launch();
+    } else if (p.U % p.SB != 0) {
+        cfg.gridDim = dim3(static_cast<unsigned>(g.tiles), static_cast<unsigned>((p.part_rows + 3) / 4));
+        cfg.blockDim = dim3(MODE == kPairSilu ? kPairTile / 8 : kPairTile / 4, MODE == kPairSilu ? 8 : 4);
+        if (MODE == kPairSilu) cfg.gridDim.y = static_cast<unsigned>((p.part_rows + 7) / 8);
+        e = cudaLaunchKernelEx(&cfg, gemm_pair_reduce_kernel<ODT, MODE>, p);
         count_launch();
     }
     return set_cuda_status(e);
 }
 
-int gemm_pair(const uint16_t* X, const PairMat* mats, int num_mats, int y_dtype, int M, int K, void* partial, size_t avail, cudaStream_t st) {
+int gemm_pair(const uint16_t* X, const PairMat* mats, int num_mats, int y_dtype, int M, int K, void* partial, size_t avail, cudaStream_t st,
+              const PairFinish& fin) {
     PairParams p = {};
     int Ns[3] = {0, 0, 0};
     for (int i = 0; i < num_mats; i++) Ns[i] = mats[i].N;
-    const PairPlan g = pair_plan(Ns, num_mats, M, K, partial != nullptr, avail);
+    const PairPlan g = pair_plan(Ns, num_mats, M, K, partial != nullptr, avail, fin.silu);
     if (g.tiles * g.SB > 0x3FFFFFFFll) return set_status(NVE_ERR_BAD_SHAPE);
     CUtensorMap xmap;
     if (!pair_x_map(&xmap, X, K, M, g.NB / 2)) return set_status(NVE_ERR_CUDA);
     int wt = 0;
     p.sc16 = (K % 128) == 0;
+    const int rows = fin.silu ? kPairTile / 2 : kPairTile;
     for (int i = 0; i < 3; i++) {
         const PairMat& m = mats[i < num_mats ? i : 0];
         p.nib[i] = m.nib;
         p.sc[i] = m.sc;
         p.Y[i] = m.Y;
         p.Nm[i] = i < num_mats ? m.N : 0;
-        if (i < num_mats) wt += (m.N + kPairTile - 1) / kPairTile;
+        if (i < (fin.silu ? 1 : num_mats)) wt += (m.N + rows - 1) / rows;
         p.wt_end[i] = wt;
         if (!aligned(m.sc, 16)) p.sc16 = 0;
+        if (!aligned(m.Y, 4)) p.y2 = 1;
     }
+    p.res = fin.res;
+    if (!aligned(fin.res, 4)) p.y2 = 1;
     p.partial = static_cast<float*>(partial);
     p.M = M;
     p.K = K;
@@ -731,13 +896,19 @@ int gemm_pair(const uint16_t* X, const PairMat* mats, int num_mats, int y_dtype,
     p.slots = min(7, (512 - p.W * p.NB) / kPairStepCols);
     // shared memory: the X rows of a step take NB * 128 bytes per CTA; at 256 rows five of them and two raw units
     // (four steps), for narrow tiles up to twelve steps of X and eight raw units, which is what hides HBM latency
+    const int extra = fin.silu ? kPairSiluBytes : 0;
     p.raw = g.NB > 192 ? 2 : (g.NB > 96 ? 4 : (g.NB > 32 ? 6 : 8));
-    p.xslots = min(12, (kPairSmemMax - 1024 - p.raw * kRawBytes) / (p.NB * 128));
-    const int smem = 1024 + p.xslots * p.NB * 128 + p.raw * kRawBytes;
-    if (y_dtype == NVE_DT_F32) return launch_pair<NVE_DT_F32>(p, g.grid_pairs, g.tiles, xmap, smem, st);
-    return y_dtype == NVE_DT_F16 ? launch_pair<NVE_DT_F16>(p, g.grid_pairs, g.tiles, xmap, smem, st)
-                                 : launch_pair<NVE_DT_BF16>(p, g.grid_pairs, g.tiles, xmap, smem, st);
+    p.xslots = min(12, (kPairSmemMax - 1024 - extra - p.raw * kRawBytes) / (p.NB * 128));
+    const int smem = 1024 + p.xslots * p.NB * 128 + p.raw * kRawBytes + extra;
+    if (fin.silu) return launch_pair<NVE_DT_F16, kPairSilu>(p, g, xmap, smem, fin, st);
+    if (fin.norm_w != nullptr) return launch_pair<NVE_DT_F16, kPairPlain>(p, g, xmap, smem, fin, st);  // the add is in the second kernel
+    if (fin.res != nullptr) return launch_pair<NVE_DT_F16, kPairAdd>(p, g, xmap, smem, fin, st);
+    if (y_dtype == NVE_DT_F32) return launch_pair<NVE_DT_F32, kPairPlain>(p, g, xmap, smem, fin, st);
+    return y_dtype == NVE_DT_F16 ? launch_pair<NVE_DT_F16, kPairPlain>(p, g, xmap, smem, fin, st)
+                                 : launch_pair<NVE_DT_BF16, kPairPlain>(p, g, xmap, smem, fin, st);
 }
+
+bool pair_norm_fits(int N) { return (N & 7) == 0 && N <= 8 * 256 * kPairNormChunks; }
 
 int gemm_pair_error(bool reset) {
     int v = 0;

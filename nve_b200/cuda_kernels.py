@@ -765,6 +765,54 @@ def gemm_w4a16_wide(x: Tensor, weights: Sequence, k: int, outs: Sequence[Tensor]
     return list(outs)
 
 
+def gemm_w4a16_silu_scratch_bytes(m: int, n: int, k: int) -> int:
+    """Workspace of gemm_w4a16_gateup_silu: its tiles are 128 rows of both matrices."""
+    return gemm_w4a16_multi_scratch_bytes(m, [256 * ((n + 127) // 128)], k)
+
+
+def gemm_w4a16_add_rmsnorm(x: Tensor, w, k: int, residual: Tensor, norm_weight: Tensor, eps: float, out: Tensor, normed: Tensor,
+                           scratch: Optional[Tensor] = None):
+    """out = residual + x . W^T and normed = RMSNorm(out) for a (nibbles, scales, n) triple, f16: the GEMM and the launch
+    that finishes it.  Bits of gemm_w4a16_wide followed by add_rms_norm_rows."""
+    nib, sc, n = w
+    m = x.shape[0]
+    if scratch is None:
+        scratch = torch.empty(max(16, gemm_w4a16_multi_scratch_bytes(m, [n], k)), dtype=torch.uint8, device=x.device)
+    _ffi.check("nve_b200_gemm_w4a16_add_rmsnorm",
+               _lib().nve_b200_gemm_w4a16_add_rmsnorm(_ptr(x, _F16, "x"), _ptr(nib, torch.uint8), _ptr(sc, torch.float32), _ptr(residual, _F16),
+                                                      _ptr(out, _F16), _ptr(norm_weight, _F16), _ptr(normed, _F16), float(eps), m, int(n), k,
+                                                      _ptr(scratch), scratch.numel() * scratch.element_size(), stream()))
+    return out, normed
+
+
+def gemm_w4a16_gateup_silu(x: Tensor, gate, up, k: int, out: Tensor, scratch: Optional[Tensor] = None) -> Tensor:
+    """out = silu(x . gate^T) * (x . up^T), f16; gate / up are (nibbles, scales, n) triples.  Bits of gemm_w4a16_wide on both
+    followed by silu_mul_inplace, up to the order of the f32 additions where the work is split differently."""
+    m = x.shape[0]
+    if scratch is None:
+        scratch = torch.empty(max(16, gemm_w4a16_silu_scratch_bytes(m, gate[2], k)), dtype=torch.uint8, device=x.device)
+    g = W4Matrix(_ptr(gate[0], torch.uint8), _ptr(gate[1], torch.float32), None, None, gate[2])
+    u = W4Matrix(_ptr(up[0], torch.uint8), _ptr(up[1], torch.float32), None, None, up[2])
+    _ffi.check("nve_b200_gemm_w4a16_gateup_silu",
+               _lib().nve_b200_gemm_w4a16_gateup_silu(_ptr(x, _F16, "x"), C.byref(g), C.byref(u), _ptr(out, _F16), m, k, _ptr(scratch),
+                                                      scratch.numel() * scratch.element_size(), stream()))
+    return out
+
+
+def prefill_layer(layer: "_ffi.RowsLayer", hidden: Tensor, start_pos: int) -> Optional[Tensor]:
+    """A whole prefill layer in one call; None when the shape is not covered."""
+    lib = _lib()
+    rows = hidden.shape[0]
+    need = lib.nve_b200_prefill_layer_workspace_bytes(C.byref(layer), rows)
+    if need == 0:
+        return None
+    ws = torch.empty(need, dtype=torch.uint8, device=hidden.device)  # blocks of the caching allocator are 512-byte aligned
+    out = torch.empty_like(hidden)
+    _ffi.check("nve_b200_prefill_layer",
+               lib.nve_b200_prefill_layer(C.byref(layer), hidden.data_ptr(), out.data_ptr(), rows, start_pos, ws.data_ptr(), need, stream()))
+    return out
+
+
 def gemm_w4a16_noalloc(x: Tensor, nibbles: Tensor, scales: Tensor, n: int, k: int, out: Tensor) -> Tensor:
     """Batched W4A16 GEMM for callers that cannot allocate: the caller passes input and output tensors only, the
     workspace for partial tiles is a fixed 4 MiB array inside the library (shapes needing more raise NVE_ERR_TOO_LARGE).

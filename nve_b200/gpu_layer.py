@@ -384,14 +384,31 @@ def gpu_layer_forward_decode(hidden: Tensor, layer_idx: int, state: GpuInference
 
 
 
+def _rows_layer(w: GpuLayerWeights, state: GpuInferenceState, layer_idx: int, hidden: int):
+    """The descriptor of nve_b200_prefill_layer for the tensors as they are now (a few microseconds)."""
+    from ._ffi import RowsLayer
+
+    d = RowsLayer()
+    for i, p in enumerate((w.q_proj, w.k_proj, w.v_proj, w.o_proj, w.gate_proj, w.up_proj, w.down_proj)):
+        d.nibbles[i], d.scales[i] = ck._ptr(p.nibbles, torch.uint8, "nibbles"), ck._ptr(p.scales, torch.float32, "scales")
+    f16 = torch.float16
+    d.input_norm, d.post_attn_norm = ck._ptr(w.input_norm, f16), ck._ptr(w.post_attn_norm, f16)
+    d.k_cache, d.v_cache = ck._ptr(state.kv_cache.k[layer_idx], f16), ck._ptr(state.kv_cache.v[layer_idx], f16)
+    d.rope_cos, d.rope_sin = ck._ptr(state.rope_cos, f16), ck._ptr(state.rope_sin, f16)
+    d.hidden, d.ffn, d.num_heads, d.num_kv_heads = hidden, w.gate_proj.n, state.num_heads, state.num_kv_heads
+    d.head_dim, d.max_seq = state.head_dim, state.kv_cache.max_seq
+    d.norm_eps, d.attn_scale = state.norm_eps, float(state.head_dim) ** -0.5
+    return d
+
+
 def gpu_layer_forward_prefill(hidden: Tensor, layer_idx: int, state: GpuInferenceState, start_pos: int) -> Tensor:
     """src/gpu_layer.rs:1086-1160 with gpu_attn_prefill (:777-890) and the batch > 1 branch of gpu_ffn (:977-996) for
     W4 weights: all S prompt positions of one sequence through one layer.  hidden [S, hidden] f16 -> same shape; the
     K/V cache of the layer receives positions start_pos .. start_pos + S - 1.
 
     The reference dequantises every projection to f16 and calls a dense GEMM, runs RMSNorm once per token and an
-    unfused masked attention; here the projections are the tensor-core GEMM on the packed weights (q/k/v and gate/up one
-    launch each per 64-row slice), RMSNorm / KV write / causal attention are one launch each.  Like the reference's
+    unfused masked attention; here the projections are the tensor-core GEMM on the packed weights, and without activation
+    multipliers the whole layer is one call into the library (nve_b200_prefill_layer).  Like the reference's
     prefill, every layer runs on 16-bit activations (the int8 route is a batch-1 path, :1017-1025)."""
     if hidden.dim() != 2:
         raise ValueError("hidden must be [S, hidden]")
@@ -402,6 +419,12 @@ def gpu_layer_forward_prefill(hidden: Tensor, layer_idx: int, state: GpuInferenc
     if start_pos < 0 or start_pos + S > max_seq:
         raise ValueError("the block does not fit the K/V cache")
     eps, scale = state.norm_eps, float(hd) ** -0.5
+    projs = (w.q_proj, w.k_proj, w.v_proj, w.o_proj, w.gate_proj, w.up_proj, w.down_proj)
+    if S > 1 and hidden.dtype == torch.float16 and hidden.is_contiguous() and hidden.data_ptr() % 16 == 0 and \
+            all(p.awq_scales is None for p in projs):
+        out = ck.prefill_layer(_rows_layer(w, state, layer_idx, hidden.shape[1]), hidden, start_pos)
+        if out is not None:
+            return out
     normed = ck.rms_norm_rows(hidden, w.input_norm, eps)
     q, k, v = matmul_x_multi(normed, [w.q_proj, w.k_proj, w.v_proj])
     ck.fused_rope_prefill(q, k, state.rope_cos, state.rope_sin, S, nh, nkv, hd, start_pos)
@@ -456,7 +479,8 @@ class BatchedDecodeScratch:
         f16 = torch.float16
         z = lambda n: torch.zeros((batch, n), dtype=f16, device=device)
         groups = [([nh * hd, nkv * hd, nkv * hd], hidden), ([hidden], nh * hd), ([ffn, ffn], hidden), ([hidden], ffn)]
-        nbytes = max(ck.gemm_w4a16_multi_scratch_bytes(min(batch, 64), ns, k) for ns, k in groups) if batch > 1 else 0
+        nbytes = max([ck.gemm_w4a16_multi_scratch_bytes(batch, ns, k) for ns, k in groups] +
+                     [ck.gemm_w4a16_silu_scratch_bytes(batch, ffn, hidden)]) if batch > 1 else 0
         return BatchedDecodeScratch(z(hidden), z(nh * hd), z(nkv * hd), z(nkv * hd), z(nh * hd), z(hidden), z(ffn), z(ffn),
                                     [z(hidden), z(hidden)], torch.empty(max(16, nbytes), dtype=torch.uint8, device=device))
 
@@ -467,9 +491,9 @@ def gpu_layer_forward_decode_batch(hidden: Tensor, layer_idx: int, state: GpuInf
     """One decode step of B independent sequences through one layer: hidden [B, hidden] f16 -> same shape.  Row b is the
     next token of sequence b at position d_pos[b] (int32 device tensors [B]); kv holds the sequences' caches.
 
-    The projections are the tensor-core GEMM on the packed weights (B <= 64 rows per launch; q/k/v and gate/up one launch
-    each), RoPE + K/V write + attention of all sequences is one launch of the fused decode kernel, RMSNorm one launch
-    over the rows.  16-bit activations on every layer, as in prefill.  Row b equals the single-sequence decode of that
+    The projections are the tensor-core GEMM on the packed weights (q/k/v and gate/up one launch each; the residual add and
+    the second RMSNorm ride on the o projection, SiLU*up on gate/up), RoPE + K/V write + attention of all sequences is one
+    launch of the fused decode kernel.  16-bit activations on every layer, as in prefill.  Row b equals the single-sequence decode of that
     sequence within the tolerance that separates the tensor-core GEMM from the integer GEMV.  With `scratch` nothing is
     allocated and the result is one of scratch.out (alternating with the layer index).
 
@@ -491,10 +515,21 @@ def gpu_layer_forward_decode_batch(hidden: Tensor, layer_idx: int, state: GpuInf
     q, k, v = matmul_x_multi(normed, [w.q_proj, w.k_proj, w.v_proj], ws, None if s is None else [s.q, s.k, s.v])
     attn = ck.attn_decode_fused_batch(q, k, v, kv.k[layer_idx], kv.v[layer_idx], state.rope_cos, state.rope_sin, d_pos,
                                       d_seqlen, nh, nkv, hd, kv.max_seq, scale, out=None if s is None else s.attn)
-    h1 = matmul_x(attn, w.o_proj, ws, None if s is None else s.h1)
-    normed2 = ck.add_rms_norm_rows(h1, hidden, w.post_attn_norm, eps, out=None if s is None else s.normed)
-    gate, up = matmul_x_multi(normed2, [w.gate_proj, w.up_proj], ws, None if s is None else [s.gate, s.up])
-    ck.silu_mul_inplace(gate, up)
+    plain = hidden.dtype == torch.float16 and all(p.awq_scales is None for p in (w.o_proj, w.gate_proj, w.up_proj))
+    h1 = torch.empty_like(hidden) if s is None else s.h1
+    if plain and hidden.shape[0] > 1 and hidden.shape[1] % 8 == 0 and hidden.shape[1] <= 8192:
+        # the launch that sums the GEMM's partial tiles also adds the residual and normalises
+        _, normed2 = ck.gemm_w4a16_add_rmsnorm(attn, w.o_proj.triple(), w.o_proj.k, hidden, w.post_attn_norm, eps, h1,
+                                               torch.empty_like(hidden) if s is None else s.normed, ws)
+    else:
+        matmul_x(attn, w.o_proj, ws, h1)
+        normed2 = ck.add_rms_norm_rows(h1, hidden, w.post_attn_norm, eps, out=None if s is None else s.normed)
+    if plain and hidden.shape[0] > 1:
+        gate = torch.empty((hidden.shape[0], w.gate_proj.n), dtype=hidden.dtype, device=hidden.device) if s is None else s.gate
+        ck.gemm_w4a16_gateup_silu(normed2, w.gate_proj.triple(), w.up_proj.triple(), w.gate_proj.k, gate, ws)
+    else:
+        gate, up = matmul_x_multi(normed2, [w.gate_proj, w.up_proj], ws, None if s is None else [s.gate, s.up])
+        ck.silu_mul_inplace(gate, up)
     out = matmul_x(gate, w.down_proj, ws, None if s is None else s.out[layer_idx & 1])
     if defer_add:
         return out, h1
