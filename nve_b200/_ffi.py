@@ -225,3 +225,23 @@ def check_last(fn: str) -> None:
     st = lib.nve_b200_last_status()
     if st != 0:
         raise NveKernelError(fn, st, lib.nve_b200_last_cuda_error())
+
+
+_host = None
+
+
+def host():
+    """The native torch-tensor wrappers (nve_b200/_host.so); raises if they are not built."""
+    global _host
+    if _host is None:
+        load()
+        import torch
+
+        try:
+            from . import _host as mod
+        except ImportError as e:
+            raise ImportError(f"nve_b200/_host.so cannot be imported ({e}): build it with `python -m nve_b200.build`") from e
+
+        mod.set_raise(check, torch.OutOfMemoryError)
+        _host = mod
+    return _host

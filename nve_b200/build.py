@@ -2,7 +2,8 @@
 
 The library is the product: a plain C-ABI shared object with no torch or Python types in its
 signatures (see include/nve_kernels.h).  ``python -m nve_b200.build`` compiles every ``.cu`` file
-under ``csrc/`` in parallel and links ``nve_b200/lib/libnve_kernels.so``.
+under ``csrc/`` in parallel and links ``nve_b200/lib/libnve_kernels.so``, then builds the Python
+module ``nve_b200/_host.so`` (csrc/host/), native wrappers over the library for torch tensors.
 """
 from __future__ import annotations
 
@@ -18,6 +19,8 @@ CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_DIR = os.path.join(PKG_DIR, "lib")
 OBJ_DIR = os.path.join(PKG_DIR, "build")
 LIB_PATH = os.path.join(LIB_DIR, "libnve_kernels.so")
+HOST_SRC = os.path.join(CSRC, "host", "torch_calls.cpp")
+HOST_PATH = os.path.join(PKG_DIR, "_host.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -69,6 +72,38 @@ def _compile_one(src: str, verbose: bool, ptxas_v: bool) -> str:
     return obj
 
 
+def build_host(verbose: bool = False, force: bool = False) -> str:
+    """Compile the torch-tensor wrappers against the installed torch; rebuilt when the source, the C ABI or torch changes."""
+    import sysconfig
+
+    import torch
+
+    stamp = os.path.join(OBJ_DIR, "_host.sha")
+    h = hashlib.sha256(f"{torch.__version__} {sys.version}".encode())
+    for dep in (HOST_SRC, os.path.join(PKG_DIR, "..", "include", "nve_kernels.h")):
+        with open(dep, "rb") as fh:
+            h.update(fh.read())
+    if not force and os.path.exists(HOST_PATH) and os.path.exists(stamp) and open(stamp).read() == h.hexdigest():
+        return HOST_PATH
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           HOST_SRC, "-o", HOST_PATH]
+    for inc in (sysconfig.get_paths()["include"], os.path.join(root, "include"),
+                os.path.join(root, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include")):
+        cmd += ["-isystem", inc]
+    cmd += ["-L", LIB_DIR, "-lnve_kernels", "-Wl,-rpath,$ORIGIN/lib", "-L", os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu",
+            "-ltorch_cuda", "-ltorch_python"]
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed for {HOST_SRC}:\n{res.stdout}\n{res.stderr}")
+    with open(stamp, "w") as fh:
+        fh.write(h.hexdigest())
+    return HOST_PATH
+
+
 def build(verbose: bool = False, ptxas_v: bool = False, force: bool = False) -> str:
     """Compile and link the library; returns its path.  Incremental unless ``force``."""
     os.makedirs(LIB_DIR, exist_ok=True)
@@ -87,6 +122,7 @@ def build(verbose: bool = False, ptxas_v: bool = False, force: bool = False) -> 
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
+    build_host(verbose, force)
     return LIB_PATH
 
 

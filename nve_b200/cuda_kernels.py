@@ -33,17 +33,19 @@ def stream() -> int:
     s = getattr(_tls, "capture_stream", None)
     if s is not None:
         return s
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def set_graph_capture_stream(s: int) -> None:
     """src/cuda_kernels.rs:46-49."""
     _tls.capture_stream = int(s) if s else None
+    _ffi.host().set_capture_stream(int(s) if s else 0)
 
 
 def clear_graph_capture_stream() -> None:
     """src/cuda_kernels.rs:51-53."""
     _tls.capture_stream = None
+    _ffi.host().set_capture_stream(0)
 
 
 # --------------------------------------------------------------------------- pointer helpers
@@ -181,9 +183,7 @@ def fused_matvec_into(x: Tensor, w: Tensor, out: Tensor, n: int, k: int) -> None
 def fused_matvec_w4a16(x: Tensor, nibbles: Tensor, scales: Tensor, awq_scales: Optional[Tensor], n: int,
                        k: int) -> Tensor:
     """src/cuda_kernels.rs:463-486: returns [1, n] f16."""
-    out = torch.empty((1, n), dtype=_F16, device=x.device)
-    fused_matvec_w4a16_into(x, nibbles, scales, awq_scales, out, n, k)
-    return out
+    return _ffi.host().matvec_w4a16(x, nibbles, scales, awq_scales, n, k)
 
 
 def fused_matvec_w4a16_into(x: Tensor, nibbles: Tensor, scales: Tensor, awq_scales: Optional[Tensor], out: Tensor,
@@ -206,24 +206,12 @@ def dequant_w4a16(nibbles: Tensor, scales: Tensor, awq_scales: Optional[Tensor],
 
 def quantize_f16_q8(x: Tensor) -> Tuple[Tensor, Tensor]:
     """src/cuda_kernels.rs:525-540: returns (xq [K] int8, xq_scales [K/32] f32)."""
-    k = x.numel()
-    if k % 32 != 0:
-        raise ValueError("quantize_f16_q8: K must be multiple of 32")
-    xq = torch.empty(k, dtype=torch.int8, device=x.device)
-    scales = torch.empty(k // 32, dtype=torch.float32, device=x.device)
-    _lib().nve_quantize_f16_q8(_ptr(x, _F16, "x"), _ptr(xq), _ptr(scales), k, stream())
-    _ffi.check_last("nve_quantize_f16_q8")
-    return xq, scales
+    return _ffi.host().quantize_f16_q8(x)
 
 
 def matvec_w4a8(xq: Tensor, xq_scales: Tensor, nibbles: Tensor, wt_scales: Tensor, n: int, k: int) -> Tensor:
     """src/cuda_kernels.rs:552-573: returns [1, n] f16."""
-    out = torch.empty((1, n), dtype=_F16, device=xq.device)
-    _lib().nve_matvec_w4a8(_ptr(xq, _Q8, "xq"), _ptr(xq_scales, torch.float32, "xq_scales"),
-                           _ptr(nibbles, torch.uint8, "nibbles"), _ptr(wt_scales, torch.float32, "wt_scales"),
-                           _ptr(out), n, k, stream())
-    _ffi.check_last("nve_matvec_w4a8")
-    return out
+    return _ffi.host().matvec_w4a8(xq, xq_scales, nibbles, wt_scales, n, k)
 
 
 def flash_decode_f16(q: Tensor, k_cache: Tensor, v_cache: Tensor, num_heads: int, num_kv_heads: int,
@@ -753,16 +741,10 @@ def gemm_w4a16_multi(x: Tensor, weights: Sequence, k: int, out_dtype=None, outs:
     return list(outs)
 
 
-def gemm_w4a16_wide(x: Tensor, weights: Sequence, k: int, outs: Sequence[Tensor], scratch: Optional[Tensor] = None):
-    """gemm_w4a16_multi for any number of rows of x, into `outs`.  Without `scratch` the workspace is allocated here."""
-    m = x.shape[0]
-    if scratch is None:
-        scratch = torch.empty(max(16, gemm_w4a16_multi_scratch_bytes(m, [w[2] for w in weights], k)), dtype=torch.uint8, device=x.device)
-    arr = _mats(weights, outs, None, x.dtype)
-    _ffi.check("nve_b200_gemm_w4a16_wide",
-               _lib().nve_b200_gemm_w4a16_wide(_ptr(x, (torch.float16, torch.bfloat16), "x"), _dt(x), arr, len(weights), _dt(x), m, k,
-                                               _ptr(scratch), scratch.numel() * scratch.element_size(), stream()))
-    return list(outs)
+def gemm_w4a16_wide(x: Tensor, weights: Sequence, k: int, outs: Optional[Sequence[Tensor]] = None, scratch: Optional[Tensor] = None):
+    """gemm_w4a16_multi for any number of rows of x; outputs of x's type.  Without `scratch` the workspace is allocated
+    here."""
+    return _ffi.host().gemm_w4a16_wide(x, weights, k, outs, scratch)
 
 
 def gemm_w4a16_silu_scratch_bytes(m: int, n: int, k: int) -> int:
@@ -847,13 +829,7 @@ def dequant_w4a16_any(nibbles: Tensor, scales: Tensor, awq: Optional[Tensor], n:
 
 def q4_quantize(w: Tensor, awq_scales: Optional[Tensor] = None) -> Tuple[Tensor, Tensor]:
     """On-device Q4 quantisation of an f32 [N,K] matrix -> (nibbles [N,K/2] u8, scales [N,K/32] f32)."""
-    n, k = w.shape
-    nib = torch.empty((n, k // 2), dtype=torch.uint8, device=w.device)
-    sc = torch.empty((n, k // 32), dtype=torch.float32, device=w.device)
-    _ffi.check("nve_b200_q4_quantize", _lib().nve_b200_q4_quantize(_ptr(w, torch.float32, "W"),
-                                                                   _ptr(awq_scales, torch.float32), _ptr(nib), _ptr(sc),
-                                                                   n, k, stream()))
-    return nib, sc
+    return _ffi.host().q4_quantize(w, awq_scales)
 
 
 def q4_repack_blocks(cpu_blocks: Tensor, n: int, k: int) -> Tuple[Tensor, Tensor]:

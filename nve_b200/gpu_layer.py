@@ -60,8 +60,7 @@ def matmul_x(x: Tensor, w: GpuW4, scratch: Optional[Tensor] = None, out: Optiona
         return ck.matvec_w4a16_multi(x, w.awq_scales, [w.triple()], w.k, outs=[out])[0]
     if w.awq_scales is not None:
         x = (x.float() * w.awq_scales.view(1, -1)).to(x.dtype)
-    out = torch.empty((m, w.n), dtype=x.dtype, device=x.device) if out is None else out
-    return ck.gemm_w4a16_wide(x, [w.triple()], w.k, outs=[out], scratch=scratch)[0]
+    return ck.gemm_w4a16_wide(x, (w.triple(),), w.k, None if out is None else (out,), scratch)[0]
 
 
 def matmul_x_multi(x: Tensor, ws: Sequence[GpuW4], scratch: Optional[Tensor] = None,
@@ -72,8 +71,7 @@ def matmul_x_multi(x: Tensor, ws: Sequence[GpuW4], scratch: Optional[Tensor] = N
     m, k = x.shape
     if m == 1 or any(w.awq_scales is not None for w in ws):
         return [matmul_x(x, w, scratch, None if outs is None else outs[i]) for i, w in enumerate(ws)]
-    outs = [torch.empty((m, w.n), dtype=x.dtype, device=x.device) for w in ws] if outs is None else list(outs)
-    return ck.gemm_w4a16_wide(x, [w.triple() for w in ws], k, outs=outs, scratch=scratch)
+    return ck.gemm_w4a16_wide(x, [w.triple() for w in ws], k, outs, scratch)
 
 
 @dataclass
