@@ -96,49 +96,113 @@ template <int ODT> __global__ void dequant_scalar_kernel(const uint8_t* nibbles,
 // On-device Q4 quantisation (bit-identical to the host quantizer of the reference project):
 //   amax = max|v| ; scale = amax > 0 ? amax/7 : 0 ; inv = scale > 0 ? 1/scale : 0
 //   q = clamp(round_half_away(v*inv), -8, 7) + 8 ; device byte j = q[j] | q[j+16] << 4
-// One thread per block of 32 weights.
+// HBM is the floor (4 bytes in, 0.625 out per weight), the instruction count what has to be kept below it: at 25 instructions
+// per weight-lane and two IEEE divisions per lane and block the kernel was bound by issue, as the form with one thread per
+// block (whose warp-wide loads touched 32 cache lines each) was by its loads.  So: eight lanes share a block, one 16-byte
+// load each (512 contiguous bytes per warp-wide load, four in flight per thread); the four blocks of a lane group are
+// reduced together, so that lane t holds the maximum of block t & 3, divides for it alone and hands the factor back.
 // ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ int round_half_away_sat(float v) {
-    if (v != v) return 0;                 // NaN -> 0, as a saturating float->int8 cast gives
-    const float r = roundf(v);            // half away from zero
-    return static_cast<int>(fminf(fmaxf(r, -128.0f), 127.0f));
+// clamp(round_half_away(v), -8, 7), NaN -> 0 as a saturating float->int8 cast gives.
+__device__ __forceinline__ int round_q4(float v) {
+    if (v != v) return 0;
+    return static_cast<int>(fminf(fmaxf(roundf(v), -8.0f), 7.0f));
+}
+// Four codes q + 8, one per byte, of products p with |p| <= 7.01: floor(p + 8.5) is round-half-away(p) + 8 except where p is a
+// negative tie, and adding one to the bits of a negative p (one ulp away from zero) settles those.  The sum with 2^22 + 8.5,
+// rounded down, holds floor(2 * (p + 8.5)) in its low bits.
+__device__ __forceinline__ uint32_t pack_q4(float p0, float p1, float p2, float p3) {
+    auto low = [](float p) {
+        const uint32_t b = __float_as_uint(p);
+        return __float_as_uint(__fadd_rd(__uint_as_float(b + (b >> 31)), 4194312.5f));
+    };
+    constexpr uint32_t kBase = 0x4A800000u * 0x01010101u;  // 2^22 in each summand
+    const uint32_t t = low(p0) + low(p1) * 0x100u + low(p2) * 0x10000u + low(p3) * 0x1000000u;
+    return ((t - kBase) >> 1) & 0x0F0F0F0Fu;
+}
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
 }
 
-__global__ void __launch_bounds__(256) q4_quantize_kernel(const float* W, const float* awq_scales, uint8_t* nibbles,
-                                                          float* scales, long long total_blocks, int nb) {
-    const long long blk = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (blk >= total_blocks) return;
-    const int b = static_cast<int>(blk % nb);
-    float v[32];
-    const float4* src = reinterpret_cast<const float4*>(W + blk * 32);
+constexpr int kQ4Loads = 4;  // 16-byte loads per thread = blocks per group of eight lanes
+template <bool AWQ>
+__global__ void __launch_bounds__(256) q4_quantize_kernel(const float* W, const float* awq_scales, uint8_t* nibbles, float* scales,
+                                                          long long total_blocks, int nb) {
+    pdl_wait();
+    const int t = threadIdx.x & 7;  // elements 4t .. 4t + 3 of the blocks blk0 + 32 * i
+    const long long blk0 = static_cast<long long>(blockIdx.x) * (32 * kQ4Loads) + (threadIdx.x >> 3);
+    float v[kQ4Loads][4];
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const float4 f = src[i];
-        v[4 * i] = f.x; v[4 * i + 1] = f.y; v[4 * i + 2] = f.z; v[4 * i + 3] = f.w;
+    for (int i = 0; i < kQ4Loads; i++) {
+        const long long blk = blk0 + 32 * i;
+        uint4 r = make_uint4(0, 0, 0, 0);
+        if (blk < total_blocks) r = ld_stream_u4(W + blk * 32 + 4 * t);
+        v[i][0] = __uint_as_float(r.x);
+        v[i][1] = __uint_as_float(r.y);
+        v[i][2] = __uint_as_float(r.z);
+        v[i][3] = __uint_as_float(r.w);
     }
-    if (awq_scales != nullptr) {
+    if (AWQ) {
 #pragma unroll
-        for (int e = 0; e < 32; e++) v[e] = __fmul_rn(v[e], awq_scales[b * 32 + e]);
+        for (int i = 0; i < kQ4Loads; i++) {
+            const float* a = awq_scales + static_cast<int>((blk0 + 32 * i) % nb) * 32 + 4 * t;
+#pragma unroll
+            for (int e = 0; e < 4; e++) v[i][e] = __fmul_rn(v[i][e], a[e]);
+        }
     }
-    float amax = 0.0f;
+    // maxima of the four blocks over the eight lanes: lane t ends up with block t & 3
+    float m[kQ4Loads];
 #pragma unroll
-    for (int e = 0; e < 32; e++) {
-        const float a = fabsf(v[e]);
-        if (a > amax) amax = a;  // NaN never wins, matching f32::max folding from 0
+    for (int i = 0; i < kQ4Loads; i++) m[i] = max_nan(max_nan(fabsf(v[i][0]), fabsf(v[i][1])), max_nan(fabsf(v[i][2]), fabsf(v[i][3])));
+    {
+        const bool up2 = (t & 2) != 0, up1 = (t & 1) != 0;
+#pragma unroll
+        for (int i = 0; i < 2; i++) m[i] = max_nan(up2 ? m[i + 2] : m[i], __shfl_xor_sync(0xffffffffu, up2 ? m[i] : m[i + 2], 2));
+        m[0] = max_nan(up1 ? m[1] : m[0], __shfl_xor_sync(0xffffffffu, up1 ? m[0] : m[1], 1));
+        m[0] = max_nan(m[0], __shfl_xor_sync(0xffffffffu, m[0], 4));
+    }
+    float amax = m[0];
+    // a NaN or infinity in the block, or a maximum so small that the reciprocal of its scale overflows: one by one below
+    const bool plain = !__any_sync(0xffffffffu, !(amax == 0.0f || (amax >= 1e-30f && amax < INFINITY)));
+    if (!plain) {
+#pragma unroll
+        for (int i = 0; i < kQ4Loads; i++) {
+            // fmaxf: NaN never wins, matching f32::max folding from 0
+            float a = fmaxf(fmaxf(fmaxf(fmaxf(0.0f, fabsf(v[i][0])), fabsf(v[i][1])), fabsf(v[i][2])), fabsf(v[i][3]));
+            for (int k = 1; k < 8; k <<= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, k));
+            if ((t & 3) == i) amax = a;
+        }
     }
     const float scale = amax > 0.0f ? __fdiv_rn(amax, 7.0f) : 0.0f;
     const float inv = scale > 0.0f ? __fdiv_rn(1.0f, scale) : 0.0f;
-    uint32_t packed[4] = {0, 0, 0, 0};
+    if (t < 4 && blk0 + 32 * t < total_blocks) scales[blk0 + 32 * t] = scale;
+    uint32_t q[kQ4Loads];
 #pragma unroll
-    for (int j = 0; j < 16; j++) {
-        int q0 = round_half_away_sat(__fmul_rn(v[j], inv));
-        int q1 = round_half_away_sat(__fmul_rn(v[j + 16], inv));
-        q0 = max(-8, min(7, q0)) + 8;
-        q1 = max(-8, min(7, q1)) + 8;
-        packed[j >> 2] |= static_cast<uint32_t>(q0 | (q1 << 4)) << (8 * (j & 3));
+    for (int i = 0; i < kQ4Loads; i++) {
+        const float f = __shfl_sync(0xffffffffu, inv, i, 8);
+        float p[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) p[e] = __fmul_rn(v[i][e], f);
+        if (plain) {
+            q[i] = pack_q4(p[0], p[1], p[2], p[3]);
+        } else {
+            q[i] = 0;
+#pragma unroll
+            for (int e = 0; e < 4; e++) q[i] |= static_cast<uint32_t>(round_q4(p[e]) + 8) << (8 * e);
+        }
     }
-    reinterpret_cast<uint4*>(nibbles)[blk] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-    scales[blk] = scale;
+    // byte j of a block is element j | element j + 16 << 4: lane t < 4 has the low, lane t + 4 the high halves of word t.  Of
+    // every two blocks the lower lanes store the first, the upper lanes the second.
+    const bool hi = (t & 4) != 0;
+#pragma unroll
+    for (int i = 0; i < kQ4Loads; i += 2) {
+        const uint32_t own = hi ? q[i + 1] : q[i];
+        const uint32_t got = __shfl_xor_sync(0xffffffffu, hi ? q[i] : q[i + 1], 4);
+        const uint32_t w = hi ? got | (own << 4) : own | (got << 4);
+        const long long blk = blk0 + 32 * (i + (hi ? 1 : 0));
+        if (blk < total_blocks) reinterpret_cast<uint32_t*>(nibbles)[blk * 4 + (t & 3)] = w;
+    }
 }
 
 // CPU block (f32 scale + 16 bytes of {2i, 2i+1}) -> device layout.
@@ -225,10 +289,21 @@ extern "C" int nve_b200_q4_quantize(const float* W, const float* awq_scales, uin
     if (N <= 0 || K <= 0 || (K % 32) != 0) return set_status(NVE_ERR_BAD_SHAPE);
     if (!aligned(W, 16) || !aligned(nibbles, 16)) return set_status(NVE_ERR_BAD_ALIGNMENT);
     const long long blocks = static_cast<long long>(N) * (K / 32);
-    q4_quantize_kernel<<<grid_for(blocks, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(W, awq_scales, nibbles, scales,
-                                                                                            blocks, K / 32);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid_for(blocks, 32 * kQ4Loads));
+    cfg.blockDim = dim3(256);
+    cfg.stream = static_cast<cudaStream_t>(stream);
+    cudaLaunchAttribute attr[1];
+    if (pdl_enabled()) {
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    const cudaError_t e = awq_scales != nullptr ? cudaLaunchKernelEx(&cfg, q4_quantize_kernel<true>, W, awq_scales, nibbles, scales, blocks, K / 32)
+                                                : cudaLaunchKernelEx(&cfg, q4_quantize_kernel<false>, W, awq_scales, nibbles, scales, blocks, K / 32);
     count_launch();
-    return check_launch();
+    return set_cuda_status(e);
 }
 
 extern "C" int nve_b200_q4_repack_blocks(const uint8_t* cpu_blocks, uint8_t* nibbles, float* scales, int N, int K,
