@@ -328,13 +328,12 @@ NVE_API int nve_b200_quantize_matvec_w4a8_allreduce(const void* x, int x_dtype, 
  * the output is also quantised to int8 per group of 32 (the call at src/gpu_layer.rs:739).  head_dim 64 or
  * 128.  Results -- cache row, output and int8 codes -- are bit-identical to the separate RoPE, KV-write,
  * flash-decode and quantise launches of this library.
- * Two attention kernels exist and nve_flash_decode_f16 / _dyn, nve_b200_attn_prefill_causal (small blocks) and this
- * entry point always run the same one: by default a tensor-core kernel (a cluster of 8 CTAs per KV head, all its
- * query heads as rows of mma.sync, f16 probabilities) when there are up to 8 query heads per KV head and the
- * pointers are 16-byte aligned; nve_b200_set_attn_decode_kernel(1) selects the CUDA-core kernel for all of them
- * (also used for other shapes; it is the arithmetic of the persistent one-kernel step), 0 restores the default.  The
- * two kernels agree within 5e-3 of the largest output.  The setting is process-wide, a captured graph keeps the
- * kernel it was recorded with; the previous setting is returned. */
+ * By default this entry point, nve_flash_decode_f16 / _dyn and the small blocks of nve_b200_attn_prefill_causal run the
+ * tensor-core kernels (all query heads of a KV head as rows of mma.sync, f16 probabilities; which of them follows from the
+ * size of the cache) when there are up to 8 query heads per KV head and the pointers are 16-byte aligned;
+ * nve_b200_set_attn_decode_kernel(1) selects the CUDA-core kernel for all of them (also used for other shapes; it is the
+ * arithmetic of the persistent one-kernel step), 0 restores the default.  They agree within 5e-3 of the largest output.
+ * The setting is process-wide, a captured graph keeps the kernel it was recorded with; the previous setting is returned. */
 NVE_API int nve_b200_attn_decode_fused(const uint16_t* q, const uint16_t* k_new, const uint16_t* v_new,
                                        uint16_t* k_cache, uint16_t* v_cache, const uint16_t* cos_tab,
                                        const uint16_t* sin_tab, const int* d_pos, const int* d_seq_len, uint16_t* out,
@@ -344,12 +343,10 @@ NVE_API int nve_b200_set_attn_decode_kernel(int mode);
 /* The same launch for `batch` independent sequences (batched decode; the reference has none): row b of q
  * [batch, nh*hd] and of k_new / v_new [batch, nkv*hd] belongs to sequence b, whose caches are k_cache / v_cache +
  * b * nkv * max_seq_len * hd, whose position is d_pos[b] and whose valid length is d_seq_len[b] (device arrays).
- * The cache row written is bit-identical to a single-sequence call.  Up to 63 (sequence, KV head) units the clustered
- * decode kernel that nve_b200_attn_decode_fused would launch (see nve_b200_set_attn_decode_kernel) runs with the
- * sequence as second grid dimension and row b of out [batch, nh*hd] is bit-identical too;
- * from 64 units on (and up to 8 query heads per KV head) one CTA per unit streams all positions and computes
- * q.K^T and p.V with mma.sync (probabilities rounded to f16): rows then agree with the single-sequence call to about
- * 1e-3 of their RMS.  q / k_new / v_new and the caches 16-byte aligned. */
+ * The cache row written is bit-identical to a single-sequence call; rows of out [batch, nh*hd] agree with it to about 1e-3
+ * of their RMS (the split of the positions over CTAs follows the batch) and are bit-identical below 64 (sequence, KV head)
+ * units with max_seq_len up to 128.  Fewer than 64 units follow nve_b200_set_attn_decode_kernel, more always run the streaming tensor-core kernel
+ * (up to 8 query heads per KV head).  q / k_new / v_new and the caches 16-byte aligned. */
 NVE_API int nve_b200_attn_decode_fused_batch(const uint16_t* q, const uint16_t* k_new, const uint16_t* v_new,
                                              uint16_t* k_cache, uint16_t* v_cache, const uint16_t* cos_tab,
                                              const uint16_t* sin_tab, const int* d_pos, const int* d_seq_len,

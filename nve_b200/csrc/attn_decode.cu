@@ -213,6 +213,16 @@ static bool attn_decode_dispatch(const AttnParams& p, int hd, cudaStream_t st, c
 // 0: tensor-core kernels where they cover the shape (default); 1: always the CUDA-core kernel (nve_b200_set_attn_decode_kernel)
 static std::atomic<int> g_attn_decode_kernel{0};
 
+// The tensor-core kernels.  One row: the latency kernel where one tile of 16 positions per warp all but covers the cache (128 to
+// 1280 positions; us per launch back to back, 8B shape, latency / streaming kernel: 256: 3.7 / 4.5, 1024: 4.3 / 4.7, 1500:
+// 5.5 / 5.0, 4096: 9.7 / 7.0, 16384: 27.5 / 17.4), otherwise the streaming one.  Up to 128 positions the latter does not split a
+// row over CTAs: a row then has the same bits in any batch of fewer than 64 units.  Several rows: always the streaming kernel (2 sequences of 1000:
+// 6.3 / 4.7, 7 of 200: 12.9 / 4.5, 7 of 500 - 2000 with 3 heads per KV head: 22.0 / 10.7, 64 of 256 - 1024: 30.7).
+static bool attn_mma_try(const AttnParams& p, int hd, cudaStream_t st, cudaError_t& err, bool fused) {
+    if (p.rows <= 1 && p.kv_stride > 128 && p.kv_stride <= 1280) return attn_decode_mma_try(p, hd, st, err, fused);
+    return attn_stream_mma_try(p, hd, st, err, fused);
+}
+
 // Used by the reference-signature flash-decode entry points (attn_glue.cu).
 bool attn_decode_try(const uint16_t* q, const uint16_t* kc, const uint16_t* vc, uint16_t* out, int nh, int nkv, int seq_len,
                      const int* d_seq_len, int kv_stride, int hd, float scale, cudaStream_t st) {
@@ -229,7 +239,7 @@ bool attn_decode_try(const uint16_t* q, const uint16_t* kc, const uint16_t* vc, 
     p.scale = scale;
     cudaError_t e = cudaSuccess;
     const bool mma = g_attn_decode_kernel.load(std::memory_order_relaxed) == 0 && aligned(q, 16) && aligned(kc, 16) && aligned(vc, 16) &&
-                     attn_decode_mma_try(p, hd, st, e, false);
+                     attn_mma_try(p, hd, st, e, false);
     if (!mma && !attn_decode_dispatch<false>(p, hd, st, e)) return false;
     count_launch();
     set_cuda_status(e);
@@ -259,7 +269,7 @@ extern "C" int nve_b200_attn_decode_fused(const uint16_t* q, const uint16_t* k_n
     p.num_heads = num_heads; p.num_kv_heads = num_kv_heads; p.kv_stride = max_seq_len; p.scale = scale;
     cudaError_t e = cudaSuccess;
     if (g_attn_decode_kernel.load(std::memory_order_relaxed) == 0 && aligned(q, 16) && aligned(k_new, 16) && aligned(v_new, 16) &&
-        attn_decode_mma_try(p, head_dim, static_cast<cudaStream_t>(stream), e)) {
+        attn_mma_try(p, head_dim, static_cast<cudaStream_t>(stream), e, true)) {
         count_launch();
         return set_cuda_status(e);
     }
@@ -306,7 +316,7 @@ extern "C" int nve_b200_attn_prefill_causal(const uint16_t* q, const uint16_t* k
         count_launch();
         return set_cuda_status(e);
     }
-    if (g_attn_decode_kernel.load(std::memory_order_relaxed) == 0 && attn_decode_mma_try(p, head_dim, static_cast<cudaStream_t>(stream), e, false)) {
+    if (g_attn_decode_kernel.load(std::memory_order_relaxed) == 0 && attn_mma_try(p, head_dim, static_cast<cudaStream_t>(stream), e, false)) {
         count_launch();
         return set_cuda_status(e);
     }
@@ -317,9 +327,8 @@ extern "C" int nve_b200_attn_prefill_causal(const uint16_t* q, const uint16_t* k
 
 /* nve_b200_attn_decode_fused for `batch` independent sequences in one launch: row b of q [batch, nh*hd] and of
  * k_new / v_new [batch, nkv*hd] belongs to sequence b, whose caches are k_cache / v_cache + b * nkv * max_seq_len * hd,
- * whose position is d_pos[b] and whose valid length is d_seq_len[b].  Small batches run the clustered kernel that
- * nve_b200_attn_decode_fused would run (row b bit-identical to a single-sequence call under the same
- * nve_b200_set_attn_decode_kernel setting), large ones the streaming tensor-core kernel of attn_batch_mma.cu. */
+ * whose position is d_pos[b] and whose valid length is d_seq_len[b].  The streaming tensor-core kernel; fewer than 64
+ * (sequence, KV head) units follow nve_b200_set_attn_decode_kernel. */
 extern "C" int nve_b200_attn_decode_fused_batch(const uint16_t* q, const uint16_t* k_new, const uint16_t* v_new,
                                                 uint16_t* k_cache, uint16_t* v_cache, const uint16_t* cos_tab,
                                                 const uint16_t* sin_tab, const int* d_pos, const int* d_seq_len, uint16_t* out,
@@ -341,17 +350,9 @@ extern "C" int nve_b200_attn_decode_fused_batch(const uint16_t* q, const uint16_
     p.cache_stride = static_cast<long long>(num_kv_heads) * max_seq_len * head_dim;
     cudaError_t e = cudaSuccess;
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
-    // enough (sequence, head pair) units to fill every SM twice: one CTA per unit over all positions, streaming;
-    // otherwise the clustered kernel, which splits a sequence's positions over eight CTAs
-    // one CTA per (sequence, KV head) on the tensor cores (attn_batch_mma.cu) from 64 such units on: measured at 8
-    // KV heads and context 1024, 8 sequences take 21 us there against 23 us on the clustered tensor-core kernel (29 us
-    // on the CUDA-core one), 16 sequences 22 against 41, 64 sequences 63 against 188; below that the clustered
-    // kernels, which split a sequence's positions over eight CTAs, are faster (2 sequences 8.7 us, 4 sequences 13.4 us)
-    if (static_cast<long long>(batch) * num_kv_heads >= 64 && attn_batch_mma_try(p, head_dim, cs, e)) {
-        count_launch();
-        return set_cuda_status(e);
-    }
-    if (g_attn_decode_kernel.load(std::memory_order_relaxed) == 0 && attn_decode_mma_try(p, head_dim, cs, e)) {
+    // few sequences follow nve_b200_set_attn_decode_kernel like a single one
+    if ((static_cast<long long>(batch) * num_kv_heads >= 64 || g_attn_decode_kernel.load(std::memory_order_relaxed) == 0) &&
+        attn_mma_try(p, head_dim, cs, e, true)) {
         count_launch();
         return set_cuda_status(e);
     }

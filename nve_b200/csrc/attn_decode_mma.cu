@@ -1,8 +1,7 @@
 // Decode attention on the tensor cores, one cluster per KV head: RoPE + K/V write + single-query GQA attention +
 // optional int8 quantisation of the output, the fused step between the q/k/v GEMV and o_proj of a decode layer
-// (FUSED); the plain flash-decode form of the same arithmetic (nve_flash_decode_f16, the rows of a small causal
-// block), so that the fused launch equals the un-fused launch sequence bit for bit; and a few independent sequences
-// in one launch (batched decode).
+// (FUSED); and the plain flash-decode form of the same arithmetic (nve_flash_decode_f16), so that the fused launch equals
+// the un-fused launch sequence bit for bit.  One sequence; several, or a long context, run attn_stream_mma.cu.
 //
 // Same interface and the same place in the step as the clustered CUDA-core kernel (attn_decode.cu), which spends
 // most of its time on dot products with shuffle reductions (about 1200 instructions per thread for 1024 positions).
@@ -60,31 +59,12 @@ template <int HD, int G> struct AdmSmem {
     __align__(8) unsigned long long pbar;
 };
 
-// With `rows` > 1 (batched decode) blockIdx.y selects one of several independent sequences: row b of q / k_new /
-// v_new / out, the b-th K/V cache and the b-th position and length words.
-// FUSED = false is the plain flash-decode form (nve_flash_decode_f16 and the rows of a small causal block): q is
-// already rotated, nothing is written to the cache, the length is *d_seq_len or seq_len, and blockIdx.y selects one of
-// `rows` query rows, row r reading q + r * row_stride and attending to seq_len + r positions.
+// FUSED = false is the plain flash-decode form: q is already rotated, nothing is written to the cache, the length is
+// *d_seq_len or seq_len.
 template <int HD, int G, bool FUSED>
 __global__ void __launch_bounds__(kAmThreads, 1) attn_decode_mma_kernel(const AttnParams pin) {
-    AttnParams p = pin;
-    int seq_len_row = p.seq_len;
-    if constexpr (!FUSED) {
-        p.q += static_cast<long long>(blockIdx.y) * p.row_stride;
-        p.out += static_cast<long long>(blockIdx.y) * p.row_stride;
-        seq_len_row += static_cast<int>(blockIdx.y);
-    }
-    if (FUSED && p.rows > 1) {
-        const long long b = blockIdx.y;
-        p.q += b * (static_cast<long long>(p.num_heads) * HD);
-        p.out += b * (static_cast<long long>(p.num_heads) * HD);
-        p.k_new += b * (static_cast<long long>(p.num_kv_heads) * HD);
-        p.v_new += b * (static_cast<long long>(p.num_kv_heads) * HD);
-        p.k_cache += b * p.cache_stride;
-        p.v_cache += b * p.cache_stride;
-        p.d_pos += b;
-        p.d_seq_len += b;
-    }
+    const AttnParams& p = pin;
+    const int seq_len_row = p.seq_len;
     constexpr int DC = HD / 8;
     constexpr int NT = HD / 8;
     static_assert((HD == 64 || HD == 128) && G >= 1 && G <= 8, "head_dim 64 or 128, up to 8 query heads per KV head");
@@ -312,7 +292,7 @@ template <int HD, int G, bool FUSED> static cudaError_t launch_adm_f(const AttnP
     if (ensure_dynamic_smem(reinterpret_cast<const void*>(attn_decode_mma_kernel<HD, G, FUSED>), smem) != NVE_OK) return cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = {};
     cfg.dynamicSmemBytes = smem;
-    cfg.gridDim = dim3(p.num_kv_heads * kAdCluster, p.rows > 1 ? p.rows : 1);  // fused: sequences; else: query rows
+    cfg.gridDim = dim3(p.num_kv_heads * kAdCluster);
     cfg.blockDim = dim3(kAmThreads);
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
@@ -347,7 +327,7 @@ template <int HD> static bool launch_adm_groups(const AttnParams& p, cudaStream_
     }
 }
 
-// Decode attention of one or a few sequences; false when the shape is not covered (more than 8 query heads per KV head,
+// Decode attention of one sequence; false when the shape is not covered (more than 8 query heads per KV head,
 // other head sizes): the caller then uses the CUDA-core kernel.
 bool attn_decode_mma_try(const AttnParams& p, int head_dim, cudaStream_t st, cudaError_t& err, bool fused) {
     if (head_dim == 128) return launch_adm_groups<128>(p, st, err, fused);

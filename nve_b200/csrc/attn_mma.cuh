@@ -1,7 +1,17 @@
-// Tile arithmetic shared by the tensor-core attention kernels (attn_batch_mma.cu: many sequences, one CTA per
-// sequence and KV head; attn_decode_mma.cu: one sequence, a cluster per KV head): one warp, one tile of 16 cached
-// positions, all G <= 8 query heads of the KV head as rows of mma.sync.m16n8k16.  The operand layouts are described
-// at the top of attn_batch_mma.cu.
+// Tile arithmetic of the latency form of decode attention (attn_decode_mma.cu): one warp, one tile of 16 cached positions held
+// in registers, all G <= 8 query heads of the KV head as rows of mma.sync.m16n8k16; mma_f16_16816 and pack_f16x2 are shared
+// with the streaming and the prefill kernels.
+//
+// Operand layouts without any shuffle or shared-memory staging of K/V -- the contraction index of a dot product may be
+// permuted freely as long as both operands use the same permutation, and so may the labels of the output columns:
+//   * scores:  S[16 x 8 positions] += Qa[16 x 16] . Kb[16 x 8].  Lane (g = lane / 4, t = lane % 4) supplies K row
+//     p0 + g, and for the kk-th MMA the four elements k = 2t, 2t+1, 2t+8, 2t+9 of the 16-wide slice.  Slice kk, slot
+//     s of lane t is mapped to the physical dim DPT*t + 4*kk + s (DPT = HD/4): every lane reads DPT contiguous dims
+//     (64 bytes at HD = 128) of its row with 128-bit loads; the q fragments use the same map.
+//   * outputs: O[16 x 8 dims] += Pa[16 x 16 positions] . Vb[16 x 8].  Pa is the score fragment of two consecutive
+//     position tiles converted to f16 (the usual register reuse); lane (g, t) supplies V rows p0 + {2t, 2t+1, 2t+8,
+//     2t+9} and output column n = g of every dim tile j, which is mapped to the physical dim NT*g + j (NT = HD/8): the
+//     lane reads NT contiguous dims (32 bytes at HD = 128) of its four rows and pairs them up with byte permutes.
 #pragma once
 #include "attn_core.cuh"
 
@@ -16,14 +26,6 @@ constexpr int kAmWarps = kAmThreads / 32;
 __host__ __device__ constexpr int am_wo_row(int hd) { return hd + 8; }
 template <int HD> __device__ __forceinline__ int am_wo_index(int d) { return d + d / (HD / 8); }
 
-template <int HD, int G> struct AmShared {
-    float q_s[G][HD];
-    __align__(16) uint16_t knew_s[HD];
-    __align__(16) uint16_t vnew_s[HD];
-    float wm[kAmWarps][G], wl[kAmWarps][G];
-    float wo[kAmWarps][G][am_wo_row(HD)];
-};
-
 __device__ __forceinline__ void mma_f16_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile(
         "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -33,24 +35,6 @@ __device__ __forceinline__ void mma_f16_16816(float (&d)[4], const uint32_t (&a)
 __device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
     const __half2 h = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&h);
-}
-
-// q fragments of lane (g, t) from the staged (rotated, f16-rounded) q rows: rows g < G are heads, the others zero
-template <int HD, int G, class SH> __device__ __forceinline__ void am_q_fragments(const SH& sh, int g, int t, uint32_t (&qa)[HD / 16][4]) {
-    constexpr int DPT = HD / 4, KK = HD / 16;
-#pragma unroll
-    for (int kk = 0; kk < KK; kk++) {
-        qa[kk][1] = 0;
-        qa[kk][3] = 0;
-        if (g < G) {
-            const float* qp = &sh.q_s[g][DPT * t + 4 * kk];
-            qa[kk][0] = pack_f16x2(qp[0], qp[1]);  // exact: q_s holds f16-rounded values
-            qa[kk][2] = pack_f16x2(qp[2], qp[3]);
-        } else {
-            qa[kk][0] = 0;
-            qa[kk][2] = 0;
-        }
-    }
 }
 
 // Loads of the tile at p0: K rows p0 + g, p0 + 8 + g (dims DPT*t ..), V rows p0 + {2t, 2t+1, 2t+8, 2t+9} (dims

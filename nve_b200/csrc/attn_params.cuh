@@ -1,4 +1,4 @@
-// Launch parameters of the decode attention kernels (attn_decode.cu, attn_batch_mma.cu).
+// Launch parameters of the decode attention kernels (attn_decode.cu, attn_decode_mma.cu, attn_stream_mma.cu, attn_prefill_mma.cu).
 #pragma once
 #include "common.cuh"
 
@@ -27,15 +27,15 @@ struct AttnParams {
     long long cache_stride;
 };
 
-// attn_batch_mma.cu: `rows` independent sequences with RoPE and the K/V write inside; false when the shape is not
-// covered (the caller then uses another kernel).
-bool attn_batch_mma_try(const AttnParams& p, int head_dim, cudaStream_t st, cudaError_t& err);
+// attn_stream_mma.cu: fused (`rows` independent sequences with RoPE and the K/V write inside) or plain form, positions split
+// over clusters chosen for the grid; false when the shape is not covered (the caller then uses another kernel).
+bool attn_stream_mma_try(const AttnParams& p, int head_dim, cudaStream_t st, cudaError_t& err, bool fused = true);
 
 // attn_prefill_mma.cu: the causal block described above, in tiles of query rows; false when the shape is not covered.
 bool attn_prefill_mma_try(const AttnParams& p, int head_dim, cudaStream_t st, cudaError_t& err);
 
-// attn_decode_mma.cu: the fused decode attention of one sequence on the tensor cores; false when the shape is not
-// covered.
+// attn_decode_mma.cu: decode attention of one sequence (or query row) on the tensor cores, built for latency; false when the
+// shape is not covered.
 bool attn_decode_mma_try(const AttnParams& p, int head_dim, cudaStream_t st, cudaError_t& err, bool fused = true);
 
 }  // namespace nve

@@ -1,0 +1,60 @@
+"""GPU: the streaming decode attention against an f64 softmax over the same 16-bit inputs: every group size, lengths around its
+16-position tiles, its slices per CTA and its 128-position and 1280-position limits, one and several sequences, few enough for
+clusters and too many, with a cache row of the new token that holds NaN before the call."""
+import pytest
+
+from helpers import dev
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nh,nkv,hd,max_seq,lens", [
+    (8, 8, 64, 40, [40, 1, 16, 17]),
+    (10, 5, 128, 128, [128]),
+    (24, 8, 128, 129, [129, 128, 113, 2]),
+    (16, 4, 64, 1281, [1281]),
+    (5, 1, 128, 1100, [1024, 15, 1100]),
+    (12, 2, 64, 2500, [2047, 2500]),
+    (7, 1, 64, 1500, [1500]),
+    (64, 8, 128, 3000, [3000]),                         # clusters of eight, two stages per warp
+    (32, 8, 128, 300, [1 + 37 * i % 300 for i in range(40)]),  # four warps per unit
+    (16, 16, 64, 70, [1 + 11 * i % 70 for i in range(33)]),
+])
+def test_streaming_decode_attention(cuda, orc, nh, nkv, hd, max_seq, lens):
+    from nve_b200 import cuda_kernels as ck
+
+    torch = cuda
+    B, G = len(lens), nh // nkv
+    f16 = torch.float16
+    q = dev(orc.to_act16(orc.fill_normal(B * nh * hd, 891, 1)), f16).view(B, nh * hd)
+    k = dev(orc.to_act16(orc.fill_normal(B * nkv * hd, 891, 2)), f16).view(B, nkv * hd)
+    v = dev(orc.to_act16(orc.fill_normal(B * nkv * hd, 891, 3)), f16).view(B, nkv * hd)
+    kc = dev(orc.to_act16(orc.fill_normal(B * nkv * max_seq * hd, 891, 4)), f16).view(B, nkv, max_seq, hd)
+    vc = dev(orc.to_act16(orc.fill_normal(B * nkv * max_seq * hd, 891, 5)), f16).view(B, nkv, max_seq, hd)
+    cos, sin = orc.rope_tables_f32(hd, max_seq, 10000.0)
+    cos, sin = dev(orc.to_act16(cos), f16), dev(orc.to_act16(sin), f16)
+    for b, n in enumerate(lens):
+        kc[b, :, n - 1:] = float("nan")
+        vc[b, :, n - 1:] = float("nan")
+    d_len = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    d_pos = d_len - 1
+    kc0, vc0 = kc.clone(), vc.clone()
+    got = ck.attn_decode_fused_batch(q, k, v, kc, vc, cos, sin, d_pos, d_len, nh, nkv, hd, max_seq, hd ** -0.5)
+    for b, n in enumerate(lens):
+        q1, k1 = q[b].clone().view(nh, hd), k[b].clone().view(nkv, hd)
+        ck.rope_decode_dyn_inplace(q1, k1, cos, sin, nh, nkv, hd, d_pos[b:b + 1].data_ptr())
+        kc0[b, :, n - 1], vc0[b, :, n - 1] = k1, v[b].view(nkv, hd)
+        s = torch.einsum("kgd,kld->kgl", q1.double().view(nkv, G, hd), kc0[b, :, :n].double()) * hd ** -0.5
+        want = torch.einsum("kgl,kld->kgd", s.softmax(-1), vc0[b, :, :n].double()).reshape(-1)
+        # f16 probabilities (2^-11 of the largest |v| at most), one f16 rounding of the result, f32 scores in the exponent
+        bound = (2.0 ** -10 + 2.0 ** -11) * vc0[b, :, :n].double().abs().max().item()
+        assert (got[b].double() - want).abs().max().item() < bound, f"sequence {b}"
+        # the plain form on the same cache, one row: same bits where neither splits a row and both take eight warps per unit
+        # (below 64 units and up to 128 positions), within the same bound otherwise
+        one = torch.empty((nh, hd), dtype=f16, device="cuda")
+        ck.flash_decode_dyn_into(q1, kc0[b], vc0[b], one, nh, nkv, d_len[b:b + 1].data_ptr(), hd, hd ** -0.5, max_seq)
+        if max_seq <= 128 and B * nkv < 64:
+            assert torch.equal(one.view(-1), got[b])
+        assert (one.view(-1).double() - want).abs().max().item() < bound
+    assert torch.equal(torch.nan_to_num(kc, nan=77.0), torch.nan_to_num(kc0, nan=77.0))
+    assert torch.equal(torch.nan_to_num(vc, nan=77.0), torch.nan_to_num(vc0, nan=77.0))
