@@ -465,12 +465,19 @@ template <typename Kern> static int launch_gemv(Kern kern, const GemvParams& p, 
     cfg.blockDim = dim3(kGemvThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    // Shared memory for two CTAs and no more: the rest of the 228 KB is the L1 that the streamed weights pass through.  Without a
+    // stated preference the SM keeps the division of the kernel before it, and behind an attention kernel that takes all of it
+    // as shared memory a layer of the 8B shape lost 5 us.
+    const size_t want = 2 * (smem + 2048) * 100 / (228 * 1024) + 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[0].val.sharedMemCarveout = static_cast<unsigned>(want < 30 ? 30 : (want > 100 ? 100 : want));
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
     if (pdl_enabled()) {
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.numAttrs = 2;
     }
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p);
     count_launch();
