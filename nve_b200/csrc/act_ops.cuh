@@ -29,26 +29,7 @@ __device__ __forceinline__ uint4 pack8(const uint16_t (&h)[8]) {
 // With `awq_inv` (the per-column divisor a weight matrix was pre-scaled by, src/quantize.rs:271-304) the values
 // are multiplied by it first, so that the W4A8 route sees the same activations as the W4A16 one.
 __device__ __forceinline__ float quantize_quad_codes(const float (&v)[8], uint32_t& lo, uint32_t& hi, int& sum) {
-    float amax = 0.0f;
-#pragma unroll
-    for (int e = 0; e < 8; e++) amax = fmaxf(amax, fabsf(v[e]));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-    const float scale = amax > 0.0f ? __fdiv_rn(amax, 127.0f) : 1.0f;
-    const float inv = __fdiv_rn(1.0f, scale);
-    lo = 0;
-    hi = 0;
-    sum = 0;
-#pragma unroll
-    for (int e = 0; e < 8; e++) {
-        int q = __float2int_rn(__fmul_rn(v[e], inv));
-        q = max(-127, min(127, q));
-        sum += q;
-        const uint32_t byte = static_cast<uint32_t>(q) & 0xFFu;
-        if (e < 4) lo |= byte << (8 * e);
-        else hi |= byte << (8 * (e - 4));
-    }
-    return scale;
+    return q8_codes(v, lo, hi, sum);
 }
 
 // Quantise the 8 values of this thread and store codes / scale to global arrays.

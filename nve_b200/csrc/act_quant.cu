@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(kActThreads) rmsnorm_kernel(const uint16_t* x,
         pdl_launch_dependents();
         load_row_reg(x, chunks, xr);
         const float total = sum_squares_reg<DT>(xr, chunks);
-        const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(n)), eps)));
+        const float r = __frcp_rn(__fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(n)), eps)));
 #pragma unroll
         for (int j = 0; j < kRegChunks; j++)
             if (j < iters) {
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(kActThreads) rmsnorm_kernel(const uint16_t* x,
     pdl_wait();
     pdl_launch_dependents();
     const float total = sum_squares<DT, VEC>(x, n);
-    const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(n)), eps)));
+    const float r = __frcp_rn(__fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(n)), eps)));
     for (int it = 0; it < iters; it++) {
         const int c = it * kActThreads + threadIdx.x;
         uint16_t hx[8] = {0, 0, 0, 0, 0, 0, 0, 0}, hw[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -229,7 +229,7 @@ template <int DT> __global__ void __launch_bounds__(kActThreads) add_rmsnorm_row
             if (c < chunks) store_chunk<true>(x, c, n, hd);
         }
         const float total = sum_squares_reg<DT>(xr, chunks);
-        const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(n)), eps)));
+        const float r = __frcp_rn(__fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(n)), eps)));
 #pragma unroll
         for (int j = 0; j < kRegChunks; j++) {
             const int c = j * kActThreads + threadIdx.x;
@@ -252,7 +252,7 @@ template <int DT> __global__ void __launch_bounds__(kActThreads) add_rmsnorm_row
     }
     __syncthreads();  // the CTA reads back what it stored
     const float total = sum_squares<DT, true>(x, n);
-    const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(n)), eps)));
+    const float r = __frcp_rn(__fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(n)), eps)));
     for (int c = threadIdx.x; c < chunks; c += kActThreads) {
         uint16_t hx[8], hw[8], ho[8];
         load_chunk<true>(x, c, n, hx);
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(kActThreads) layer_norm_kernel(const uint16_t*
     }
     const float mean = ta / static_cast<float>(n);
     const float var = tb / static_cast<float>(n) - mean * mean;
-    const float istd = __fdiv_rn(1.0f, __fsqrt_rn(var + eps));
+    const float istd = __frcp_rn(__fsqrt_rn(var + eps));
     for (int i = threadIdx.x; i < n; i += kActThreads) {
         const float v = (Act16<NVE_DT_F16>::to_f32(x[i]) - mean) * istd;
         const float bb = bias != nullptr ? Act16<NVE_DT_F16>::to_f32(bias[i]) : 0.0f;

@@ -35,6 +35,8 @@ template <> struct Act16<NVE_DT_F16> {
     using T = __half;
     __device__ static __forceinline__ float to_f32(uint16_t v) { return __half2float(__ushort_as_half(v)); }
     __device__ static __forceinline__ uint16_t from_f32(float v) { return __half_as_ushort(__float2half_rn(v)); }
+    // both values rounded to the type and back, one conversion each way
+    __device__ static __forceinline__ float2 round2(float a, float b) { return __half22float2(__floats2half2_rn(a, b)); }
 };
 template <> struct Act16<NVE_DT_BF16> {
     using T = __nv_bfloat16;
@@ -42,6 +44,7 @@ template <> struct Act16<NVE_DT_BF16> {
     __device__ static __forceinline__ uint16_t from_f32(float v) {
         return __bfloat16_as_ushort(__float2bfloat16_rn(v));
     }
+    __device__ static __forceinline__ float2 round2(float a, float b) { return __bfloat1622float2(__floats2bfloat162_rn(a, b)); }
 };
 
 // Store one result element in the requested output type.
@@ -203,31 +206,86 @@ __host__ __device__ __forceinline__ float gen_normal(unsigned long long st, unsi
     return static_cast<float>(s - 262140) * 0x1.3988e2p-16f;
 }
 
+// ---------------------------------------------------------------------------------------------
+// Group quantisation of 8 values per thread, 32 per quad.  This arithmetic runs in the prologue of every GEMV CTA, between the
+// arrival of the activations and the first dot product, so its length counts; the codes are those of
+//   scale = amax > 0 ? RN(amax / kMax) : 1;  q = clamp(rint(RN(x * RN(1 / scale))), -kMax, kMax)
+// operation by operation (group_codes_plain), computed with fewer instructions where amax is an ordinary number.
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+// RN(a / D) for a constant D, 1e-30 <= a <= 3e38: Markstein's correction of a quotient by its exact residual ("Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990): with y = RN(1/D) and q = RN(a y), q + (a - D q) y
+// rounds to the correctly rounded quotient.
+template <int D> __device__ __forceinline__ float div_const(float a) {
+    constexpr float y = static_cast<float>(1.0 / D);
+    const float q = __fmul_rn(a, y);
+    return __fmaf_rn(__fmaf_rn(-static_cast<float>(D), q, a), y, q);
+}
+template <int kMax> __device__ __forceinline__ float group_codes_plain(const float (&v)[8], float amax, int (&q)[8]) {
+    const float scale = amax > 0.0f ? __fdiv_rn(amax, static_cast<float>(kMax)) : 1.0f;
+    const float inv = __fdiv_rn(1.0f, scale);
+#pragma unroll
+    for (int e = 0; e < 8; e++) q[e] = max(-kMax, min(kMax, __float2int_rn(__fmul_rn(v[e], inv))));
+    return scale;
+}
+// Codes of the thread's values as numbers whose low 16 bits are the two's complement code; returns the group's scale.  All 32
+// lanes of the warp take part.
+template <int kMax> __device__ __forceinline__ float group_codes(const float (&v)[8], uint32_t (&q)[8]) {
+    float amax = max_nan(max_nan(max_nan(fabsf(v[0]), fabsf(v[1])), max_nan(fabsf(v[2]), fabsf(v[3]))),
+                         max_nan(max_nan(fabsf(v[4]), fabsf(v[5])), max_nan(fabsf(v[6]), fabsf(v[7]))));
+    amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    const bool plain = amax == 0.0f || (amax >= 1e-30f && amax <= 3.0e38f);
+    if (__any_sync(0xffffffffu, !plain)) {  // a NaN, an infinity or a vanishing maximum somewhere in the warp
+        amax = 0.0f;
+#pragma unroll
+        for (int e = 0; e < 8; e++) amax = fmaxf(amax, fabsf(v[e]));
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+        int qi[8];
+        const float scale = group_codes_plain<kMax>(v, amax, qi);
+        const bool lost = kMax == 32767 && !(amax <= 3.0e38f);  // the 16-bit form has no code for it: a NaN scale and zeros
+#pragma unroll
+        for (int e = 0; e < 8; e++) q[e] = lost ? 0u : static_cast<uint32_t>(qi[e]);
+        return lost ? __int_as_float(0x7FC00000) : scale;
+    }
+    const float scale = amax > 0.0f ? div_const<kMax>(amax) : 1.0f;
+    const float inv = __frcp_rn(scale);
+    // |x * inv| <= kMax * (1 + 2^-22): no clamp; adding 1.5 * 2^23 rounds to the nearest integer, ties to even, and leaves it in
+    // the low bits
+#pragma unroll
+    for (int e = 0; e < 8; e++) q[e] = __float_as_uint(__fadd_rn(__fmul_rn(v[e], inv), 12582912.0f));
+    return scale;
+}
+// int8 codes of 8 values: two words, and their sum
+__device__ __forceinline__ float q8_codes(const float (&v)[8], uint32_t& w0, uint32_t& w1, int& sum) {
+    uint32_t q[8];
+    const float scale = group_codes<127>(v, q);
+    w0 = __byte_perm(__byte_perm(q[0], q[1], 0x0040), __byte_perm(q[2], q[3], 0x0040), 0x5410);
+    w1 = __byte_perm(__byte_perm(q[4], q[5], 0x0040), __byte_perm(q[6], q[7], 0x0040), 0x5410);
+    sum = __dp4a(static_cast<int>(w0), 0x01010101, __dp4a(static_cast<int>(w1), 0x01010101, 0));
+    return scale;
+}
+
 // 16-bit fixed point of one 32-wide group held by the 4 threads of a quad (8 values each): v = rint(x * 32767 / amax),
 // split into an unsigned low-byte plane and a signed high-byte plane (the form the W4A16 GEMV multiplies with dp4a).
-// Returns the group's scale; `sum` is the sum of the group's 32 codes.
+// Returns the group's scale (NaN when amax is not finite); `sum` is the sum of the group's 32 codes.
 __device__ __forceinline__ float x16_quad_convert(const float (&xe)[8], uint32_t& l0, uint32_t& l1, uint32_t& h0, uint32_t& h1,
                                                   int& sum) {
-    float amax = 0.0f;
-#pragma unroll
-    for (int e = 0; e < 8; e++) amax = fmaxf(amax, fabsf(xe[e]));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-    float scale = amax > 0.0f ? __fdiv_rn(amax, 32767.0f) : 1.0f;
-    if (!(amax <= 3.0e38f)) scale = __int_as_float(0x7FC00000);
-    const float inv = __fdiv_rn(1.0f, scale);
-    l0 = l1 = h0 = h1 = 0;
-    sum = 0;
-#pragma unroll
-    for (int e = 0; e < 8; e++) {
-        int q = __float2int_rn(__fmul_rn(xe[e], inv));
-        q = max(-32767, min(32767, q));
-        sum += q;
-        const uint32_t lo8 = static_cast<uint32_t>(q) & 0xFFu;
-        const uint32_t hi8 = static_cast<uint32_t>(q >> 8) & 0xFFu;
-        if (e < 4) { l0 |= lo8 << (8 * e); h0 |= hi8 << (8 * e); }
-        else { l1 |= lo8 << (8 * (e - 4)); h1 |= hi8 << (8 * (e - 4)); }
-    }
+    uint32_t q[8];
+    const float scale = group_codes<32767>(xe, q);
+    const uint32_t a = __byte_perm(q[0], q[1], 0x5410), b = __byte_perm(q[2], q[3], 0x5410);
+    const uint32_t c = __byte_perm(q[4], q[5], 0x5410), d = __byte_perm(q[6], q[7], 0x5410);
+    l0 = __byte_perm(a, b, 0x6420);
+    h0 = __byte_perm(a, b, 0x7531);
+    l1 = __byte_perm(c, d, 0x6420);
+    h1 = __byte_perm(c, d, 0x7531);
+    sum = 256 * __dp4a(static_cast<int>(h0), 0x01010101, __dp4a(static_cast<int>(h1), 0x01010101, 0)) +
+          static_cast<int>(dp4a_uu(l0, 0x01010101u, static_cast<int>(dp4a_uu(l1, 0x01010101u, 0))));
     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
     sum += __shfl_xor_sync(0xffffffffu, sum, 2);
     return scale;

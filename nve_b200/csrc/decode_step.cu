@@ -451,7 +451,7 @@ __device__ __forceinline__ void ds_stage_norm(const uint16_t* x, const uint16_t*
     float total = warp_part[0];
 #pragma unroll
     for (int w = 1; w < kGemvThreads / 32; w++) total = __fadd_rn(total, warp_part[w]);
-    const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(K)), eps)));
+    const float r = __frcp_rn(__fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(K)), eps)));
 #pragma unroll
     for (int it = 0; it < kDsStageIters; it++) {
         if (it < iters) {  // uniform over the CTA: the quad shuffles inside stage_chunk_* need whole warps

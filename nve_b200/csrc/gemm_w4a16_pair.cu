@@ -743,7 +743,7 @@ __global__ void __launch_bounds__(256) gemm_pair_reduce_norm_kernel(const PairPa
     float total = warp_part[0];
 #pragma unroll
     for (int i = 1; i < 8; i++) total = __fadd_rn(total, warp_part[i]);
-    const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(N)), eps)));
+    const float r = __frcp_rn(__fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(N)), eps)));
 #pragma unroll
     for (int j = 0; j < kPairNormChunks; j++) {
         const int c = j * 256 + static_cast<int>(threadIdx.x);

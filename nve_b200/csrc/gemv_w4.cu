@@ -36,6 +36,7 @@
 namespace nve {
 
 
+constexpr int kMaxOwnGroups = 16;  // groups of 32 values that a gate/up CTA converts from its own shared memory
 constexpr unsigned kTpSpinLimit = 1u << 22;  // bounded wait for a peer's slot (local polls of >= 32 ns each)
 
 // One warp item: R rows x C consecutive column sets (R * C = 8 blocks per lane), all 16 loads in flight at once.
@@ -83,6 +84,8 @@ __device__ __forceinline__ void load_item(const GemvParams& p, int tile, int cg,
             if constexpr (C > 2) {
                 t.w[2][r] = ld_stream_u4_off<1024>(nrow);
                 t.s[2][r] = ld_stream_f32_off<256>(srow);
+            }
+            if constexpr (C > 3) {
                 t.w[3][r] = ld_stream_u4_off<1536>(nrow);
                 t.s[3][r] = ld_stream_f32_off<384>(srow);
             }
@@ -102,19 +105,25 @@ __device__ __forceinline__ void load_item(const GemvParams& p, int tile, int cg,
     }
 }
 
-template <int PLANES, int XDT, int ODT, bool IDOT, int PRO, int R, int C, bool PAIR = false>
+// PAIRED: 0 rows of one to three matrices, 1 gate/up, 2 gate/up with whole groups of the converted product per CTA (p.pq_own)
+template <int PLANES, int XDT, int ODT, bool IDOT, int PRO, int R, int C, int PAIRED = 0>
 __global__ void __launch_bounds__(kGemvThreads, 2) gemv_w4_kernel(const GemvParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     constexpr int W = kGemvThreads / 32;
+    constexpr bool PAIR = PAIRED != 0;
     const int S = p.S;
     const int CG = (S + C - 1) / C;  // column groups per row
     Smem<PLANES> sm(smem_raw, S * kWarp);
 
     const int tiles = (p.n_total + R - 1) / R;
-    const int tile_begin = static_cast<int>(static_cast<long long>(tiles) * blockIdx.x / gridDim.x);
-    const int tile_end = static_cast<int>(static_cast<long long>(tiles) * (blockIdx.x + 1) / gridDim.x);
+    int tile_begin = static_cast<int>(static_cast<long long>(tiles) * blockIdx.x / gridDim.x);
+    int tile_end = static_cast<int>(static_cast<long long>(tiles) * (blockIdx.x + 1) / gridDim.x);
+    if constexpr (PAIRED == 2) {  // whole 32-wide groups
+        tile_begin = min(tiles, static_cast<int>(blockIdx.x) * p.pq_own * (64 / R));
+        tile_end = min(tiles, tile_begin + p.pq_own * (64 / R));
+    }
     const int chunk_tiles_max = max(1, kPartFloats / (R * CG));
 
     // Weights do not depend on the producer kernel: start streaming them before waiting for it.
@@ -149,7 +158,9 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_w4_kernel(const GemvPara
             }
         }
     }
-    stage_activations<PLANES, XDT, PRO>(p, sm, nr);
+    XRegs xr;
+    if constexpr (PRO == 1) load_x_regs(p, xr);
+    stage_activations<PLANES, XDT, PRO>(p, sm, nr, xr);
     // tensor parallel: this launch's epoch is this CTA's own launch counter + 1; slots of the parity it selects
     // are used (a peer can be at most one all-reduce ahead, so two parities never collide)
     __shared__ unsigned tp_epoch_s;
@@ -161,6 +172,89 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_w4_kernel(const GemvPara
     // offset of the plane [parity][source = this rank] inside any rank's buffer
     const size_t tp_plane = (static_cast<size_t>(tp_epoch & 1u) * p.tp.world + p.tp.rank) * p.tp.rows_cap;
 
+    // the item in registers: per lane and row the sum over its column sets
+    auto dot_item = [&](auto even_tag, int cg, float (&a)[R]) {
+        constexpr bool EVEN = decltype(even_tag)::value;
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+            // < nbp; idle column sets carry zero weights
+            const int bs = (EVEN ? (cg * C + c) : min((cg * C + c), S - 1)) * kWarp + lane;
+            XTile<PLANES> x;
+#pragma unroll
+            for (int pl = 0; pl < PLANES; pl++) {
+                x.lo[pl] = sm.plane[(pl * 2 + 0) * sm.nbp + bs];
+                x.hi[pl] = sm.plane[(pl * 2 + 1) * sm.nbp + bs];
+            }
+            x.xs = sm.xs[bs];
+            x.bias = sm.bias[bs];
+            const bool live = EVEN || (cg * C + c) < S;
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const int I = block_dot<PLANES>(it.w[c][r], x);
+                if constexpr (IDOT) {
+                    const int grow = it.row0 + r;
+                    const int b = (cg * C + c) * kWarp + lane;
+                    if (live && grow < p.n_total && b < p.nb) p.idot[static_cast<long long>(grow) * p.nb + b] = I;
+                    a[r] = 0.0f;
+                } else {
+                    // per lane the C column sets of the group are added in ascending order, first term exact
+                    const float v = live ? __fmul_rn(__fmul_rn(it.s[c][r], x.xs), static_cast<float>(I)) : 0.0f;
+                    a[r] = (c == 0) ? v : __fadd_rn(a[r], v);
+                }
+            }
+        }
+    };
+
+    // ---- gate/up, the groups of 32 values dealt out whole, rows of one column group: a warp has whole rows and stores its values
+    // itself, the CTA converts its groups from shared memory.  No partial sums, and no counting, which costs 2 us after the last
+    // dot product of a launch (two fences, an atomic and a read in series): 1B shape 22.4 -> 20.5 us per layer, 3B 29.8 -> 27.0.
+    // (8B: 448 groups on 296 CTAs.  The groups that do not divide, computed first and counted while the CTA goes on, cost 1.5 us
+    // more than they saved: a fence waits for the weights that the warp has under way.)
+    if constexpr (PAIRED == 2) {
+        constexpr int H = R / 2;
+        __shared__ uint16_t own_mid[kMaxOwnGroups * 32];
+        auto run = [&](auto even_tag) {
+            for (int tile = tile_begin + warp; tile < tile_end; tile += W) {
+                float a[R];
+                dot_item(even_tag, 0, a);
+                if (tile + W < tile_end) load_item<R, C, PAIR, decltype(even_tag)::value>(p, tile + W, 0, lane, it);
+                warp_sum_multi<R>(a, lane);
+                const float up = __shfl_xor_sync(0xffffffffu, a[0], 16);  // the up row of the gate row that this lane holds
+                if (multi_row_writer<R>(lane) && lane < 16) {
+                    const int idx = tile * H + multi_row_of<R>(lane);
+                    const float g = Act16<ODT>::to_f32(Act16<ODT>::from_f32(a[0]));
+                    const uint16_t m16 = Act16<ODT>::from_f32(silu_mul_f32(g, Act16<ODT>::to_f32(Act16<ODT>::from_f32(up))));
+                    static_cast<uint16_t*>(p.out[0])[idx] = m16;
+                    own_mid[idx - tile_begin * H] = m16;
+                }
+            }
+        };
+        if ((p.nb % kWarp) == 0 && (S % C) == 0) run(std::true_type{});
+        else run(std::false_type{});
+        __syncthreads();
+        const int own = (tile_end - tile_begin) / (64 / R);
+        for (int g0 = 8 * warp; g0 < own; g0 += 8 * W) {  // eight groups per warp, a quad each
+            const int g = g0 + (lane >> 2);
+            const bool mine = g < own;
+            const long long chunk = (static_cast<long long>(blockIdx.x) * p.pq_own + g) * 4 + (lane & 3);
+            float v[8];
+#pragma unroll
+            for (int e = 0; e < 8; e++) v[e] = mine ? Act16<ODT>::to_f32(own_mid[(g * 4 + (lane & 3)) * 8 + e]) : 0.0f;
+            if (p.pq_mode == 1) {
+                quantize_quad(v, p.pq_xq, p.pq_xs, chunk, mine);
+            } else {
+                if (mine && p.pq_awq != nullptr) {
+#pragma unroll
+                    for (int e = 0; e < 8; e++) v[e] = __fmul_rn(v[e], p.pq_awq[chunk * 8 + e]);
+                }
+                x16_quad(v, p.pq_xlo, p.pq_xq, p.pq_xs, chunk, mine);
+            }
+            // every launch adds 32 to every counter, whichever way its group was converted
+            if (mine && (lane & 3) == 0) atomicAdd(p.pq_cnt + (chunk >> 2), 32u);
+        }
+        return;
+    }
+
     bool first_chunk = true;
     // The streaming loop is compiled twice: with and without the bounds checks of ragged rows (see load_item).
     auto stream = [&](auto even_tag) {
@@ -169,34 +263,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_w4_kernel(const GemvPara
         const int n_items = chunk_tiles * CG;
         while (q < n_items) {
             float a[R];
-#pragma unroll
-            for (int c = 0; c < C; c++) {
-                // < nbp; idle column sets carry zero weights
-                const int bs = (EVEN ? (cg * C + c) : min((cg * C + c), S - 1)) * kWarp + lane;
-                XTile<PLANES> x;
-#pragma unroll
-                for (int pl = 0; pl < PLANES; pl++) {
-                    x.lo[pl] = sm.plane[(pl * 2 + 0) * sm.nbp + bs];
-                    x.hi[pl] = sm.plane[(pl * 2 + 1) * sm.nbp + bs];
-                }
-                x.xs = sm.xs[bs];
-                x.bias = sm.bias[bs];
-                const bool live = EVEN || (cg * C + c) < S;
-#pragma unroll
-                for (int r = 0; r < R; r++) {
-                    const int I = block_dot<PLANES>(it.w[c][r], x);
-                    if constexpr (IDOT) {
-                        const int grow = it.row0 + r;
-                        const int b = (cg * C + c) * kWarp + lane;
-                        if (live && grow < p.n_total && b < p.nb) p.idot[static_cast<long long>(grow) * p.nb + b] = I;
-                        a[r] = 0.0f;
-                    } else {
-                        // per lane the C column sets of the group are added in ascending order, first term exact
-                        const float v = live ? __fmul_rn(__fmul_rn(it.s[c][r], x.xs), static_cast<float>(I)) : 0.0f;
-                        a[r] = (c == 0) ? v : __fadd_rn(a[r], v);
-                    }
-                }
-            }
+            dot_item(even_tag, cg, a);
             // issue the next item's loads before reducing this one
             const int qn = q + W;
             int tln = tl + step_t, cgn = cg + step_c;
@@ -448,7 +515,7 @@ __global__ void gemv_w4_unaligned_kernel(const GemvParams p) {
 // ---------------------------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------------------------
-template <typename Kern> static int launch_gemv(Kern kern, const GemvParams& p, int planes, int rows_per_item, cudaStream_t stream) {
+template <typename Kern> static int launch_gemv(Kern kern, const GemvParams& p, int planes, int rows_per_item, cudaStream_t stream, int own = 0) {
     const size_t smem = gemv_smem_bytes(planes, p.S);
     if (smem > static_cast<size_t>(kMaxGemvSmem)) return set_status(NVE_ERR_TOO_LARGE);
     if (smem > 48 * 1024) {
@@ -479,7 +546,10 @@ template <typename Kern> static int launch_gemv(Kern kern, const GemvParams& p, 
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.numAttrs = 2;
     }
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p);
+    GemvParams pl = p;
+    pl.pq_own = own;
+    if (own > 0) cfg.gridDim = dim3((p.row_end[0] / 32 + own - 1) / own);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, pl);
     count_launch();
     return set_cuda_status(e);
 }
@@ -492,13 +562,33 @@ static bool all_aligned(const GemvParams& p, int num_mats, int planes, int pro) 
     return aligned(p.x16, 16);  // PRO 1 and 2 and W4A16 read the 16-bit vector
 }
 
+// Whole groups of 32 values per gate/up CTA, where that takes no more rounds of eight warps than an even split of the tiles
+// and every row is one column group: the number of groups, else 0.
+static int own_groups(const GemvParams& p, int rows_per_item, int sets_per_item) {
+    if (p.pq_mode == 0 || p.S > sets_per_item || p.row_end[0] % 32 != 0) return 0;
+    const int grid = 2 * sm_count(), groups = p.row_end[0] / 32, group_tiles = 64 / rows_per_item, tiles = groups * group_tiles;
+    const int own = (groups + grid - 1) / grid, rounds = ((tiles + grid - 1) / grid + 7) / 8;
+    return own <= kMaxOwnGroups && (own * group_tiles + 7) / 8 <= rounds ? own : 0;
+}
+
 template <int PLANES, int XDT, int ODT, int PRO, bool PAIR = false>
 static int dispatch_aligned(const GemvParams& p, int num_mats, cudaStream_t st) {
     if (all_aligned(p, num_mats, PLANES, PRO)) {
-        // 8 blocks per lane and item: 2 rows x 4 column sets, or more rows when a row has fewer column sets
-        if (p.S >= 3) return launch_gemv(gemv_w4_kernel<PLANES, XDT, ODT, false, PRO, 2, 4, PAIR>, p, PLANES, 2, st);
-        if (p.S == 2) return launch_gemv(gemv_w4_kernel<PLANES, XDT, ODT, false, PRO, 4, 2, PAIR>, p, PLANES, 4, st);
-        return launch_gemv(gemv_w4_kernel<PLANES, XDT, ODT, false, PRO, 8, 1, PAIR>, p, PLANES, 8, st);
+        // 8 blocks per lane and item: 2 rows x 4 column sets, or more rows when a row has fewer column sets.  Three column sets
+        // are one group of their own: no idle fourth (3B shape, 3072 columns: 30.0 -> 29.0 us per layer).
+        auto run = [&](auto rows, auto sets) {
+            constexpr int R = decltype(rows)::value, C = decltype(sets)::value;
+            if constexpr (PAIR && ODT != NVE_DT_F32) {
+                if (const int own = own_groups(p, R, C); own > 0)
+                    return launch_gemv(gemv_w4_kernel<PLANES, XDT, ODT, false, PRO, R, C, 2>, p, PLANES, R, st, own);
+            }
+            return launch_gemv(gemv_w4_kernel<PLANES, XDT, ODT, false, PRO, R, C, PAIR ? 1 : 0>, p, PLANES, R, st);
+        };
+        using std::integral_constant;
+        if (p.S == 3) return run(integral_constant<int, 2>(), integral_constant<int, 3>());
+        if (p.S > 3) return run(integral_constant<int, 2>(), integral_constant<int, 4>());
+        if (p.S == 2) return run(integral_constant<int, 4>(), integral_constant<int, 2>());
+        return run(integral_constant<int, 8>(), integral_constant<int, 1>());
     }
     if constexpr (PRO != 0) {
         return set_status(NVE_ERR_BAD_ALIGNMENT);  // the fused prologue needs 16-byte aligned vectors
@@ -544,6 +634,7 @@ static int fill_params(GemvParams& p, const nve_b200_w4_matrix* mats, int num_ma
     p.xq = nullptr; p.xs = nullptr; p.x16 = nullptr; p.xlo = nullptr; p.awq = nullptr; p.idot = nullptr;
     p.paired = 0;
     p.pq_mode = 0;
+    p.pq_own = 0;
     p.pq_cnt = nullptr;
     p.pq_xq = nullptr;
     p.pq_xlo = nullptr;

@@ -40,6 +40,7 @@ struct GemvParams {
     const void* x16;    // W4A16 activations
     const uint8_t* xlo; // W4A16 activations already in fixed point: low-byte plane (high bytes in xq, scales in xs)
     const float* awq;   // optional per-column multiplier (W4A16)
+    int awq16;          // awq is 16-byte aligned
     const void* norm_w; // RMSNorm weight of the fused prologue (16-bit, same type as x16)
     float eps;
     int32_t* idot;      // debug: per-block integer dots [n_total, nb]
@@ -50,6 +51,7 @@ struct GemvParams {
     // activation kernel and no per-CTA quantiser prologue is needed.  pq_cnt[g] counts the values written to group g
     // (32 per launch, never reset; the test is on the count modulo 32, so the wrap of the 32-bit counter is harmless).
     int pq_mode;
+    int pq_own;         // > 0: whole groups per CTA; else the groups are counted
     unsigned* pq_cnt;
     int8_t* pq_xq;      // int8 codes (mode 1) / high-byte plane (mode 2)
     uint8_t* pq_xlo;    // low-byte plane (mode 2)
@@ -171,24 +173,9 @@ template <int PLANES> __device__ __forceinline__ void store_chunk_planes(Smem<PL
 // W4A8 codes from 8 already-rounded 16-bit values per thread (same arithmetic as the stand-alone quantizer:
 // scale = amax > 0 ? amax/127 : 1 ; q = clamp(rint(v * (1/scale)), -127, 127)).
 __device__ __forceinline__ void stage_chunk_q8(Smem<1>& sm, int c, const float (&v)[8], bool active) {
-    float amax = 0.0f;
-#pragma unroll
-    for (int e = 0; e < 8; e++) amax = fmaxf(amax, fabsf(v[e]));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-    const float scale = amax > 0.0f ? __fdiv_rn(amax, 127.0f) : 1.0f;
-    const float inv = __fdiv_rn(1.0f, scale);
-    uint32_t w0 = 0, w1 = 0;
-    int sum = 0;
-#pragma unroll
-    for (int e = 0; e < 8; e++) {
-        int q = __float2int_rn(__fmul_rn(v[e], inv));
-        q = max(-127, min(127, q));
-        sum += q;
-        const uint32_t byte = static_cast<uint32_t>(q) & 0xFFu;
-        if (e < 4) w0 |= byte << (8 * e);
-        else w1 |= byte << (8 * (e - 4));
-    }
+    uint32_t w0, w1;
+    int sum;
+    const float scale = q8_codes(v, w0, w1, sum);
     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
     sum += __shfl_xor_sync(0xffffffffu, sum, 2);
     if (active) {
@@ -283,6 +270,19 @@ __device__ __forceinline__ void load_norm_regs(const GemvParams& p, NormRegs& nr
         if (c < chunks && chunks <= kNormRegChunks * kGemvThreads) nr.w[j] = reinterpret_cast<const uint4*>(p.norm_w)[c];
     }
 }
+// The 16-bit vector of the fused RMSNorm prologue, all loads in flight together (K <= 8192).
+struct XRegs {
+    uint4 x[kNormRegChunks];
+};
+__device__ __forceinline__ void load_x_regs(const GemvParams& p, XRegs& xr) {
+    const int chunks = p.K >> 3;
+#pragma unroll
+    for (int j = 0; j < kNormRegChunks; j++) {
+        const int c = j * kGemvThreads + threadIdx.x;
+        xr.x[j] = make_uint4(0, 0, 0, 0);
+        if (c < chunks && chunks <= kNormRegChunks * kGemvThreads) xr.x[j] = reinterpret_cast<const uint4*>(p.x16)[c];
+    }
+}
 // Stage the activations.  PRO = 0: the caller's vector (int8 codes for W4A8, 16-bit values for W4A16).
 // PRO = 2: the caller's 16-bit vector, quantised here (W4A8: the int8 codes of the stand-alone quantiser).
 // PRO = 1: RMSNorm of the caller's 16-bit vector first, in the library's fixed order (256 threads; thread t
@@ -290,7 +290,8 @@ __device__ __forceinline__ void load_norm_regs(const GemvParams& p, NormRegs& nr
 // order; r = 1/sqrt(sum/n + eps); o = round16((x*r)*w)), then quantised exactly as the separate kernels do.
 template <int PLANES, int XDT, int PRO> __device__ __forceinline__ void stage_activations(const GemvParams& p,
                                                                                            Smem<PLANES>& sm,
-                                                                                           const NormRegs& nr) {
+                                                                                           const NormRegs& nr,
+                                                                                           const XRegs& xr) {
     zero_padding<PLANES>(p, sm);
     if constexpr (PLANES == 1 && PRO == 0) {
         stage_q8(p, sm);
@@ -307,22 +308,15 @@ template <int PLANES, int XDT, int PRO> __device__ __forceinline__ void stage_ac
         float r = 1.0f;
         if constexpr (PRO == 1) {
             if (chunks <= kNormRegChunks * kGemvThreads) {
-                // Register-resident form: the vector is read once (all loads in flight together), the norm weights
-                // came in before the dependency wait.  Same arithmetic and the same summation order as below.
+                // Register-resident form: the vector is read once (load_x_regs), the norm weights came in before the
+                // dependency wait.  Same arithmetic and the same summation order as below.
                 __shared__ float warp_part_r[kGemvThreads / 32];
-                uint4 xr[kNormRegChunks];
-#pragma unroll
-                for (int j = 0; j < kNormRegChunks; j++) {
-                    const int c = j * kGemvThreads + threadIdx.x;
-                    xr[j] = make_uint4(0, 0, 0, 0);
-                    if (c < chunks) xr[j] = reinterpret_cast<const uint4*>(x)[c];
-                }
                 float acc = 0.0f;
 #pragma unroll
                 for (int j = 0; j < kNormRegChunks; j++) {
                     if (j * kGemvThreads + static_cast<int>(threadIdx.x) < chunks) {
                         uint16_t h[8];
-                        unpack8(xr[j], h);
+                        unpack8(xr.x[j], h);
 #pragma unroll
                         for (int e = 0; e < 8; e++) {
                             const float v = Act16<XDT>::to_f32(h[e]);
@@ -336,7 +330,7 @@ template <int PLANES, int XDT, int PRO> __device__ __forceinline__ void stage_ac
                 float total = warp_part_r[0];
 #pragma unroll
                 for (int w = 1; w < kGemvThreads / 32; w++) total = __fadd_rn(total, warp_part_r[w]);
-                r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(p.K)), p.eps)));
+                r = __frcp_rn(__fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(p.K)), p.eps)));
                 const int iters_r = (chunks + kGemvThreads - 1) / kGemvThreads;
 #pragma unroll
                 for (int j = 0; j < kNormRegChunks; j++) {
@@ -346,16 +340,27 @@ template <int PLANES, int XDT, int PRO> __device__ __forceinline__ void stage_ac
                         float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
                         if (active) {
                             uint16_t h[8], hw[8];
-                            unpack8(xr[j], h);
+                            unpack8(xr.x[j], h);
                             unpack8(nr.w[j], hw);
 #pragma unroll
-                            for (int e = 0; e < 8; e++) {
-                                const float o = __fmul_rn(__fmul_rn(Act16<XDT>::to_f32(h[e]), r), Act16<XDT>::to_f32(hw[e]));
-                                v[e] = Act16<XDT>::to_f32(Act16<XDT>::from_f32(o));
+                            for (int e = 0; e < 8; e += 2) {
+                                const float2 o = Act16<XDT>::round2(__fmul_rn(__fmul_rn(Act16<XDT>::to_f32(h[e]), r), Act16<XDT>::to_f32(hw[e])),
+                                                                   __fmul_rn(__fmul_rn(Act16<XDT>::to_f32(h[e + 1]), r), Act16<XDT>::to_f32(hw[e + 1])));
+                                v[e] = o.x;
+                                v[e + 1] = o.y;
                             }
                             if (p.awq != nullptr) {  // W4A16 always; W4A8 only through the *_awq entry point
+                                // two 16-byte loads where the vector allows them (the entry points take any float pointer)
+                                float a[8];
+                                if (p.awq16) {
+                                    const float4 a0 = reinterpret_cast<const float4*>(p.awq)[2 * c], a1 = reinterpret_cast<const float4*>(p.awq)[2 * c + 1];
+                                    a[0] = a0.x, a[1] = a0.y, a[2] = a0.z, a[3] = a0.w, a[4] = a1.x, a[5] = a1.y, a[6] = a1.z, a[7] = a1.w;
+                                } else {
 #pragma unroll
-                                for (int e = 0; e < 8; e++) v[e] = __fmul_rn(v[e], p.awq[c * 8 + e]);
+                                    for (int e = 0; e < 8; e++) a[e] = p.awq[c * 8 + e];
+                                }
+#pragma unroll
+                                for (int e = 0; e < 8; e++) v[e] = __fmul_rn(v[e], a[e]);
                             }
                         }
                         if constexpr (PLANES == 1) stage_chunk_q8(sm, c, v, active);
@@ -383,7 +388,7 @@ template <int PLANES, int XDT, int PRO> __device__ __forceinline__ void stage_ac
             float total = warp_part[0];
 #pragma unroll
             for (int w = 1; w < kGemvThreads / 32; w++) total = __fadd_rn(total, warp_part[w]);
-            r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(p.K)), p.eps)));
+            r = __frcp_rn(__fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(p.K)), p.eps)));
         }
         const int iters = (chunks + kGemvThreads - 1) / kGemvThreads;
         for (int it = 0; it < iters; it++) {
@@ -406,8 +411,16 @@ template <int PLANES, int XDT, int PRO> __device__ __forceinline__ void stage_ac
                     for (int e = 0; e < 8; e++) v[e] = Act16<XDT>::to_f32(h[e]);
                 }
                 if (p.awq != nullptr) {
+                    float a[8];
+                    if (p.awq16) {
+                        const float4 a0 = reinterpret_cast<const float4*>(p.awq)[2 * c], a1 = reinterpret_cast<const float4*>(p.awq)[2 * c + 1];
+                        a[0] = a0.x, a[1] = a0.y, a[2] = a0.z, a[3] = a0.w, a[4] = a1.x, a[5] = a1.y, a[6] = a1.z, a[7] = a1.w;
+                    } else {
 #pragma unroll
-                    for (int e = 0; e < 8; e++) v[e] = __fmul_rn(v[e], p.awq[c * 8 + e]);
+                        for (int e = 0; e < 8; e++) a[e] = p.awq[c * 8 + e];
+                    }
+#pragma unroll
+                    for (int e = 0; e < 8; e++) v[e] = __fmul_rn(v[e], a[e]);
                 }
             }
             if constexpr (PLANES == 1) stage_chunk_q8(sm, c, v, active);

@@ -119,11 +119,6 @@ __device__ __forceinline__ uint32_t pack_q4(float p0, float p1, float p2, float 
     const uint32_t t = low(p0) + low(p1) * 0x100u + low(p2) * 0x10000u + low(p3) * 0x1000000u;
     return ((t - kBase) >> 1) & 0x0F0F0F0Fu;
 }
-__device__ __forceinline__ float max_nan(float a, float b) {
-    float r;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-    return r;
-}
 
 constexpr int kQ4Loads = 4;  // 16-byte loads per thread = blocks per group of eight lanes
 template <bool AWQ>
