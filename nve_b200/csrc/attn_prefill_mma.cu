@@ -1,18 +1,20 @@
-// Causal attention of a block of new positions (prefill) on the tensor cores: tiles of 128 query rows against tiles
+// Causal attention of a block of new positions (prefill) on the tensor cores: tiles of 64 query rows against tiles
 // of 64 cached positions, online softmax, K/V staged in shared memory once per tile and used by all its rows.
 //
 // What bounds it: with one CTA per (row, KV head) every row read the whole K/V prefix through L2 by itself (1777 rows
-// of an 8B model: 1.58 M (row, position) pairs x 512 bytes x 8 KV heads = 6.5 GB per layer); a tile of 128 rows reads
-// it 128 / G times less often and the kernel is bound by the mma.sync rate instead.  Whole prefill passes before / after:
-// 8B, 1777 positions 57.4 -> 31.8 ms; 3B (3 query heads per KV head), 300 positions at 700 20.7 -> 7.6 ms.
+// of an 8B model: 1.58 M (row, position) pairs x 512 bytes x 8 KV heads = 6.5 GB per layer); a tile of 64 rows reads
+// it 64 / G times less often and the kernel is bound by the mma.sync rate (about 1000 multiply-adds per cycle and SM) and by
+// what stands between the two products of a step.  Tiles of 64 rows, not 128: twice the CTAs where the block is short, half the
+// registers of a step, and faster at every size (8B, us: 61 rows 7.8 -> 4.7, 300 rows 25.5 -> 12.0, 600 rows 36.8 -> 20.8,
+// 1777 rows 126 -> 107).  The queries stay in shared memory: in registers they leave room for a third CTA per SM, and all
+// of it was slower (1777 rows 122, 3B 300 rows at 700 21.5 -> 29.7).
 //
 // A query row of a tile is a (position, head) pair of ONE KV head: row r of a tile is position t * PT + r / G, head
-// h0 + r % G with PT = 128 / G positions per tile.  All G heads of the group share the staged K/V, and a short block
-// (61 rows x 4 heads) fills its tiles; any group size works.  Four warps take 32 rows each (two m16 row blocks, so that
-// every K / V fragment that is read from shared memory feeds two MMAs).
+// h0 + r % G with PT = 64 / G positions per tile.  All G heads of the group share the staged K/V, and a short block
+// fills its tiles; any group size up to 64 works.  Four warps take 16 rows each.
 //
 // Few tiles (a short block behind a long prefix) would leave most SMs idle: a cluster of 2, 4 or 8 CTAs then splits
-// the positions of one tile, leaves unnormalised partials in shared memory and every CTA merges 128 / C of the rows
+// the positions of one tile, leaves unnormalised partials in shared memory and every CTA merges 64 / C of the rows
 // through distributed shared memory.
 #include <cooperative_groups.h>
 
@@ -23,9 +25,9 @@ namespace cg = cooperative_groups;
 
 namespace nve {
 
-constexpr int kApRows = 128;     // query rows per tile
+constexpr int kApRows = 64;      // query rows per tile
 constexpr int kApKeys = 64;      // cached positions per step
-constexpr int kApThreads = 128;  // four warps of 32 rows
+constexpr int kApThreads = 128;  // four warps of 16 rows
 
 __device__ __forceinline__ uint32_t ap_smem(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void ap_cp16(uint32_t dst, const void* src) {
@@ -56,7 +58,7 @@ template <int HD> __device__ __forceinline__ uint32_t ap_off(int r, int c) {
 
 template <int HD> constexpr int ap_smem_bytes() {
     constexpr int stage = kApRows * HD * 2 + 4 * kApKeys * HD * 2;  // Q, two K and two V tiles
-    constexpr int part = kApRows * (HD + 4) * 4 + kApRows * 8;      // f32 partials of a split tile + their m, l
+    constexpr int part = kApRows * (HD + 4) * 4 + kApRows * 8 + kApRows * 32;  // f32 partials of a split tile + their m, l + weights
     return stage > part ? stage : part;
 }
 
@@ -107,26 +109,16 @@ __global__ void __launch_bounds__(kApThreads, 2) attn_prefill_mma_kernel(const A
     if (kt0 < kt1) load_kv(kt0, 0);
     asm volatile("cp.async.commit_group;" ::: "memory");
 
-    // this thread's four query rows: row block mt (16 rows), rows g and g + 8 of it; lim = positions the row may see
-    int lim[2][2];
+    // this thread's two query rows: g and g + 8 of the warp's sixteen; lim = positions the row may see
+    int lim[2];
 #pragma unroll
-    for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-        for (int hh = 0; hh < 2; hh++) {
-            const int r = warp * 32 + mt * 16 + hh * 8 + g;
-            lim[mt][hh] = start + pos0 + min(r, nrows - 1) / groups + 1;
-        }
+    for (int hh = 0; hh < 2; hh++) lim[hh] = start + pos0 + min(warp * 16 + hh * 8 + g, nrows - 1) / groups + 1;
     const int lim_min = start + pos0 + 1;
     const float sl2 = p.scale * 1.4426950408889634f;  // exponentials in base 2
-    float m[2][2], l[2][2];
-    float o[2][CH][4];
+    float m[2] = {-1e30f, -1e30f}, l[2] = {0.0f, 0.0f};
+    float o[CH][4];
 #pragma unroll
-    for (int mt = 0; mt < 2; mt++) {
-        m[mt][0] = m[mt][1] = -1e30f;
-        l[mt][0] = l[mt][1] = 0.0f;
-#pragma unroll
-        for (int j = 0; j < CH; j++) o[mt][j][0] = o[mt][j][1] = o[mt][j][2] = o[mt][j][3] = 0.0f;
-    }
+    for (int j = 0; j < CH; j++) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.0f;
 
     for (int kt = kt0; kt < kt1; kt++) {
         const int buf = (kt - kt0) & 1;
@@ -135,72 +127,60 @@ __global__ void __launch_bounds__(kApThreads, 2) attn_prefill_mma_kernel(const A
         if (kt + 1 < kt1) load_kv(kt + 1, buf ^ 1);
         asm volatile("cp.async.commit_group;" ::: "memory");
 
-        float s[2][8][4];
+        float s[8][4];
 #pragma unroll
-        for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-            for (int n = 0; n < 8; n++) s[mt][n][0] = s[mt][n][1] = s[mt][n][2] = s[mt][n][3] = 0.0f;
+        for (int n = 0; n < 8; n++) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.0f;
         const uint32_t kb = sk + buf * KVB, vb = sv + buf * KVB;
 #pragma unroll
         for (int kk = 0; kk < HD / 16; kk++) {
-            uint32_t qa[2][4];
-#pragma unroll
-            for (int mt = 0; mt < 2; mt++)
-                ap_ldm4(sq + ap_off<HD>(warp * 32 + mt * 16 + (lane & 15), 2 * kk + (lane >> 4)), qa[mt]);
+            uint32_t qa[4];
+            ap_ldm4(sq + ap_off<HD>(warp * 16 + (lane & 15), 2 * kk + (lane >> 4)), qa);
 #pragma unroll
             for (int np = 0; np < 4; np++) {
                 uint32_t b[4];  // positions np*16 .. +7 (b0, b1) and +8 .. +15 (b2, b3)
                 ap_ldm4(kb + ap_off<HD>(np * 16 + (lane & 7) + ((lane >> 4) << 3), 2 * kk + ((lane >> 3) & 1)), b);
-#pragma unroll
-                for (int mt = 0; mt < 2; mt++) {
-                    mma_f16_16816(s[mt][2 * np], qa[mt], b[0], b[1]);
-                    mma_f16_16816(s[mt][2 * np + 1], qa[mt], b[2], b[3]);
-                }
+                mma_f16_16816(s[2 * np], qa, b[0], b[1]);
+                mma_f16_16816(s[2 * np + 1], qa, b[2], b[3]);
             }
         }
         if ((kt + 1) * kApKeys > lim_min) {  // some row does not see the whole tile
 #pragma unroll
-            for (int mt = 0; mt < 2; mt++)
+            for (int n = 0; n < 8; n++)
 #pragma unroll
-                for (int n = 0; n < 8; n++)
-#pragma unroll
-                    for (int e = 0; e < 4; e++)
-                        if (kt * kApKeys + n * 8 + 2 * t + (e & 1) >= lim[mt][e >> 1]) s[mt][n][e] = -INFINITY;
+                for (int e = 0; e < 4; e++)
+                    if (kt * kApKeys + n * 8 + 2 * t + (e & 1) >= lim[e >> 1]) s[n][e] = -INFINITY;
         }
-        uint32_t pa[2][4][4];
 #pragma unroll
-        for (int mt = 0; mt < 2; mt++) {
+        for (int hh = 0; hh < 2; hh++) {
+            float mx = s[0][2 * hh];
 #pragma unroll
-            for (int hh = 0; hh < 2; hh++) {
-                float mx = s[mt][0][2 * hh];
+            for (int n = 0; n < 8; n++) mx = fmaxf(mx, fmaxf(s[n][2 * hh], s[n][2 * hh + 1]));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+            const float mn = fmaxf(m[hh], mx * sl2);  // stays finite: the masked value is below -1e30
+            const float corr = ap_exp2(m[hh] - mn);
+            m[hh] = mn;
+            float sum = 0.0f;
 #pragma unroll
-                for (int n = 0; n < 8; n++) mx = fmaxf(mx, fmaxf(s[mt][n][2 * hh], s[mt][n][2 * hh + 1]));
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-                const float mn = fmaxf(m[mt][hh], mx * sl2);  // stays finite: the masked value is below -1e30
-                const float corr = ap_exp2(m[mt][hh] - mn);
-                m[mt][hh] = mn;
-                float sum = 0.0f;
-#pragma unroll
-                for (int n = 0; n < 8; n++) {
-                    s[mt][n][2 * hh] = ap_exp2(fmaf(s[mt][n][2 * hh], sl2, -mn));
-                    s[mt][n][2 * hh + 1] = ap_exp2(fmaf(s[mt][n][2 * hh + 1], sl2, -mn));
-                    sum += s[mt][n][2 * hh] + s[mt][n][2 * hh + 1];
-                }
-                l[mt][hh] = l[mt][hh] * corr + sum;
-#pragma unroll
-                for (int j = 0; j < CH; j++) {
-                    o[mt][j][2 * hh] *= corr;
-                    o[mt][j][2 * hh + 1] *= corr;
-                }
+            for (int n = 0; n < 8; n++) {
+                s[n][2 * hh] = ap_exp2(fmaf(s[n][2 * hh], sl2, -mn));
+                s[n][2 * hh + 1] = ap_exp2(fmaf(s[n][2 * hh + 1], sl2, -mn));
+                sum += s[n][2 * hh] + s[n][2 * hh + 1];
             }
+            l[hh] = l[hh] * corr + sum;
 #pragma unroll
-            for (int kp = 0; kp < 4; kp++) {  // probabilities of 16 positions as the A operand of the second product
-                pa[mt][kp][0] = pack_f16x2(s[mt][2 * kp][0], s[mt][2 * kp][1]);
-                pa[mt][kp][1] = pack_f16x2(s[mt][2 * kp][2], s[mt][2 * kp][3]);
-                pa[mt][kp][2] = pack_f16x2(s[mt][2 * kp + 1][0], s[mt][2 * kp + 1][1]);
-                pa[mt][kp][3] = pack_f16x2(s[mt][2 * kp + 1][2], s[mt][2 * kp + 1][3]);
+            for (int j = 0; j < CH; j++) {
+                o[j][2 * hh] *= corr;
+                o[j][2 * hh + 1] *= corr;
             }
+        }
+        uint32_t pa[4][4];
+#pragma unroll
+        for (int kp = 0; kp < 4; kp++) {  // probabilities of 16 positions as the A operand of the second product
+            pa[kp][0] = pack_f16x2(s[2 * kp][0], s[2 * kp][1]);
+            pa[kp][1] = pack_f16x2(s[2 * kp][2], s[2 * kp][3]);
+            pa[kp][2] = pack_f16x2(s[2 * kp + 1][0], s[2 * kp + 1][1]);
+            pa[kp][3] = pack_f16x2(s[2 * kp + 1][2], s[2 * kp + 1][3]);
         }
 #pragma unroll
         for (int kp = 0; kp < 4; kp++)
@@ -208,39 +188,31 @@ __global__ void __launch_bounds__(kApThreads, 2) attn_prefill_mma_kernel(const A
             for (int dp = 0; dp < HD / 16; dp++) {
                 uint32_t b[4];  // dims dp*16 .. +7 (b0, b1) and +8 .. +15 (b2, b3) of positions kp*16 .. +15
                 ap_ldm4t(vb + ap_off<HD>(kp * 16 + (lane & 15), 2 * dp + (lane >> 4)), b);
-#pragma unroll
-                for (int mt = 0; mt < 2; mt++) {
-                    mma_f16_16816(o[mt][2 * dp], pa[mt][kp], b[0], b[1]);
-                    mma_f16_16816(o[mt][2 * dp + 1], pa[mt][kp], b[2], b[3]);
-                }
+                mma_f16_16816(o[2 * dp], pa[kp], b[0], b[1]);
+                mma_f16_16816(o[2 * dp + 1], pa[kp], b[2], b[3]);
             }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
-    for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-        for (int hh = 0; hh < 2; hh++) {
-            l[mt][hh] += __shfl_xor_sync(0xffffffffu, l[mt][hh], 1);
-            l[mt][hh] += __shfl_xor_sync(0xffffffffu, l[mt][hh], 2);
-        }
+    for (int hh = 0; hh < 2; hh++) {
+        l[hh] += __shfl_xor_sync(0xffffffffu, l[hh], 1);
+        l[hh] += __shfl_xor_sync(0xffffffffu, l[hh], 2);
+    }
     __syncthreads();  // the staged tiles are no longer read: the buffers are free
 
     if (csize == 1) {
-        // rows through shared memory (each warp its own 32) so that they leave in 16-byte pieces
+        // rows through shared memory (each warp its own 16) so that they leave in 16-byte pieces
 #pragma unroll
-        for (int mt = 0; mt < 2; mt++)
+        for (int hh = 0; hh < 2; hh++) {
+            const int r = warp * 16 + hh * 8 + g;
+            const float inv = l[hh] > 0.0f ? 1.0f / l[hh] : 0.0f;
 #pragma unroll
-            for (int hh = 0; hh < 2; hh++) {
-                const int r = warp * 32 + mt * 16 + hh * 8 + g;
-                const float inv = l[mt][hh] > 0.0f ? 1.0f / l[mt][hh] : 0.0f;
-#pragma unroll
-                for (int j = 0; j < CH; j++)
-                    *reinterpret_cast<uint32_t*>(ap_raw + ap_off<HD>(r, j) + 4 * t) =
-                        pack_f16x2(o[mt][j][2 * hh] * inv, o[mt][j][2 * hh + 1] * inv);
-            }
+            for (int j = 0; j < CH; j++)
+                *reinterpret_cast<uint32_t*>(ap_raw + ap_off<HD>(r, j) + 4 * t) = pack_f16x2(o[j][2 * hh] * inv, o[j][2 * hh + 1] * inv);
+        }
         __syncwarp();
-        for (int id = lane; id < 32 * CH; id += 32) {
-            const int r = warp * 32 + id / CH, c = id % CH;
+        for (int id = lane; id < 16 * CH; id += 32) {
+            const int r = warp * 16 + id / CH, c = id % CH;
             if (r < nrows) {
                 const int pr = r / groups, h = r - pr * groups;
                 *reinterpret_cast<uint4*>(p.out + static_cast<long long>(pos0 + pr) * p.row_stride + (h0 + h) * HD + c * 8) =
@@ -255,40 +227,77 @@ __global__ void __launch_bounds__(kApThreads, 2) attn_prefill_mma_kernel(const A
     float* pm = part + kApRows * PR;
     float* pl = pm + kApRows;
 #pragma unroll
-    for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-        for (int hh = 0; hh < 2; hh++) {
-            const int r = warp * 32 + mt * 16 + hh * 8 + g;
-            if (t == 0) {
-                pm[r] = m[mt][hh];
-                pl[r] = l[mt][hh];
-            }
-#pragma unroll
-            for (int j = 0; j < CH; j++)
-                *reinterpret_cast<float2*>(part + r * PR + j * 8 + 2 * t) = make_float2(o[mt][j][2 * hh], o[mt][j][2 * hh + 1]);
+    for (int hh = 0; hh < 2; hh++) {
+        const int r = warp * 16 + hh * 8 + g;
+        if (t == 0) {
+            pm[r] = m[hh];
+            pl[r] = l[hh];
         }
+#pragma unroll
+        for (int j = 0; j < CH; j++)
+            *reinterpret_cast<float2*>(part + r * PR + j * 8 + 2 * t) = make_float2(o[j][2 * hh], o[j][2 * hh + 1]);
+    }
     cluster.sync();
-    const int rows_per = kApRows / csize;
-    for (int id = tid; id < rows_per * (HD / 4); id += kApThreads) {
-        const int r = rank * rows_per + id / (HD / 4), c = id % (HD / 4);
-        if (r >= nrows) continue;
-        float mm = -1e30f;
-        for (int k = 0; k < csize; k++) mm = fmaxf(mm, cluster.map_shared_rank(pm, k)[r]);
-        float ss = 0.0f;
-        float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        for (int k = 0; k < csize; k++) {  // ranks in ascending order
-            const float w = ap_exp2(cluster.map_shared_rank(pm, k)[r] - mm);
-            ss = fmaf(cluster.map_shared_rank(pl, k)[r], w, ss);
-            const float4 v = *reinterpret_cast<const float4*>(cluster.map_shared_rank(part, k) + r * PR + c * 4);
-            a.x = fmaf(v.x, w, a.x);
-            a.y = fmaf(v.y, w, a.y);
-            a.z = fmaf(v.z, w, a.z);
-            a.w = fmaf(v.w, w, a.w);
-        }
+    // This CTA's share of the rows: first the weights of the ranks' partials, then the sums with the loads of all ranks and of
+    // several pieces on their way together.  One dependent remote load after the other, this took 10 us.
+    float* pw = pl + kApRows;  // [8][kApRows]
+    const int rows_per = kApRows / csize, r0 = rank * rows_per;
+    const int rows_here = min(rows_per, nrows - r0);
+    for (int r = r0 + tid; r < r0 + rows_here; r += kApThreads) {
+        float mk[8], lk[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (k < csize) {
+                mk[k] = cluster.map_shared_rank(pm, k)[r];
+                lk[k] = cluster.map_shared_rank(pl, k)[r];
+            }
+        float mm = -1e30f, ss = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (k < csize) mm = fmaxf(mm, mk[k]);
+#pragma unroll
+        for (int k = 0; k < 8; k++)  // ranks in ascending order
+            if (k < csize) {
+                mk[k] = ap_exp2(mk[k] - mm);
+                ss = fmaf(lk[k], mk[k], ss);
+            }
         const float inv = ss > 0.0f ? 1.0f / ss : 0.0f;
-        const int pr = r / groups, h = r - pr * groups;
-        *reinterpret_cast<uint2*>(p.out + static_cast<long long>(pos0 + pr) * p.row_stride + (h0 + h) * HD + c * 4) =
-            make_uint2(pack_f16x2(a.x * inv, a.y * inv), pack_f16x2(a.z * inv, a.w * inv));
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (k < csize) pw[k * kApRows + r] = mk[k] * inv;
+    }
+    __syncthreads();
+    constexpr int kFly = 2;  // pieces of four dims a thread has under way
+    for (int id0 = tid; id0 < rows_here * (HD / 4); id0 += kFly * kApThreads) {
+        float4 v[kFly][8];
+#pragma unroll
+        for (int f = 0; f < kFly; f++) {
+            const int id = id0 + f * kApThreads, r = r0 + id / (HD / 4), c = id % (HD / 4);
+            if (id < rows_here * (HD / 4)) {
+#pragma unroll
+                for (int k = 0; k < 8; k++)
+                    if (k < csize) v[f][k] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(part, k) + r * PR + c * 4);
+            }
+        }
+#pragma unroll
+        for (int f = 0; f < kFly; f++) {
+            const int id = id0 + f * kApThreads, r = r0 + id / (HD / 4), c = id % (HD / 4);
+            if (id < rows_here * (HD / 4)) {
+                float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+                for (int k = 0; k < 8; k++)  // ranks in ascending order
+                    if (k < csize) {
+                        const float w = pw[k * kApRows + r];
+                        a.x = fmaf(v[f][k].x, w, a.x);
+                        a.y = fmaf(v[f][k].y, w, a.y);
+                        a.z = fmaf(v[f][k].z, w, a.z);
+                        a.w = fmaf(v[f][k].w, w, a.w);
+                    }
+                const int pr = r / groups, h = r - pr * groups;
+                *reinterpret_cast<uint2*>(p.out + static_cast<long long>(pos0 + pr) * p.row_stride + (h0 + h) * HD + c * 4) =
+                    make_uint2(pack_f16x2(a.x, a.y), pack_f16x2(a.z, a.w));
+            }
+        }
     }
     cluster.sync();  // nobody leaves while its shared memory is read
 }
@@ -300,10 +309,10 @@ template <int HD> static cudaError_t launch_ap(const AttnParams& p, cudaStream_t
     const int PT = kApRows / groups;
     const int tiles = (p.rows + PT - 1) / PT;
     const int nkt = (p.seq_len - 1 + p.rows + kApKeys - 1) / kApKeys;
-    // Split the positions of a tile while the larger grid still fits two CTAs per SM (what shared memory allows) and
-    // every CTA keeps two steps: more CTAs than that only add merging.
+    // Split the positions of a tile while the larger grid still fits two CTAs per SM and it pays: a step of 64 positions takes
+    // about 1.2 us, merging two to four CTAs 2.5 us, eight another one or two.
     int csize = 1;
-    while (csize < 8 && static_cast<long long>(tiles) * p.num_kv_heads * csize * 2 <= 2 * sm_count() && nkt >= 4 * csize) csize *= 2;
+    while (csize < 8 && static_cast<long long>(tiles) * p.num_kv_heads * csize * 2 <= 2 * sm_count() && nkt >= max(8, 4 * csize)) csize *= 2;
     cudaLaunchConfig_t cfg = {};
     cfg.dynamicSmemBytes = smem;
     cfg.gridDim = dim3(tiles * csize, p.num_kv_heads);

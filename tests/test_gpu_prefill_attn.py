@@ -1,5 +1,5 @@
 """GPU: the tiled causal attention of a block of new positions against an f64 softmax over the same 16-bit inputs, at
-the edges of its tiles (128 query rows, 64 positions per step) and with the positions of a tile split over a cluster."""
+the edges of its tiles (64 query rows, 64 positions per step) and with the positions of a tile split over a cluster."""
 import pytest
 
 from helpers import dev
@@ -8,14 +8,17 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("nh,nkv,hd,S,start", [
-    (32, 8, 128, 32, 32),    # one full tile of 32 positions x 4 heads per KV head, 64 positions in all: one step
-    (32, 8, 128, 33, 31),    # one row more than a tile
-    (24, 8, 128, 43, 0),     # 3 heads per KV head: 42 positions (126 rows) per tile, one position in the second
-    (24, 8, 128, 8, 1013),   # few rows behind a long prefix: eight CTAs share the positions, the last one has fewer
+    (32, 8, 128, 32, 32),    # 32 positions x 4 heads per KV head, 64 positions in all
+    (32, 8, 128, 33, 31),    # one position more than two tiles
+    (24, 8, 128, 43, 0),     # 3 heads per KV head: 21 positions (63 rows) per tile, one position in the third
+    (24, 8, 128, 8, 1013),   # few rows behind a longer prefix
     (8, 8, 64, 129, 64),     # one head per KV head, a tile of a single row
     (5, 1, 64, 70, 250),     # odd group
     (16, 1, 128, 64, 5),     # more heads per KV head than the decode kernels take
     (64, 2, 128, 300, 700),  # several tiles, split in two or four
+    (32, 8, 128, 38, 2050),  # three tiles per KV head, the last of six positions, four CTAs each
+    (32, 8, 128, 16, 500),   # a short block: the streaming kernel, row by row
+    (32, 8, 128, 33, 3000),  # few rows, but too much K/V to read row by row
 ])
 def test_tiled_causal_attention(cuda, orc, nh, nkv, hd, S, start):
     from nve_b200 import cuda_kernels as ck
