@@ -41,6 +41,8 @@ static int run_gemm_multi(const void* X, int x_dtype, const PairMat* mats, int n
     unsigned char* sp = static_cast<unsigned char*>(scratch);
     const uint16_t* x = static_cast<const uint16_t*>(X);
     if (x_dtype == NVE_DT_BF16) {
+        int status;  // few rows: converted on the way into shared memory
+        if (aligned(sp, 16) && gemm_rows_try(X, x_dtype, mats, num_mats, y_dtype, M, K, sp, scratch_bytes, st, PairFinish(), &status)) return status;
         const size_t xb = x16_region_bytes(M, K);
         if (sp == nullptr || scratch_bytes < xb) return set_status(NVE_ERR_TOO_LARGE);
         if (!aligned(sp, 16)) return set_status(NVE_ERR_BAD_ALIGNMENT);
@@ -74,7 +76,7 @@ extern "C" size_t nve_b200_gemm_w4a16_multi_scratch_bytes(int M, const int* Ns, 
     if (M <= 0 || K <= 0 || (K % kKBlock) != 0 || Ns == nullptr || num_mats < 1 || num_mats > 3) return 0;
     for (int m = 0; m < num_mats; m++)
         if (Ns[m] <= 0) return 0;
-    return x16_region_bytes(M, K) + pair_plan(Ns, num_mats, M, K, true, ~static_cast<size_t>(0)).partial_bytes;
+    return x16_region_bytes(M, K) + gemm_partial_bytes(Ns, num_mats, M, K);
 }
 
 extern "C" size_t nve_b200_gemm_w4a16_scratch_bytes(int M, int N, int K) { return nve_b200_gemm_w4a16_multi_scratch_bytes(M, &N, 1, K); }

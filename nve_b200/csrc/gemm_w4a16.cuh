@@ -81,8 +81,18 @@ struct PairFinish {
     bool silu = false;                 // two matrices of the same N: Y of the first = silu(first product) * second product
 };
 PairPlan pair_plan(const int* Ns, int num_mats, int M, int K, bool have_scratch, size_t avail, bool silu = false);
+// Workspace that a call of these sizes can use, whichever kernel takes it
+size_t rows_partial_bytes(const int* Ns, int num_mats, int M, int K, bool silu);
+inline size_t gemm_partial_bytes(const int* Ns, int num_mats, int M, int K, bool silu = false) {
+    const size_t a = pair_plan(Ns, num_mats, M, K, true, ~static_cast<size_t>(0), silu).partial_bytes, b = rows_partial_bytes(Ns, num_mats, M, K, silu);
+    return a > b ? a : b;
+}
 int gemm_pair(const uint16_t* X, const PairMat* mats, int num_mats, int y_dtype, int M, int K, void* partial, size_t avail, cudaStream_t st,
               const PairFinish& fin = PairFinish());
+// The kernel for few rows (gemm_w4a16_rows.cuh), X in f16 or bf16; false: not its sizes, or a workspace too small, and nothing was
+// launched.  gemm_pair asks it first.
+bool gemm_rows_try(const void* X, int x_dtype, const PairMat* mats, int num_mats, int y_dtype, int M, int K, void* partial, size_t avail,
+                   cudaStream_t st, const PairFinish& fin, int* status);
 bool pair_norm_fits(int N);
 int gemm_pair_error(bool reset);
 

@@ -29,6 +29,8 @@
 // (nve_b200_gemm_error) and both CTAs leave through the normal path.
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "act_ops.cuh"
 #include "gemm_w4a16.cuh"
 
@@ -69,6 +71,7 @@ struct PairParams {
     int total;       // units
     int sc16;        // 1: rows of scales are 16-byte aligned
     int y2;          // 1: an output is not 4-byte aligned
+    int by_tile;     // 1: every segment is in the workspace, that of (run, tile) in slot run + tile (the kernel for few rows)
     const uint16_t* res;  // kPairAdd: [M, N] f16, added to the rounded product
 };
 // What happens to the product on its way out
@@ -637,16 +640,27 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 // Sum of four consecutive columns of row mm of a tile over the pairs that worked on it, in ascending K order.
 __device__ __forceinline__ float4 pair_sum4(const PairParams& p, int tile, int first, int last, int mm, int col) {
     auto part = [&](int c) {
-        const int slot = 2 * c + (c * p.U >= tile * p.SB ? 0 : 1);  // the pair's first segment when its run starts inside this tile
+        // by pair: its first segment when its run starts inside this tile
+        const int slot = p.by_tile ? c + tile : 2 * c + (c * p.U >= tile * p.SB ? 0 : 1);
         return __ldcg(reinterpret_cast<const float4*>(p.partial + (static_cast<long long>(slot) * p.part_rows + mm) * kPairTile + col));
     };
+    // Eight loads on their way at a time: one after the other each cost an L2 round trip, and that was most of the call for a row
+    // or two of tiles cut into a dozen segments.
+    constexpr int kFly = 8;
     float4 y = part(first);
-    for (int c = first + 1; c <= last; c++) {
-        const float4 v = part(c);
-        y.x = __fadd_rn(y.x, v.x);
-        y.y = __fadd_rn(y.y, v.y);
-        y.z = __fadd_rn(y.z, v.z);
-        y.w = __fadd_rn(y.w, v.w);
+    for (int c = first + 1; c <= last; c += kFly) {
+        float4 v[kFly];
+#pragma unroll
+        for (int i = 0; i < kFly; i++)
+            if (c + i <= last) v[i] = part(c + i);
+#pragma unroll
+        for (int i = 0; i < kFly; i++)
+            if (c + i <= last) {
+                y.x = __fadd_rn(y.x, v[i].x);
+                y.y = __fadd_rn(y.y, v[i].y);
+                y.z = __fadd_rn(y.z, v[i].z);
+                y.w = __fadd_rn(y.w, v[i].w);
+            }
     }
     return y;
 }
@@ -658,7 +672,7 @@ template <int ODT, int MODE> __global__ void __launch_bounds__(256) gemm_pair_re
     pdl_launch_dependents();
     const int tile = blockIdx.x;
     const int first = (tile * p.SB) / p.U, last = ((tile + 1) * p.SB - 1) / p.U;
-    if (first == last) return;
+    if (first == last && !p.by_tile) return;
     const PairTile tl = pair_locate<MODE>(p, tile);
     const int Nloc = p.Nm[tl.mi];
     const int c4 = static_cast<int>(threadIdx.x) * 4, n = tl.n0 + c4;
@@ -689,64 +703,79 @@ template <int ODT, int MODE> __global__ void __launch_bounds__(256) gemm_pair_re
 
 // The same for one matrix whose product goes through the residual add and an RMSNorm: one block per row of X finishes
 // the row -- Y = res + round16(product), normed = RMSNorm(Y) -- with the arithmetic and the summation order of the separate
-// kernels (thread t takes the 8-element chunks t, t + 256, ...).  Tiles that one pair covered are in Y already.
+// kernels (of 256 threads, thread t takes the 8-element chunks t, t + 256, ...).  Tiles that one pair covered are in Y already.
+// The sums over segments are spread over all THREADS, four columns each: with few rows of X they are a chain of L2 round trips.
 constexpr int kPairNormChunks = 4;  // 8-element chunks per thread: N <= 8192
-__global__ void __launch_bounds__(256) gemm_pair_reduce_norm_kernel(const PairParams p, const uint16_t* norm_w, uint16_t* normed, float eps) {
+template <int THREADS> __global__ void __launch_bounds__(THREADS) gemm_pair_reduce_norm_kernel(const PairParams p, const uint16_t* norm_w, uint16_t* normed, float eps) {
     __shared__ float warp_part[8];
+    __shared__ uint2 row16[8 * 256 * kPairNormChunks / 4];  // Y of the row
     const int m = blockIdx.x, N = p.Nm[0], chunks = N >> 3;
     const int xt = m / p.NB, mm = m - xt * p.NB;
     const long long row = static_cast<long long>(m) * N;
-    uint4 w[kPairNormChunks], rs[kPairNormChunks], h[kPairNormChunks];
+    const int tid = static_cast<int>(threadIdx.x);
+    uint4 w[kPairNormChunks];
+    if (tid < 256) {
 #pragma unroll
-    for (int j = 0; j < kPairNormChunks; j++) {
-        const int c = j * 256 + static_cast<int>(threadIdx.x);
-        if (c < chunks) w[j] = reinterpret_cast<const uint4*>(norm_w)[c];  // static, unlike what follows
+        for (int j = 0; j < kPairNormChunks; j++) {
+            const int c = j * 256 + tid;
+            if (c < chunks) w[j] = reinterpret_cast<const uint4*>(norm_w)[c];  // static, unlike what follows
+        }
     }
     pdl_wait();
     pdl_launch_dependents();
     uint16_t* y16 = static_cast<uint16_t*>(p.Y[0]);
-#pragma unroll
-    for (int j = 0; j < kPairNormChunks; j++) {
-        const int c = j * 256 + static_cast<int>(threadIdx.x);
-        if (c < chunks) rs[j] = reinterpret_cast<const uint4*>(p.res + row)[c];
-    }
-    float acc = 0.0f;
-#pragma unroll
-    for (int j = 0; j < kPairNormChunks; j++) {
-        const int c = j * 256 + static_cast<int>(threadIdx.x);
-        if (c < chunks) {
-            const int wt = c >> 5, col = (c & 31) * 8, tile = wt * p.XT + xt;
-            const int first = (tile * p.SB) / p.U, last = ((tile + 1) * p.SB - 1) / p.U;
-            uint16_t a[8], b[8];
-            if (first == last) {
-                unpack8(__ldcg(reinterpret_cast<const uint4*>(y16 + row) + c), a);
-            } else {
-                const float4 lo = pair_sum4(p, tile, first, last, mm, col), hi = pair_sum4(p, tile, first, last, mm, col + 4);
-                const float f[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-#pragma unroll
-                for (int e = 0; e < 8; e++) a[e] = Act16<NVE_DT_F16>::from_f32(f[e]);
-            }
-            unpack8(rs[j], b);
-#pragma unroll
-            for (int e = 0; e < 8; e++) {
-                a[e] = Act16<NVE_DT_F16>::from_f32(__fadd_rn(Act16<NVE_DT_F16>::to_f32(a[e]), Act16<NVE_DT_F16>::to_f32(b[e])));
-                const float v = Act16<NVE_DT_F16>::to_f32(a[e]);
-                acc = __fmaf_rn(v, v, acc);
-            }
-            h[j] = pack8(a);
-            reinterpret_cast<uint4*>(y16 + row)[c] = h[j];
+    for (int q = tid; q < (N >> 2); q += THREADS) {
+        const int wt = q >> 6, col = (q & 63) * 4, tile = wt * p.XT + xt;
+        const int first = (tile * p.SB) / p.U, last = ((tile + 1) * p.SB - 1) / p.U;
+        const uint2 r2 = reinterpret_cast<const uint2*>(p.res + row)[q];
+        uint2 y2;
+        if (first == last && !p.by_tile) {
+            y2 = __ldcg(reinterpret_cast<const uint2*>(y16 + row) + q);
+        } else {
+            const float4 f = pair_sum4(p, tile, first, last, mm, col);
+            y2.x = static_cast<uint32_t>(Act16<NVE_DT_F16>::from_f32(f.x)) | (static_cast<uint32_t>(Act16<NVE_DT_F16>::from_f32(f.y)) << 16);
+            y2.y = static_cast<uint32_t>(Act16<NVE_DT_F16>::from_f32(f.z)) | (static_cast<uint32_t>(Act16<NVE_DT_F16>::from_f32(f.w)) << 16);
         }
+        auto add = [](uint32_t a, uint32_t b) {
+            auto one = [](uint16_t u, uint16_t v) { return Act16<NVE_DT_F16>::from_f32(__fadd_rn(Act16<NVE_DT_F16>::to_f32(u), Act16<NVE_DT_F16>::to_f32(v))); };
+            return static_cast<uint32_t>(one(static_cast<uint16_t>(a), static_cast<uint16_t>(b))) |
+                   (static_cast<uint32_t>(one(static_cast<uint16_t>(a >> 16), static_cast<uint16_t>(b >> 16))) << 16);
+        };
+        y2 = make_uint2(add(y2.x, r2.x), add(y2.y, r2.y));
+        reinterpret_cast<uint2*>(y16 + row)[q] = y2;
+        row16[q] = y2;
     }
-    acc = warp_sum(acc);
-    if ((threadIdx.x & 31) == 0) warp_part[threadIdx.x >> 5] = acc;
     __syncthreads();
+    uint4 h[kPairNormChunks];
+    if (tid < 256) {
+        float acc = 0.0f;
+#pragma unroll
+        for (int j = 0; j < kPairNormChunks; j++) {
+            const int c = j * 256 + tid;
+            if (c < chunks) {
+                const uint2 lo = row16[2 * c], hi = row16[2 * c + 1];
+                h[j] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+                uint16_t a[8];
+                unpack8(h[j], a);
+#pragma unroll
+                for (int e = 0; e < 8; e++) {
+                    const float v = Act16<NVE_DT_F16>::to_f32(a[e]);
+                    acc = __fmaf_rn(v, v, acc);
+                }
+            }
+        }
+        acc = warp_sum(acc);
+        if ((tid & 31) == 0) warp_part[tid >> 5] = acc;
+    }
+    __syncthreads();
+    if (tid >= 256) return;
     float total = warp_part[0];
 #pragma unroll
     for (int i = 1; i < 8; i++) total = __fadd_rn(total, warp_part[i]);
     const float r = __frcp_rn(__fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(N)), eps)));
 #pragma unroll
     for (int j = 0; j < kPairNormChunks; j++) {
-        const int c = j * 256 + static_cast<int>(threadIdx.x);
+        const int c = j * 256 + tid;
         if (c < chunks) {
             uint16_t a[8], b[8];
             unpack8(h[j], a);
@@ -758,6 +787,10 @@ __global__ void __launch_bounds__(256) gemm_pair_reduce_norm_kernel(const PairPa
         }
     }
 }
+
+}  // namespace nve
+#include "gemm_w4a16_rows.cuh"
+namespace nve {
 
 using PairEncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -820,6 +853,35 @@ PairPlan pair_plan(const int* Ns, int num_mats, int M, int K, bool have_scratch,
     return g;
 }
 
+// What a GEMM kernel left to be finished: tiles in several segments, or a row that goes through a norm.
+template <int ODT, int MODE> static int launch_finish(const PairParams& p, unsigned tiles, const PairFinish& fin, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    if (pdl_enabled()) {
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    cudaError_t e = cudaSuccess;
+    if (fin.norm_w != nullptr) {
+        cfg.gridDim = dim3(static_cast<unsigned>(p.M));
+        // one block per SM or less: every thread four columns; more: the blocks hide each other's latency
+        const bool wide = p.M <= sm_count();
+        cfg.blockDim = dim3(wide ? 1024 : 256);
+        e = cudaLaunchKernelEx(&cfg, wide ? gemm_pair_reduce_norm_kernel<1024> : gemm_pair_reduce_norm_kernel<256>, p, fin.norm_w, fin.normed, fin.eps);
+        count_launch();
+    } else if (p.by_tile || p.U % p.SB != 0) {
+        cfg.gridDim = dim3(tiles, static_cast<unsigned>((p.part_rows + 3) / 4));
+        cfg.blockDim = dim3(MODE == kPairSilu ? kPairTile / 8 : kPairTile / 4, MODE == kPairSilu ? 8 : 4);
+        if (MODE == kPairSilu) cfg.gridDim.y = static_cast<unsigned>((p.part_rows + 7) / 8);
+        e = cudaLaunchKernelEx(&cfg, gemm_pair_reduce_kernel<ODT, MODE>, p);
+        count_launch();
+    }
+    return set_cuda_status(e);
+}
+
 template <int ODT, int MODE>
 static int launch_pair(const PairParams& p, const PairPlan& g, const CUtensorMap& xmap, int smem, const PairFinish& fin, cudaStream_t st) {
     auto kern = gemm_w4a16_pair_kernel<ODT, MODE>;
@@ -836,34 +898,14 @@ static int launch_pair(const PairParams& p, const PairPlan& g, const CUtensorMap
         cfg.attrs = attr;
         cfg.numAttrs = 1;
     }
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p, xmap);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p, xmap);
     count_launch();
     if (e != cudaSuccess) return set_cuda_status(e);
-    cfg.dynamicSmemBytes = 0;
-    if (fin.norm_w != nullptr) {
-        cfg.gridDim = dim3(static_cast<unsigned>(p.M));
-        cfg.blockDim = dim3(256);
-        e = cudaLaunchKernelEx(&cfg, gemm_pair_reduce_norm_kernel, p, fin.norm_w, fin.normed, fin.eps);
-        count_launch();
-    } else if (p.U % p.SB != 0) {
-        cfg.gridDim = dim3(static_cast<unsigned>(g.tiles), static_cast<unsigned>((p.part_rows + 3) / 4));
-        cfg.blockDim = dim3(MODE == kPairSilu ? kPairTile / 8 : kPairTile / 4, MODE == kPairSilu ? 8 : 4);
-        if (MODE == kPairSilu) cfg.gridDim.y = static_cast<unsigned>((p.part_rows + 7) / 8);
-        e = cudaLaunchKernelEx(&cfg, gemm_pair_reduce_kernel<ODT, MODE>, p);
-        count_launch();
-    }
-    return set_cuda_status(e);
+    return launch_finish<ODT, MODE>(p, static_cast<unsigned>(g.tiles), fin, st);
 }
 
-int gemm_pair(const uint16_t* X, const PairMat* mats, int num_mats, int y_dtype, int M, int K, void* partial, size_t avail, cudaStream_t st,
-              const PairFinish& fin) {
-    PairParams p = {};
-    int Ns[3] = {0, 0, 0};
-    for (int i = 0; i < num_mats; i++) Ns[i] = mats[i].N;
-    const PairPlan g = pair_plan(Ns, num_mats, M, K, partial != nullptr, avail, fin.silu);
-    if (g.tiles * g.SB > 0x3FFFFFFFll) return set_status(NVE_ERR_BAD_SHAPE);
-    CUtensorMap xmap;
-    if (!pair_x_map(&xmap, X, K, M, g.NB / 2)) return set_status(NVE_ERR_CUDA);
+// Outputs and matrices of a call, common to the kernels
+static void set_matrices(PairParams& p, const PairMat* mats, int num_mats, int M, int K, void* partial, const PairFinish& fin) {
     int wt = 0;
     p.sc16 = (K % 128) == 0;
     const int rows = fin.silu ? kPairTile / 2 : kPairTile;
@@ -884,6 +926,57 @@ int gemm_pair(const uint16_t* X, const PairMat* mats, int num_mats, int y_dtype,
     p.M = M;
     p.K = K;
     p.nb = K / 32;
+}
+// f(ODT, MODE) of a call
+template <typename F> static int by_finish(const PairFinish& fin, int y_dtype, F f) {
+    using std::integral_constant;
+    const integral_constant<int, kPairPlain> plain;
+    if (fin.silu) return f(integral_constant<int, NVE_DT_F16>(), integral_constant<int, kPairSilu>());
+    if (fin.norm_w != nullptr) return f(integral_constant<int, NVE_DT_F16>(), plain);  // the add is in the second kernel
+    if (fin.res != nullptr) return f(integral_constant<int, NVE_DT_F16>(), integral_constant<int, kPairAdd>());
+    if (y_dtype == NVE_DT_F32) return f(integral_constant<int, NVE_DT_F32>(), plain);
+    if (y_dtype == NVE_DT_F16) return f(integral_constant<int, NVE_DT_F16>(), plain);
+    return f(integral_constant<int, NVE_DT_BF16>(), plain);
+}
+
+size_t rows_partial_bytes(const int* Ns, int num_mats, int M, int K, bool silu) { return rows_plan(Ns, num_mats, M, K, silu).partial_bytes; }
+
+bool gemm_rows_try(const void* X, int x_dtype, const PairMat* mats, int num_mats, int y_dtype, int M, int K, void* partial, size_t avail,
+                   cudaStream_t st, const PairFinish& fin, int* status) {
+    int Ns[3] = {0, 0, 0};
+    for (int i = 0; i < num_mats; i++) Ns[i] = mats[i].N;
+    const RowsPlan r = rows_plan(Ns, num_mats, M, K, fin.silu);
+    if (r.grid == 0 || partial == nullptr || r.partial_bytes > avail) return false;
+    PairParams p = {};
+    set_matrices(p, mats, num_mats, M, K, partial, fin);
+    p.NB = p.part_rows = M;
+    p.XT = 1;
+    p.SB = r.SB;
+    p.U = r.U;
+    p.total = r.total;
+    p.by_tile = 1;
+    const uint16_t* x = static_cast<const uint16_t*>(X);
+    int s;
+    if (fin.silu) s = launch_rows<NVE_DT_F16, true>(p, r, x, st);
+    else s = x_dtype == NVE_DT_F16 ? launch_rows<NVE_DT_F16, false>(p, r, x, st) : launch_rows<NVE_DT_BF16, false>(p, r, x, st);
+    if (s == NVE_OK)
+        s = by_finish(fin, y_dtype, [&](auto odt, auto mode) { return launch_finish<odt.value, mode.value>(p, static_cast<unsigned>(r.tiles), fin, st); });
+    *status = s;
+    return true;
+}
+
+int gemm_pair(const uint16_t* X, const PairMat* mats, int num_mats, int y_dtype, int M, int K, void* partial, size_t avail, cudaStream_t st,
+              const PairFinish& fin) {
+    int status;
+    if (gemm_rows_try(X, NVE_DT_F16, mats, num_mats, y_dtype, M, K, partial, avail, st, fin, &status)) return status;
+    PairParams p = {};
+    int Ns[3] = {0, 0, 0};
+    for (int i = 0; i < num_mats; i++) Ns[i] = mats[i].N;
+    const PairPlan g = pair_plan(Ns, num_mats, M, K, partial != nullptr, avail, fin.silu);
+    if (g.tiles * g.SB > 0x3FFFFFFFll) return set_status(NVE_ERR_BAD_SHAPE);
+    CUtensorMap xmap;
+    if (!pair_x_map(&xmap, X, K, M, g.NB / 2)) return set_status(NVE_ERR_CUDA);
+    set_matrices(p, mats, num_mats, M, K, partial, fin);
     p.NB = g.NB;
     p.part_rows = M < g.NB ? M : g.NB;
     p.XT = g.XT;
@@ -900,12 +993,7 @@ int gemm_pair(const uint16_t* X, const PairMat* mats, int num_mats, int y_dtype,
     p.raw = g.NB > 192 ? 2 : (g.NB > 96 ? 4 : (g.NB > 32 ? 6 : 8));
     p.xslots = min(12, (kPairSmemMax - 1024 - extra - p.raw * kRawBytes) / (p.NB * 128));
     const int smem = 1024 + p.xslots * p.NB * 128 + p.raw * kRawBytes + extra;
-    if (fin.silu) return launch_pair<NVE_DT_F16, kPairSilu>(p, g, xmap, smem, fin, st);
-    if (fin.norm_w != nullptr) return launch_pair<NVE_DT_F16, kPairPlain>(p, g, xmap, smem, fin, st);  // the add is in the second kernel
-    if (fin.res != nullptr) return launch_pair<NVE_DT_F16, kPairAdd>(p, g, xmap, smem, fin, st);
-    if (y_dtype == NVE_DT_F32) return launch_pair<NVE_DT_F32, kPairPlain>(p, g, xmap, smem, fin, st);
-    return y_dtype == NVE_DT_F16 ? launch_pair<NVE_DT_F16, kPairPlain>(p, g, xmap, smem, fin, st)
-                                 : launch_pair<NVE_DT_BF16, kPairPlain>(p, g, xmap, smem, fin, st);
+    return by_finish(fin, y_dtype, [&](auto odt, auto mode) { return launch_pair<odt.value, mode.value>(p, g, xmap, smem, fin, st); });
 }
 
 bool pair_norm_fits(int N) { return (N & 7) == 0 && N <= 8 * 256 * kPairNormChunks; }

@@ -78,10 +78,9 @@ static RowsPlan rows_plan(const nve_b200_rows_layer& L, int S) {
     r.h1 = take(s2 * L.hidden);
     r.mid = take(s2 * L.ffn);
     const int qkv[3] = {static_cast<int>(qd), static_cast<int>(kvd), static_cast<int>(kvd)}, gu[2] = {L.ffn, L.ffn}, one[1] = {L.hidden};
-    const size_t any = ~static_cast<size_t>(0);
-    r.part_bytes = pair_plan(qkv, 3, S, L.hidden, true, any).partial_bytes;
-    for (size_t b : {pair_plan(one, 1, S, static_cast<int>(qd), true, any).partial_bytes, pair_plan(gu, 2, S, L.hidden, true, any, true).partial_bytes,
-                     pair_plan(one, 1, S, L.ffn, true, any).partial_bytes})
+    r.part_bytes = gemm_partial_bytes(qkv, 3, S, L.hidden);
+    for (size_t b : {gemm_partial_bytes(one, 1, S, static_cast<int>(qd)), gemm_partial_bytes(gu, 2, S, L.hidden, true),
+                     gemm_partial_bytes(one, 1, S, L.ffn)})
         if (b > r.part_bytes) r.part_bytes = b;
     r.part = take(r.part_bytes);
     r.total = at;
