@@ -442,11 +442,11 @@ def gemm_batch_table(torch, ck, state, shape, peak):
 
 
 def prefill_entry(torch, ck, state, shape, lengths=(64, 256, 1024)):
-    """A prompt block of S positions through all layers with gpu_layer_forward_prefill: projections through
-    matmul_x (the fused tensor-core GEMM in 64-row slices up to 128 rows, dequantisation + dense GEMM above, as the
-    reference does for every prompt), one-launch RMSNorm rows / KV rows / causal attention.  Eager launches,
-    allocations included: the reference has no graph for prefill either (src/gpu_layer.rs:1086-1160)."""
-    from nve_b200.gpu_layer import DENSE_ROWS, gpu_layer_forward_prefill
+    """A prompt block of S positions through all layers with gpu_layer_forward_prefill: one native
+    call per layer that issues the W4A16 GEMMs with what follows them finished inside, RoPE + K/V write and the causal
+    attention.  Eager launches, allocations included: the reference has no graph for prefill either
+    (src/gpu_layer.rs:1086-1160)."""
+    from nve_b200.gpu_layer import gpu_layer_forward_prefill
 
     layers = len(state.layer_weights)
     res = {}
@@ -464,7 +464,7 @@ def prefill_entry(torch, ck, state, shape, lengths=(64, 256, 1024)):
         finite = bool(torch.isfinite(out.float()).all())
         ms = time_events(torch, run, 3)
         res[str(S)] = {"ms": round(ms, 3), "prompt_tok_s": round(S / (ms * 1e-3), 1), "output_finite": finite,
-                       "projections": "dequantise + dense GEMM" if S > DENSE_ROWS else "fused W4A16 GEMM, 64-row slices"}
+                       "projections": "fused W4A16 GEMM"}
     res["workload"] = f"prompt block of S positions through all {layers} layers (positions 0..S-1, 16-bit route)"
     res["gemm_error"] = ck.gemm_error()
     return res

@@ -398,7 +398,7 @@ NVE_API int nve_b200_gemm_w4a16(const void* X, int x_dtype, const uint8_t* nibbl
                                 int y_dtype, int M, int N, int K, void* scratch, size_t scratch_bytes,
                                 nve_stream_t stream);
 /* The same GEMM over 1..3 matrices that share X (q/k/v, gate/up) in one launch: mats[i].{nibbles, scales, out, N},
- * out [M, N_i] row-major, residual must be NULL.  Their 128-row tiles follow one another in one unit sequence and the
+ * out [M, N_i] row-major, residual must be NULL.  Their 256-row tiles follow one another in one unit sequence and the
  * runs are chosen for the total, which is what lets the narrow k and v projections fill the GPU. */
 NVE_API size_t nve_b200_gemm_w4a16_multi_scratch_bytes(int M, const int* Ns, int num_mats, int K);
 NVE_API int nve_b200_gemm_w4a16_multi(const void* X, int x_dtype, const nve_b200_w4_matrix* mats, int num_mats,

@@ -7,9 +7,9 @@
 // is the limit at NB = 64, and at NB = 256 the tensor pipe is.
 //
 //   step  = 128 elements of K: A slot of 64 TMEM columns, X slot of NB / 2 rows x 256 bytes, one phase of the "full"
-//           (A), "xfull" (X) and "empty" barriers, eight tcgen05.mma (M = 256, N = NB, K = 16).  The X ring is deeper than
+//           (A and X) and "empty" barriers, eight tcgen05.mma (M = 256, N = NB, K = 16).  The X ring is deeper than
 //           the A ring: a slot that waits for a TMA load from L2 (about a microsecond) would set the pace otherwise.
-//   unit  = 2 steps = 256 elements of K: one raw stage (128 rows x 128 nibble bytes by TMA, 128 rows x 8 scales)
+//   unit  = 2 steps = 256 elements of K: one raw stage (128 rows x 128 nibble bytes and 8 scales, by cp.async)
 //   tile  = SB units;  the sequence of all (tile, unit) is dealt out in equal contiguous runs, one per pair
 //
 // Roles (768 threads per CTA):
@@ -23,7 +23,7 @@
 // TMEM: W accumulator sets of NB columns, then the A slots.  X is loaded without multicast.
 //
 // Ring discipline: a parity wait is only meaningful when the waiter knows the barrier's previous phase to be complete.
-// full / empty barriers are indexed by the step modulo kBarRing = 12 (a multiple of the number of dequantiser groups
+// full / empty barriers are indexed by the step modulo kBarRing = 24 (a multiple of the number of dequantiser groups
 // and of issuing warps), raw barriers by the unit modulo an even ring: consecutive phases of a barrier are always
 // awaited by the same threads, in order.  Every wait is bounded in time; an expired one latches an error code
 // (nve_b200_gemm_error) and both CTAs leave through the normal path.
