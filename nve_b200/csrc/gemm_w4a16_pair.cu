@@ -704,9 +704,11 @@ template <int ODT, int MODE> __global__ void __launch_bounds__(256) gemm_pair_re
 // The same for one matrix whose product goes through the residual add and an RMSNorm: one block per row of X finishes
 // the row -- Y = res + round16(product), normed = RMSNorm(Y) -- with the arithmetic and the summation order of the separate
 // kernels (of 256 threads, thread t takes the 8-element chunks t, t + 256, ...).  Tiles that one pair covered are in Y already.
-// The sums over segments are spread over all THREADS, four columns each: with few rows of X they are a chain of L2 round trips.
+// The sums over segments are spread over all threads, four columns each: with few rows of X (at most one block per SM) they are
+// a chain of L2 round trips.
 constexpr int kPairNormChunks = 4;  // 8-element chunks per thread: N <= 8192
-template <int THREADS> __global__ void __launch_bounds__(THREADS) gemm_pair_reduce_norm_kernel(const PairParams p, const uint16_t* norm_w, uint16_t* normed, float eps) {
+constexpr int kPairNormThreads = 1024;
+__global__ void __launch_bounds__(kPairNormThreads) gemm_pair_reduce_norm_kernel(const PairParams p, const uint16_t* norm_w, uint16_t* normed, float eps) {
     __shared__ float warp_part[8];
     __shared__ uint2 row16[8 * 256 * kPairNormChunks / 4];  // Y of the row
     const int m = blockIdx.x, N = p.Nm[0], chunks = N >> 3;
@@ -724,7 +726,7 @@ template <int THREADS> __global__ void __launch_bounds__(THREADS) gemm_pair_redu
     pdl_wait();
     pdl_launch_dependents();
     uint16_t* y16 = static_cast<uint16_t*>(p.Y[0]);
-    for (int q = tid; q < (N >> 2); q += THREADS) {
+    for (int q = tid; q < (N >> 2); q += kPairNormThreads) {
         const int wt = q >> 6, col = (q & 63) * 4, tile = wt * p.XT + xt;
         const int first = (tile * p.SB) / p.U, last = ((tile + 1) * p.SB - 1) / p.U;
         const uint2 r2 = reinterpret_cast<const uint2*>(p.res + row)[q];
@@ -776,6 +778,77 @@ template <int THREADS> __global__ void __launch_bounds__(THREADS) gemm_pair_redu
 #pragma unroll
     for (int j = 0; j < kPairNormChunks; j++) {
         const int c = j * 256 + tid;
+        if (c < chunks) {
+            uint16_t a[8], b[8];
+            unpack8(h[j], a);
+            unpack8(w[j], b);
+#pragma unroll
+            for (int e = 0; e < 8; e++)
+                a[e] = Act16<NVE_DT_F16>::from_f32(__fmul_rn(__fmul_rn(Act16<NVE_DT_F16>::to_f32(a[e]), r), Act16<NVE_DT_F16>::to_f32(b[e])));
+            reinterpret_cast<uint4*>(normed + row)[c] = pack8(a);
+        }
+    }
+}
+
+// More rows of X than SMs: the blocks hide each other's latency and a thread keeps its chunks of the row in registers, all of
+// their loads under way together (o projection with its finish, 8B, 1777 rows: 89.7 us with the form above, 73.8 with this one; 300
+// rows 25.6 and 23.5; at 147 and 149 rows, each with its own form, 15.5 and 16.5).
+__global__ void __launch_bounds__(256) gemm_pair_reduce_norm_rows_kernel(const PairParams p, const uint16_t* norm_w, uint16_t* normed, float eps) {
+    __shared__ float warp_part[8];
+    const int m = blockIdx.x, N = p.Nm[0], chunks = N >> 3;
+    const int xt = m / p.NB, mm = m - xt * p.NB;
+    const long long row = static_cast<long long>(m) * N;
+    uint4 w[kPairNormChunks], rs[kPairNormChunks], h[kPairNormChunks];
+#pragma unroll
+    for (int j = 0; j < kPairNormChunks; j++) {
+        const int c = j * 256 + static_cast<int>(threadIdx.x);
+        if (c < chunks) w[j] = reinterpret_cast<const uint4*>(norm_w)[c];  // static, unlike what follows
+    }
+    pdl_wait();
+    pdl_launch_dependents();
+    uint16_t* y16 = static_cast<uint16_t*>(p.Y[0]);
+#pragma unroll
+    for (int j = 0; j < kPairNormChunks; j++) {
+        const int c = j * 256 + static_cast<int>(threadIdx.x);
+        if (c < chunks) rs[j] = reinterpret_cast<const uint4*>(p.res + row)[c];
+    }
+    float acc = 0.0f;
+#pragma unroll
+    for (int j = 0; j < kPairNormChunks; j++) {
+        const int c = j * 256 + static_cast<int>(threadIdx.x);
+        if (c < chunks) {
+            const int wt = c >> 5, col = (c & 31) * 8, tile = wt * p.XT + xt;
+            const int first = (tile * p.SB) / p.U, last = ((tile + 1) * p.SB - 1) / p.U;
+            uint16_t a[8], b[8];
+            if (first == last && !p.by_tile) {
+                unpack8(__ldcg(reinterpret_cast<const uint4*>(y16 + row) + c), a);
+            } else {
+                const float4 lo = pair_sum4(p, tile, first, last, mm, col), hi = pair_sum4(p, tile, first, last, mm, col + 4);
+                const float f[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+                for (int e = 0; e < 8; e++) a[e] = Act16<NVE_DT_F16>::from_f32(f[e]);
+            }
+            unpack8(rs[j], b);
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+                a[e] = Act16<NVE_DT_F16>::from_f32(__fadd_rn(Act16<NVE_DT_F16>::to_f32(a[e]), Act16<NVE_DT_F16>::to_f32(b[e])));
+                const float v = Act16<NVE_DT_F16>::to_f32(a[e]);
+                acc = __fmaf_rn(v, v, acc);
+            }
+            h[j] = pack8(a);
+            reinterpret_cast<uint4*>(y16 + row)[c] = h[j];
+        }
+    }
+    acc = warp_sum(acc);
+    if ((threadIdx.x & 31) == 0) warp_part[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    float total = warp_part[0];
+#pragma unroll
+    for (int i = 1; i < 8; i++) total = __fadd_rn(total, warp_part[i]);
+    const float r = __frcp_rn(__fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(N)), eps)));
+#pragma unroll
+    for (int j = 0; j < kPairNormChunks; j++) {
+        const int c = j * 256 + static_cast<int>(threadIdx.x);
         if (c < chunks) {
             uint16_t a[8], b[8];
             unpack8(h[j], a);
@@ -867,10 +940,9 @@ template <int ODT, int MODE> static int launch_finish(const PairParams& p, unsig
     cudaError_t e = cudaSuccess;
     if (fin.norm_w != nullptr) {
         cfg.gridDim = dim3(static_cast<unsigned>(p.M));
-        // one block per SM or less: every thread four columns; more: the blocks hide each other's latency
         const bool wide = p.M <= sm_count();
-        cfg.blockDim = dim3(wide ? 1024 : 256);
-        e = cudaLaunchKernelEx(&cfg, wide ? gemm_pair_reduce_norm_kernel<1024> : gemm_pair_reduce_norm_kernel<256>, p, fin.norm_w, fin.normed, fin.eps);
+        cfg.blockDim = dim3(wide ? kPairNormThreads : 256);
+        e = cudaLaunchKernelEx(&cfg, wide ? gemm_pair_reduce_norm_kernel : gemm_pair_reduce_norm_rows_kernel, p, fin.norm_w, fin.normed, fin.eps);
         count_launch();
     } else if (p.by_tile || p.U % p.SB != 0) {
         cfg.gridDim = dim3(tiles, static_cast<unsigned>((p.part_rows + 3) / 4));
