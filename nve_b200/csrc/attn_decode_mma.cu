@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kAmThreads, 1) attn_decode_mma_kernel(const At
     for (int p0 = t_begin + warp * 16; p0 < t_end; p0 += kAmWarps * 16) {
         if (!have) am_load_tile<HD>(kh, vh, p0, t_end - 1, g, t, kr, vr);
         have = false;
-        if (pos_ok) am_patch_tile<HD>(sh.knew_s, sh.vnew_s, p0, pos, g, t, kr, vr);
+        if (pos_ok) am_patch_tile<HD>(sh.knew_s, sh.vnew_s, p0, t_end - 1, pos, g, t, kr, vr);
         am_tile<HD>(qa, kr, vr, p0, t_end, p.scale, t, m, l, o);
     }
 

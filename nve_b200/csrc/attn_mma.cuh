@@ -58,20 +58,21 @@ template <int HD> __device__ __forceinline__ void am_load_tile(const uint16_t* k
 }
 
 // Rows of the tile that are position `pos` take the new token's k / v (f16, in shared memory) instead of what was
-// loaded from the cache.
-template <int HD> __device__ __forceinline__ void am_patch_tile(const uint16_t* knew_s, const uint16_t* vnew_s, int p0, int pos, int g, int t,
+// loaded from the cache; so do the rows beyond `last` that repeat it: their weight is zero, which a NaN of a cache row that was
+// never written would survive.
+template <int HD> __device__ __forceinline__ void am_patch_tile(const uint16_t* knew_s, const uint16_t* vnew_s, int p0, int last, int pos, int g, int t,
                                                               uint4 (&kr)[2][HD / 32], uint4 (&vr)[4][HD / 64]) {
     constexpr int DPT = HD / 4, KQ = DPT / 8, NT = HD / 8, VQ = NT / 8;
     if (pos < p0 || pos >= p0 + 16) return;
 #pragma unroll
     for (int r = 0; r < 2; r++)
-        if (p0 + 8 * r + g == pos) {
+        if (min(p0 + 8 * r + g, last) == pos) {
 #pragma unroll
             for (int i = 0; i < KQ; i++) kr[r][i] = *reinterpret_cast<const uint4*>(knew_s + DPT * t + 8 * i);
         }
 #pragma unroll
     for (int r = 0; r < 4; r++)
-        if (p0 + 2 * t + (r & 1) + 8 * (r >> 1) == pos) {
+        if (min(p0 + 2 * t + (r & 1) + 8 * (r >> 1), last) == pos) {
 #pragma unroll
             for (int i = 0; i < VQ; i++) vr[r][i] = *reinterpret_cast<const uint4*>(vnew_s + NT * g + 8 * i);
         }

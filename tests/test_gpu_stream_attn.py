@@ -58,3 +58,36 @@ def test_streaming_decode_attention(cuda, orc, nh, nkv, hd, max_seq, lens):
         assert (one.view(-1).double() - want).abs().max().item() < bound
     assert torch.equal(torch.nan_to_num(kc, nan=77.0), torch.nan_to_num(kc0, nan=77.0))
     assert torch.equal(torch.nan_to_num(vc, nan=77.0), torch.nan_to_num(vc0, nan=77.0))
+
+
+@pytest.mark.parametrize("cuda_core", [False, True])
+@pytest.mark.parametrize("nh,nkv,hd,max_seq,pos", [(24, 8, 128, 1000, 777), (32, 8, 128, 1280, 130), (8, 8, 64, 129, 0), (16, 2, 64, 300, 299),
+                                                   (32, 8, 128, 4096, 777), (16, 4, 64, 64, 33)])
+def test_rows_never_written_do_not_reach_the_output(cuda, orc, nh, nkv, hd, max_seq, pos, cuda_core):
+    """One sequence: the cache from the position on holds NaN before the call, in caches for each of the kernels; the last tile of
+    16 positions is cut at the new row."""
+    from nve_b200 import cuda_kernels as ck
+
+    torch = cuda
+    f16, G = torch.float16, nh // nkv
+    q, k, v = (dev(orc.to_act16(orc.fill_normal(h * hd, 893, i)), f16).view(h, hd) for i, h in enumerate((nh, nkv, nkv)))
+    kc, vc = (dev(orc.to_act16(orc.fill_normal(nkv * max_seq * hd, 893, 4 + i)), f16).view(nkv, max_seq, hd) for i in range(2))
+    kc[:, pos:], vc[:, pos:] = float("nan"), float("nan")
+    cos, sin = orc.rope_tables_f32(hd, max_seq, 10000.0)
+    cos, sin = dev(orc.to_act16(cos), f16), dev(orc.to_act16(sin), f16)
+    d_pos = torch.tensor([pos], dtype=torch.int32, device="cuda")
+    d_len = d_pos + 1
+    got = torch.empty((nh, hd), dtype=f16, device="cuda")
+    prev = ck.set_attn_decode_kernel(cuda_core)
+    try:
+        ck.attn_decode_fused(q, k, v, kc, vc, cos, sin, d_pos.data_ptr(), d_len.data_ptr(), got, nh, nkv, hd, max_seq, hd ** -0.5)
+    finally:
+        ck.set_attn_decode_kernel(prev)
+    q1, k1 = q.clone(), k.clone()
+    ck.rope_decode_dyn_inplace(q1, k1, cos, sin, nh, nkv, hd, d_pos.data_ptr())
+    assert torch.equal(kc[:, pos], k1) and torch.equal(vc[:, pos], v)
+    s = torch.einsum("kgd,kld->kgl", q1.double().view(nkv, G, hd), kc[:, :pos + 1].double()) * hd ** -0.5
+    want = torch.einsum("kgl,kld->kgd", s.softmax(-1), vc[:, :pos + 1].double()).reshape(nh, hd)
+    # f16 probabilities (2^-11 of the largest |v| at most), one f16 rounding of the result, f32 scores in the exponent
+    bound = (2.0 ** -10 + 2.0 ** -11) * vc[:, :pos + 1].double().abs().max().item()
+    assert (got.double() - want).abs().max().item() < bound
