@@ -79,8 +79,10 @@ __global__ void __launch_bounds__(kAdThreads) attn_decode_kernel(const AttnParam
     // Fused form: the cache rows of earlier positions were written by earlier steps, so the first batches of K/V
     // loads can be in flight while the kernel still waits for its predecessor (which produces q and the new k/v,
     // not the cache).  The scalars read here are only a guess used for addressing: they are read again after the
-    // wait and the prefetched rows are dropped if anything differs.
+    // wait and the prefetched rows are dropped if anything differs, or if the row before the position is among them: the
+    // attention launch of that position may be in front and lets this one start before it has stored.
     int pre_seq = -1, pre_pos = -2;
+    bool settled = false;
     AdPrefetch pre;
     if constexpr (FUSED) {
         pre_seq = max(0, min(*p.d_seq_len, p.kv_stride));
@@ -88,6 +90,7 @@ __global__ void __launch_bounds__(kAdThreads) attn_decode_kernel(const AttnParam
         const int pchunk = (pre_seq + kAdRanks - 1) / kAdRanks;
         const int pb = rank * pchunk, pe = min(pre_seq, pb + pchunk);
         const int safe = pb < p.kv_stride ? pb : 0;
+        settled = min(pe, pb + kAdPre * PL * kAdUnroll) < pre_pos;
 #pragma unroll
         for (int b = 0; b < kAdPre; b++) {
 #pragma unroll
@@ -113,7 +116,7 @@ __global__ void __launch_bounds__(kAdThreads) attn_decode_kernel(const AttnParam
     }
     seq_len = max(0, min(seq_len, p.kv_stride));
     const bool pos_ok = FUSED && pos >= 0 && pos < p.kv_stride;
-    const bool pre_ok = FUSED && pre_seq == seq_len && pre_pos == pos;
+    const bool pre_ok = FUSED && settled && pre_seq == seq_len && pre_pos == pos;
     if (!FUSED || pos != pre_pos) {  // uniform over the grid
         if constexpr (FUSED) __syncthreads();
         attn_stage_q<HD, QH, FUSED>(sh, tid, q_row, p.k_new, p.v_new, p.cos_tab, p.sin_tab, h0, kvh, pos, pos_ok);

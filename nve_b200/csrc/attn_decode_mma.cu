@@ -96,14 +96,17 @@ __global__ void __launch_bounds__(kAmThreads, 1) attn_decode_mma_kernel(const At
     const uint16_t* vh = p.v_cache + static_cast<long long>(kvh) * p.kv_stride * HD;
 
     // ---- this warp's first tile, addressed with the position words as they are now (read again after the wait; the tile is
-    // loaded again if they changed).  Before the wait only in the fused form: in the plain form the launch in front may be writing the
-    // rows that this one reads, and it may let its dependents start before it has stored.
+    // loaded again if they changed).  Fused form: before the wait, if the tile ends below the row before the position -- the
+    // attention launch of that position may be in front, and it lets its dependents start before it has stored.  Plain form: the
+    // launch in front may be writing any row.  After the wait then, next to the new token's q, k and v: one round trip for both
+    // (8B at 1024 positions: the token takes 1249 us with every tile early, 1260 with the late one requested behind the staging).
     const int pre_seq = max(0, min(p.d_seq_len != nullptr ? *p.d_seq_len : seq_len_row, p.kv_stride));
     const int pre_pos = FUSED ? *p.d_pos : -1;
     uint4 kr[2][HD / 32], vr[4][HD / 64];
     const int pchunk = (pre_seq + kAdRanks - 1) / kAdRanks;
     const int pre_p0 = rank * pchunk + warp * 16, pre_end = min(pre_seq, (rank + 1) * pchunk);
-    if (FUSED && pre_p0 < pre_end) am_load_tile<HD>(kh, vh, pre_p0, pre_end - 1, g, t, kr, vr);
+    const bool early = FUSED && min(pre_p0 + 16, pre_end) < pre_pos;
+    if (early && pre_p0 < pre_end) am_load_tile<HD>(kh, vh, pre_p0, pre_end - 1, g, t, kr, vr);
     // the RoPE row of the guessed position does not depend on the producer either; rows g >= G of the q fragments are zero
     // this thread's element pairs (qe, qe + HALF) of the heads qh, qh + HPP, ... (those below G) ...
     constexpr int HPP = kAmThreads / HALF;        // heads covered by one pass of the CTA's threads
@@ -117,7 +120,7 @@ __global__ void __launch_bounds__(kAmThreads, 1) attn_decode_mma_kernel(const At
     }
     for (int i = tid; i < (HD / 16) * 32 * 2; i += kAmThreads) reinterpret_cast<uint32_t*>(sh.qf)[i] = 0;
     pdl_wait();
-    if (!FUSED && pre_p0 < pre_end) am_load_tile<HD>(kh, vh, pre_p0, pre_end - 1, g, t, kr, vr);
+    if (!early && pre_p0 < pre_end) am_load_tile<HD>(kh, vh, pre_p0, pre_end - 1, g, t, kr, vr);
     // one round trip: the position words are read again while q, k and v of the new token come in; everything that
     // was addressed with the guess is redone in the rare case that the words changed
     uint16_t x0[QI], x1[QI];

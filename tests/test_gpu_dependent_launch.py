@@ -88,3 +88,42 @@ def test_plain_attention_behind_the_launch_that_writes_the_row(cuda, orc, nh, nk
     off, on = _both(ck, torch, run)
     assert all(torch.isfinite(t.float()).all() for t in off[:3])
     assert all(torch.equal(a, b) for a, b in zip(off, on))
+
+
+@pytest.mark.parametrize("cuda_core", [False, True])
+@pytest.mark.parametrize("nh,nkv,hd,max_seq,pos", [(32, 8, 128, 64, 14), (24, 8, 128, 1000, 777), (16, 16, 64, 3000, 2000)])
+def test_fused_attention_of_successive_positions(cuda, orc, nh, nkv, hd, max_seq, pos, cuda_core):
+    """Three positions one after the other on the same cache, nothing in between: each reads the row that the launch in front writes.
+    One sequence and several."""
+    from nve_b200 import cuda_kernels as ck
+
+    torch = cuda
+    B, steps, f16, scale = 4, 3, torch.float16, hd ** -0.5
+    q, k, v = (_normal(torch, orc, (steps, B, h * hd), 1120, i) for i, h in enumerate((nh, nkv, nkv)))
+    cos, sin = orc.rope_tables_f32(hd, max_seq, 10000.0)
+    cos, sin = dev(orc.to_act16(cos), f16), dev(orc.to_act16(sin), f16)
+    old = [_normal(torch, orc, (B, nkv, max_seq, hd), 1121, i) for i in range(2)]
+    d_pos = torch.arange(pos, pos + steps, dtype=torch.int32, device="cuda").view(steps, 1).repeat(1, B)
+    d_len = d_pos + 1
+
+    def run():
+        out = torch.zeros((2, steps, B, nh * hd), dtype=f16, device="cuda")
+        (kc, vc), (kb, vb) = ([t.clone() for t in old] for _ in range(2))
+        for t in (kc, vc, kb, vb):
+            t[:, :, pos:] = float("nan")
+        torch.cuda.synchronize()
+        for b in range(B):
+            for s in range(steps):
+                ck.attn_decode_fused(q[s, b], k[s, b], v[s, b], kc[b], vc[b], cos, sin, d_pos[s, b:].data_ptr(), d_len[s, b:].data_ptr(),
+                                     out[0, s, b], nh, nkv, hd, max_seq, scale)
+        for s in range(steps):
+            ck.attn_decode_fused_batch(q[s], k[s], v[s], kb, vb, cos, sin, d_pos[s], d_len[s], nh, nkv, hd, max_seq, scale, out=out[1, s])
+        return [out] + [t[:, :, :pos + steps].clone() for t in (kc, vc, kb, vb)]
+
+    prev = ck.set_attn_decode_kernel(cuda_core)
+    try:
+        off, on = _both(ck, torch, run)
+    finally:
+        ck.set_attn_decode_kernel(prev)
+    assert torch.isfinite(off[0].float()).all()
+    assert all(torch.equal(a, b) for a, b in zip(off, on))
