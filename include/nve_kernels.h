@@ -334,8 +334,8 @@ NVE_API int nve_b200_quantize_matvec_w4a8_allreduce(const void* x, int x_dtype, 
  * nve_b200_set_attn_decode_kernel(1) selects the CUDA-core kernel for all of them (also used for other shapes; it is the
  * arithmetic of the persistent one-kernel step), 0 restores the default.  They agree within 5e-3 of the largest output.
  * The setting is process-wide, a captured graph keeps the kernel it was recorded with; the previous setting is returned.
- * With dependent launch on (nve_b200_set_pdl) the fused forms may read rows below *d_pos - 1 while the launch in front still
- * runs: those rows have to come from launches before that one (as the rows of earlier steps do). */
+ * With dependent launch on (nve_b200_set_pdl) it may read rows below *d_pos - 1 while the launch in front still runs: those
+ * rows have to come from launches before that one (as the rows of earlier steps do). */
 NVE_API int nve_b200_attn_decode_fused(const uint16_t* q, const uint16_t* k_new, const uint16_t* v_new,
                                        uint16_t* k_cache, uint16_t* v_cache, const uint16_t* cos_tab,
                                        const uint16_t* sin_tab, const int* d_pos, const int* d_seq_len, uint16_t* out,

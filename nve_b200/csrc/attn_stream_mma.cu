@@ -10,8 +10,8 @@
 //     always under way, eight warps per SM, 130 KB or more per SM;
 //   * the positions of a unit are split over a cluster of 1 .. 8 CTAs (distributed-shared-memory merge in rank 0, as in the
 //     latency kernel), chosen so that the grid fills the GPU whatever the batch; the slices follow the sequence's own length;
-//   * fused form: the first tiles that hold settled rows only are requested before the grid dependency resolves, from the
-//     position words as they are then (read again after the wait; requested again in the rare case that they changed).
+//   * the position words are read before the grid dependency resolves, for the slices and the RoPE row, and again after it (both
+//     are redone in the rare case that they changed); the first tiles are requested then.
 // Tile layout in shared memory: rows of HD f16, 16-byte chunks XORed with the row, so that ldmatrix reads eight rows of a
 // chunk from eight bank groups; K as the B operand of q.K^T as it is, V through ldmatrix.trans for p.V.
 #include <cooperative_groups.h>
@@ -131,13 +131,6 @@ template <int HD, int G, int NW, int NS, bool FUSED> __global__ void __launch_bo
         as_commit();
     };
     slice();
-    // Which of the first tiles may be requested before the wait.  A launch in front that writes this cache lets its dependents
-    // start before it has stored: the K/V write of a prompt block (plain form: any row may be new, so none), and the attention
-    // launch of the preceding position (fused form: the tiles that end below that row).  A warp's early tiles come before its others.
-    auto early = [&](int i) { return FUSED && min(t_begin + 16 * (warp + NW * i) + 16, t_end) < pos; };
-#pragma unroll
-    for (int i = 0; i < NS; i++)
-        if (early(i)) load(t_begin + 16 * (warp + NW * i), i);
     const int qe = tid % HALF, qh = tid / HALF;  // this thread's element pairs (qe, qe + HALF) of the heads qh, qh + HPP, ...
     constexpr int HPP = (32 * NW) / HALF, QI = (G + HPP - 1) / HPP;
     uint16_t c16 = 0, s16 = 0;
@@ -168,21 +161,21 @@ template <int HD, int G, int NW, int NS, bool FUSED> __global__ void __launch_bo
     {
         const int now = max(0, min(p.d_seq_len != nullptr ? *reinterpret_cast<const volatile int*>(p.d_seq_len) : seq_len_row, p.kv_stride));
         const int now_pos = FUSED ? *reinterpret_cast<const volatile int*>(p.d_pos) : -1;
-        const bool moved = now != seq_len || now_pos != pos;  // uniform over the CTA
         if (FUSED && now_pos != pos) {
             pos = now_pos;
             rope_row();
         }
-        if (moved) {
-            as_wait<0>();
-            __syncwarp();
+        if (now != seq_len) {  // uniform over the CTA
             seq_len = now;
             slice();
         }
-#pragma unroll
-        for (int i = 0; i < NS; i++)
-            if (moved || !early(i)) load(t_begin + 16 * (warp + NW * i), i);
     }
+    // Nothing of the cache before the wait: the launch in front may be writing it, and it may let its dependents start before it
+    // has stored.  Behind q, k and v, which everything waits for: tiles requested before the wait hold them up where there is much
+    // K/V (us per token with early tiles and so: 8B at 16384 positions 1772 and 1725; 3B, 7 sequences 1492 and 1459; 8B, 64
+    // sequences 3314 and 3305; tiles right after the wait, in front of q: 1776, 1504 and 3344).
+#pragma unroll
+    for (int i = 0; i < NS; i++) load(t_begin + 16 * (warp + NW * i), i);
     const bool pos_ok = FUSED && pos >= 0 && pos < p.kv_stride;
     {
         // the rotation of the stand-alone RoPE kernel: same IEEE operations, same 16-bit rounding
