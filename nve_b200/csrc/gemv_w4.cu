@@ -553,6 +553,7 @@ template <typename Kern> static int launch_gemv(Kern kern, const GemvParams& p, 
     }
     GemvParams pl = p;
     pl.pq_own = own;
+    pl.awq16 = pl.awq != nullptr && aligned(pl.awq, 16);
     if (own > 0) cfg.gridDim = dim3((p.row_end[0] / 32 + own - 1) / own);
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, pl);
     count_launch();
@@ -658,7 +659,7 @@ using namespace nve;
 
 extern "C" int nve_b200_matvec_w4a8_multi(const int8_t* xq, const float* xq_scales, const nve_b200_w4_matrix* mats,
                                           int num_mats, int K, int out_dtype, nve_stream_t stream) {
-    GemvParams p;
+    GemvParams p = {};
     int st = fill_params(p, mats, num_mats, K);
     if (st != NVE_OK) return set_status(st);
     if (!xq || !xq_scales) return set_status(NVE_ERR_BAD_POINTER);
@@ -669,7 +670,7 @@ extern "C" int nve_b200_matvec_w4a8_multi(const int8_t* xq, const float* xq_scal
 
 extern "C" int nve_b200_matvec_w4a16_multi(const void* x, int x_dtype, const float* awq, const nve_b200_w4_matrix* mats,
                                            int num_mats, int K, int out_dtype, nve_stream_t stream) {
-    GemvParams p;
+    GemvParams p = {};
     int st = fill_params(p, mats, num_mats, K);
     if (st != NVE_OK) return set_status(st);
     if (!x) return set_status(NVE_ERR_BAD_POINTER);
@@ -684,7 +685,7 @@ extern "C" int nve_b200_matvec_w4a16_multi(const void* x, int x_dtype, const flo
 extern "C" int nve_b200_matvec_w4a16_planes_multi(const uint8_t* x_lo, const int8_t* x_hi, const float* x_scales,
                                                   const nve_b200_w4_matrix* mats, int num_mats, int K, int out_dtype,
                                                   nve_stream_t stream) {
-    GemvParams p;
+    GemvParams p = {};
     int st = fill_params(p, mats, num_mats, K);
     if (st != NVE_OK) return set_status(st);
     if (!x_lo || !x_hi || !x_scales) return set_status(NVE_ERR_BAD_POINTER);
@@ -701,7 +702,7 @@ extern "C" int nve_b200_matvec_w4a16_planes_multi(const uint8_t* x_lo, const int
 extern "C" int nve_b200_w4a8_idot(const int8_t* xq, const uint8_t* nibbles, int32_t* I, int N, int K,
                                   nve_stream_t stream) {
     nve_b200_w4_matrix m = {nibbles, reinterpret_cast<const float*>(nibbles), I, nullptr, N};
-    GemvParams p;
+    GemvParams p = {};
     int st = fill_params(p, &m, 1, K);
     if (st != NVE_OK) return set_status(st);
     if (!xq || !I) return set_status(NVE_ERR_BAD_POINTER);
@@ -715,7 +716,7 @@ extern "C" int nve_b200_w4a8_idot(const int8_t* xq, const uint8_t* nibbles, int3
 extern "C" int nve_b200_rmsnorm_matvec_w4a8_multi(const void* h, const void* norm_weight, float eps, int act_dtype,
                                                   const nve_b200_w4_matrix* mats, int num_mats, int K, int out_dtype,
                                                   nve_stream_t stream) {
-    GemvParams p;
+    GemvParams p = {};
     int st = fill_params(p, mats, num_mats, K);
     if (st != NVE_OK) return set_status(st);
     if (!h || !norm_weight) return set_status(NVE_ERR_BAD_POINTER);
@@ -731,7 +732,7 @@ extern "C" int nve_b200_rmsnorm_matvec_w4a8_multi(const void* h, const void* nor
 extern "C" int nve_b200_rmsnorm_matvec_w4a8_awq_multi(const void* h, const void* norm_weight, float eps, int act_dtype,
                                                       const float* awq_inv, const nve_b200_w4_matrix* mats, int num_mats,
                                                       int K, int out_dtype, nve_stream_t stream) {
-    GemvParams p;
+    GemvParams p = {};
     int st = fill_params(p, mats, num_mats, K);
     if (st != NVE_OK) return set_status(st);
     if (!h || !norm_weight) return set_status(NVE_ERR_BAD_POINTER);
@@ -748,7 +749,7 @@ extern "C" int nve_b200_rmsnorm_matvec_w4a8_awq_multi(const void* h, const void*
 extern "C" int nve_b200_rmsnorm_matvec_w4a16_multi(const void* h, const void* norm_weight, float eps, int act_dtype,
                                                    const float* awq, const nve_b200_w4_matrix* mats, int num_mats, int K,
                                                    int out_dtype, nve_stream_t stream) {
-    GemvParams p;
+    GemvParams p = {};
     int st = fill_params(p, mats, num_mats, K);
     if (st != NVE_OK) return set_status(st);
     if (!h || !norm_weight) return set_status(NVE_ERR_BAD_POINTER);
@@ -786,7 +787,7 @@ static int fill_gateup(GemvParams& p, const nve_b200_w4_matrix* gate, const nve_
 extern "C" int nve_b200_rmsnorm_gateup_silu_w4a8(const void* h, const void* norm_weight, float eps, int act_dtype,
                                                  const float* awq_inv, const nve_b200_w4_matrix* gate,
                                                  const nve_b200_w4_matrix* up, void* mid_out, int K, nve_stream_t stream) {
-    GemvParams p;
+    GemvParams p = {};
     int st = fill_gateup(p, gate, up, mid_out, K);
     if (st != NVE_OK) return set_status(st);
     if (!h || !norm_weight) return set_status(NVE_ERR_BAD_POINTER);
@@ -800,7 +801,7 @@ extern "C" int nve_b200_rmsnorm_gateup_silu_w4a8(const void* h, const void* norm
 extern "C" int nve_b200_rmsnorm_gateup_silu_w4a16(const void* h, const void* norm_weight, float eps, int act_dtype,
                                                   const float* awq, const nve_b200_w4_matrix* gate,
                                                   const nve_b200_w4_matrix* up, void* mid_out, int K, nve_stream_t stream) {
-    GemvParams p;
+    GemvParams p = {};
     int st = fill_gateup(p, gate, up, mid_out, K);
     if (st != NVE_OK) return set_status(st);
     if (!h || !norm_weight) return set_status(NVE_ERR_BAD_POINTER);
@@ -829,7 +830,7 @@ extern "C" int nve_b200_rmsnorm_gateup_silu_q8_w4a8(const void* h, const void* n
                                                     const float* awq_inv, const nve_b200_w4_matrix* gate,
                                                     const nve_b200_w4_matrix* up, void* mid_out, int K, int8_t* mid_q,
                                                     float* mid_scales, unsigned* group_counters, nve_stream_t stream) {
-    GemvParams p;
+    GemvParams p = {};
     int st = fill_gateup(p, gate, up, mid_out, K);
     if (st != NVE_OK) return set_status(st);
     if (!h || !norm_weight) return set_status(NVE_ERR_BAD_POINTER);
@@ -847,7 +848,7 @@ extern "C" int nve_b200_rmsnorm_gateup_silu_x16_w4a16(const void* h, const void*
                                                       const nve_b200_w4_matrix* up, void* mid_out, int K, uint8_t* mid_lo,
                                                       int8_t* mid_hi, float* mid_scales, const float* down_awq,
                                                       unsigned* group_counters, nve_stream_t stream) {
-    GemvParams p;
+    GemvParams p = {};
     int st = fill_gateup(p, gate, up, mid_out, K);
     if (st != NVE_OK) return set_status(st);
     if (!h || !norm_weight) return set_status(NVE_ERR_BAD_POINTER);
@@ -862,7 +863,7 @@ extern "C" int nve_b200_rmsnorm_gateup_silu_x16_w4a16(const void* h, const void*
 
 static int quantize_matvec_w4a8(const void* x, int x_dtype, const float* awq_inv, const nve_b200_w4_matrix* mats, int num_mats,
                                 int K, bool allreduce, cudaStream_t cs) {
-    GemvParams p;
+    GemvParams p = {};
     int st = fill_params(p, mats, num_mats, K);
     if (st != NVE_OK) return set_status(st);
     if (!x) return set_status(NVE_ERR_BAD_POINTER);
@@ -900,7 +901,7 @@ static int attach_tp(GemvParams& p) {
 
 extern "C" int nve_b200_matvec_w4a8_allreduce(const int8_t* xq, const float* xq_scales, const nve_b200_w4_matrix* mat,
                                               int K, int out_dtype, nve_stream_t stream) {
-    GemvParams p;
+    GemvParams p = {};
     int st = fill_params(p, mat, 1, K);
     if (st != NVE_OK) return set_status(st);
     if (!xq || !xq_scales) return set_status(NVE_ERR_BAD_POINTER);
@@ -915,7 +916,7 @@ extern "C" int nve_b200_matvec_w4a8_allreduce(const int8_t* xq, const float* xq_
 extern "C" int nve_b200_matvec_w4a16_planes_allreduce(const uint8_t* x_lo, const int8_t* x_hi, const float* x_scales,
                                                       const nve_b200_w4_matrix* mat, int K, int out_dtype,
                                                       nve_stream_t stream) {
-    GemvParams p;
+    GemvParams p = {};
     int st = fill_params(p, mat, 1, K);
     if (st != NVE_OK) return set_status(st);
     if (!x_lo || !x_hi || !x_scales) return set_status(NVE_ERR_BAD_POINTER);
@@ -931,7 +932,7 @@ extern "C" int nve_b200_matvec_w4a16_planes_allreduce(const uint8_t* x_lo, const
 
 extern "C" int nve_b200_matvec_w4a16_allreduce(const void* x, int x_dtype, const float* awq, const nve_b200_w4_matrix* mat,
                                                int K, int out_dtype, nve_stream_t stream) {
-    GemvParams p;
+    GemvParams p = {};
     int st = fill_params(p, mat, 1, K);
     if (st != NVE_OK) return set_status(st);
     if (!x) return set_status(NVE_ERR_BAD_POINTER);

@@ -391,3 +391,36 @@ def test_w4a16_fixed_point_hostile_ranges(cuda, orc, case):
     ref = orc.q4_matvec(blocks, orc.from_act16(x16), awq_inv=awq)
     assert np.all(np.isfinite(y.cpu().numpy()))
     assert rel_rms_err(y.cpu().numpy(), ref) < TOL
+
+
+@pytest.mark.parametrize("bf", [False, True])
+@pytest.mark.parametrize("K", [96, 2048, 8192, 8224, 14336])
+def test_activation_multipliers_of_any_alignment(cuda, orc, K, bf):
+    """A multiplier vector that is a float pointer into a larger one gives the bits of an aligned one: W4A16 and W4A8, from the plain
+    vector and from the RMSNorm prologue (in registers up to K = 8192, in two passes above)."""
+    from nve_b200 import cuda_kernels as ck
+    from oracle import np_oracle as npo
+
+    torch = cuda
+    dt = torch.bfloat16 if bf else torch.float16
+    N = 48
+    nib, sc = orc.extract_for_gpu(orc.quantize_q4(orc.fill_normal(N * K, 621, 3, scale=0.02).reshape(N, K)))
+    mats = [(dev(nib), dev(sc), N)]
+    h = dev(orc.to_act16(orc.fill_normal(K, 621, 1), bf), dt).view(1, -1)
+    nw = dev(orc.to_act16(1.0 + 0.1 * orc.fill_normal(K, 621, 4), bf), dt)
+    big = dev((0.5 + np.abs(orc.fill_normal(K + 4, 621, 2))).astype(np.float32))
+    res = []
+    for off in range(4):
+        awq = torch.empty(K + 4, dtype=torch.float32, device="cuda")[off:off + K]
+        awq.copy_(big[:K])
+        assert awq.data_ptr() % 16 == 4 * off
+        res.append([ck.matvec_w4a16_multi(h, awq, mats, K, out_dtype=dt)[0], ck.rmsnorm_matvec_w4a16_multi(h, nw, 1e-5, awq, mats, K, out_dtype=dt)[0],
+                    ck.rmsnorm_matvec_w4a8_awq_multi(h, nw, 1e-5, awq, mats, K, out_dtype=dt)[0],
+                    ck.quantize_matvec_w4a8_multi(h, awq, mats, K)[0]])
+    for other in res[1:]:
+        for a, b in zip(res[0], other):
+            assert torch.equal(a, b)
+    xf = h.double().cpu().numpy() * big[:K].double().cpu().numpy()
+    Wq = npo.unpack_gpu(nib).astype(np.float64) * np.repeat(sc.astype(np.float64), 32, axis=1)
+    # one 16-bit rounding of the result on top of the route's tolerance
+    assert rel_rms_err(res[0][0].float().cpu().numpy(), xf @ Wq.T) < TOL + (2.0 ** -6 if bf else 0.0)
