@@ -56,14 +56,21 @@ template <int HD> __device__ __forceinline__ uint32_t ap_off(int r, int c) {
     return static_cast<uint32_t>(r * (HD * 2) + ((c ^ (r & 7)) << 4));
 }
 
+// bits 15 and 31: which half of a word is an infinity or a NaN (all exponent bits set)
+__device__ __forceinline__ uint32_t ap_not_finite(uint32_t w) { return ((w & 0x7C007C00u) + 0x04000400u) & 0x80008000u; }
+
 template <int HD> constexpr int ap_smem_bytes() {
     constexpr int stage = kApRows * HD * 2 + 4 * kApKeys * HD * 2;  // Q, two K and two V tiles
     constexpr int part = kApRows * (HD + 4) * 4 + kApRows * 8 + kApRows * 32;  // f32 partials of a split tile + their m, l + weights
     return stage > part ? stage : part;
 }
 
-template <int HD>
-__global__ void __launch_bounds__(kApThreads, 2) attn_prefill_mma_kernel(const AttnParams p, int groups, int tiles) {
+// One CTA's work.  A position that some rows of the tile do not see yet may hold an infinity or a NaN in v, which their zero probability
+// would turn into NaN.  So a CTA that finds an output that is not finite stores nothing and says false, and the tile is computed once more,
+// CAREFUL: in the steps that are cut such elements go to the rows that see them one by one and are zeros in the product.  (In line, as a
+// branch of the steps, this cost 0.7 to 3 us per launch in a prefill of 61 rows, 8B; so 0.3.)
+template <int HD, bool CAREFUL>
+__device__ __forceinline__ bool ap_tile(const AttnParams& p, int groups, int tiles) {
     extern __shared__ __align__(128) unsigned char ap_raw[];
     constexpr int CH = HD / 8;  // 16-byte chunks per row
     constexpr int KVB = kApKeys * HD * 2;
@@ -88,8 +95,10 @@ __global__ void __launch_bounds__(kApThreads, 2) attn_prefill_mma_kernel(const A
     const int per = (nkt + csize - 1) / csize;
     const int kt0 = rank * per, kt1 = min(nkt, kt0 + per);
 
-    pdl_wait();
-    pdl_launch_dependents();
+    if (!CAREFUL) {
+        pdl_wait();
+        pdl_launch_dependents();
+    }
     auto load_kv = [&](int kt, int buf) {
 #pragma unroll
         for (int i = 0; i < kApKeys * CH / kApThreads; i++) {
@@ -143,7 +152,8 @@ __global__ void __launch_bounds__(kApThreads, 2) attn_prefill_mma_kernel(const A
                 mma_f16_16816(s[2 * np + 1], qa, b[2], b[3]);
             }
         }
-        if ((kt + 1) * kApKeys > lim_min) {  // some row does not see the whole tile
+        const bool cut = (kt + 1) * kApKeys > lim_min;  // some row does not see the whole tile
+        if (cut) {
 #pragma unroll
             for (int n = 0; n < 8; n++)
 #pragma unroll
@@ -174,6 +184,37 @@ __global__ void __launch_bounds__(kApThreads, 2) attn_prefill_mma_kernel(const A
                 o[j][2 * hh + 1] *= corr;
             }
         }
+        if (CAREFUL && cut) {
+            float ps[32];
+#pragma unroll
+            for (int i = 0; i < 32; i++) ps[i] = s[i >> 2][i & 3];
+#pragma unroll 1
+            for (int r = 0; r < kApKeys; r++) {
+                const int i = (r >> 3) * 4 + (r & 1), from = (lane & ~3) | ((r & 7) >> 1), col = kt * kApKeys + r;
+                const float p0 = __shfl_sync(0xffffffffu, ps[i], from), p1 = __shfl_sync(0xffffffffu, ps[i + 2], from);
+#pragma unroll
+                for (int j = 0; j < CH; j++) {
+                    uint32_t w;
+                    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(w) : "r"(vb + ap_off<HD>(r, j) + 4 * t) : "memory");
+#pragma unroll
+                    for (int d = 0; d < 2; d++)
+                        if (ap_not_finite(w) & (d == 0 ? 0x8000u : 0x80000000u)) {
+                            const float v = Act16<NVE_DT_F16>::to_f32(static_cast<uint16_t>(w >> (16 * d)));
+                            if (col < lim[0]) o[j][d] = fmaf(p0, v, o[j][d]);
+                            if (col < lim[1]) o[j][2 + d] = fmaf(p1, v, o[j][2 + d]);
+                        }
+                }
+            }
+            __syncthreads();
+#pragma unroll 1
+            for (int i = tid; i < kApKeys * (HD / 2); i += kApThreads) {
+                uint32_t w;
+                asm volatile("ld.shared.b32 %0, [%1];" : "=r"(w) : "r"(vb + i * 4) : "memory");
+                const uint32_t bad = ap_not_finite(w), keep = ((bad & 0x8000u) ? 0u : 0xFFFFu) | ((bad & 0x80000000u) ? 0u : 0xFFFF0000u);
+                asm volatile("st.shared.b32 [%0], %1;" ::"r"(vb + i * 4), "r"(w & keep) : "memory");
+            }
+            __syncthreads();
+        }
         uint32_t pa[4][4];
 #pragma unroll
         for (int kp = 0; kp < 4; kp++) {  // probabilities of 16 positions as the A operand of the second product
@@ -198,7 +239,17 @@ __global__ void __launch_bounds__(kApThreads, 2) attn_prefill_mma_kernel(const A
         l[hh] += __shfl_xor_sync(0xffffffffu, l[hh], 1);
         l[hh] += __shfl_xor_sync(0xffffffffu, l[hh], 2);
     }
-    __syncthreads();  // the staged tiles are no longer read: the buffers are free
+    // barrier: the staged tiles are no longer read, the buffers are free
+    if (CAREFUL) {
+        __syncthreads();
+    } else {
+        float probe[4] = {};
+#pragma unroll
+        for (int j = 0; j < CH; j++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) probe[e] += o[j][e];
+        if (__syncthreads_or(!(fabsf((probe[0] + probe[1]) + (probe[2] + probe[3])) <= 3.0e38f))) return false;
+    }
 
     if (csize == 1) {
         // rows through shared memory (each warp its own 16) so that they leave in 16-byte pieces
@@ -219,7 +270,7 @@ __global__ void __launch_bounds__(kApThreads, 2) attn_prefill_mma_kernel(const A
                     *reinterpret_cast<const uint4*>(ap_raw + ap_off<HD>(r, c));
             }
         }
-        return;
+        return true;
     }
     // ---- split tile: unnormalised partials in shared memory, merged across the cluster
     constexpr int PR = HD + 4;  // floats per partial row
@@ -300,6 +351,14 @@ __global__ void __launch_bounds__(kApThreads, 2) attn_prefill_mma_kernel(const A
         }
     }
     cluster.sync();  // nobody leaves while its shared memory is read
+    return true;
+}
+
+template <int HD> __device__ __noinline__ void ap_tile_careful(const AttnParams& p, int groups, int tiles) { ap_tile<HD, true>(p, groups, tiles); }
+
+template <int HD>
+__global__ void __launch_bounds__(kApThreads, 2) attn_prefill_mma_kernel(const __grid_constant__ AttnParams p, int groups, int tiles) {
+    if (!ap_tile<HD, false>(p, groups, tiles)) ap_tile_careful<HD>(p, groups, tiles);
 }
 
 template <int HD> static cudaError_t launch_ap(const AttnParams& p, cudaStream_t st) {

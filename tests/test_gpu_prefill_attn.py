@@ -41,3 +41,25 @@ def test_tiled_causal_attention(cuda, orc, nh, nkv, hd, S, start):
     # plus f32 scores and sums (2^-16 of a score of at most ~60 in the exponent)
     bound = (2.0 ** -10 + 2.0 ** -11) * vc[:, :L].double().abs().max().item()
     assert (got.double() - want).abs().max().item() < bound
+
+
+@pytest.mark.parametrize("nh,nkv,hd,S,start", [(32, 8, 128, 40, 21), (24, 8, 128, 130, 0), (8, 8, 64, 129, 64), (64, 2, 128, 300, 700),
+                                               (32, 8, 128, 16, 5), (5, 1, 64, 70, 250)])
+def test_infinities_do_not_reach_earlier_rows(cuda, orc, nh, nkv, hd, S, start):
+    """An infinity and a NaN in v, and a NaN in k, at positions inside the block: rows that do not see them keep their bits, rows that
+    do are not finite where they have to be."""
+    from nve_b200 import cuda_kernels as ck
+
+    torch = cuda
+    max_seq = start + S
+    q = dev(orc.to_act16(orc.fill_normal(S * nh * hd, 885, 1)), torch.float16).view(S, nh * hd)
+    kc, vc = (dev(orc.to_act16(orc.fill_normal(nkv * max_seq * hd, 885, 2 + i)), torch.float16).view(nkv, max_seq, hd) for i in range(2))
+    clean = ck.attn_prefill_causal(q, kc, vc, start, nh, nkv, hd, max_seq, hd ** -0.5).view(S, nkv, -1, hd)
+    inf, nan, key = S // 3, S // 2, S - 1  # rows of the block
+    vc[:, start + inf, 3] = float("inf")
+    vc[:, start + nan, hd - 1] = float("nan")
+    kc[:, start + key] = float("nan")
+    got = ck.attn_prefill_causal(q, kc, vc, start, nh, nkv, hd, max_seq, hd ** -0.5).view(S, nkv, -1, hd)
+    assert torch.equal(got[:inf], clean[:inf])
+    assert torch.equal(got[inf:key, ..., 4:hd - 1], clean[inf:key, ..., 4:hd - 1]) and torch.equal(got[inf:nan, ..., hd - 1], clean[inf:nan, ..., hd - 1])
+    assert not torch.isfinite(got[inf:key, ..., 3]).any() and not torch.isfinite(got[nan:key, ..., hd - 1]).any()
