@@ -393,7 +393,8 @@ NVE_API int nve_b200_fill_normal_16(void* out, long long n, unsigned long long s
  * of the SM count is balanced; tiles that several pairs share are summed in ascending K order by a second kernel
  * (reproducible for a given SM count).  Its size comes from nve_b200_gemm_w4a16_scratch_bytes.  bf16 activations
  * without enough scratch for their copy are refused with NVE_ERR_TOO_LARGE; a scratch too small for the partial
- * tiles only lengthens the runs (fewer CTAs), down to one whole tile per pair, which needs none.
+ * tiles only lengthens the runs (fewer CTAs), down to one whole tile per pair, which needs none. f16 activations
+ * take a workspace of any alignment and use it from its first 16-byte boundary on; bf16 ones want it 16-byte aligned.
  * nve_b200_gemm_error returns the code latched by an expired bounded wait. */
 NVE_API size_t nve_b200_gemm_w4a16_scratch_bytes(int M, int N, int K);
 NVE_API int nve_b200_gemm_w4a16(const void* X, int x_dtype, const uint8_t* nibbles, const float* scales, void* Y,

@@ -29,6 +29,8 @@
 // (nve_b200_gemm_error) and both CTAs leave through the normal path.
 #include <cuda.h>
 
+#include <algorithm>
+#include <cstdint>
 #include <type_traits>
 
 #include "act_ops.cuh"
@@ -1039,6 +1041,11 @@ bool gemm_rows_try(const void* X, int x_dtype, const PairMat* mats, int num_mats
 
 int gemm_pair(const uint16_t* X, const PairMat* mats, int num_mats, int y_dtype, int M, int K, void* partial, size_t avail, cudaStream_t st,
               const PairFinish& fin) {
+    // partial tiles are read four floats at a time: of a workspace that is not aligned to that, the part from the first boundary on
+    if (const size_t over = reinterpret_cast<uintptr_t>(partial) % 16; over != 0) {
+        partial = static_cast<unsigned char*>(partial) + (16 - over);
+        avail -= std::min(avail, 16 - over);
+    }
     int status;
     if (gemm_rows_try(X, NVE_DT_F16, mats, num_mats, y_dtype, M, K, partial, avail, st, fin, &status)) return status;
     PairParams p = {};

@@ -98,3 +98,29 @@ def test_prefill_layer_equals_separate_launches(cuda, orc, S, start, nh, nkv, hd
     for a, b in ((got, want), (k1, st.kv_cache.k[0]), (v1, st.kv_cache.v[0])):
         assert rel_rms_err(a.float().cpu().numpy(), b.float().cpu().numpy()) < 5e-3
     assert torch.equal(k1[:, :start], k0[:, :start]) and torch.equal(k1[:, start + S:], k0[:, start + S:])
+
+
+@pytest.mark.parametrize("M,N,K", [(5, 640, 2048), (16, 640, 4096), (200, 520, 1024)])
+@pytest.mark.parametrize("off", [4, 8, 12])
+def test_workspace_of_any_alignment(cuda, orc, M, N, K, off):
+    """A workspace that starts between two 16-byte boundaries gives the bits of an aligned one, also where it is so much too small that
+    runs get longer; the bytes around it stay as they are."""
+    from nve_b200 import cuda_kernels as ck
+
+    torch = cuda
+    x, (g, _), (u, _) = _x(torch, orc, M, K, 1030), _weights(torch, orc, N, K, 1031), _weights(torch, orc, N, K, 1032)
+    res, norm = _x(torch, orc, M, N, 1033), dev(orc.to_act16(1.0 + 0.1 * orc.fill_normal(N, 1034, 3)), torch.float16)
+    need = max(ck.gemm_w4a16_multi_scratch_bytes(M, [N], K), ck.gemm_w4a16_silu_scratch_bytes(M, N, K))
+    out = []
+    for o, nbytes in ((0, need), (off, need), (0, 8), (off, 8)):
+        buf = torch.full((nbytes + 32,), 255, dtype=torch.uint8, device="cuda")
+        ws = buf[o:o + nbytes + 16]
+        y, h, normed, mid = (torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda") for _ in range(4))
+        ck.gemm_w4a16_wide(x, [g], K, [y], ws)
+        ck.gemm_w4a16_add_rmsnorm(x, g, K, res, norm, 1e-5, h, normed, ws)
+        ck.gemm_w4a16_gateup_silu(x, g, u, K, mid, ws)
+        torch.cuda.synchronize()
+        assert ck.gemm_error() == 0 and (buf[:o] == 255).all() and (buf[o + nbytes + 16:] == 255).all()
+        out.append((y, h, normed, mid))
+    for a, b in ((0, 1), (2, 3)):
+        assert all(torch.equal(s, t) for s, t in zip(out[a], out[b]))
