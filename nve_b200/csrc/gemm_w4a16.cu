@@ -6,6 +6,7 @@
 // dequantised to f16, the type the reference dequantises to; bf16 activations are converted to f16 by a small pre-pass
 // into the caller's scratch (bf16 weights would cost 2^-8 per weight and leave no tolerance margin; tcgen05.mma
 // kind::f16 takes both operands in one format).
+#include <algorithm>
 #include <mutex>
 
 #include "common.cuh"
@@ -166,8 +167,8 @@ extern "C" int nve_b200_gemm_error(int reset) { return gemm_pair_error(reset != 
 // caller-provided buffer.
 //
 // Cost and limits: the array is kStaticScratchFloats * 4 bytes (4 MiB) of device memory on every GPU that loads
-// the library, until the process exits.  A call whose partial tiles (nve_b200_gemm_w4a16_scratch_bytes) exceed
-// it is rejected with NVE_ERR_TOO_LARGE.  All calls share the one array: two such GEMMs that overlap on the same
+// the library, until the process exits.  A call whose partial tiles exceed it, counted
+// as noalloc_partial_bytes does, is rejected with NVE_ERR_TOO_LARGE; what the kernel could use beyond it only lengthens its runs.  All calls share the one array: two such GEMMs that overlap on the same
 // GPU (different streams) race on it; issue them on one stream.  The array keeps whatever the previous call
 // left in it; nothing in it has to start at zero, because every partial a call reads was written by that same
 // call's first kernel.
@@ -179,6 +180,17 @@ namespace nve {
 
 constexpr size_t kStaticScratchFloats = static_cast<size_t>(1) << 20;  // 1 Mi floats = 4 MiB
 static __device__ __align__(256) float g_gemm_static_scratch[kStaticScratchFloats];
+
+// What counts against the limit: partial tiles of M x 128 floats, two per SM, of runs of at least two units of 256 along K that are cut
+// evenly over the SMs, where K is a multiple of 256 and not (M > 32 and a whole tile for every SM).  The sizes that are taken are part of the
+// interface and do not follow the tiles of the kernel behind it.
+static size_t noalloc_partial_bytes(int M, int N, int K) {
+    const long long tiles = (static_cast<long long>(N) + 127) / 128, sb = K / 256, sms = sm_count();
+    if (K % 256 != 0 || (M > 32 && tiles >= sms)) return 0;
+    const long long total = tiles * sb;
+    const long long U = std::max((total + sms - 1) / sms, std::min(sb, 2ll));
+    return U % sb == 0 ? 0 : static_cast<size_t>(2 * ((total + U - 1) / U) * M * 128) * sizeof(float);
+}
 
 // Device address of g_gemm_static_scratch on the current device.  In host code the symbol itself is only a
 // stand-in and must never be passed to a kernel; the address comes from the runtime, once per device.
@@ -210,8 +222,7 @@ extern "C" int nve_b200_gemm_w4a16_noalloc(const void* X, int x_dtype, const uin
     if (x_dtype != NVE_DT_F16 && x_dtype != NVE_DT_BF16) return set_status(NVE_ERR_BAD_DTYPE);
     if (y_dtype != x_dtype && y_dtype != NVE_DT_F32) return set_status(NVE_ERR_BAD_DTYPE);
     if (!aligned(X, 16) || !aligned(nibbles, 16) || !aligned(scales, 8)) return set_status(NVE_ERR_BAD_ALIGNMENT);
-    const size_t need = (x_dtype == NVE_DT_BF16 ? x16_region_bytes(M, K) : 0) +
-                        pair_plan(&N, 1, M, K, true, ~static_cast<size_t>(0)).partial_bytes;
+    const size_t need = (x_dtype == NVE_DT_BF16 ? x16_region_bytes(M, K) : 0) + noalloc_partial_bytes(M, N, K);
     if (need > kStaticScratchFloats * sizeof(float)) return set_status(NVE_ERR_TOO_LARGE);
     float* scratch = nullptr;
     int st = static_scratch_address(&scratch);

@@ -87,3 +87,22 @@ def test_noalloc_gemm_refuses_oversized_workspace(cuda):
     with pytest.raises(_ffi.NveKernelError) as ei:
         ck.gemm_w4a16_noalloc(x, nib, sc, N, K, out)
     assert ei.value.status == 5  # NVE_ERR_TOO_LARGE
+
+
+@pytest.mark.parametrize("M,N,K", [(64, 512, 320), (33, 19072, 512), (64, 4000, 64), (50, 300, 4160)])
+def test_noalloc_gemm_takes_sizes_without_split_tiles(cuda, orc, M, N, K):
+    """Sizes that need no partial tiles of 128 rows (K no multiple of 256; as many tiles as SMs and more than 32 rows): taken, although
+    the kernel could use more workspace than there is."""
+    from nve_b200 import cuda_kernels as ck
+    from oracle import np_oracle as npo
+
+    torch = cuda
+    nib, sc, X16 = _inputs(orc, M, N, K, 931)
+    dx, dn, ds = dev(X16, torch.float16), dev(nib), dev(sc)
+    got = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
+    for _ in range(2):
+        ck.gemm_w4a16_noalloc(dx, dn, ds, N, K, got)
+    torch.cuda.synchronize()
+    assert ck.gemm_error() == 0
+    ref = orc.from_act16(X16).astype(np.float64) @ (npo.unpack_gpu(nib).astype(np.float64) * np.repeat(sc.astype(np.float64), 32, axis=1)).T
+    assert rel_rms_err(got.cpu().numpy(), ref) < 3e-3  # f16 rounding of the weights, f32 sums
