@@ -39,9 +39,35 @@ class GpuW4:
         return (self.nibbles, self.scales, self.n)
 
 
-# Rows of x from which on the product is bound by arithmetic rather than by the packed weights (an 8B projection group on
-# B200: 64 rows take 1.2 times as long as 8, 256 rows twice as long, above that the time grows with the rows).
+# Rows of x up to which only what the packed GEMM takes is accepted (and a workspace too small for all rows is used for 64 of
+# them at a time); above it everything that the reference's route takes.
 DENSE_ROWS = 128
+
+
+def _matmul_dense(x: Tensor, w: GpuW4, out: Optional[Tensor]) -> Tensor:
+    """x [M, K] . W^T as src/gpu_layer.rs:220-239 does it for every M > 1, `nve_b200_dequant_w4a16` and a dense library GEMM: for
+    what the packed GEMM does not take (_gemm_takes).  Weights are dequantised to f16 (the reference's type), other activation types
+    converted to f16 with saturation, the result is rounded once to x's type."""
+    wf = ck.dequant_w4a16_any(w.nibbles, w.scales, None, w.n, w.k, out_dtype=torch.float16)
+    xf = x if x.dtype == torch.float16 else x.float().clamp_(-65504.0, 65504.0).to(torch.float16)
+    if out is not None and out.dtype == torch.float16 and out.is_contiguous():
+        return torch.matmul(xf, wf.t(), out=out)
+    y = torch.matmul(xf, wf.t())
+    if out is None:
+        return y if y.dtype == x.dtype else y.to(x.dtype)
+    out.copy_(y)
+    return out
+
+
+def _gemm_takes(x: Tensor, w: GpuW4, out: Optional[Tensor]) -> bool:
+    """K in multiples of 64, 16-bit x and an output of its type and shape, contiguous, x and the nibbles on 16-byte boundaries."""
+    return (w.k % 64 == 0 and x.dtype in (torch.float16, torch.bfloat16) and x.is_cuda and x.is_contiguous() and
+            (x.data_ptr() | w.nibbles.data_ptr()) % 16 == 0 and w.scales.data_ptr() % 8 == 0 and
+            (out is None or (out.dtype == x.dtype and out.shape == (x.shape[0], w.n) and out.is_contiguous())))
+
+
+def _workspace_holds(scratch: Optional[Tensor], m: int, ns: Sequence[int], k: int) -> bool:
+    return scratch is None or m <= 64 or scratch.numel() * scratch.element_size() >= ck.gemm_w4a16_multi_scratch_bytes(m, ns, k)
 
 
 def matmul_x(x: Tensor, w: GpuW4, scratch: Optional[Tensor] = None, out: Optional[Tensor] = None) -> Tensor:
@@ -49,29 +75,51 @@ def matmul_x(x: Tensor, w: GpuW4, scratch: Optional[Tensor] = None, out: Optiona
 
     The reference sends M == 1 to `fused_matvec_w4a16` and M > 1 through `dequant_w4a16` + a dense matmul (the whole
     matrix materialised in f16, 4.6 bytes of traffic per weight).  Here M > 1 goes to the tensor-core GEMM that reads the
-    packed weights and dequantises them on their way into tensor memory, whatever M is.  The activation multiplier
-    `awq_scales`, which the GEMM has no argument for, is applied to x first as the GEMV does per element."""
+    packed weights and dequantises them on their way into tensor memory, whatever M is; above DENSE_ROWS rows, x and outputs
+    that it does not take go the reference's way (_matmul_dense).  The activation multiplier `awq_scales`, which the GEMM has no
+    argument for, is applied to x first as the GEMV does per element.  `scratch` is sized by gemm_w4a16_scratch_bytes for M rows; one
+    that is smaller serves 64 rows at a time, above DENSE_ROWS rows it is left aside."""
     if x.dim() != 2 or x.shape[1] != w.k:
         raise ValueError(f"x must be [M, {w.k}]")
     m = x.shape[0]
+    if m == 0:
+        return torch.empty((0, w.n), dtype=x.dtype, device=x.device) if out is None else out
     if m == 1 and out is None:
         return ck.fused_matvec_w4a16(x, w.nibbles, w.scales, w.awq_scales, w.n, w.k)
     if m == 1:
         return ck.matvec_w4a16_multi(x, w.awq_scales, [w.triple()], w.k, outs=[out])[0]
     if w.awq_scales is not None:
         x = (x.float() * w.awq_scales.view(1, -1)).to(x.dtype)
+    if m > DENSE_ROWS and not _gemm_takes(x, w, out):
+        return _matmul_dense(x, w, out)
+    if not _workspace_holds(scratch, m, [w.n], w.k):
+        if m <= DENSE_ROWS:
+            out = torch.empty((m, w.n), dtype=x.dtype, device=x.device) if out is None else out
+            for r in range(0, m, 64):
+                ck.gemm_w4a16_wide(x[r:r + 64], (w.triple(),), w.k, (out[r:r + 64],), scratch)
+            return out
+        scratch = None
     return ck.gemm_w4a16_wide(x, (w.triple(),), w.k, None if out is None else (out,), scratch)[0]
 
 
 def matmul_x_multi(x: Tensor, ws: Sequence[GpuW4], scratch: Optional[Tensor] = None,
                    outs: Optional[Sequence[Tensor]] = None) -> List[Tensor]:
     """matmul_x for several projections of the same x (q/k/v, gate/up) in one GEMM launch: their tiles share the grid, so
-    narrow projections do not run as few-CTA kernels.  M == 1 and weights with an activation multiplier go through
-    matmul_x one by one."""
+    narrow projections do not run as few-CTA kernels.  M == 1, weights with an activation multiplier and what the GEMM does
+    not take go through matmul_x one by one."""
     m, k = x.shape
-    if m == 1 or any(w.awq_scales is not None for w in ws):
+    if m <= 1 or any(w.awq_scales is not None for w in ws) or (m > DENSE_ROWS and not (
+            1 <= len(ws) <= 3 and all(w.k == k and _gemm_takes(x, w, None if outs is None else outs[i]) for i, w in enumerate(ws)))):
         return [matmul_x(x, w, scratch, None if outs is None else outs[i]) for i, w in enumerate(ws)]
-    return ck.gemm_w4a16_wide(x, [w.triple() for w in ws], k, outs, scratch)
+    triples = [w.triple() for w in ws]
+    if not _workspace_holds(scratch, m, [w.n for w in ws], k):
+        if m <= DENSE_ROWS:
+            outs = [torch.empty((m, w.n), dtype=x.dtype, device=x.device) for w in ws] if outs is None else list(outs)
+            for r in range(0, m, 64):
+                ck.gemm_w4a16_wide(x[r:r + 64], triples, k, [o[r:r + 64] for o in outs], scratch)
+            return outs
+        scratch = None
+    return ck.gemm_w4a16_wide(x, triples, k, outs, scratch)
 
 
 @dataclass

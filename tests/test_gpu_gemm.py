@@ -157,6 +157,69 @@ def test_matmul_x_dense_route_bf16(cuda, orc):
     assert torch.equal(out, y)
 
 
+@pytest.mark.parametrize("form", ["k32", "f32", "strided", "offset", "nibbles", "out_strided", "out_f32", "out_bf16", "small_scratch", "awq_k32"])
+def test_matmul_x_forms_above_128_rows(cuda, orc, form):
+    """What the packed GEMM does not take: K % 64 == 32, f32 or strided or unaligned x, unaligned nibbles, strided or other outputs,
+    a workspace made for 64 rows."""
+    from nve_b200 import cuda_kernels as ck
+    from nve_b200.gpu_layer import GpuW4, matmul_x, matmul_x_multi
+
+    torch = cuda
+    M, N, K = 150, 264, 288 if form.endswith("k32") else 512
+    nib, sc, X16, _ = _case(orc, M, N, K, 983, False)
+    x, dn, awq, out, scratch = dev(X16, torch.float16), dev(nib), None, None, None
+    if form == "f32":
+        x = x.float()
+    elif form == "strided":
+        x = torch.cat([x, x], 1)[:, :K]
+    elif form == "offset":
+        x = torch.cat([x.flatten()[:1], x.flatten()])[1:].view(M, K)
+    elif form == "nibbles":
+        dn = torch.cat([dn.flatten()[:1], dn.flatten()])[1:].view(N, K // 2)
+    elif form == "out_strided":
+        out = torch.full((M, 2 * N), float("nan"), dtype=torch.float16, device="cuda")[:, ::2]
+    elif form.startswith("out_"):
+        out = torch.full((M, N), float("nan"), dtype=torch.float32 if form == "out_f32" else torch.bfloat16, device="cuda")
+    elif form == "small_scratch":
+        x = x.bfloat16()
+        scratch = torch.empty(ck.gemm_w4a16_scratch_bytes(64, N, K), dtype=torch.uint8, device="cuda")
+    elif form == "awq_k32":
+        awq = dev((0.5 + np.abs(orc.fill_normal(K, 983, 3))).astype(np.float32))
+    w = GpuW4(dn, dev(sc), awq, N, K)
+    Wq = npo.unpack_gpu(nib).astype(np.float64) * np.repeat(sc.astype(np.float64), 32, axis=1)
+    ref = (x.double() if awq is None else x.double() * awq.double()).cpu().numpy() @ Wq.T
+    # weights and x * multiplier rounded to f16 (3e-3 of the RMS at most), and the rounding of results of up to ten times the RMS
+    bound = 3e-3 + 5 * torch.finfo(torch.bfloat16 if form in ("out_bf16", "small_scratch") else torch.float16).eps
+    for got in (matmul_x(x, w, scratch, out), matmul_x_multi(x, [w] * 2, scratch, None if out is None else [out] * 2)[1]):
+        assert got is out or (out is None and got.dtype == x.dtype)
+        assert tuple(got.shape) == (M, N) and rel_rms_err(got.float().cpu().numpy(), ref) < bound
+    got = matmul_x_multi(x, [w] * 4, scratch)  # more than one launch takes
+    assert len(got) == 4 and rel_rms_err(got[3].float().cpu().numpy(), ref) < bound
+
+
+def test_matmul_x_of_a_workspace_for_64_rows_and_of_no_rows(cuda, orc):
+    """Up to 128 rows a workspace made for 64 serves them in slices, with nothing allocated; zero rows give an empty result."""
+    from nve_b200 import cuda_kernels as ck
+    from nve_b200.gpu_layer import GpuW4, matmul_x, matmul_x_multi
+
+    torch = cuda
+    M, N, K = 100, 520, 1024
+    for dt in (torch.float16, torch.bfloat16):
+        nib, sc, X16, ref = _case(orc, M, N, K, 987, dt == torch.bfloat16)
+        w, x = GpuW4(dev(nib), dev(sc), None, N, K), dev(X16, dt)
+        scratch = torch.full((ck.gemm_w4a16_multi_scratch_bytes(64, [N, N], K) + 64,), 255, dtype=torch.uint8, device="cuda")
+        out = [torch.full((M, N), float("nan"), dtype=dt, device="cuda") for _ in range(2)]
+        before = torch.cuda.memory_allocated()
+        assert matmul_x(x, w, scratch[:-64], out[0]) is out[0]
+        assert all(a is b for a, b in zip(matmul_x_multi(x, [w, w], scratch[:-64], out), out))
+        torch.cuda.synchronize()
+        assert torch.cuda.memory_allocated() == before and (scratch[-64:] == 255).all()
+        for o in out:
+            assert rel_rms_err(o.float().cpu().numpy(), ref) < 3e-3 + 5 * torch.finfo(dt).eps
+        assert tuple(matmul_x(x[:0], w).shape) == (0, N) and matmul_x(x[:0], w).dtype == dt
+        assert [tuple(t.shape) for t in matmul_x_multi(x[:0], [w, w])] == [(0, N)] * 2
+
+
 @pytest.mark.parametrize("kernel", ["mma", "tc"])
 def test_gemm_parity_with_each_kernel_forced(cuda, kernel):
     """The library picks the kernel by batch size; NVE_B200_GEMM_KERNEL (read once per process) forces one.  The
