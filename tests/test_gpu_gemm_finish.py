@@ -124,3 +124,28 @@ def test_workspace_of_any_alignment(cuda, orc, M, N, K, off):
         out.append((y, h, normed, mid))
     for a, b in ((0, 1), (2, 3)):
         assert all(torch.equal(s, t) for s, t in zip(out[a], out[b]))
+
+
+def test_prefill_layer_refuses_what_does_not_fit(cuda, orc):
+    """Rows on the host, rows of another width, projections of another size: errors as from the separate launches, not a read past the end."""
+    from dataclasses import replace
+
+    from nve_b200 import gpu_layer as gl
+    from test_gpu_glue import _make_state
+
+    torch = cuda
+    hidden, ffn = 512, 1024
+    st = _make_state(torch, orc, hidden, ffn, 8, 2, 64, 1, 64, 1045, True)
+    x = _x(torch, orc, 4, hidden, 1046)
+    assert tuple(gl.gpu_layer_forward_prefill(x, 0, st, 0).shape) == (4, hidden)
+    with pytest.raises(ValueError):
+        gl.gpu_layer_forward_prefill(x.cpu(), 0, st, 0)
+    w = st.layer_weights[0]
+    for bad in (dict(o_proj=gl.GpuW4(w.down_proj.nibbles, w.down_proj.scales, None, hidden, ffn)),
+                dict(down_proj=gl.GpuW4(w.q_proj.nibbles, w.q_proj.scales, None, hidden, hidden))):
+        st.layer_weights[0] = replace(w, **bad)
+        with pytest.raises(ValueError):
+            gl.gpu_layer_forward_prefill(x, 0, st, 0)
+        st.layer_weights[0] = w
+    with pytest.raises(ValueError):
+        gl.gpu_layer_forward_prefill(_x(torch, orc, 4, hidden // 2, 1046), 0, st, 0)
