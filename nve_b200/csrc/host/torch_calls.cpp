@@ -80,6 +80,12 @@ void status(const char* name, int st) {
     if (!PyErr_Occurred()) PyErr_Format(PyExc_RuntimeError, "%s: status %d", name, st);
     throw Failed();
 }
+// Other Python threads run while this one allocates and launches: either can wait for the device (a full launch queue, an allocation
+// that has to free memory first).
+struct WithoutGil {
+    PyThreadState* state = PyEval_SaveThread();
+    ~WithoutGil() { PyEval_RestoreThread(state); }
+};
 at::Tensor empty(at::IntArrayRef size, at::ScalarType type, const at::Tensor& like) {
     return at::detail::empty_cuda(size, type, like.device(), c10::nullopt);
 }
@@ -109,9 +115,15 @@ PyObject* matvec_w4a16(PyObject*, PyObject* const* a, Py_ssize_t na) {
         const auto* sc = static_cast<const float*>(typed_ptr(tensor(a[2], "scales"), at::kFloat, "scales"));
         const auto* awq = static_cast<const float*>(optional_ptr(a[3], at::kFloat, "awq"));
         const long n = integer(a[4]), k = integer(a[5]);
-        at::Tensor out = empty({1, n}, at::kHalf, x);
-        nve_matvec_w4a16(xp, nib, sc, awq, static_cast<uint16_t*>(out.data_ptr()), static_cast<int>(n), static_cast<int>(k), current_stream());
-        status("nve_matvec_w4a16", nve_b200_last_status());
+        at::Tensor out;
+        int st;
+        {
+            WithoutGil others;
+            out = empty({1, n}, at::kHalf, x);
+            nve_matvec_w4a16(xp, nib, sc, awq, static_cast<uint16_t*>(out.data_ptr()), static_cast<int>(n), static_cast<int>(k), current_stream());
+            st = nve_b200_last_status();
+        }
+        status("nve_matvec_w4a16", st);
         return wrap(std::move(out));
     });
 }
@@ -124,9 +136,16 @@ PyObject* quantize_f16_q8(PyObject*, PyObject* const* a, Py_ssize_t na) {
         const int64_t k = x.numel();
         if (k % 32 != 0) fail(PyExc_ValueError, "%s: K must be multiple of 32", "quantize_f16_q8");
         const auto* xp = static_cast<const uint16_t*>(typed_ptr(x, at::kHalf, "x"));
-        at::Tensor xq = empty({k}, at::kChar, x), xs = empty({k / 32}, at::kFloat, x);
-        nve_quantize_f16_q8(xp, static_cast<int8_t*>(xq.data_ptr()), static_cast<float*>(xs.data_ptr()), static_cast<int>(k), current_stream());
-        status("nve_quantize_f16_q8", nve_b200_last_status());
+        at::Tensor xq, xs;
+        int st;
+        {
+            WithoutGil others;
+            xq = empty({k}, at::kChar, x);
+            xs = empty({k / 32}, at::kFloat, x);
+            nve_quantize_f16_q8(xp, static_cast<int8_t*>(xq.data_ptr()), static_cast<float*>(xs.data_ptr()), static_cast<int>(k), current_stream());
+            st = nve_b200_last_status();
+        }
+        status("nve_quantize_f16_q8", st);
         PyObject* r = PyTuple_New(2);
         PyTuple_SET_ITEM(r, 0, wrap(std::move(xq)));
         PyTuple_SET_ITEM(r, 1, wrap(std::move(xs)));
@@ -144,9 +163,15 @@ PyObject* matvec_w4a8(PyObject*, PyObject* const* a, Py_ssize_t na) {
         const auto* nib = static_cast<const uint8_t*>(typed_ptr(tensor(a[2], "nibbles"), at::kByte, "nibbles"));
         const auto* sc = static_cast<const float*>(typed_ptr(tensor(a[3], "wt_scales"), at::kFloat, "wt_scales"));
         const long n = integer(a[4]), k = integer(a[5]);
-        at::Tensor out = empty({1, n}, at::kHalf, xq);
-        nve_matvec_w4a8(qp, qs, nib, sc, static_cast<uint16_t*>(out.data_ptr()), static_cast<int>(n), static_cast<int>(k), current_stream());
-        status("nve_matvec_w4a8", nve_b200_last_status());
+        at::Tensor out;
+        int st;
+        {
+            WithoutGil others;
+            out = empty({1, n}, at::kHalf, xq);
+            nve_matvec_w4a8(qp, qs, nib, sc, static_cast<uint16_t*>(out.data_ptr()), static_cast<int>(n), static_cast<int>(k), current_stream());
+            st = nve_b200_last_status();
+        }
+        status("nve_matvec_w4a8", st);
         return wrap(std::move(out));
     });
 }
@@ -182,23 +207,36 @@ PyObject* gemm_w4a16_wide(PyObject*, PyObject* const* a, Py_ssize_t na) {
             mats[i].scales = static_cast<const float*>(typed_ptr(tensor(PyTuple_GET_ITEM(w, 1), "scales"), at::kFloat, "scales"));
             mats[i].residual = nullptr;
             mats[i].N = ns[i] = static_cast<int>(integer(PyTuple_GET_ITEM(w, 2)));
-            made[i] = outs.o != nullptr ? tensor(PySequence_Fast_GET_ITEM(outs.o, i), "out") : empty({m, ns[i]}, x.scalar_type(), x);
-            mats[i].out = typed_ptr(made[i], x.scalar_type(), "out");
+            if (outs.o != nullptr) {
+                made[i] = tensor(PySequence_Fast_GET_ITEM(outs.o, i), "out");
+                typed_ptr(made[i], x.scalar_type(), "out");
+            }
         }
         void* scratch = nullptr;
         size_t bytes = 0;
-        at::Tensor own;
         if (a[4] != Py_None) {
             const at::Tensor& s = tensor(a[4], "scratch");
             scratch = cuda_ptr(s, "scratch");
             bytes = s.nbytes();
-        } else if (const size_t need = nve_b200_gemm_w4a16_multi_scratch_bytes(static_cast<int>(m), ns, static_cast<int>(count), k); need > 0) {
-            own = empty({static_cast<int64_t>(need)}, at::kByte, x);
-            scratch = own.data_ptr();
-            bytes = need;
         }
-        status("nve_b200_gemm_w4a16_wide",
-               nve_b200_gemm_w4a16_wide(xp, dt, mats, static_cast<int>(count), dt, static_cast<int>(m), k, scratch, bytes, current_stream()));
+        int st;
+        at::Tensor own;
+        {
+            WithoutGil others;
+            for (Py_ssize_t i = 0; i < count; i++) {
+                if (outs.o == nullptr) made[i] = empty({m, ns[i]}, x.scalar_type(), x);
+                mats[i].out = made[i].data_ptr();
+            }
+            if (a[4] == Py_None) {
+                bytes = nve_b200_gemm_w4a16_multi_scratch_bytes(static_cast<int>(m), ns, static_cast<int>(count), k);
+                if (bytes > 0) {
+                    own = empty({static_cast<int64_t>(bytes)}, at::kByte, x);
+                    scratch = own.data_ptr();
+                }
+            }
+            st = nve_b200_gemm_w4a16_wide(xp, dt, mats, static_cast<int>(count), dt, static_cast<int>(m), k, scratch, bytes, current_stream());
+        }
+        status("nve_b200_gemm_w4a16_wide", st);
         PyObject* r = PyList_New(count);
         for (Py_ssize_t i = 0; i < count; i++) PyList_SET_ITEM(r, i, wrap(std::move(made[i])));
         return r;
@@ -214,9 +252,16 @@ PyObject* q4_quantize(PyObject*, PyObject* const* a, Py_ssize_t na) {
         const int64_t n = w.size(0), k = w.size(1);
         const auto* wp = static_cast<const float*>(typed_ptr(w, at::kFloat, "W"));
         const auto* awq = static_cast<const float*>(optional_ptr(a[1], at::kFloat, "awq_scales"));
-        at::Tensor nib = empty({n, k / 2}, at::kByte, w), sc = empty({n, k / 32}, at::kFloat, w);
-        status("nve_b200_q4_quantize", nve_b200_q4_quantize(wp, awq, static_cast<uint8_t*>(nib.data_ptr()), static_cast<float*>(sc.data_ptr()),
-                                                            static_cast<int>(n), static_cast<int>(k), current_stream()));
+        at::Tensor nib, sc;
+        int st;
+        {
+            WithoutGil others;
+            nib = empty({n, k / 2}, at::kByte, w);
+            sc = empty({n, k / 32}, at::kFloat, w);
+            st = nve_b200_q4_quantize(wp, awq, static_cast<uint8_t*>(nib.data_ptr()), static_cast<float*>(sc.data_ptr()), static_cast<int>(n),
+                                      static_cast<int>(k), current_stream());
+        }
+        status("nve_b200_q4_quantize", st);
         PyObject* r = PyTuple_New(2);
         PyTuple_SET_ITEM(r, 0, wrap(std::move(nib)));
         PyTuple_SET_ITEM(r, 1, wrap(std::move(sc)));

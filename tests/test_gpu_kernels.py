@@ -424,3 +424,40 @@ def test_activation_multipliers_of_any_alignment(cuda, orc, K, bf):
     Wq = npo.unpack_gpu(nib).astype(np.float64) * np.repeat(sc.astype(np.float64), 32, axis=1)
     # one 16-bit rounding of the result on top of the route's tolerance
     assert rel_rms_err(res[0][0].float().cpu().numpy(), xf @ Wq.T) < TOL + (2.0 ** -6 if bf else 0.0)
+
+
+def test_native_calls_let_other_threads_run(cuda, orc):
+    """A thread that fills the launch queue of a busy device waits without holding the interpreter lock."""
+    import threading
+    import time
+
+    from nve_b200 import cuda_kernels as ck
+
+    torch = cuda
+    N, K = 64, 64
+    nib, sc = orc.extract_for_gpu(orc.quantize_q4(orc.fill_normal(N * K, 631, 3, scale=0.02).reshape(N, K)))
+    dn, ds, x = dev(nib), dev(sc), dev(orc.to_act16(orc.fill_normal(K, 631, 1)), torch.float16).view(1, K)
+    want = ck.fused_matvec_w4a16(x, dn, ds, None, N, K)
+    torch.cuda.synchronize()
+    stop, gap = threading.Event(), [0.0]
+
+    def tick():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            gap[0], last = max(gap[0], now - last), now
+
+    t = threading.Thread(target=tick)
+    t.start()
+    t0 = time.perf_counter()
+    torch.cuda._sleep(1_500_000_000)  # most of a second at 1.9 GHz
+    for _ in range(4000):  # the queue holds about a thousand launches
+        got = ck.fused_matvec_w4a16(x, dn, ds, None, N, K)
+    issued = time.perf_counter() - t0
+    stop.set()
+    t.join()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    assert issued > 0.3, "the launch queue did not fill"
+    assert gap[0] < 0.5 * issued, f"another thread stood still for {gap[0]:.3f} of {issued:.3f} s"
