@@ -410,17 +410,20 @@ template <int HD, int G, int NW, int NS, bool FUSED> struct AsLaunch {
     static int prepare() {
         return ensure_dynamic_smem(reinterpret_cast<const void*>(attn_stream_mma_kernel<HD, G, NW, NS, FUSED>), as_smem_bytes<HD, G, NW, NS>(kAsMaxCluster));
     }
-    // How many clusters of `csize` CTAs the device holds at a time (clusters do not straddle the SM groups of the chip, so this is
-    // less than SMs / csize: 15 clusters of 8 on 148 SMs); asked once.
+    // How many clusters of `csize` CTAs the current device holds at a time (clusters do not straddle the SM groups of the chip, so this
+    // is less than SMs / csize: 15 clusters of 8 on 148 SMs); asked once per device.
     static int active(const AttnParams& p, int csize) {
-        static std::atomic<int> known[kAsMaxCluster + 1];
-        int n = known[csize].load(std::memory_order_relaxed);
+        constexpr int kDevices = 64;
+        static std::atomic<int> known[kDevices][kAsMaxCluster + 1];
+        int dev = 0;
+        const bool keep = cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kDevices;
+        int n = keep ? known[dev][csize].load(std::memory_order_relaxed) : 0;
         if (n == 0) {
             cudaLaunchConfig_t cfg;
             cudaLaunchAttribute attr[2];
             config(cfg, attr, p, 1, csize, nullptr);
             if (cudaOccupancyMaxActiveClusters(&n, attn_stream_mma_kernel<HD, G, NW, NS, FUSED>, &cfg) != cudaSuccess || n < 1) n = 1;
-            known[csize].store(n, std::memory_order_relaxed);
+            if (keep) known[dev][csize].store(n, std::memory_order_relaxed);
         }
         return n;
     }
