@@ -58,11 +58,11 @@ __global__ void __launch_bounds__(kRowThreads) rope_kv_rows_kernel(uint16_t* q, 
 static size_t up256(size_t n) { return (n + 255) & ~static_cast<size_t>(255); }
 
 // Workspace: normed | q | k | v | attention output | h1 | SiLU*up | GEMM partial tiles
-struct RowsPlan {
+struct LayerPlan {
     size_t normed, q, k, v, attn, h1, mid, part, part_bytes, total;
 };
-static RowsPlan rows_plan(const nve_b200_rows_layer& L, int S) {
-    RowsPlan r;
+static LayerPlan layer_plan(const nve_b200_rows_layer& L, int S) {
+    LayerPlan r;
     const size_t qd = static_cast<size_t>(L.num_heads) * L.head_dim, kvd = static_cast<size_t>(L.num_kv_heads) * L.head_dim, s2 = 2 * static_cast<size_t>(S);
     size_t at = 0;
     auto take = [&](size_t bytes) {
@@ -111,7 +111,7 @@ using namespace nve;
 extern "C" size_t nve_b200_prefill_layer_workspace_bytes(const nve_b200_rows_layer* layer, int rows) {
     const int st = check_rows_layer(layer, rows);
     set_status(st);
-    return st == NVE_OK ? rows_plan(*layer, rows).total : 0;
+    return st == NVE_OK ? layer_plan(*layer, rows).total : 0;
 }
 
 extern "C" int nve_b200_prefill_layer(const nve_b200_rows_layer* layer, const uint16_t* hidden, uint16_t* out, int rows, int start_pos,
@@ -121,7 +121,7 @@ extern "C" int nve_b200_prefill_layer(const nve_b200_rows_layer* layer, const ui
     if (!hidden || !out || !workspace) return set_status(NVE_ERR_BAD_POINTER);
     if (start_pos < 0 || start_pos + rows > L.max_seq) return set_status(NVE_ERR_BAD_SHAPE);
     if (!aligned(hidden, 16) || !aligned(out, 16) || !aligned(workspace, 256)) return set_status(NVE_ERR_BAD_ALIGNMENT);
-    const RowsPlan r = rows_plan(L, rows);
+    const LayerPlan r = layer_plan(L, rows);
     if (workspace_bytes < r.total) return set_status(NVE_ERR_TOO_LARGE);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     unsigned char* ws = static_cast<unsigned char*>(workspace);
