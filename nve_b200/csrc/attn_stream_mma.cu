@@ -300,7 +300,7 @@ template <int HD, int G, int NW, int NS, bool FUSED> __global__ void __launch_bo
     if (csize > 1) cg::this_cluster().barrier_wait();  // all CTAs of the cluster run
     AdCtaPartial<HD, G>* parts = sm.parts;
     auto finish = [&](int i, float a, float ss, bool arrived) {
-        const uint16_t o16 = arrived ? Act16<NVE_DT_F16>::from_f32(ss > 0.0f ? a / ss : 0.0f) : static_cast<uint16_t>(0x7E00);  // NaN
+        const uint16_t o16 = arrived ? Act16<NVE_DT_F16>::from_f32(ss == 0.0f ? 0.0f : a / ss) : static_cast<uint16_t>(0x7E00);  // NaN
         const long long oi = static_cast<long long>(h0) * HD + i;
         p.out[oi] = o16;
         if (p.out_q != nullptr) {

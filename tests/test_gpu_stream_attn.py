@@ -91,3 +91,24 @@ def test_rows_never_written_do_not_reach_the_output(cuda, orc, nh, nkv, hd, max_
     # f16 probabilities (2^-11 of the largest |v| at most), one f16 rounding of the result, f32 scores in the exponent
     bound = (2.0 ** -10 + 2.0 ** -11) * vc[:, :pos + 1].double().abs().max().item()
     assert (got.double() - want).abs().max().item() < bound
+
+
+@pytest.mark.parametrize("B,max_seq", [(1, 2000), (3, 300), (40, 100)])
+def test_a_nan_score_gives_nan(cuda, orc, B, max_seq):
+    """A NaN in a key that a sequence sees, as in a softmax: NaN for the query heads of that KV head, the others keep their bits."""
+    from nve_b200 import cuda_kernels as ck
+
+    torch = cuda
+    nh, nkv, hd, f16 = 12, 4, 64, torch.float16
+    mk = lambda sid, *shape: dev(orc.to_act16(orc.fill_normal(int(torch.tensor(shape).prod()), 899, sid)), f16).view(*shape)
+    q, k, v, kc, vc = mk(1, B, nh * hd), mk(2, B, nkv * hd), mk(3, B, nkv * hd), mk(4, B, nkv, max_seq, hd), mk(5, B, nkv, max_seq, hd)
+    cos, sin = orc.rope_tables_f32(hd, max_seq, 10000.0)
+    cos, sin = dev(orc.to_act16(cos), f16), dev(orc.to_act16(sin), f16)
+    d_len = torch.full((B,), max_seq, dtype=torch.int32, device="cuda")
+    run = lambda: ck.attn_decode_fused_batch(q, k, v, kc, vc, cos, sin, d_len - 1, d_len, nh, nkv, hd, max_seq, hd ** -0.5).view(B, nkv, 3, hd).clone()
+    clean = run()
+    kc[B // 2, 1, max_seq // 3, 7] = float("nan")
+    got = run()
+    assert torch.isnan(got[B // 2, 1]).all()
+    got[B // 2, 1] = clean[B // 2, 1]
+    assert torch.equal(got, clean)
