@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kAmThreads, 1) attn_decode_mma_kernel(const At
         if (!have) am_load_tile<HD>(kh, vh, p0, t_end - 1, g, t, kr, vr);
         have = false;
         if (pos_ok) am_patch_tile<HD>(sh.knew_s, sh.vnew_s, p0, t_end - 1, pos, g, t, kr, vr);
-        am_tile<HD>(qa, kr, vr, p0, t_end, p.scale, t, m, l, o);
+        am_tile<HD, am_split(G)>(qa, kr, vr, p0, t_end, p.scale, t, m, l, o);
     }
 
     // ---- level 1: the warps' partials meet in shared memory; level 2: every CTA's partial goes to rank 0

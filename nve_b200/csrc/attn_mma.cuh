@@ -37,6 +37,19 @@ __device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
+// Group sizes whose probabilities are two f16 numbers, the upper 11 bits and the rest: as good as the 32-bit ones of the CUDA-core
+// kernel, which used to serve these sizes.  1, 2, 4 and 8 query heads per KV head take one f16 number, as they always did.  In a decode tile
+// the rests are unused rows of the A operand; in the tiled prefill they are half as many products again.  Probabilities and their sums are
+// scaled by 1024 then: f16 ends at 2^-24.  Error of 24 heads over 8 KV heads, 2-norm against 64 bits, one number / two / CUDA cores: 2000
+// positions 2.52e-4 / 2.08e-4 / 2.08e-4, a block of 300 behind 700 2.71e-4 / 2.07e-4 / -.  us: 7 sequences of a 3B model 1467 per step either
+// way, 300 rows at 700 of it 3503 / 3654.
+__host__ __device__ constexpr bool am_split(int groups) { return groups != 1 && groups != 2 && groups != 4 && groups != 8; }
+constexpr float kAmSplitLog2 = 10.0f, kAmSplitScale = 1024.0f;
+__device__ __forceinline__ uint32_t pack_f16x2_rest(float lo, float hi, uint32_t packed) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&packed));
+    return pack_f16x2(lo - f.x, hi - f.y);
+}
+
 // Loads of the tile at p0: K rows p0 + g, p0 + 8 + g (dims DPT*t ..), V rows p0 + {2t, 2t+1, 2t+8, 2t+9} (dims
 // NT*g ..); rows beyond `last` are clamped to it (their scores are masked by am_tile).
 template <int HD> __device__ __forceinline__ void am_load_tile(const uint16_t* kh, const uint16_t* vh, int p0, int last, int g, int t,
@@ -79,8 +92,9 @@ template <int HD> __device__ __forceinline__ void am_patch_tile(const uint16_t* 
 }
 
 // One tile into the warp's online-softmax state: m = running maximum of row g (equal on the four lanes of a row),
-// l = this lane's share of the sum of exponentials, o[j] = columns of the weighted V sum (o[j][0], o[j][1]: row g).
-template <int HD> __device__ __forceinline__ void am_tile(const uint32_t (&qa)[HD / 16][4], const uint4 (&kr)[2][HD / 32],
+// l = this lane's share of the sum of exponentials, o[j] = columns of the weighted V sum (o[j][0], o[j][1]: row g; SPLIT: o[j][2],
+// o[j][3]: the same for the rests of the probabilities).
+template <int HD, bool SPLIT> __device__ __forceinline__ void am_tile(const uint32_t (&qa)[HD / 16][4], const uint4 (&kr)[2][HD / 32],
                                                         const uint4 (&vr)[4][HD / 64], int p0, int seq_len, float scale, int t,
                                                         float& m, float& l, float (&o)[HD / 8][4]) {
     constexpr int NT = HD / 8, KK = HD / 16;
@@ -106,20 +120,24 @@ template <int HD> __device__ __forceinline__ void am_tile(const uint32_t (&qa)[H
     const float corr = __expf(m - m_new);
     float pe[4];
 #pragma unroll
-    for (int i = 0; i < 4; i++) pe[i] = sc[i] > -1e29f ? __expf(sc[i] - m_new) : 0.0f;
+    for (int i = 0; i < 4; i++) pe[i] = sc[i] > -1e29f ? (SPLIT ? kAmSplitScale * __expf(sc[i] - m_new) : __expf(sc[i] - m_new)) : 0.0f;
     l = l * corr + ((pe[0] + pe[1]) + (pe[2] + pe[3]));
     m = m_new;
 #pragma unroll
     for (int j = 0; j < NT; j++) {
         o[j][0] *= corr;
         o[j][1] *= corr;
+        if (SPLIT) {
+            o[j][2] *= corr;
+            o[j][3] *= corr;
+        }
     }
     // ---- outputs: p (f16) . V
     uint32_t pa[4];
     pa[0] = pack_f16x2(pe[0], pe[1]);
-    pa[1] = 0;
+    pa[1] = SPLIT ? pack_f16x2_rest(pe[0], pe[1], pa[0]) : 0;
     pa[2] = pack_f16x2(pe[2], pe[3]);
-    pa[3] = 0;
+    pa[3] = SPLIT ? pack_f16x2_rest(pe[2], pe[3], pa[2]) : 0;
     const uint32_t* v0 = reinterpret_cast<const uint32_t*>(&vr[0][0]);  // row p0 + 2t
     const uint32_t* v1 = reinterpret_cast<const uint32_t*>(&vr[1][0]);  // row p0 + 2t + 1
     const uint32_t* v2 = reinterpret_cast<const uint32_t*>(&vr[2][0]);  // row p0 + 8 + 2t
@@ -147,8 +165,9 @@ template <int HD, int G, class SH> __device__ __forceinline__ void am_store_warp
         }
 #pragma unroll
         for (int j = 0; j < NT; j++) {
-            sh.wo[warp][g][(NT + 1) * (2 * t) + j] = o[j][0];  // = am_wo_index(NT * (2t) + j)
-            sh.wo[warp][g][(NT + 1) * (2 * t + 1) + j] = o[j][1];
+            // = am_wo_index(NT * (2t) + j)
+            sh.wo[warp][g][(NT + 1) * (2 * t) + j] = am_split(G) ? o[j][0] + o[j][2] : o[j][0];
+            sh.wo[warp][g][(NT + 1) * (2 * t + 1) + j] = am_split(G) ? o[j][1] + o[j][3] : o[j][1];
         }
     }
 }

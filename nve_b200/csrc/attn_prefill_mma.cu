@@ -69,7 +69,7 @@ template <int HD> constexpr int ap_smem_bytes() {
 // would turn into NaN.  So a CTA that finds an output that is not finite stores nothing and says false, and the tile is computed once more,
 // CAREFUL: in the steps that are cut such elements go to the rows that see them one by one and are zeros in the product.  (In line, as a
 // branch of the steps, this cost 0.7 to 3 us per launch in a prefill of 61 rows, 8B; so 0.3.)
-template <int HD, bool CAREFUL>
+template <int HD, bool SPLIT, bool CAREFUL>
 __device__ __forceinline__ bool ap_tile(const AttnParams& p, int groups, int tiles) {
     extern __shared__ __align__(128) unsigned char ap_raw[];
     constexpr int CH = HD / 8;  // 16-byte chunks per row
@@ -168,13 +168,13 @@ __device__ __forceinline__ bool ap_tile(const AttnParams& p, int groups, int til
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
             const float mn = fmaxf(m[hh], mx * sl2);  // stays finite: the masked value is below -1e30
-            const float corr = ap_exp2(m[hh] - mn);
+            const float corr = ap_exp2(m[hh] - mn), shift = SPLIT ? kAmSplitLog2 - mn : -mn;
             m[hh] = mn;
             float sum = 0.0f;
 #pragma unroll
             for (int n = 0; n < 8; n++) {
-                s[n][2 * hh] = ap_exp2(fmaf(s[n][2 * hh], sl2, -mn));
-                s[n][2 * hh + 1] = ap_exp2(fmaf(s[n][2 * hh + 1], sl2, -mn));
+                s[n][2 * hh] = ap_exp2(fmaf(s[n][2 * hh], sl2, shift));
+                s[n][2 * hh + 1] = ap_exp2(fmaf(s[n][2 * hh + 1], sl2, shift));
                 sum += s[n][2 * hh] + s[n][2 * hh + 1];
             }
             l[hh] = l[hh] * corr + sum;
@@ -215,14 +215,15 @@ __device__ __forceinline__ bool ap_tile(const AttnParams& p, int groups, int til
             }
             __syncthreads();
         }
-        uint32_t pa[4][4];
+        uint32_t pa[4][4], pb[4][4];
 #pragma unroll
-        for (int kp = 0; kp < 4; kp++) {  // probabilities of 16 positions as the A operand of the second product
-            pa[kp][0] = pack_f16x2(s[2 * kp][0], s[2 * kp][1]);
-            pa[kp][1] = pack_f16x2(s[2 * kp][2], s[2 * kp][3]);
-            pa[kp][2] = pack_f16x2(s[2 * kp + 1][0], s[2 * kp + 1][1]);
-            pa[kp][3] = pack_f16x2(s[2 * kp + 1][2], s[2 * kp + 1][3]);
-        }
+        for (int kp = 0; kp < 4; kp++)  // probabilities of 16 positions as the A operand of the second product
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float p0 = s[2 * kp + (i >> 1)][2 * (i & 1)], p1 = s[2 * kp + (i >> 1)][2 * (i & 1) + 1];
+                pa[kp][i] = pack_f16x2(p0, p1);
+                pb[kp][i] = SPLIT ? pack_f16x2_rest(p0, p1, pa[kp][i]) : 0;
+            }
 #pragma unroll
         for (int kp = 0; kp < 4; kp++)
 #pragma unroll
@@ -231,6 +232,10 @@ __device__ __forceinline__ bool ap_tile(const AttnParams& p, int groups, int til
                 ap_ldm4t(vb + ap_off<HD>(kp * 16 + (lane & 15), 2 * dp + (lane >> 4)), b);
                 mma_f16_16816(o[2 * dp], pa[kp], b[0], b[1]);
                 mma_f16_16816(o[2 * dp + 1], pa[kp], b[2], b[3]);
+                if (SPLIT) {
+                    mma_f16_16816(o[2 * dp], pb[kp], b[0], b[1]);
+                    mma_f16_16816(o[2 * dp + 1], pb[kp], b[2], b[3]);
+                }
             }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -354,16 +359,18 @@ __device__ __forceinline__ bool ap_tile(const AttnParams& p, int groups, int til
     return true;
 }
 
-template <int HD> __device__ __noinline__ void ap_tile_careful(const AttnParams& p, int groups, int tiles) { ap_tile<HD, true>(p, groups, tiles); }
-
-template <int HD>
-__global__ void __launch_bounds__(kApThreads, 2) attn_prefill_mma_kernel(const __grid_constant__ AttnParams p, int groups, int tiles) {
-    if (!ap_tile<HD, false>(p, groups, tiles)) ap_tile_careful<HD>(p, groups, tiles);
+template <int HD, bool SPLIT> __device__ __noinline__ void ap_tile_careful(const AttnParams& p, int groups, int tiles) {
+    ap_tile<HD, SPLIT, true>(p, groups, tiles);
 }
 
-template <int HD> static cudaError_t launch_ap(const AttnParams& p, cudaStream_t st) {
+template <int HD, bool SPLIT>
+__global__ void __launch_bounds__(kApThreads, 2) attn_prefill_mma_kernel(const __grid_constant__ AttnParams p, int groups, int tiles) {
+    if (!ap_tile<HD, SPLIT, false>(p, groups, tiles)) ap_tile_careful<HD, SPLIT>(p, groups, tiles);
+}
+
+template <int HD, bool SPLIT> static cudaError_t launch_ap(const AttnParams& p, cudaStream_t st) {
     constexpr int smem = ap_smem_bytes<HD>();
-    if (ensure_dynamic_smem(reinterpret_cast<const void*>(attn_prefill_mma_kernel<HD>), smem) != NVE_OK) return cudaErrorInvalidValue;
+    if (ensure_dynamic_smem(reinterpret_cast<const void*>(attn_prefill_mma_kernel<HD, SPLIT>), smem) != NVE_OK) return cudaErrorInvalidValue;
     const int groups = p.num_heads / p.num_kv_heads;
     const int PT = kApRows / groups;
     const int tiles = (p.rows + PT - 1) / PT;
@@ -389,13 +396,14 @@ template <int HD> static cudaError_t launch_ap(const AttnParams& p, cudaStream_t
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.numAttrs = 2;
     }
-    return cudaLaunchKernelEx(&cfg, attn_prefill_mma_kernel<HD>, p, groups, tiles);
+    return cudaLaunchKernelEx(&cfg, attn_prefill_mma_kernel<HD, SPLIT>, p, groups, tiles);
 }
 
 bool attn_prefill_mma_try(const AttnParams& p, int head_dim, cudaStream_t st, cudaError_t& err) {
     if (p.num_heads / p.num_kv_heads > kApRows || p.num_kv_heads > 65535) return false;
-    if (head_dim == 128) err = launch_ap<128>(p, st);
-    else if (head_dim == 64) err = launch_ap<64>(p, st);
+    const bool split = am_split(p.num_heads / p.num_kv_heads);
+    if (head_dim == 128) err = split ? launch_ap<128, true>(p, st) : launch_ap<128, false>(p, st);
+    else if (head_dim == 64) err = split ? launch_ap<64, true>(p, st) : launch_ap<64, false>(p, st);
     else return false;
     return true;
 }

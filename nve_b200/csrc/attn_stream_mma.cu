@@ -86,6 +86,7 @@ template <int HD, int G, int NW, int NS, bool FUSED> __global__ void __launch_bo
         seq_len_row += static_cast<int>(b);
     }
     constexpr int HALF = HD / 2, DC = HD / 8, NT = HD / 8;
+    constexpr bool SPLIT = am_split(G);
     static_assert((HD == 64 || HD == 128) && G >= 1 && G <= 8, "head_dim 64 or 128, up to 8 query heads per KV head");
     static_assert(HD <= (32 * NW) && G * (HD + 8) * 4 <= NS * 2 * 16 * HD * 2, "one element of v per thread; a partial fits its ring");
     extern __shared__ __align__(16) unsigned char as_raw[];
@@ -261,9 +262,13 @@ template <int HD, int G, int NW, int NS, bool FUSED> __global__ void __launch_bo
         const float corr = as_exp2(m - mn);
         m = mn;
 #pragma unroll
-        for (int e = 0; e < 4; e++) sc[e] = as_exp2(sc[e] - mn);
+        for (int e = 0; e < 4; e++) sc[e] = as_exp2(SPLIT ? sc[e] - (mn - kAmSplitLog2) : sc[e] - mn);
         l = l * corr + ((sc[0] + sc[1]) + (sc[2] + sc[3]));
-        const uint32_t pa[4] = {pack_f16x2(sc[0], sc[1]), 0, pack_f16x2(sc[2], sc[3]), 0};
+        uint32_t pa[4] = {pack_f16x2(sc[0], sc[1]), 0, pack_f16x2(sc[2], sc[3]), 0};
+        if (SPLIT) {  // the rests in rows g + 8
+            pa[1] = pack_f16x2_rest(sc[0], sc[1], pa[0]);
+            pa[3] = pack_f16x2_rest(sc[2], sc[3], pa[2]);
+        }
 #pragma unroll
         for (int j = 0; j < NT; j += 2) {
             uint32_t vb[4];  // dims 8j .. + 7 (vb[0], vb[1]) and the next eight (vb[2], vb[3]) of the sixteen positions
@@ -271,10 +276,10 @@ template <int HD, int G, int NW, int NS, bool FUSED> __global__ void __launch_bo
             float d0[4] = {o[j][0] * corr, o[j][1] * corr, 0, 0}, d1[4] = {o[j + 1][0] * corr, o[j + 1][1] * corr, 0, 0};
             mma_f16_16816(d0, pa, vb[0], vb[1]);
             mma_f16_16816(d1, pa, vb[2], vb[3]);
-            o[j][0] = d0[0];
-            o[j][1] = d0[1];
-            o[j + 1][0] = d1[0];
-            o[j + 1][1] = d1[1];
+            o[j][0] = SPLIT ? d0[0] + d0[2] : d0[0];
+            o[j][1] = SPLIT ? d0[1] + d0[3] : d0[1];
+            o[j + 1][0] = SPLIT ? d1[0] + d1[2] : d1[0];
+            o[j + 1][1] = SPLIT ? d1[1] + d1[3] : d1[1];
         }
         __syncwarp();  // every lane has read the tile
         load(p0 + 16 * NW * NS, st);

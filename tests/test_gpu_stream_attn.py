@@ -112,3 +112,52 @@ def test_a_nan_score_gives_nan(cuda, orc, B, max_seq):
     assert torch.isnan(got[B // 2, 1]).all()
     got[B // 2, 1] = clean[B // 2, 1]
     assert torch.equal(got, clean)
+
+
+@pytest.mark.parametrize("nh,nkv,hd,max_seq,lens,S", [
+    (24, 8, 128, 700, [700], 0),                          # the latency kernel
+    (21, 3, 64, 1280, [1111], 0),
+    (12, 2, 64, 2500, [2500], 0),                         # the streaming kernel over clusters
+    (24, 8, 128, 4000, [4000, 1733, 901], 0),
+    (10, 2, 128, 900, [900 - 7 * i for i in range(80)], 0),  # four warps per unit
+    (24, 8, 128, 1000, [1], 300),                         # blocks of positions: in tiles, the positions split over a cluster or not
+    (5, 1, 64, 3000, [1], 70),
+    (16, 1, 128, 600, [1], 200),
+    (24, 8, 128, 500, [1], 3),                            # row by row
+])
+def test_probabilities_of_the_other_group_sizes_keep_32_bits(cuda, orc, nh, nkv, hd, max_seq, lens, S):
+    """Group sizes other than 1, 2, 4 and 8: what is left of the error is the rounding of the result to f16 (2.0e-4 of its 2-norm); one f16
+    number per probability would add as much again (2.9e-4 in all)."""
+    from nve_b200 import cuda_kernels as ck
+
+    torch = cuda
+    B, G, f16 = len(lens), nh // nkv, torch.float16
+    mk = lambda sid, *shape: dev(orc.to_act16(orc.fill_normal(int(torch.tensor(shape).prod()), 897, sid)), f16).view(*shape)
+    kc, vc = mk(4, B, nkv, max_seq, hd), mk(5, B, nkv, max_seq, hd)
+    if S:
+        start = max_seq - S
+        q = mk(1, S, nh * hd)
+        got = ck.attn_prefill_causal(q, kc[0], vc[0], start, nh, nkv, hd, max_seq, hd ** -0.5).view(S, nkv, G, hd)
+        seen = torch.arange(max_seq, device="cuda")[None, :] <= torch.arange(start, max_seq, device="cuda")[:, None]
+        s = torch.einsum("skgd,kld->skgl", q.double().view(S, nkv, G, hd), kc[0].double()) * hd ** -0.5
+        want = torch.einsum("skgl,kld->skgd", s.masked_fill(~seen[:, None, None, :], float("-inf")).softmax(-1), vc[0].double())
+    else:
+        q, k, v = mk(1, B, nh * hd), mk(2, B, nkv * hd), mk(3, B, nkv * hd)
+        cos, sin = orc.rope_tables_f32(hd, max_seq, 10000.0)
+        cos, sin = dev(orc.to_act16(cos), f16), dev(orc.to_act16(sin), f16)
+        d_len = torch.tensor(lens, dtype=torch.int32, device="cuda")
+        d_pos = d_len - 1
+        got = torch.empty((B, nh * hd), dtype=f16, device="cuda")
+        if B == 1:
+            ck.attn_decode_fused(q, k, v, kc, vc, cos, sin, d_pos.data_ptr(), d_len.data_ptr(), got, nh, nkv, hd, max_seq, hd ** -0.5)
+        else:
+            ck.attn_decode_fused_batch(q, k, v, kc, vc, cos, sin, d_pos, d_len, nh, nkv, hd, max_seq, hd ** -0.5, out=got)
+        want = []
+        for b, n in enumerate(lens):
+            q1, k1 = q[b].clone().view(nh, hd), k[b].clone().view(nkv, hd)
+            ck.rope_decode_dyn_inplace(q1, k1, cos, sin, nh, nkv, hd, d_pos[b:b + 1].data_ptr())
+            s = torch.einsum("kgd,kld->kgl", q1.double().view(nkv, G, hd), kc[b, :, :n].double()) * hd ** -0.5
+            want.append(torch.einsum("kgl,kld->kgd", s.softmax(-1), vc[b, :, :n].double()).reshape(-1))
+        want = torch.stack(want)
+    want = want.reshape(got.shape)
+    assert ((got.double() - want).norm() / want.norm()).item() < 2.3e-4
