@@ -39,3 +39,21 @@ def cuda():
     _ffi.load()
     torch.cuda.set_device(0)
     return torch
+
+
+def pytest_generate_tests(metafunc):
+    """Every test on one GPU runs twice: with programmatic dependent launch off (the library's default) and on (what decoding programs and the
+    benchmark switch on), where a kernel may start while the one in front still runs."""
+    gpu = metafunc.definition.get_closest_marker("gpu") is not None
+    if gpu and "cuda" in metafunc.fixturenames and metafunc.module.__name__ != "test_gpu_tp":
+        metafunc.fixturenames.append("dependent_launch")
+        metafunc.parametrize("dependent_launch", [False, True], ids=["launch_after", "dependent_launch"], indirect=True)
+
+
+@pytest.fixture
+def dependent_launch(request, cuda):
+    from nve_b200 import cuda_kernels as ck
+
+    was = ck.set_pdl(request.param)
+    yield request.param
+    ck.set_pdl(was)
