@@ -1,10 +1,6 @@
-"""GPU parity: the batched W4A16 GEMM (mma.sync kernel up to 8 batch rows, tcgen05 kernel above) against the
+"""GPU parity: the batched W4A16 GEMM (mma.sync kernel up to 8 batch rows where it has a workspace, tcgen05 kernel otherwise) against the
 reference's CPU semantics (q4_linear: one f32 GEMV per row of X, src/quantize.rs:1057-1075) on the same
 16-bit-rounded activations."""
-import os
-import subprocess
-import sys
-
 import numpy as np
 import pytest
 
@@ -119,8 +115,7 @@ def test_gemm_rejects_bad_arguments(cuda):
 @pytest.mark.parametrize("M", [1, 5, 64, 100, 130, 300])
 @pytest.mark.parametrize("with_awq", [False, True])
 def test_matmul_x_matches_q4_linear(cuda, orc, M, with_awq):
-    """gpu_layer.matmul_x (the batch > 1 call site: GEMV at M == 1, the fused GEMM walked in 64-row slices up to
-    128 rows, dequantisation + dense GEMM above)
+    """gpu_layer.matmul_x (the batch > 1 call site: GEMV at M == 1, the packed GEMM for any number of rows)
     against the reference's CPU semantics q4_linear on the same 16-bit activations."""
     from nve_b200.gpu_layer import GpuW4, matmul_x
 
@@ -139,8 +134,7 @@ def test_matmul_x_matches_q4_linear(cuda, orc, M, with_awq):
 
 
 def test_matmul_x_dense_route_bf16(cuda, orc):
-    """Above 128 rows matmul_x dequantises to f16 and calls the dense GEMM; bf16 activations are converted to f16
-    for it and the result is rounded to bf16 once (judged on the f32 reference within bf16's own rounding)."""
+    """bf16 activations above 128 rows: converted to f16 for the GEMM, the result rounded to bf16 once (judged on the f32 reference within bf16's own rounding)."""
     from nve_b200.gpu_layer import DENSE_ROWS, GpuW4, matmul_x
 
     torch = cuda
@@ -220,15 +214,22 @@ def test_matmul_x_of_a_workspace_for_64_rows_and_of_no_rows(cuda, orc):
         assert [tuple(t.shape) for t in matmul_x_multi(x[:0], [w, w])] == [(0, N)] * 2
 
 
-@pytest.mark.parametrize("kernel", ["mma", "tc"])
-def test_gemm_parity_with_each_kernel_forced(cuda, kernel):
-    """The library picks the kernel by batch size; NVE_B200_GEMM_KERNEL (read once per process) forces one.  The
-    parity cases above are run again in a child process with each kernel forced, so that the mma.sync kernel is
-    also checked at 16 and 32 batch rows and the tcgen05 kernel at 8 and fewer."""
-    if os.environ.get("NVE_B200_GEMM_KERNEL_CHILD"):
-        pytest.skip("already inside the forced-kernel child run")
-    env = dict(os.environ, NVE_B200_GEMM_KERNEL=kernel, NVE_B200_GEMM_KERNEL_CHILD="1")
-    res = subprocess.run([sys.executable, "-m", "pytest", os.path.abspath(__file__), "-q", "-x", "-m", "gpu", "-k",
-                          "tensor_core or multi_matrix", "-p", "no:cacheprovider"],
-                         env=env, capture_output=True, text=True, timeout=900, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
-    assert res.returncode == 0, res.stdout[-3000:] + res.stderr[-2000:]
+@pytest.mark.parametrize("M,N,K", [(1, 256, 64), (3, 300, 320), (8, 384, 2048), (7, 1000, 4096), (2, 19000, 1280), (5, 40000, 128)])
+def test_few_rows_on_each_kernel(cuda, orc, M, N, K):
+    """Up to eight rows: the kernel for few rows (two launches: it always leaves partial tiles) where the workspace holds its partial
+    tiles and no run is longer than a tile, else the two-SM kernel, in whole tiles (one launch) where the workspace holds nothing."""
+    from nve_b200 import cuda_kernels as ck
+
+    torch = cuda
+    nib, sc, X16, ref = _case(orc, M, N, K, 990, False)
+    dx, dn, ds = dev(X16, torch.float16), dev(nib), dev(sc)
+    tall = -(-N // 256) > torch.cuda.get_device_properties(0).multi_processor_count  # more tiles than SMs: runs of whole tiles
+    full = torch.empty(ck.gemm_w4a16_scratch_bytes(M, N, K), dtype=torch.uint8, device="cuda")
+    for scratch, launches in ((None, 1), (full[:16], 1), (full, None if tall else 2)):
+        out = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
+        before = ck.launch_count()
+        ck.gemm_w4a16(dx, dn, ds, N, K, out_dtype=torch.float32, out=out, scratch=scratch)
+        assert launches is None or ck.launch_count() - before == launches
+        torch.cuda.synchronize()
+        assert ck.gemm_error() == 0
+        assert rel_rms_err(out.cpu().numpy(), ref) < 3e-3  # f16 rounding of the weights, as above
