@@ -218,11 +218,11 @@ NVE_API int nve_b200_silu_mul(void* gate, const void* up, int n, int dtype, nve_
  *   src/gpu_layer.rs:814-818.
  * nve_b200_attn_prefill_causal: row r of q [rows, num_heads * head_dim] attends to positions [0, start_pos + r] of the
  *   caches (which already hold the block); out has q's layout.  Replaces the unfused masked SDPA of
- *   src/gpu_layer.rs:846-885.  Blocks of fewer than 64 (row, KV head) pairs run the decode kernel with the row as
- *   second grid dimension: every row equals a nve_flash_decode_f16 call of length start_pos + r + 1 bit for bit.
- *   Larger blocks run a tiled tensor-core kernel (128 query rows share the K/V they read; f16 probabilities, another
- *   summation order): equal to those calls within 5e-3 of the largest output.  head_dim 64 or 128; q and caches 16-byte
- *   aligned. */
+ *   src/gpu_layer.rs:846-885.  Blocks of fewer than 64 (row, KV head) pairs, and of up to two such pairs per SM behind
+ *   a short prefix, run the streaming decode kernel with the row as second grid dimension, others a tiled tensor-core kernel
+ *   (64 query rows share the K/V they read).  A row equals a nve_flash_decode_f16 call of length start_pos + r + 1 within
+ *   5e-3 of the largest output (the order of the sums follows kernel and split), and bit for bit with fewer than 64 pairs and
+ *   max_seq_len up to 128.  head_dim 64 or 128; q and caches 16-byte aligned. */
 NVE_API int nve_b200_rms_norm_rows(const void* x, const void* weight, void* out, int rows, int n, float eps, int dtype,
                                    nve_stream_t stream);
 /* x[r] += delta[r] in place (nve_b200_add_inplace's arithmetic) and out[r] = RMSNorm(x[r]) for every row, one launch:
@@ -329,7 +329,8 @@ NVE_API int nve_b200_quantize_matvec_w4a8_allreduce(const void* x, int x_dtype, 
  * 128.  Results -- cache row, output and int8 codes -- are bit-identical to the separate RoPE, KV-write,
  * flash-decode and quantise launches of this library.
  * By default this entry point, nve_flash_decode_f16 / _dyn and the small blocks of nve_b200_attn_prefill_causal run the
- * tensor-core kernels (all query heads of a KV head as rows of mma.sync, f16 probabilities; which of them follows from the
+ * tensor-core kernels (all query heads of a KV head as rows of mma.sync, probabilities in f16, with 3, 5, 6 or 7 heads in two
+ * f16 numbers; which of them follows from the
  * size of the cache) when there are up to 8 query heads per KV head and the pointers are 16-byte aligned;
  * nve_b200_set_attn_decode_kernel(1) selects the CUDA-core kernel for all of them (also used for other shapes; it is the
  * arithmetic of the persistent one-kernel step), 0 restores the default.  They agree within 5e-3 of the largest output.
@@ -383,7 +384,8 @@ NVE_API int nve_b200_fill_normal_16(void* out, long long n, unsigned long long s
 
 /* Batched W4A16 GEMM for decode batches 1 < M <= 64 on the tensor cores: Y[M,N] = X[M,K] . W^T with the packed
  * weights read once and dequantised on the fly (replaces nve_dequant_w4a16 + dense GEMM,
- * src/gpu_layer.rs:220-239): they go to tensor memory and pairs of SMs multiply them with tcgen05.mma.
+ * src/gpu_layer.rs:220-239): they go to tensor memory and pairs of SMs multiply them with tcgen05.mma, or, up to 8
+ * rows with a workspace for it, stay in registers for mma.sync.
  * X and Y are row-major; x_dtype f16 or bf16, y_dtype = x_dtype or f32; K % 64 == 0; X and nibbles 16-byte aligned,
  * scales 8-byte aligned.  Weights are rounded to f16 as (q-8)*scale like the reference's dequantisation;
  * accumulation is f32.

@@ -793,7 +793,7 @@ __global__ void __launch_bounds__(kPairNormThreads) gemm_pair_reduce_norm_kernel
 }
 
 // More rows of X than SMs: the blocks hide each other's latency and a thread keeps its chunks of the row in registers, all of
-// their loads under way together (o projection with its finish, 8B, 1777 rows: 89.7 us with the form above, 73.8 with this one; 300
+// their loads under way together (o projection with its finish, 8B, 1777 rows: 78.7 us with the form above, 73.4 with this one; 300
 // rows 25.6 and 23.5; at 147 and 149 rows, each with its own form, 15.5 and 16.5).
 __global__ void __launch_bounds__(256) gemm_pair_reduce_norm_rows_kernel(const PairParams p, const uint16_t* norm_w, uint16_t* normed, float eps) {
     __shared__ float warp_part[8];

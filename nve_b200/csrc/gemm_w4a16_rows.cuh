@@ -4,7 +4,8 @@
 // With so few rows the two-SM kernel's fixed costs (cluster start, TMEM, operand rings, the drain of a tile) are a large part of
 // a call.  Here a warp streams 16 weight rows like a decode GEMV does -- 16 bytes (a block of 32) per lane and row, kRowsDepth
 // units ahead, the first of them before the grid dependency resolves -- and multiplies them by mma.sync (m16n8k16).  The four
-// GEMMs of a layer with 7 rows, us: 1B 41.4 -> 36, 3B 50.0 -> 44.7, 8B 69.3 -> 66; with more rows than fill one mma (15: 74 against
+// GEMMs of a layer with 7 rows, us: 1B 41.4 -> 36, 3B 50.0 -> 44.7, 8B 69.3 -> 66 (not the largest matrices: 8B gate/up and down take
+// 27.3 and 16.6 here with 8 rows, 24.2 and 15.2 there with 16); with more rows than fill one mma (15: 74 against
 // 70) the multiplications no longer hide behind the weights.  What is left is the dequantisation (two thirds of the issue
 // slots), the weights' latency and the two launches.  Taken back: two CTAs per SM (small matrices 1 to 2 us slower), more units
 // in flight with them (slower still).
