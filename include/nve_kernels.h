@@ -327,7 +327,7 @@ NVE_API int nve_b200_quantize_matvec_w4a8_allreduce(const void* x, int x_dtype, 
  * [nkv, max_seq_len, hd]; tables [max_seq_len, hd/2]; out [nh,hd] f16.  When out_q / out_scales are given
  * the output is also quantised to int8 per group of 32 (the call at src/gpu_layer.rs:739).  head_dim 64 or
  * 128.  Results -- cache row, output and int8 codes -- are bit-identical to the separate RoPE, KV-write,
- * flash-decode and quantise launches of this library.
+ * flash-decode (nve_flash_decode_dyn with the same max_seq_len) and quantise launches of this library.
  * By default this entry point, nve_flash_decode_f16 / _dyn and the small blocks of nve_b200_attn_prefill_causal run the
  * tensor-core kernels (all query heads of a KV head as rows of mma.sync, probabilities in f16, with 3, 5, 6 or 7 heads in two
  * f16 numbers; which of them follows from the
