@@ -348,6 +348,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
             }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
+        // not before the kernel in front is complete: what starts then may read what was written two launches ahead of it
+        pdl_wait();
         pdl_launch_dependents();
         pg_cluster_wait();
     } else {

@@ -127,3 +127,39 @@ def test_fused_attention_of_successive_positions(cuda, orc, nh, nkv, hd, max_seq
         ck.set_attn_decode_kernel(prev)
     assert torch.isfinite(off[0].float()).all()
     assert all(torch.equal(a, b) for a, b in zip(off, on))
+
+
+@pytest.mark.parametrize("M,N,K", [(9, 64, 64), (64, 2048, 256)])
+def test_fused_attention_two_launches_behind(cuda, orc, M, N, K):
+    """Attention of a position, a GEMM of another size, attention two positions on: rows that the first wrote are read early by the last, which
+    may start when the GEMM's loads are done -- but not before the first is complete."""
+    from nve_b200 import cuda_kernels as ck
+
+    torch = cuda
+    nh, nkv, hd, max_seq, pos, f16 = 64, 8, 128, 1200, 1000, torch.float16
+    q, k, v = (_normal(torch, orc, (2, h * hd), 1130, i) for i, h in enumerate((nh, nkv, nkv)))
+    cos, sin = orc.rope_tables_f32(hd, max_seq, 10000.0)
+    cos, sin = dev(orc.to_act16(cos), f16), dev(orc.to_act16(sin), f16)
+    old = [_normal(torch, orc, (nkv, max_seq, hd), 1131, i) for i in range(2)]
+    d_pos = torch.tensor([pos, pos + 40], dtype=torch.int32, device="cuda")
+    d_len = d_pos + 1
+    nib, sc = ck.q4_quantize(ck.fill_normal(N * K, 1132, 1, scale=0.02).view(N, K))
+    x = _normal(torch, orc, (M, K), 1133, 1)
+
+    def run():
+        outs = []
+        y = torch.empty((M, N), dtype=f16, device="cuda")
+        for _ in range(8):
+            kc, vc = (t.clone() for t in old)
+            kc[:, pos], vc[:, pos], kc[:, pos + 40:], vc[:, pos + 40:] = (float("nan"),) * 4
+            out = torch.zeros((2, nh, hd), dtype=f16, device="cuda")
+            torch.cuda.synchronize()
+            ck.attn_decode_fused(q[0], k[0], v[0], kc, vc, cos, sin, d_pos.data_ptr(), d_len.data_ptr(), out[0], nh, nkv, hd, max_seq, hd ** -0.5)
+            ck.gemm_w4a16(x, nib, sc, N, K, out=y)
+            ck.attn_decode_fused(q[1], k[1], v[1], kc, vc, cos, sin, d_pos[1:].data_ptr(), d_len[1:].data_ptr(), out[1], nh, nkv, hd, max_seq, hd ** -0.5)
+            outs.append(out)
+        return outs
+
+    off, on = _both(ck, torch, run)
+    assert all(torch.isfinite(t.float()).all() for t in off)
+    assert all(torch.equal(a, b) for a, b in zip(off, on))
