@@ -68,6 +68,11 @@ long integer(PyObject* o) {
     if (v == -1 && PyErr_Occurred()) throw Failed();
     return v;
 }
+double number(PyObject* o) {
+    const double v = PyFloat_AsDouble(o);
+    if (v == -1.0 && PyErr_Occurred()) throw Failed();
+    return v;
+}
 void expect(Py_ssize_t have, Py_ssize_t want, const char* name) {
     if (have != want) fail(PyExc_TypeError, "%s: wrong number of arguments", name);
 }
@@ -269,6 +274,71 @@ PyObject* q4_quantize(PyObject*, PyObject* const* a, Py_ssize_t na) {
     });
 }
 
+// prefill_layer(hidden [S, H] f16, ((nibbles, scales, n, k) of q, k, v, o, gate, up, down), input norm, post-attention norm, K cache, V cache,
+//               rope cos, rope sin, heads, KV heads, head_dim, max_seq, eps, scale, start_pos) -> [S, H] f16, or None where the
+// sizes do not fit together or the library does not cover them: the caller then issues the launches one by one.
+PyObject* prefill_layer(PyObject*, PyObject* const* a, Py_ssize_t na) {
+    return guarded([&]() -> PyObject* {
+        expect(na, 15, "prefill_layer");
+        const at::Tensor& x = tensor(a[0], "hidden");
+        const auto* xp = static_cast<const uint16_t*>(typed_ptr(x, at::kHalf, "hidden"));
+        if (x.dim() != 2) fail(PyExc_ValueError, "%s must be [S, hidden]", "hidden");
+        if (!PyTuple_Check(a[1]) || PyTuple_GET_SIZE(a[1]) != 7) fail(PyExc_TypeError, "%s: seven projections", "prefill_layer");
+        const int64_t rows = x.size(0), h = x.size(1), nh = integer(a[8]), nkv = integer(a[9]), hd = integer(a[10]), max_seq = integer(a[11]);
+        nve_b200_rows_layer L;
+        int64_t n[7], k[7];
+        bool fits = rows <= 65535 && h <= 0x7FFFFFFF && nh > 0 && nkv > 0 && nh <= 65536 && nkv <= 65536 && hd > 0 && hd <= 65536 && max_seq > 0 &&
+                    max_seq <= 0x7FFFFFFF;
+        for (int i = 0; i < 7; i++) {
+            PyObject* p = PyTuple_GET_ITEM(a[1], i);
+            if (!PyTuple_Check(p) || PyTuple_GET_SIZE(p) != 4) fail(PyExc_TypeError, "%s: a projection is (nibbles, scales, n, k)", "prefill_layer");
+            const at::Tensor &nib = tensor(PyTuple_GET_ITEM(p, 0), "nibbles"), &sc = tensor(PyTuple_GET_ITEM(p, 1), "scales");
+            L.nibbles[i] = static_cast<const uint8_t*>(typed_ptr(nib, at::kByte, "nibbles"));
+            L.scales[i] = static_cast<const float*>(typed_ptr(sc, at::kFloat, "scales"));
+            n[i] = integer(PyTuple_GET_ITEM(p, 2));
+            k[i] = integer(PyTuple_GET_ITEM(p, 3));
+            fits = fits && n[i] > 0 && n[i] <= 0x7FFFFFFF && k[i] > 0 && k[i] <= 0x7FFFFFFF && nib.numel() == n[i] * k[i] / 2 && sc.numel() == n[i] * k[i] / 32;
+        }
+        const int64_t q = nh * hd, kv = nkv * hd, ffn = n[4];
+        const int64_t want_n[7] = {q, kv, kv, h, ffn, ffn, h}, want_k[7] = {h, h, h, q, h, h, ffn};
+        for (int i = 0; i < 7; i++) fits = fits && n[i] == want_n[i] && k[i] == want_k[i];
+        auto vec = [&](int i, const char* name, int64_t least, bool exact) {
+            const at::Tensor& t = tensor(a[i], name);
+            fits = fits && (exact ? t.numel() == least : t.numel() >= least);
+            return static_cast<uint16_t*>(typed_ptr(t, at::kHalf, name));
+        };
+        L.input_norm = vec(2, "input norm", h, true);
+        L.post_attn_norm = vec(3, "post-attention norm", h, true);
+        L.k_cache = vec(4, "k cache", kv * max_seq, true);
+        L.v_cache = vec(5, "v cache", kv * max_seq, true);
+        L.rope_cos = vec(6, "rope cos", max_seq * (hd / 2), false);
+        L.rope_sin = vec(7, "rope sin", max_seq * (hd / 2), false);
+        L.norm_eps = static_cast<float>(number(a[12]));
+        L.attn_scale = static_cast<float>(number(a[13]));
+        const int64_t start = integer(a[14]);
+        at::Tensor out;
+        int st = NVE_OK;
+        if (fits && start >= 0 && start + rows <= max_seq) {
+            L.hidden = static_cast<int>(h);
+            L.ffn = static_cast<int>(ffn);
+            L.num_heads = static_cast<int>(nh);
+            L.num_kv_heads = static_cast<int>(nkv);
+            L.head_dim = static_cast<int>(hd);
+            L.max_seq = static_cast<int>(max_seq);
+            WithoutGil others;
+            if (const size_t need = nve_b200_prefill_layer_workspace_bytes(&L, static_cast<int>(rows)); need > 0) {
+                at::Tensor ws = empty({static_cast<int64_t>(need)}, at::kByte, x);  // blocks of the caching allocator are 512-byte aligned
+                out = empty({rows, h}, at::kHalf, x);
+                st = nve_b200_prefill_layer(&L, xp, static_cast<uint16_t*>(out.data_ptr()), static_cast<int>(rows), static_cast<int>(start), ws.data_ptr(),
+                                            need, current_stream());
+            }
+        }
+        status("nve_b200_prefill_layer", st);
+        if (!out.defined()) Py_RETURN_NONE;
+        return wrap(std::move(out));
+    });
+}
+
 // set_capture_stream(stream | 0): where this thread's calls go while a graph is recorded
 PyObject* set_capture_stream(PyObject*, PyObject* const* a, Py_ssize_t na) {
     return guarded([&] {
@@ -298,7 +368,7 @@ PyObject* set_raise(PyObject*, PyObject* const* a, Py_ssize_t na) {
 
 #define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
 PyMethodDef kMethods[] = {FAST(matvec_w4a16), FAST(quantize_f16_q8),    FAST(matvec_w4a8), FAST(gemm_w4a16_wide),
-                          FAST(q4_quantize),  FAST(set_capture_stream), FAST(set_raise),   {nullptr, nullptr, 0, nullptr}};
+                          FAST(q4_quantize),  FAST(prefill_layer),      FAST(set_capture_stream), FAST(set_raise), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", "torch-tensor calls into libnve_kernels.so", -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

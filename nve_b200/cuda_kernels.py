@@ -781,18 +781,13 @@ def gemm_w4a16_gateup_silu(x: Tensor, gate, up, k: int, out: Tensor, scratch: Op
     return out
 
 
-def prefill_layer(layer: "_ffi.RowsLayer", hidden: Tensor, start_pos: int) -> Optional[Tensor]:
-    """A whole prefill layer in one call; None when the shape is not covered."""
-    lib = _lib()
-    rows = hidden.shape[0]
-    need = lib.nve_b200_prefill_layer_workspace_bytes(C.byref(layer), rows)
-    if need == 0:
-        return None
-    ws = torch.empty(need, dtype=torch.uint8, device=hidden.device)  # blocks of the caching allocator are 512-byte aligned
-    out = torch.empty_like(hidden)
-    _ffi.check("nve_b200_prefill_layer",
-               lib.nve_b200_prefill_layer(C.byref(layer), hidden.data_ptr(), out.data_ptr(), rows, start_pos, ws.data_ptr(), need, stream()))
-    return out
+def prefill_layer(hidden: Tensor, projs: Sequence, input_norm: Tensor, post_attn_norm: Tensor, k_cache: Tensor, v_cache: Tensor,
+                  rope_cos: Tensor, rope_sin: Tensor, num_heads: int, num_kv_heads: int, head_dim: int, max_seq: int, eps: float,
+                  scale: float, start_pos: int) -> Optional[Tensor]:
+    """A whole prefill layer in one call; `projs` are (nibbles, scales, n, k) of q, k, v, o, gate, up and down.  None when its sizes do
+    not fit together or are not covered."""
+    return _ffi.host().prefill_layer(hidden, projs, input_norm, post_attn_norm, k_cache, v_cache, rope_cos, rope_sin, num_heads,
+                                     num_kv_heads, head_dim, max_seq, eps, scale, start_pos)
 
 
 def gemm_w4a16_noalloc(x: Tensor, nibbles: Tensor, scales: Tensor, n: int, k: int, out: Tensor) -> Tensor:

@@ -430,36 +430,6 @@ def gpu_layer_forward_decode(hidden: Tensor, layer_idx: int, state: GpuInference
 
 
 
-def _rows_layer(w: GpuLayerWeights, state: GpuInferenceState, layer_idx: int, hidden: int):
-    """The descriptor of nve_b200_prefill_layer for the tensors as they are now (a few microseconds)."""
-    from ._ffi import RowsLayer
-
-    d = RowsLayer()
-    for i, p in enumerate((w.q_proj, w.k_proj, w.v_proj, w.o_proj, w.gate_proj, w.up_proj, w.down_proj)):
-        d.nibbles[i], d.scales[i] = ck._ptr(p.nibbles, torch.uint8, "nibbles"), ck._ptr(p.scales, torch.float32, "scales")
-    f16 = torch.float16
-    d.input_norm, d.post_attn_norm = ck._ptr(w.input_norm, f16), ck._ptr(w.post_attn_norm, f16)
-    d.k_cache, d.v_cache = ck._ptr(state.kv_cache.k[layer_idx], f16), ck._ptr(state.kv_cache.v[layer_idx], f16)
-    d.rope_cos, d.rope_sin = ck._ptr(state.rope_cos, f16), ck._ptr(state.rope_sin, f16)
-    d.hidden, d.ffn, d.num_heads, d.num_kv_heads = hidden, w.gate_proj.n, state.num_heads, state.num_kv_heads
-    d.head_dim, d.max_seq = state.head_dim, state.kv_cache.max_seq
-    d.norm_eps, d.attn_scale = state.norm_eps, float(state.head_dim) ** -0.5
-    return d
-
-
-def _fits_together(w: GpuLayerWeights, state: GpuInferenceState, layer_idx: int, hidden: int) -> bool:
-    """Whether the sizes of a layer are those that the one native call takes for granted; others go through the separate calls, which
-    check or accept them one by one."""
-    q, kv, rows = state.num_heads * state.head_dim, state.num_kv_heads * state.head_dim, state.kv_cache.max_seq
-    ffn = w.gate_proj.n
-    shapes = ((w.q_proj, q, hidden), (w.k_proj, kv, hidden), (w.v_proj, kv, hidden), (w.o_proj, hidden, q),
-              (w.gate_proj, ffn, hidden), (w.up_proj, ffn, hidden), (w.down_proj, hidden, ffn))
-    return (all(p.n == n and p.k == k and p.nibbles.numel() == n * k // 2 and p.scales.numel() == n * k // 32 for p, n, k in shapes) and
-            w.input_norm.numel() == w.post_attn_norm.numel() == hidden and
-            state.kv_cache.k[layer_idx].numel() == state.kv_cache.v[layer_idx].numel() == kv * rows and
-            min(state.rope_cos.numel(), state.rope_sin.numel()) >= rows * (state.head_dim // 2))
-
-
 def gpu_layer_forward_prefill(hidden: Tensor, layer_idx: int, state: GpuInferenceState, start_pos: int) -> Tensor:
     """src/gpu_layer.rs:1086-1160 with gpu_attn_prefill (:777-890) and the batch > 1 branch of gpu_ffn (:977-996) for
     W4 weights: all S prompt positions of one sequence through one layer.  hidden [S, hidden] f16 -> same shape; the
@@ -480,8 +450,11 @@ def gpu_layer_forward_prefill(hidden: Tensor, layer_idx: int, state: GpuInferenc
     eps, scale = state.norm_eps, float(hd) ** -0.5
     projs = (w.q_proj, w.k_proj, w.v_proj, w.o_proj, w.gate_proj, w.up_proj, w.down_proj)
     if S > 1 and hidden.dtype == torch.float16 and hidden.is_cuda and hidden.is_contiguous() and hidden.data_ptr() % 16 == 0 and \
-            all(p.awq_scales is None for p in projs) and _fits_together(w, state, layer_idx, hidden.shape[1]):
-        out = ck.prefill_layer(_rows_layer(w, state, layer_idx, hidden.shape[1]), hidden, start_pos)
+            all(p.awq_scales is None for p in projs):
+        # None: sizes that do not fit together or are not covered go through the separate calls, which check or accept them one by one
+        out = ck.prefill_layer(hidden, tuple((p.nibbles, p.scales, p.n, p.k) for p in projs), w.input_norm, w.post_attn_norm,
+                               state.kv_cache.k[layer_idx], state.kv_cache.v[layer_idx], state.rope_cos, state.rope_sin, nh, nkv, hd,
+                               max_seq, eps, scale, start_pos)
         if out is not None:
             return out
     normed = ck.rms_norm_rows(hidden, w.input_norm, eps)
