@@ -16,21 +16,13 @@ namespace nve {
 
 constexpr int kKBlock = 64;  // K is a multiple of this
 
-// bf16 -> f16, eight elements per thread.  Exact for 6.1e-5 <= |x| <= 65504 (every bf16 significand fits f16);
-// larger magnitudes saturate to +-65504, smaller ones round into the f16 subnormal range.
+// bf16 -> f16, eight elements per thread.
 __global__ void bf16_to_f16_kernel(const uint4* in, uint4* out, long long n8) {
     pdl_wait();
     const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n8) return;
     const uint4 v = in[i];
-    auto cvt = [](uint32_t w) {
-        float lo = __uint_as_float(w << 16), hi = __uint_as_float(w & 0xFFFF0000u);
-        lo = fminf(fmaxf(lo, -65504.0f), 65504.0f);
-        hi = fminf(fmaxf(hi, -65504.0f), 65504.0f);
-        const __half2 h = __floats2half2_rn(lo, hi);
-        return *reinterpret_cast<const uint32_t*>(&h);
-    };
-    out[i] = make_uint4(cvt(v.x), cvt(v.y), cvt(v.z), cvt(v.w));
+    out[i] = make_uint4(bf16x2_to_f16x2(v.x), bf16x2_to_f16x2(v.y), bf16x2_to_f16x2(v.z), bf16x2_to_f16x2(v.w));
 }
 
 static size_t x16_region_bytes(int M, int K) { return (static_cast<size_t>(M) * K * 2 + 255) & ~static_cast<size_t>(255); }

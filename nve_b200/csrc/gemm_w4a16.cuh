@@ -8,6 +8,15 @@ namespace nve {
 
 __device__ __forceinline__ uint32_t s_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
+// bf16 -> f16 of two elements.  Exact for 6.1e-5 <= |x| <= 65504 (every bf16 significand fits f16); larger magnitudes saturate to
+// +-65504, smaller ones round into the f16 subnormal range.
+__device__ __forceinline__ uint32_t bf16x2_to_f16x2(uint32_t w) {
+    const float lo = fminf(fmaxf(__uint_as_float(w << 16), -65504.0f), 65504.0f);
+    const float hi = fminf(fmaxf(__uint_as_float(w & 0xFFFF0000u), -65504.0f), 65504.0f);
+    const __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+
 // Dequantisation of two nibbles.  0x6400 is 1024.0 in f16 with one ulp = 1, so OR-ing a nibble into mantissa bits
 // 0-3 gives 1024 + q exactly; 0x5400 is 64.0 with one ulp = 1/16, so a nibble left in place at bits 4-7 gives
 // 64 + q exactly (no shift needed).  Subtracting 1032 (72) gives q - 8 exactly, and one multiply by the f16 scale

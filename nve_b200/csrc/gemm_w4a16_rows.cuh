@@ -36,14 +36,6 @@ __device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1,
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// bf16 -> f16 of two elements, as the conversion pass does: magnitudes beyond f16 saturate
-__device__ __forceinline__ uint32_t bf16x2_to_f16x2(uint32_t w) {
-    const float lo = fminf(fmaxf(__uint_as_float(w << 16), -65504.0f), 65504.0f);
-    const float hi = fminf(fmaxf(__uint_as_float(w & 0xFFFF0000u), -65504.0f), 65504.0f);
-    const __half2 h = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<const uint32_t*>(&h);
-}
-
 template <int XDT, bool SILU>
 __global__ void __launch_bounds__(kRowsThreads, 1) gemm_w4a16_rows_kernel(const PairParams p, const uint16_t* X) {
     extern __shared__ __align__(16) unsigned char rows_x[];
