@@ -37,19 +37,15 @@ bool pdl_enabled() { return g_pdl.load(std::memory_order_relaxed) != 0; }
 int check_launch() { return set_cuda_status(cudaPeekAtLastError()); }
 
 int sm_count() {
-    static std::mutex mu;
-    static int cached[64];
-    static bool have[64];
+    static std::atomic<int> cached[64];  // asked by every launch: no lock
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-    std::lock_guard<std::mutex> lock(mu);
-    if (!have[dev]) {
-        int n = 0;
+    int n = cached[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
         if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-        cached[dev] = n;
-        have[dev] = true;
+        cached[dev].store(n, std::memory_order_relaxed);
     }
-    return cached[dev];
+    return n;
 }
 
 int ensure_dynamic_smem(const void* kernel, int bytes) {
