@@ -217,10 +217,10 @@ static bool attn_decode_dispatch(const AttnParams& p, int hd, cudaStream_t st, c
 static std::atomic<int> g_attn_decode_kernel{0};
 
 // The tensor-core kernels.  One row: the latency kernel where one tile of 16 positions per warp all but covers the cache (128 to
-// 1280 positions; us per launch back to back, 8B shape, latency / streaming kernel: 256: 3.7 / 4.5, 1024: 4.3 / 4.7, 1500:
-// 5.5 / 5.0, 4096: 9.7 / 7.0, 16384: 27.5 / 17.4), otherwise the streaming one.  Up to 128 positions the latter does not split a
+// 1280 positions; us per launch back to back, 8B shape, latency / streaming kernel: 256: 3.3 / 3.5, 1024: 3.7 / 4.3; where the first
+// version of the latter stood at 1500: 5.5 / 5.0, 4096: 9.7 / 7.0, 16384: 27.5 / 17.4, it takes 4.8, 6.6 and 14.7 now), otherwise the streaming one.  Up to 128 positions the latter does not split a
 // row over CTAs: a row then has the same bits in any batch of fewer than 64 units.  Several rows: always the streaming kernel (2 sequences of 1000:
-// 6.3 / 4.7, 7 of 200: 12.9 / 4.5, 7 of 500 - 2000 with 3 heads per KV head: 22.0 / 10.7, 64 of 256 - 1024: 30.7).
+// 6.3 / 5.0, 7 of 200: 12.9 / 4.4, 7 of 500 - 2000 with 3 heads per KV head: 22.0 / 10.8, 64 of 256 - 1024: 28.7).
 static bool attn_mma_try(const AttnParams& p, int hd, cudaStream_t st, cudaError_t& err, bool fused) {
     if (p.rows <= 1 && p.kv_stride > 128 && p.kv_stride <= 1280) return attn_decode_mma_try(p, hd, st, err, fused);
     return attn_stream_mma_try(p, hd, st, err, fused);

@@ -174,7 +174,8 @@ template <int HD, int G, int NW, int NS, bool FUSED> __global__ void __launch_bo
     // Nothing of the cache before the wait: the launch in front may be writing it, and it may let its dependents start before it
     // has stored.  Behind q, k and v, which everything waits for: tiles requested before the wait hold them up where there is much
     // K/V (us per token with early tiles and so: 8B at 16384 positions 1772 and 1725; 3B, 7 sequences 1492 and 1459; 8B, 64
-    // sequences 3314 and 3305; tiles right after the wait, in front of q: 1776, 1504 and 3344).
+    // sequences 3314 and 3305; tiles right after the wait, in front of q: 1776, 1504 and 3344).  Only attention launches right behind one another
+    // were shorter with early tiles: 7 sequences of 500 - 2000 8.9 us, 10.8 so.
 #pragma unroll
     for (int i = 0; i < NS; i++) load(t_begin + 16 * (warp + NW * i), i);
     const bool pos_ok = FUSED && pos >= 0 && pos < p.kv_stride;
@@ -445,7 +446,8 @@ template <int HD, int G, int NW, int NS, bool FUSED> struct AsLaunch {
     }
 };
 
-// The split.  us per launch on B200 (HD 128, 4 heads per KV head; 4 warps x 3 stages, two CTAs per SM / 8 warps, one CTA per SM):
+// The split.  us per launch on B200 (HD 128, 4 heads per KV head; 4 warps x 3 stages, two CTAs per SM / 8 warps, one CTA per SM), as
+// measured when it was chosen; back to back the chosen forms take 28.7, 27.6, 10.8, 14.7 and 14.7 now:
 //   512 units of 256 - 1024 positions   one CTA per unit 30.7 / 40.1, clusters of two 48.9 / 59.5 (HBM floor 25.6)
 //   160 units of 750 - 3000             34.8 / 28.8, clusters of two 30.2 / 35.6 (23.5)
 //   56 units of 500 - 2000              clusters of four 10.7 / of two 10.7, one CTA per unit 18.5 / 15.0 (5.5)
