@@ -13,8 +13,8 @@
 //   tile  = SB units;  the sequence of all (tile, unit) is dealt out in equal contiguous runs, one per pair
 //
 // Roles (768 threads per CTA):
-//   warps 0-1    issue the MMAs (leader, cluster rank 0, only): warp w < W the steps w, w + W, ... of a segment into
-//                accumulator set w (warp 2 has no part)
+//   warps 0-2    issue the MMAs (leader, cluster rank 0, only): warp w < W the steps w, w + W, ... of a segment into
+//                accumulator set w
 //   warp 3       X loader: TMA of this CTA's half of the X rows, bytes counted on the leader's full barrier
 //   warps 4-7    raw loaders: run ahead by the depth of the raw ring; start before the grid dependency resolves
 //   warps 8-23   dequantisers: four groups of four warps (thread = weight row = TMEM lane), group s % 4 takes step s.
@@ -41,7 +41,7 @@ namespace nve {
 constexpr int kPairRows = 128;           // weight rows per CTA
 constexpr int kPairTile = 256;           // per pair
 constexpr int kPairStepCols = 64;        // TMEM columns of an A slot (128 f16 per row)
-constexpr int kPairIssueWarp = 0;        // first of up to two issuing warps
+constexpr int kPairIssueWarp = 0;        // first of up to three issuing warps
 constexpr int kPairRawWarp = 4, kPairRawWarps = 4;
 constexpr int kPairDeqWarp = 8, kPairDeqWarps = 16;
 constexpr int kPairXWarp = 3;
@@ -1127,8 +1127,10 @@ int gemm_pair(const uint16_t* X, const PairMat* mats, int num_mats, int y_dtype,
     p.total = static_cast<int>(g.tiles * g.SB);
     // Accumulator sets = issuing warps: a step costs an issuing warp about a thousand cycles of waiting and issuing, the
     // MMAs themselves 8 * NB / 2.  The sets of a step follow its index in the segment.
-    // (8B layer, us, one / two / three sets: 24 rows 67.2 / 61.5 / 61.4, 61 rows 72.9 / 67.6 / 68.6: a third set takes an operand slot's columns.)
-    p.W = g.NB <= 128 ? 2 : 1;
+    // Up to 64 rows the third set is there for the sums: an MMA rounds its accumulator towards zero, so that the error of a sum grows with the
+    // length of its chain (4096 x 4096, 24 rows, against 64 bits: 4.6e-7 of the result, 6.4e-7 with two sets).  It takes an operand
+    // slot's columns (8B layer, us, one / two / three sets: 24 rows 67.2 / 61.5 / 61.4, 61 rows 72.9 / 67.6 / 68.6).
+    p.W = g.NB <= 64 ? 3 : (g.NB <= 128 ? 2 : 1);
     p.slots = min(7, (512 - p.W * p.NB) / kPairStepCols);
     // shared memory: the X rows of a step take NB * 128 bytes per CTA; at 256 rows five of them and two raw units
     // (four steps), for narrow tiles up to twelve steps of X and eight raw units, which is what hides HBM latency

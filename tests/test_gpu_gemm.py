@@ -233,3 +233,37 @@ def test_few_rows_on_each_kernel(cuda, orc, M, N, K):
         torch.cuda.synchronize()
         assert ck.gemm_error() == 0
         assert rel_rms_err(out.cpu().numpy(), ref) < 3e-3  # f16 rounding of the weights, as above
+
+
+def _sums_error(N, K, sets, pairs):
+    """Expected error of the f32 sums over K, relative to the result.  An MMA (16 elements of K) rounds its accumulator towards zero, by half
+    an ulp on average: 2^-24 / (2 ln 2) of a sum with an even exponent distribution.  The sum after j of c MMAs is on average j / c of what
+    the chain ends with, which is thus (c + 1) / 2 times that too small.  `sets` chains share the steps (eight MMAs) of a segment; segments are
+    where the runs of two-SM pairs (units of two steps) cut a tile of 256 rows."""
+    units, tiles = -(-K // 256), -(-N // 256)
+    run = max(2, -(-tiles * units // pairs))
+    total = 0.0
+    for t in range(0, tiles * units, units):
+        cuts = sorted({t, t + units} | set(range(-(-t // run) * run, t + units, run)))
+        for a, b in zip(cuts, cuts[1:]):
+            chains = [8 * len(range(w, 2 * (b - a), sets)) for w in range(sets)]
+            total += sum(c * (c + 1) / 2 for c in chains) / (16 * units * tiles)
+    return 2.0**-24 / (2 * np.log(2)) * total
+
+
+@pytest.mark.parametrize("M,N,K", [(17, 4096, 4096), (32, 1024, 14336), (61, 2048, 2048), (64, 14336, 4096)])
+def test_sums_over_k(cuda, orc, M, N, K):
+    """f32 results against an f64 product of the weights as the kernel has them (f16), which leaves the error of the sums: three accumulator
+    sets up to 64 rows (a tenth for the spread; two sets are 1.3 to 1.5 times further off)."""
+    from nve_b200 import cuda_kernels as ck
+
+    torch = cuda
+    nib, sc, X16, _ = _case(orc, M, N, K, 992, False)
+    dx, dn, ds = dev(X16, torch.float16), dev(nib), dev(sc)
+    y = ck.gemm_w4a16(dx, dn, ds, N, K, out_dtype=torch.float32,
+                      scratch=torch.empty(ck.gemm_w4a16_scratch_bytes(M, N, K), dtype=torch.uint8, device="cuda"))
+    b = dn.view(N, K // 32, 16)
+    q = torch.cat([(b & 15).half() - 8, (b >> 4).half() - 8], dim=2)
+    want = dx.double() @ (q * ds.half()[:, :, None]).view(N, K).double().t()
+    pairs = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    assert float((y.double() - want).norm() / want.norm()) < 1.1 * _sums_error(N, K, 3, pairs)
