@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemm_w4a16_rows_kernel(const 
     }
 }
 
-// How a call is cut: equal runs, one per SM; grid == 0 when this kernel is not the one to take: too many rows, or X of a run larger
+// How a call is cut: equal runs, at most one per SM; grid == 0 when this kernel is not the one to take: too many rows, or X of a run larger
 // than shared memory.
 struct RowsPlan {
     int grid = 0, SB = 0, U = 0, total = 0, tiles = 0, nt = 0, depth = 0;
@@ -222,7 +222,9 @@ static RowsPlan rows_plan(const int* Ns, int num_mats, int M, int K, bool silu) 
     const long long total = tiles * r.SB;
     if (total > 0x3FFFFFFFll) return r;
     const int sm = max(1, sm_count());
-    const long long U = (total + sm - 1) / sm;
+    // A tile in many segments costs the finish more than a second unit costs the run: 512 x 14336 (56 units a tile), 8 rows, 9.0 us in runs of one,
+    // 7.7 of two, 16 rows 9.4 and 8.2; 28 units 6.2 and 6.1; 16 units 4.9 and 5.4.
+    const long long U = std::max((total + sm - 1) / sm, r.SB >= 28 ? 2ll : 1ll);
     r.nt = (M + 7) / 8;
     const size_t x = static_cast<size_t>(std::min<long long>(U, r.SB)) * r.nt * kRowsSlab;
     // No more stages than units: 37888 x 512 (runs of two units, 8 rows) 7.3 us with three stages, 6.9 with two; 3072 x 3072 (one unit) 6.9

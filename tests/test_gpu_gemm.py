@@ -1,4 +1,4 @@
-"""GPU parity: the batched W4A16 GEMM (mma.sync kernel up to 8 batch rows where it has a workspace, tcgen05 kernel otherwise) against the
+"""GPU parity: the batched W4A16 GEMM (mma.sync kernel up to 16 batch rows where it has a workspace, tcgen05 kernel otherwise) against the
 reference's CPU semantics (q4_linear: one f32 GEMV per row of X, src/quantize.rs:1057-1075) on the same
 16-bit-rounded activations."""
 import numpy as np
@@ -214,25 +214,28 @@ def test_matmul_x_of_a_workspace_for_64_rows_and_of_no_rows(cuda, orc):
         assert [tuple(t.shape) for t in matmul_x_multi(x[:0], [w, w])] == [(0, N)] * 2
 
 
-@pytest.mark.parametrize("M,N,K", [(1, 256, 64), (3, 300, 320), (8, 384, 2048), (7, 1000, 4096), (2, 19000, 1280), (5, 40000, 128)])
-def test_few_rows_on_each_kernel(cuda, orc, M, N, K):
-    """Up to eight rows: the kernel for few rows (two launches: it always leaves partial tiles) where the workspace holds its partial
-    tiles and no run is longer than a tile, else the two-SM kernel, in whole tiles (one launch) where the workspace holds nothing."""
+@pytest.mark.parametrize("M,N,K,one", [(1, 256, 64, False), (3, 300, 320, False), (8, 384, 2048, False), (7, 1000, 4096, False), (2, 19000, 1280, False),
+                                        (5, 40000, 128, False), (9, 1000, 4096, False), (16, 384, 2048, False), (9, 2000, 512, True),
+                                        (16, 300, 320, True), (13, 257, 7168, False), (17, 384, 2048, False)])
+def test_few_rows_on_each_kernel(cuda, orc, M, N, K, one):
+    """Up to sixteen rows: the kernel for few rows (two launches: it always leaves partial tiles) where the workspace holds its partial tiles,
+    else the two-SM kernel, in whole tiles (one launch) where the workspace holds nothing.  `one`: nine rows or more of f16 on one tile per
+    pair of SMs stay on the two-SM kernel.  bf16 rows tell the two apart: the two-SM kernel has them converted first."""
     from nve_b200 import cuda_kernels as ck
 
     torch = cuda
-    nib, sc, X16, ref = _case(orc, M, N, K, 990, False)
-    dx, dn, ds = dev(X16, torch.float16), dev(nib), dev(sc)
-    tall = -(-N // 256) > torch.cuda.get_device_properties(0).multi_processor_count  # more tiles than SMs: runs of whole tiles
-    full = torch.empty(ck.gemm_w4a16_scratch_bytes(M, N, K), dtype=torch.uint8, device="cuda")
-    for scratch, launches in ((None, 1), (full[:16], 1), (full, None if tall else 2)):
-        out = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
-        before = ck.launch_count()
-        ck.gemm_w4a16(dx, dn, ds, N, K, out_dtype=torch.float32, out=out, scratch=scratch)
-        assert launches is None or ck.launch_count() - before == launches
-        torch.cuda.synchronize()
-        assert ck.gemm_error() == 0
-        assert rel_rms_err(out.cpu().numpy(), ref) < 3e-3  # f16 rounding of the weights, as above
+    for bf in (False, True):
+        nib, sc, X16, ref = _case(orc, M, N, K, 990, bf)
+        dx, dn, ds = dev(X16, torch.bfloat16 if bf else torch.float16), dev(nib), dev(sc)
+        full = torch.empty(ck.gemm_w4a16_scratch_bytes(M, N, K), dtype=torch.uint8, device="cuda")
+        for scratch, launches in ((full, 2 if M <= 16 else 3),) if bf else ((None, 1), (full[:16], 1), (full, 1 if one else 2)):
+            out = torch.full((M, N), float("nan"), dtype=torch.float32, device="cuda")
+            before = ck.launch_count()
+            ck.gemm_w4a16(dx, dn, ds, N, K, out_dtype=torch.float32, out=out, scratch=scratch)
+            assert ck.launch_count() - before == launches
+            torch.cuda.synchronize()
+            assert ck.gemm_error() == 0
+            assert rel_rms_err(out.cpu().numpy(), ref) < 3e-3  # f16 rounding of the weights, as above
 
 
 def _sums_error(N, K, sets, pairs):
