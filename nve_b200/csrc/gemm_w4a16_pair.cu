@@ -239,7 +239,7 @@ template <int ODT, int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     gemm_w4a16_pair_kernel(const PairParams p, const __grid_constant__ CUtensorMap xmap) {
     extern __shared__ __align__(1024) unsigned char pg_raw[];
-    __shared__ __align__(8) uint64_t bars[2 * kBarRing + 2 * kMaxRaw + 2];
+    __shared__ __align__(8) uint64_t bars[2 * kBarRing + 2 * kMaxRaw + 2 + 4];
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -248,7 +248,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     const uint32_t sB = smem, sRaw = smem + p.xslots * bslot_bytes;
     const uint32_t sX = sRaw + p.raw * kRawBytes;  // kPairSilu: exchange between the halves of a tile, [4 groups][2][128 rows][16 B]
     const uint32_t full = s_addr(bars), empty = full + 8 * kBarRing, rawf = empty + 8 * kBarRing, rawe = rawf + 8 * kMaxRaw;
-    const uint32_t accum = rawe + 8 * kMaxRaw, accfree = accum + 8;
+    const uint32_t accum = rawe + 8 * kMaxRaw, accfree = accum + 8, swap = accfree + 8;
     uint32_t rank;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     const int pair = blockIdx.x >> 1;
@@ -263,6 +263,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
             pg_init(rawf + 8 * tid, 32 * kPairRawWarps);  // the copies of every loader lane
             pg_init(rawe + 8 * tid, 8);                   // the eight warps that read the stage
         }
+        if (MODE == kPairSilu && tid < 4) pg_init(swap + 8 * tid, 4);  // the four warps of a dequantiser group
         if (tid == 0) {
             pg_init(accum, p.W);
             pg_init(accfree, 2 * kPairDeqWarps);  // leader: every dequantiser (= epilogue) warp of both CTAs
@@ -381,7 +382,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
             // the MMAs stood still for 8100 of 36000 cycles (8B gate/up, 61 rows; four GEMMs of a layer 70.7 us, 68.0 as it is; 69.3
             // with as many steps ahead as there are slots).
             const uint32_t lfree = pg_map(accfree, 0);
-            int xb = 0;  // kPairSilu: half of the exchange buffer
+            int xb = 0;  // kPairSilu: half of the exchange buffer, and parity of its barrier
             int ej = 0, eseg = 0, etile = u0 / p.SB, esbi = u0 - (u0 / p.SB) * p.SB;  // first segment without its epilogue
             int eunits = min(p.SB - esbi, n_units);
             int lim = min(n_steps, 2 * eunits + 4);  // the group's steps from here on wait for the epilogue: one step of the next segment each
@@ -433,7 +434,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
                             // stored product, each half hands eight over and finishes eight rows of X
                             const bool up = r >= 64;
                             const uint32_t buf = sX + static_cast<uint32_t>((grp * 2 + xb) * 2048);
-                            xb ^= 1;  // the other half next time: one barrier per exchange is enough
                             uint32_t h[4];
 #pragma unroll
                             for (int e = 0; e < 4; e++) {
@@ -441,7 +441,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
                                 h[e] = *reinterpret_cast<const uint32_t*>(&v2);
                             }
                             asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(buf + r * 16), "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3]) : "memory");
-                            asm volatile("bar.sync %0, 128;" ::"r"(2 + grp) : "memory");
+                            __syncwarp();
+                            if (lane == 0) pg_arrive(swap + 8 * grp);
+                            if (!pg_wait(swap + 8 * grp, static_cast<unsigned>(xb))) {  // a warp of the group has given up
+                                fail(6);
+                                return false;
+                            }
+                            xb ^= 1;  // the other half next time: one barrier per exchange is enough
                             asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(h[0]), "=r"(h[1]), "=r"(h[2]), "=r"(h[3]) : "r"(buf + (r ^ 64) * 16) : "memory");
                             float z[8];
 #pragma unroll

@@ -1,4 +1,7 @@
 """CPU: host-side logic of the call sites (routing, normalisation) against the oracle restatement."""
+import os
+import re
+
 import numpy as np
 
 from nve_b200.gpu_layer import RoutingConfig, normalize_importance
@@ -39,3 +42,16 @@ def test_top_half_threshold_is_the_median(golden):
 def test_degenerate_scores():
     assert normalize_importance([2.0, 2.0]) == [0.5, 0.5]
     assert normalize_importance([1.0, 3.0]) == [0.0, 1.0]
+
+
+def test_pair_gemm_roles_wait_on_bounded_barriers_only():
+    """A warp of the two-SM GEMM whose wait expires leaves for the end of the kernel.  Its siblings must get there too: between set-up and
+    teardown no role may stand at a barrier of the whole group, which a warp that left never reaches."""
+    path = os.path.join(os.path.dirname(__file__), "..", "nve_b200", "csrc", "gemm_w4a16_pair.cu")
+    with open(path) as fh:
+        kernel = fh.read().split("gemm_w4a16_pair_kernel(const PairParams p", 1)[1]
+    loaders, rest = kernel.split("raw loaders (weights", 1)[1].split("tcgen05.alloc", 1)
+    roles = rest.split("pg_cluster_wait();", 1)[1].split("// ---- teardown", 1)[0]
+    for part in (loaders, roles):
+        assert "pg_wait(" in part  # the split above still finds the roles
+        assert not re.search(r"\bbar(rier)?\.(cta\.)?(sync|arrive|red)|__syncthreads|__barrier", part)
