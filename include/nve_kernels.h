@@ -384,8 +384,8 @@ NVE_API int nve_b200_fill_normal_16(void* out, long long n, unsigned long long s
 
 /* Batched W4A16 GEMM for decode batches 1 < M <= 64 on the tensor cores: Y[M,N] = X[M,K] . W^T with the packed
  * weights read once and dequantised on the fly (replaces nve_dequant_w4a16 + dense GEMM,
- * src/gpu_layer.rs:220-239): they go to tensor memory and pairs of SMs multiply them with tcgen05.mma, or, up to 8
- * rows with a workspace for it, stay in registers for mma.sync.
+ * src/gpu_layer.rs:220-239): they go to tensor memory and pairs of SMs multiply them with tcgen05.mma, or, up to 16
+ * rows with a workspace that holds the partial tiles, through shared memory to mma.sync.
  * X and Y are row-major; x_dtype f16 or bf16, y_dtype = x_dtype or f32; K % 64 == 0; X and nibbles 16-byte aligned,
  * scales 8-byte aligned.  Weights are rounded to f16 as (q-8)*scale like the reference's dequantisation;
  * accumulation is f32.
@@ -394,8 +394,9 @@ NVE_API int nve_b200_fill_normal_16(void* out, long long n, unsigned long long s
  * to the pairs of SMs in equal contiguous runs, so that few tiles still fill all SMs and a tile count that is not a multiple
  * of the SM count is balanced; tiles that several pairs share are summed in ascending K order by a second kernel
  * (reproducible for a given SM count).  Its size comes from nve_b200_gemm_w4a16_scratch_bytes.  bf16 activations
- * without enough scratch for their copy are refused with NVE_ERR_TOO_LARGE; a scratch too small for the partial
- * tiles only lengthens the runs (fewer CTAs), down to one whole tile per pair, which needs none. f16 activations
+ * without enough scratch for their copy are refused with NVE_ERR_TOO_LARGE, also where up to 16 rows would be converted
+ * on their way in; up to 8 rows are taken all the same where the scratch holds the partial tiles.  A scratch too small
+ * for the partial tiles only lengthens the runs (fewer CTAs), down to one whole tile per pair, which needs none. f16 activations
  * take a workspace of any alignment and use it from its first 16-byte boundary on; bf16 ones want it 16-byte aligned.
  * nve_b200_gemm_error returns the code latched by an expired bounded wait. */
 NVE_API size_t nve_b200_gemm_w4a16_scratch_bytes(int M, int N, int K);

@@ -36,8 +36,8 @@ static int run_gemm_multi(const void* X, int x_dtype, const PairMat* mats, int n
     const uint16_t* x = static_cast<const uint16_t*>(X);
     if (x_dtype == NVE_DT_BF16) {
         const size_t xb = x16_region_bytes(M, K);
-        int status;  // few rows: converted on the way into shared memory; above eight a workspace without room for the copy stays refused
-        if (aligned(sp, 16) && (M <= 8 || scratch_bytes >= xb) &&
+        int status;  // few rows: converted on the way into shared memory; above kFewRows a workspace without room for the copy stays refused
+        if (aligned(sp, 16) && (M <= kFewRows || scratch_bytes >= xb) &&
             gemm_rows_try(X, x_dtype, mats, num_mats, y_dtype, M, K, sp, scratch_bytes, st, PairFinish(), &status))
             return status;
         if (sp == nullptr || scratch_bytes < xb) return set_status(NVE_ERR_TOO_LARGE);

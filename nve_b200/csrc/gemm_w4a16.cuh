@@ -69,6 +69,10 @@ __device__ __forceinline__ void dequant_word(uint32_t w, const DequantScale& d, 
     hi1 = dequant_pair<true>(t, d, c);   // b2 high, b3 high
 }
 
+// Rows of X that fill one mma column.  Up to here the kernel for few rows takes every call whose partial tiles the workspace holds, and bf16
+// rows need no room for an f16 copy; from 9 to 16 it leaves some to the two-SM kernel.
+constexpr int kFewRows = 8;
+
 // The two-SM tcgen05 kernel (gemm_w4a16_pair.cu): any number of rows of X (f16), up to three matrices side by side.
 struct PairMat {
     const uint8_t* nib;

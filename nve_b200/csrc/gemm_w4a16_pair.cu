@@ -1118,10 +1118,10 @@ int gemm_pair(const uint16_t* X, const PairMat* mats, int num_mats, int y_dtype,
     int Ns[3] = {0, 0, 0};
     for (int i = 0; i < num_mats; i++) Ns[i] = mats[i].N;
     const PairPlan g = pair_plan(Ns, num_mats, M, K, partial != nullptr, avail, fin.silu);
-    // More than eight rows on one tile per pair of SMs, with nothing that needs a finishing launch anyway, stay here: one launch against two
+    // More than kFewRows rows on one tile per pair of SMs, with nothing that needs a finishing launch anyway, stay here: one launch against two
     // (16 rows, us: 2000 x 512 3.6 here, 4.4 in the kernel for few rows, 16384 x 1024 6.7 and 7.3, 18944 x 4096 15.5 and 16.9; where the
     // runs cut tiles, 17000 x 4096 17.6 and 16.6).
-    const bool one_launch = M > 8 && g.U == g.SB && fin.norm_w == nullptr && fin.rope == nullptr;
+    const bool one_launch = M > kFewRows && g.U == g.SB && fin.norm_w == nullptr && fin.rope == nullptr;
     int status;
     if (!one_launch && gemm_rows_try(X, NVE_DT_F16, mats, num_mats, y_dtype, M, K, partial, avail, st, fin, &status)) return status;
     PairParams p = {};

@@ -225,7 +225,7 @@ static RowsPlan rows_plan(const int* Ns, int num_mats, int M, int K, bool silu) 
     // A tile in many segments costs the finish more than a second unit costs the run: 512 x 14336 (56 units a tile), 8 rows, 9.0 us in runs of one,
     // 7.7 of two, 16 rows 9.4 and 8.2; 28 units 6.2 and 6.1; 16 units 4.9 and 5.4.
     const long long U = std::max((total + sm - 1) / sm, r.SB >= 28 ? 2ll : 1ll);
-    r.nt = (M + 7) / 8;
+    r.nt = (M + kFewRows - 1) / kFewRows;
     const size_t x = static_cast<size_t>(std::min<long long>(U, r.SB)) * r.nt * kRowsSlab;
     // No more stages than units: 37888 x 512 (runs of two units, 8 rows) 7.3 us with three stages, 6.9 with two; 3072 x 3072 (one unit) 6.9
     // with two, 5.6 with one.
