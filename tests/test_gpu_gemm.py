@@ -238,6 +238,27 @@ def test_few_rows_on_each_kernel(cuda, orc, M, N, K, one):
             assert rel_rms_err(out.cpu().numpy(), ref) < 3e-3  # f16 rounding of the weights, as above
 
 
+@pytest.mark.parametrize("M", [8, 9])
+def test_bf16_rows_without_room_for_their_copy(cuda, orc, M):
+    """Up to eight bf16 rows are taken where the workspace holds the partial tiles, though it has no room for an f16 copy; more are refused."""
+    from nve_b200 import _ffi
+    from nve_b200 import cuda_kernels as ck
+
+    torch = cuda
+    N, K = 64, 81920  # the copy is larger than the partial tiles of one tile of weights
+    x = dev(orc.to_act16(orc.fill_normal(M * K, 991, 2), True), torch.bfloat16).view(M, K)
+    nib, sc = dev(np.full((N, K // 2), 0x99, np.uint8)), dev(np.full((N, K // 32), 0.01, np.float32))  # every weight 0.01
+    scratch = torch.empty(M * K * 2 - 16, dtype=torch.uint8, device="cuda")
+    if M > 8:
+        with pytest.raises(_ffi.NveKernelError):
+            ck.gemm_w4a16(x, nib, sc, N, K, out_dtype=torch.float32, scratch=scratch)
+        return
+    y = ck.gemm_w4a16(x, nib, sc, N, K, out_dtype=torch.float32, scratch=scratch).double()
+    want = x.double().sum(1, keepdim=True).expand(M, N) * float(np.float16(0.01))
+    # f32 sums of 81920 terms against a sum that is their square root times as large: 2^-24 * sqrt(81920) / 16 of it at most
+    assert float((y - want).abs().max()) < 1e-5 * float(x.double().norm(dim=1).max()) * 0.01
+
+
 def _sums_error(N, K, sets, pairs):
     """Expected error of the f32 sums over K, relative to the result.  An MMA (16 elements of K) rounds its accumulator towards zero, by half
     an ulp on average: 2^-24 / (2 ln 2) of a sum with an even exponent distribution.  The sum after j of c MMAs is on average j / c of what

@@ -151,15 +151,18 @@ def test_prefill_layer_refuses_what_does_not_fit(cuda, orc):
         gl.gpu_layer_forward_prefill(_x(torch, orc, 4, hidden // 2, 1046), 0, st, 0)
 
 
-@pytest.mark.parametrize("S,start,nh,nkv,hd", [(9, 0, 4, 2, 128), (31, 1, 10, 2, 64), (257, 40, 6, 3, 128), (300, 3, 8, 2, 64)])
-def test_prefill_layer_rope_and_cache_write(cuda, orc, S, start, nh, nkv, hd):
+@pytest.mark.parametrize("S,start,nh,nkv,hd,hidden", [(9, 0, 4, 2, 128, 512), (31, 1, 10, 2, 64, 512), (61, 0, 20, 5, 64, 1088), (257, 40, 6, 3, 128, 1024),
+                                                       (300, 3, 8, 2, 64, 1024), (1500, 2, 18, 3, 128, 512)])
+def test_prefill_layer_rope_and_cache_write(cuda, orc, S, start, nh, nkv, hd, hidden):
     """The launch that finishes q, k and v rotates them and writes the cache: both GEMM kernels before it, more than one tile of rows, k and
-    v narrower than a tile, both head sizes, positions that start inside the cache.  Against the separate launches."""
+    v narrower than a tile, both head sizes, positions that start inside the cache.  On 148 SMs the tiles of q, k and v are whole (31 rows), cut
+    in half (257 and 300 rows, two tiles of rows), cut by runs of two units that end one tile of five and begin the next (61 rows), and some
+    whole, some cut by runs of three units over tiles of two (1500 rows).  Against the separate launches."""
     from nve_b200 import gpu_layer as gl
     from test_gpu_glue import _make_state
 
     torch = cuda
-    hidden, ffn, max_seq = 512, 768, 350
+    ffn, max_seq = 768, start + S + 50
     st = _make_state(torch, orc, hidden, ffn, nh, nkv, hd, 1, max_seq, 1070, True)
     x = _x(torch, orc, S, hidden, 1071)
     caches = st.kv_cache.k[0], st.kv_cache.v[0]
