@@ -9,10 +9,12 @@
 // instruction, the former form: 19.8 us with nothing else, 24.4 with dequantisation and mma (more loads in flight change nothing: the SM takes
 // the 32 short pieces one by one).  The same through cp.async, whole 128-byte lines: 11.8 and 14.4 us; arithmetic alone 11.8.  32-byte
 // loads into registers 14.2 and 19.  cp.async.bulk takes some 55 cycles per copy: only pieces of 2 KB and more keep up with HBM.
-// Two units of a ring ahead are enough; a third costs shared memory that X needs.
+// Two units of a ring ahead are enough; a third costs shared memory that X needs (and a ring with more stages than the run has units, time).
 //
-// The four GEMMs of a layer in turn, us: 8B 58.7 -> 46.3 with 2 rows, 60.7 -> 49.2 with 8, 61.0 -> 58.4 with 16; 3B 37.4 -> 34.8 with 8,
-// 42.2 -> 39.5 with 16; 1B 27.2 -> 26.9 and 34.9 -> 30.5.  Sixteen rows are the most: with 24 the mma rate (an SM takes
+// The four GEMMs of a layer in turn, us (before: weights into registers up to 8 rows, the two-SM kernel above): 8B 59.6 -> 46.6 with 2 rows,
+// 61.1 -> 48.4 with 8, 61.6 -> 57.6 with 16; 3B 36.4 -> 34.0 with 8, 42.9 -> 39.1 with 16; 1B 27.5 -> 26.3 and 35.9 -> 30.2.  Matrices with
+// more tiles than SMs: 40000 x 4096 30.3 -> 23.7 with one row, 31.0 -> 29.7 with 16; 128256 x 4096 82 -> 61 and 87.5 -> 78.9; 57344 x 8192 72 ->
+// 57 and 73.3 -> 74.0.  Sixteen rows are the most: with 24 the mma rate (an SM takes
 // three cycles for one) is what bounds it, 66.3 against 63.3 in the two-SM kernel (8B), 47.3 against 43.8 (3B).
 //
 //   unit  = 256 elements of K x 256 weight rows, 16 rows per warp; tile = SB units
@@ -23,7 +25,7 @@
 // X is staged once per run in the order in which the lanes read it: 16 bytes per lane and step, no bank conflicts.
 //
 // Sums: an MMA rounds its accumulator towards zero, so that the error of a sum grows with the length of its chain.  A chain is eight MMAs long
-// and added to the sum with a rounding to nearest: sums are 1.8e-7 to 2.4e-7 of the result off (against 64 bits).  One chain for a whole
+// and added to the sum with a rounding to nearest: sums are 1.7e-7 to 2.5e-7 of the result off (against 64 bits).  One chain for a whole
 // run: 3.3e-7 at 512 x 2048, 6.4e-7 at 4096 x 4096, 2.1e-6 at 4096 x 14336, where the two-SM kernel with its shorter ones has
 // 2.7e-7, 4.5e-7 and 1.3e-6 (16 rows).  It costs 1 to 2 %.
 //
