@@ -34,6 +34,9 @@ bool attn_stream_mma_try(const AttnParams& p, int head_dim, cudaStream_t st, cud
 // attn_prefill_mma.cu: the causal block described above, in tiles of query rows; false when the shape is not covered.
 bool attn_prefill_mma_try(const AttnParams& p, int head_dim, cudaStream_t st, cudaError_t& err);
 
+// attn_prefill_tc.cu: the same in tiles of 256 query rows on tcgen05; false: not its shapes, or too few of them.
+bool attn_prefill_tc_try(const AttnParams& p, int head_dim, cudaStream_t st, cudaError_t& err);
+
 // attn_decode_mma.cu: decode attention of one sequence (or query row) on the tensor cores, built for latency; false when the
 // shape is not covered.
 bool attn_decode_mma_try(const AttnParams& p, int head_dim, cudaStream_t st, cudaError_t& err, bool fused = true);

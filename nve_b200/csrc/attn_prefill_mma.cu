@@ -401,6 +401,7 @@ template <int HD, bool SPLIT> static cudaError_t launch_ap(const AttnParams& p, 
 
 bool attn_prefill_mma_try(const AttnParams& p, int head_dim, cudaStream_t st, cudaError_t& err) {
     if (p.num_heads / p.num_kv_heads > kApRows || p.num_kv_heads > 65535) return false;
+    if (attn_prefill_tc_try(p, head_dim, st, err)) return true;
     const bool split = am_split(p.num_heads / p.num_kv_heads);
     if (head_dim == 128) err = split ? launch_ap<128, true>(p, st) : launch_ap<128, false>(p, st);
     else if (head_dim == 64) err = split ? launch_ap<64, true>(p, st) : launch_ap<64, false>(p, st);
