@@ -571,10 +571,12 @@ bool attn_prefill_tc_try(const AttnParams& p, int head_dim, cudaStream_t st, cud
     // Tiles of 128 rows over all KV heads, and steps of the longest.  Below these numbers the form with tiles of 64 rows, which also cuts the
     // positions of a tile into pieces, fills the SMs better (us, that form / this one, 32 over 8 heads of 128: 128 rows 5.9 / 5.9 and at
     // 1000 16.1 / 21.7; 180 rows 7.1 / 7.9, at 300 13.8 / 12.1; 256 rows at 2500 45.8 / 47.1; 300 rows 11.9 / 10.0, at 1000 40.1 / 25.9;
-    // heads of 64: 300 rows 7.0 / 7.8, at 300 11.9 / 11.1; 400 rows 10.3 / 9.2).
+    // heads of 64: 300 rows 7.0 / 7.8, at 100 8.7 / 9.6, at 300 11.9 / 11.1; 400 rows 10.3 / 9.2).
     const long long PT = 2 * (64 / groups), ctas = (p.rows + PT - 1) / PT * p.num_kv_heads, sm = sm_count();
     const int steps = (p.seq_len - 1 + p.rows + kTcKeys - 1) / kTcKeys;
-    if (ctas * 10 < sm * 7 && !(ctas * 20 >= sm * 10 + 40 && steps >= (head_dim == 128 ? 3 : 4)) && !(ctas * 8 >= sm * 3 && steps >= 4 && steps <= 20)) return false;
+    if (ctas * 10 < sm * 7 && !(ctas * 20 >= sm * 10 + 40 && steps >= (head_dim == 128 ? 3 : 5)) &&
+        !(ctas * 8 >= sm * 3 && steps >= (head_dim == 128 ? 4 : 5) && steps <= 20))
+        return false;
     // Two tiles in a CTA take 1.4 to 1.5 times as long as one: from two waves of single tiles on, or where a second wave would be as long as
     // the first (us, one / two: 1000 rows 24.4 / 30.0, at 1000 55.9 / 51.0; 1300 rows 37.3 / 36.0; 1777 rows 59.7 / 46.2; 24 over 8 heads,
     // whose steps are longer, 1000 rows at 1000 58.4 / 59.8, 1777 rows 56.5 / 53.3).
