@@ -356,6 +356,14 @@ NVE_API int nve_b200_attn_decode_fused_batch(const uint16_t* q, const uint16_t* 
                                              uint16_t* out, int batch, int num_heads, int num_kv_heads, int head_dim,
                                              int max_seq_len, float scale, nve_stream_t stream);
 
+/* The q, k and v projections of a batch (nve_b200_gemm_w4a16_wide: X [batch, K] f16, mats = q, k, v with outputs of their own) and the
+ * attention above, with the same values of out and of the cache rows as the two calls.  The attention sums the segments of the
+ * product itself where it can, so that the outputs of mats are scratch: written or not. */
+NVE_API int nve_b200_qkv_attn_decode_batch(const uint16_t* X, const nve_b200_w4_matrix* mats, int K, void* scratch, size_t scratch_bytes,
+                                           uint16_t* k_cache, uint16_t* v_cache, const uint16_t* cos_tab, const uint16_t* sin_tab,
+                                           const int* d_pos, const int* d_seq_len, uint16_t* out, int batch, int num_heads,
+                                           int num_kv_heads, int head_dim, int max_seq_len, float scale, nve_stream_t stream);
+
 /* Exact per-block integer dot products I[N, K/32] (int32) of the W4A8 GEMV, for bit-level checks. */
 NVE_API int nve_b200_w4a8_idot(const int8_t* xq, const uint8_t* nibbles, int32_t* I, int N, int K, nve_stream_t stream);
 

@@ -334,6 +334,48 @@ extern "C" int nve_b200_attn_prefill_causal(const uint16_t* q, const uint16_t* k
     return set_cuda_status(e);
 }
 
+namespace nve {
+// Whether the sequences of a batch run a tensor-core kernel, the streaming one if there are several (else the CUDA-core one): few of them
+// follow nve_b200_set_attn_decode_kernel like a single one
+static bool batch_streams(int batch, int num_heads, int num_kv_heads) {
+    return num_heads / num_kv_heads <= 8 &&
+           (static_cast<long long>(batch) * num_kv_heads >= 64 || g_attn_decode_kernel.load(std::memory_order_relaxed) == 0);
+}
+// q, k and v of a batch: finished values, or (left) where their unfinished product lies
+static int attn_batch(const uint16_t* q, const uint16_t* k_new, const uint16_t* v_new, const PairLeft& left, uint16_t* k_cache, uint16_t* v_cache,
+                      const uint16_t* cos_tab, const uint16_t* sin_tab, const int* d_pos, const int* d_seq_len, uint16_t* out, int batch, int num_heads,
+                      int num_kv_heads, int head_dim, int max_seq_len, float scale, bool streams, cudaStream_t cs) {
+    AttnParams p = {};
+    p.q = q; p.k_new = k_new; p.v_new = v_new; p.k_cache = k_cache; p.v_cache = v_cache;
+    p.cos_tab = cos_tab; p.sin_tab = sin_tab; p.d_pos = d_pos; p.d_seq_len = d_seq_len; p.seq_len = 0;
+    p.out = out;
+    p.num_heads = num_heads; p.num_kv_heads = num_kv_heads; p.kv_stride = max_seq_len; p.scale = scale;
+    p.rows = batch;
+    p.cache_stride = static_cast<long long>(num_kv_heads) * max_seq_len * head_dim;
+    p.left = left;
+    cudaError_t e = cudaSuccess;
+    if (streams && attn_mma_try(p, head_dim, cs, e, true)) {
+        count_launch();
+        return set_cuda_status(e);
+    }
+    if (!attn_decode_dispatch<true, true>(p, head_dim, cs, e)) return set_status(NVE_ERR_BAD_SHAPE);
+    count_launch();
+    return set_cuda_status(e);
+}
+static int check_attn_batch(const uint16_t* q, const uint16_t* k_new, const uint16_t* v_new, const uint16_t* k_cache, const uint16_t* v_cache, const uint16_t* cos_tab,
+                            const uint16_t* sin_tab, const int* d_pos, const int* d_seq_len, const uint16_t* out, int batch, int num_heads, int num_kv_heads,
+                            int head_dim, int max_seq_len) {
+    if (!q || !k_new || !v_new || !k_cache || !v_cache || !cos_tab || !sin_tab || !d_pos || !d_seq_len || !out)
+        return set_status(NVE_ERR_BAD_POINTER);
+    if (batch <= 0 || batch > 65535 || num_heads <= 0 || num_kv_heads <= 0 || (num_heads % num_kv_heads) != 0 || max_seq_len <= 0)
+        return set_status(NVE_ERR_BAD_SHAPE);
+    if (head_dim != 64 && head_dim != 128) return set_status(NVE_ERR_BAD_SHAPE);
+    if (!aligned(k_cache, 16) || !aligned(v_cache, 16) || !aligned(q, 16) || !aligned(k_new, 16) || !aligned(v_new, 16))
+        return set_status(NVE_ERR_BAD_ALIGNMENT);
+    return NVE_OK;
+}
+}  // namespace nve
+
 /* nve_b200_attn_decode_fused for `batch` independent sequences in one launch: row b of q [batch, nh*hd] and of
  * k_new / v_new [batch, nkv*hd] belongs to sequence b, whose caches are k_cache / v_cache + b * nkv * max_seq_len * hd,
  * whose position is d_pos[b] and whose valid length is d_seq_len[b].  The streaming tensor-core kernel; fewer than 64
@@ -343,29 +385,36 @@ extern "C" int nve_b200_attn_decode_fused_batch(const uint16_t* q, const uint16_
                                                 const uint16_t* sin_tab, const int* d_pos, const int* d_seq_len, uint16_t* out,
                                                 int batch, int num_heads, int num_kv_heads, int head_dim, int max_seq_len,
                                                 float scale, nve_stream_t stream) {
-    if (!q || !k_new || !v_new || !k_cache || !v_cache || !cos_tab || !sin_tab || !d_pos || !d_seq_len || !out)
-        return set_status(NVE_ERR_BAD_POINTER);
-    if (batch <= 0 || batch > 65535 || num_heads <= 0 || num_kv_heads <= 0 || (num_heads % num_kv_heads) != 0 || max_seq_len <= 0)
-        return set_status(NVE_ERR_BAD_SHAPE);
-    if (head_dim != 64 && head_dim != 128) return set_status(NVE_ERR_BAD_SHAPE);
-    if (!aligned(k_cache, 16) || !aligned(v_cache, 16) || !aligned(q, 16) || !aligned(k_new, 16) || !aligned(v_new, 16))
-        return set_status(NVE_ERR_BAD_ALIGNMENT);
-    AttnParams p = {};
-    p.q = q; p.k_new = k_new; p.v_new = v_new; p.k_cache = k_cache; p.v_cache = v_cache;
-    p.cos_tab = cos_tab; p.sin_tab = sin_tab; p.d_pos = d_pos; p.d_seq_len = d_seq_len; p.seq_len = 0;
-    p.out = out;
-    p.num_heads = num_heads; p.num_kv_heads = num_kv_heads; p.kv_stride = max_seq_len; p.scale = scale;
-    p.rows = batch;
-    p.cache_stride = static_cast<long long>(num_kv_heads) * max_seq_len * head_dim;
-    cudaError_t e = cudaSuccess;
+    if (int s = check_attn_batch(q, k_new, v_new, k_cache, v_cache, cos_tab, sin_tab, d_pos, d_seq_len, out, batch, num_heads, num_kv_heads, head_dim, max_seq_len);
+        s != NVE_OK)
+        return s;
+    return attn_batch(q, k_new, v_new, PairLeft(), k_cache, v_cache, cos_tab, sin_tab, d_pos, d_seq_len, out, batch, num_heads, num_kv_heads, head_dim,
+                      max_seq_len, scale, batch_streams(batch, num_heads, num_kv_heads), static_cast<cudaStream_t>(stream));
+}
+
+/* q, k and v projections of a batch (nve_b200_gemm_w4a16_wide of X [batch, K] f16 over mats = q, k, v) and the attention above.  Where the
+ * streaming kernel takes the attention, it sums the segments of the product itself: no finishing launch between the two.  The same
+ * values of out and of the cache rows as from the two calls; the outputs of mats are scratch (written or not). */
+extern "C" int nve_b200_qkv_attn_decode_batch(const uint16_t* X, const nve_b200_w4_matrix* mats, int K, void* scratch, size_t scratch_bytes,
+                                              uint16_t* k_cache, uint16_t* v_cache, const uint16_t* cos_tab, const uint16_t* sin_tab,
+                                              const int* d_pos, const int* d_seq_len, uint16_t* out, int batch, int num_heads,
+                                              int num_kv_heads, int head_dim, int max_seq_len, float scale, nve_stream_t stream) {
+    if (!mats) return set_status(NVE_ERR_BAD_POINTER);
+    const uint16_t* y[3];
+    for (int i = 0; i < 3; i++) y[i] = static_cast<const uint16_t*>(mats[i].out);
+    if (int s = check_attn_batch(y[0], y[1], y[2], k_cache, v_cache, cos_tab, sin_tab, d_pos, d_seq_len, out, batch, num_heads, num_kv_heads, head_dim, max_seq_len);
+        s != NVE_OK)
+        return s;
+    if (mats[0].N != num_heads * head_dim || mats[1].N != num_kv_heads * head_dim || mats[2].N != mats[1].N) return set_status(NVE_ERR_BAD_SHAPE);
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
-    // few sequences follow nve_b200_set_attn_decode_kernel like a single one
-    if ((static_cast<long long>(batch) * num_kv_heads >= 64 || g_attn_decode_kernel.load(std::memory_order_relaxed) == 0) &&
-        attn_mma_try(p, head_dim, cs, e, true)) {
-        count_launch();
-        return set_cuda_status(e);
-    }
-    if (!attn_decode_dispatch<true, true>(p, head_dim, cs, e)) return set_status(NVE_ERR_BAD_SHAPE);
-    count_launch();
-    return set_cuda_status(e);
+    const bool streams = batch_streams(batch, num_heads, num_kv_heads);
+    // Unfinished, but for a few units of small heads whose positions are split over large clusters: there every CTA of a cluster sums the
+    // same segments while the launch that finishes them is at its shortest (us per layer, 1B, finished / unfinished: 2 sequences of 2000
+    // 33.7 / 34.0, of 8000 36.7 / 37.9, of 100 32.5 / 31.2; 4 of 4000 37.0 / 37.7; 5 of 8000 43.2 / 42.2, 24 of 1000 49.7 / 48.1; 3B, 2 of
+    // 8000 49.3 / 48.1).
+    const bool leave = streams && batch > 1 && !(head_dim == 64 && batch * num_kv_heads < 40 && max_seq_len > 512);
+    PairLeft left;
+    if (int s = gemm_qkv(X, mats, batch, K, scratch, scratch_bytes, leave ? &left : nullptr, cs); s != NVE_OK) return s;
+    return attn_batch(y[0], y[1], y[2], left, k_cache, v_cache, cos_tab, sin_tab, d_pos, d_seq_len, out, batch, num_heads, num_kv_heads, head_dim, max_seq_len,
+                      scale, streams, cs);
 }

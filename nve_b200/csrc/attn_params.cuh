@@ -1,6 +1,7 @@
 // Launch parameters of the decode attention kernels (attn_decode.cu, attn_decode_mma.cu, attn_stream_mma.cu, attn_prefill_mma.cu).
 #pragma once
 #include "common.cuh"
+#include "gemm_w4a16.cuh"
 
 namespace nve {
 
@@ -23,6 +24,8 @@ struct AttnParams {
     // un-fused form only: blockIdx.y selects one of `rows` query rows; row r reads q + r * row_stride, writes
     // out + r * row_stride and attends to seq_len + r positions (causal attention over a block of new positions)
     int rows, row_stride;
+    // batched fused form, streaming kernel: q, k and v may be a product whose segments are not summed yet
+    PairLeft left;
     // batched fused form: `rows` independent sequences; elements between consecutive K (or V) caches
     long long cache_stride;
 };

@@ -67,7 +67,9 @@ template <int HD, int G, int NW, int NS> struct AsSmem {
 
 // Fused: blockIdx.y is one of `rows` independent sequences (one sequence: rows <= 1).  Else: one of `rows` query rows over one
 // cache, row r attends to seq_len + r positions.  blockIdx.x = KV head * csize + rank.
-template <int HD, int G, int NW, int NS, bool FUSED> __global__ void __launch_bounds__(32 * NW, 8 / NW) attn_stream_mma_kernel(const AttnParams pin, int csize) {
+// LEFT (fused): q, k and v are a product whose segments are not summed yet; with heads of 64 two CTAs of eight warps still fit an SM.
+template <int HD, int G, int NW, int NS, bool FUSED, bool LEFT>
+__global__ void __launch_bounds__(32 * NW, LEFT && HD == 64 && NW == 8 ? 2 : 8 / NW) attn_stream_mma_kernel(const AttnParams pin, int csize) {
     AttnParams p = pin;
     int seq_len_row = p.seq_len;
     const long long b = blockIdx.y;
@@ -142,24 +144,33 @@ template <int HD, int G, int NW, int NS, bool FUSED> __global__ void __launch_bo
     };
     if constexpr (FUSED) rope_row();
     for (int i = tid; i < (8 - G) * HALF; i += (32 * NW)) reinterpret_cast<uint32_t*>(sm.q[G])[i] = 0;
+    constexpr int E = LEFT ? 2 * QI + 3 : 1;
+    const uint16_t* y[E];
+    PairFeatures<E> features;
+    if constexpr (LEFT) {
+        int tile0[E], n[E];
+#pragma unroll
+        for (int j = 0; j < QI; j++) {
+            const int h = qh + j * HPP;
+            tile0[2 * j] = tile0[2 * j + 1] = p.left.tile0[0];
+            n[2 * j] = (h0 + (h < G ? h : 0)) * HD + qe;
+            n[2 * j + 1] = n[2 * j] + HALF;
+            y[2 * j] = p.q + n[2 * j];
+            y[2 * j + 1] = p.q + n[2 * j + 1];
+        }
+        tile0[E - 3] = tile0[E - 2] = p.left.tile0[1];
+        tile0[E - 1] = p.left.tile0[2];
+        n[E - 3] = kvh * HD + qe;
+        n[E - 2] = n[E - 3] + HALF;
+        n[E - 1] = kvh * HD + (tid < HD ? tid : 0);
+        y[E - 3] = p.k_new + n[E - 3];
+        y[E - 2] = p.k_new + n[E - 2];
+        y[E - 1] = p.v_new + n[E - 1];
+        features.find(p.left, static_cast<int>(b), tile0, n);
+    }
     pdl_wait();
     uint16_t x0[QI], x1[QI], k0 = 0, k1 = 0, vv = 0;
-#pragma unroll
-    for (int j = 0; j < QI; j++) {
-        const int h = qh + j * HPP;
-        const uint16_t* qp = p.q + static_cast<long long>(h0 + (h < G ? h : 0)) * HD;
-        x0[j] = qp[qe];
-        x1[j] = qp[qe + HALF];
-    }
-    if constexpr (FUSED) {
-        const uint16_t* kp = p.k_new + static_cast<long long>(kvh) * HD;
-        if (tid < HALF) {
-            k0 = kp[qe];
-            k1 = kp[qe + HALF];
-        }
-        if (tid < HD) vv = p.v_new[static_cast<long long>(kvh) * HD + tid];
-    }
-    {
+    auto positions = [&]() {
         const int now = max(0, min(p.d_seq_len != nullptr ? *reinterpret_cast<const volatile int*>(p.d_seq_len) : seq_len_row, p.kv_stride));
         const int now_pos = FUSED ? *reinterpret_cast<const volatile int*>(p.d_pos) : -1;
         if (FUSED && now_pos != pos) {
@@ -170,14 +181,52 @@ template <int HD, int G, int NW, int NS, bool FUSED> __global__ void __launch_bo
             seq_len = now;
             slice();
         }
-    }
+    };
     // Nothing of the cache before the wait: the launch in front may be writing it, and it may let its dependents start before it
     // has stored.  Behind q, k and v, which everything waits for: tiles requested before the wait hold them up where there is much
     // K/V (us per token with early tiles and so: 8B at 16384 positions 1772 and 1725; 3B, 7 sequences 1492 and 1459; 8B, 64
     // sequences 3314 and 3305; tiles right after the wait, in front of q: 1776, 1504 and 3344).  Only attention launches right behind one another
     // were shorter with early tiles: 7 sequences of 500 - 2000 8.9 us, 10.8 so.
+    auto request = [&]() {
 #pragma unroll
-    for (int i = 0; i < NS; i++) load(t_begin + 16 * (warp + NW * i), i);
+        for (int i = 0; i < NS; i++) load(t_begin + 16 * (warp + NW * i), i);
+    };
+    if constexpr (LEFT) {
+        // No finishing launch of the GEMM in between: 3B, 7 sequences of up to 2000 positions 1308 -> 1254 us per step, 8B, 64 of up to 1024
+        // 3242 -> 3195.  What counts is the order: the segments are found before the wait and requested first, K/V behind them and in front of
+        // the sums (sums first: 1320), and the positions are read ahead all the same (1312 without).
+        uint16_t x[E];
+        features.sum(y, x, [&]() {
+            positions();
+            request();
+        });
+#pragma unroll
+        for (int j = 0; j < QI; j++) {
+            x0[j] = x[2 * j];
+            x1[j] = x[2 * j + 1];
+        }
+        k0 = x[E - 3];
+        k1 = x[E - 2];
+        vv = x[E - 1];
+    } else {
+#pragma unroll
+        for (int j = 0; j < QI; j++) {
+            const int h = qh + j * HPP;
+            const uint16_t* qp = p.q + static_cast<long long>(h0 + (h < G ? h : 0)) * HD;
+            x0[j] = qp[qe];
+            x1[j] = qp[qe + HALF];
+        }
+        if constexpr (FUSED) {
+            const uint16_t* kp = p.k_new + static_cast<long long>(kvh) * HD;
+            if (tid < HALF) {
+                k0 = kp[qe];
+                k1 = kp[qe + HALF];
+            }
+            if (tid < HD) vv = p.v_new[static_cast<long long>(kvh) * HD + tid];
+        }
+        positions();
+        request();
+    }
     const bool pos_ok = FUSED && pos >= 0 && pos < p.kv_stride;
     {
         // the rotation of the stand-alone RoPE kernel: same IEEE operations, same 16-bit rounding
@@ -399,7 +448,7 @@ template <int HD, int G, int NW, int NS> constexpr int as_smem_bytes(int csize) 
 // A CTA of eight warps takes most of an SM: three stages where they fit next to the partials of eight ranks.
 template <int HD, int G> constexpr int as_wide_stages() { return as_smem_bytes<HD, G, 8, 3>(8) <= 227 * 1024 ? 3 : 2; }
 
-template <int HD, int G, int NW, int NS, bool FUSED> struct AsLaunch {
+template <int HD, int G, int NW, int NS, bool FUSED, bool LEFT> struct AsLaunch {
     static void config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, const AttnParams& p, int rows, int csize, cudaStream_t st) {
         cfg = {};
         cfg.dynamicSmemBytes = as_smem_bytes<HD, G, NW, NS>(csize);
@@ -414,7 +463,7 @@ template <int HD, int G, int NW, int NS, bool FUSED> struct AsLaunch {
         cfg.numAttrs = 1;
     }
     static int prepare() {
-        return ensure_dynamic_smem(reinterpret_cast<const void*>(attn_stream_mma_kernel<HD, G, NW, NS, FUSED>), as_smem_bytes<HD, G, NW, NS>(kAsMaxCluster));
+        return ensure_dynamic_smem(reinterpret_cast<const void*>(attn_stream_mma_kernel<HD, G, NW, NS, FUSED, LEFT>), as_smem_bytes<HD, G, NW, NS>(kAsMaxCluster));
     }
     // How many clusters of `csize` CTAs the current device holds at a time (clusters do not straddle the SM groups of the chip, so this
     // is less than SMs / csize: 15 clusters of 8 on 148 SMs); asked once per device.
@@ -428,7 +477,7 @@ template <int HD, int G, int NW, int NS, bool FUSED> struct AsLaunch {
             cudaLaunchConfig_t cfg;
             cudaLaunchAttribute attr[2];
             config(cfg, attr, p, 1, csize, nullptr);
-            if (cudaOccupancyMaxActiveClusters(&n, attn_stream_mma_kernel<HD, G, NW, NS, FUSED>, &cfg) != cudaSuccess || n < 1) n = 1;
+            if (cudaOccupancyMaxActiveClusters(&n, attn_stream_mma_kernel<HD, G, NW, NS, FUSED, LEFT>, &cfg) != cudaSuccess || n < 1) n = 1;
             if (keep) known[dev][csize].store(n, std::memory_order_relaxed);
         }
         return n;
@@ -442,7 +491,7 @@ template <int HD, int G, int NW, int NS, bool FUSED> struct AsLaunch {
             attr[1].val.programmaticStreamSerializationAllowed = 1;
             cfg.numAttrs = 2;
         }
-        return cudaLaunchKernelEx(&cfg, attn_stream_mma_kernel<HD, G, NW, NS, FUSED>, p, csize);
+        return cudaLaunchKernelEx(&cfg, attn_stream_mma_kernel<HD, G, NW, NS, FUSED, LEFT>, p, csize);
     }
 };
 
@@ -455,9 +504,9 @@ template <int HD, int G, int NW, int NS, bool FUSED> struct AsLaunch {
 // Launching a cluster costs about 0.1 us of the whole device, so: up to one and a half units per SM slot eight warps each, the
 // largest cluster (no more than eight CTAs: seven of 16 fit) of which all units run at a time and whose warps all get a tile;
 // beyond that four warps per unit.
-template <int HD, int G, bool FUSED> static cudaError_t launch_as(const AttnParams& p, cudaStream_t st) {
-    using Wide = AsLaunch<HD, G, 8, as_wide_stages<HD, G>(), FUSED>;
-    using Narrow = AsLaunch<HD, G, 4, 3, FUSED>;
+template <int HD, int G, bool FUSED, bool LEFT> static cudaError_t launch_as_with(const AttnParams& p, cudaStream_t st) {
+    using Wide = AsLaunch<HD, G, 8, as_wide_stages<HD, G>(), FUSED, LEFT>;
+    using Narrow = AsLaunch<HD, G, 4, 3, FUSED, LEFT>;
     const int rows = p.rows > 1 ? p.rows : 1;
     const long long units = static_cast<long long>(p.num_kv_heads) * rows;
     if (Wide::prepare() != NVE_OK || Narrow::prepare() != NVE_OK) return cudaErrorInvalidValue;
@@ -465,6 +514,12 @@ template <int HD, int G, bool FUSED> static cudaError_t launch_as(const AttnPara
     int csize = kAsMaxCluster;
     while (csize > 1 && (units > Wide::active(p, csize) || p.kv_stride <= 128 * (csize - 1))) csize--;
     return Wide::launch(p, rows, csize, st);
+}
+template <int HD, int G, bool FUSED> static cudaError_t launch_as(const AttnParams& p, cudaStream_t st) {
+    if constexpr (FUSED) {
+        if (p.left.partial != nullptr) return launch_as_with<HD, G, true, true>(p, st);
+    }
+    return launch_as_with<HD, G, FUSED, false>(p, st);
 }
 template <int HD, bool FUSED> static bool launch_as_groups(const AttnParams& p, cudaStream_t st, cudaError_t& err) {
     switch (p.num_heads / p.num_kv_heads) {

@@ -96,6 +96,14 @@ static int check_gemm_multi(const void* X, int x_dtype, const nve_b200_w4_matrix
     if (cols > 0x7FFFFFF0ll) return set_status(NVE_ERR_BAD_SHAPE);
     return NVE_OK;
 }
+int gemm_qkv(const uint16_t* X, const nve_b200_w4_matrix* mats, int M, int K, void* scratch, size_t scratch_bytes, PairLeft* left, cudaStream_t st) {
+    PairMat g[3];
+    if (M < 1) return set_status(NVE_ERR_BAD_SHAPE);
+    if (int s = check_gemm_multi(X, NVE_DT_F16, mats, 3, NVE_DT_F16, K, g); s != NVE_OK) return s;
+    PairFinish fin;
+    fin.left = left;
+    return gemm_pair(X, g, 3, NVE_DT_F16, M, K, scratch, scratch != nullptr ? scratch_bytes : 0, st, fin);
+}
 }  // namespace nve
 
 extern "C" int nve_b200_gemm_w4a16_multi(const void* X, int x_dtype, const nve_b200_w4_matrix* mats, int num_mats, int y_dtype,

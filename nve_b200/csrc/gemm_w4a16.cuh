@@ -91,6 +91,12 @@ struct PairRope {
     const uint16_t *cos_t, *sin_t;
     int start_pos, hd, max_seq;
 };
+// Where a product that was left unfinished lies (rows of X in one tile): of tiles that were cut the f32 sums of their segments, of others Y.
+struct PairLeft {
+    const float* partial = nullptr;  // nullptr: everything is in Y
+    int part_rows = 0, SB = 0, U = 0, by_tile = 0;
+    int tile0[3] = {0, 0, 0};        // first tile of a matrix
+};
 // What becomes of the product (f16 outputs only; nothing set: Y = X . W^T)
 struct PairFinish {
     const uint16_t* res = nullptr;     // one matrix: Y = res + round16(product)
@@ -98,6 +104,7 @@ struct PairFinish {
     uint16_t* normed = nullptr;
     float eps = 0.0f;
     const PairRope* rope = nullptr;    // three matrices q, k, v of whole heads; the cache is written, the outputs of k and v are scratch
+    PairLeft* left = nullptr;          // no finishing launch: the caller's next kernel sums the segments (PairFeatures)
     bool silu = false;                 // two matrices of the same N: Y of the first = silu(first product) * second product
 };
 PairPlan pair_plan(const int* Ns, int num_mats, int M, int K, bool have_scratch, size_t avail, bool silu = false);
@@ -113,7 +120,60 @@ int gemm_pair(const uint16_t* X, const PairMat* mats, int num_mats, int y_dtype,
 // launched.  gemm_pair asks it first.
 bool gemm_rows_try(const void* X, int x_dtype, const PairMat* mats, int num_mats, int y_dtype, int M, int K, void* partial, size_t avail,
                    cudaStream_t st, const PairFinish& fin, int* status);
+// q, k and v of `M` rows of X (f16), left unfinished where `left` is given and the rows are one tile; the entry point's checks
+int gemm_qkv(const uint16_t* X, const nve_b200_w4_matrix* mats, int M, int K, void* scratch, size_t scratch_bytes, PairLeft* left, cudaStream_t st);
 bool pair_norm_fits(int N);
+#ifdef __CUDACC__
+// E features of row m of a product that was left unfinished, rounded to f16: element e is feature n of the matrix whose tiles begin at
+// tile0 and whose finished values are at y.  Found before the grid dependency; the segments of all E are then under way together, eight at a
+// time, and added in ascending K order like the finishing kernel does; behind() runs when the first are under way.
+template <int E> struct PairFeatures {
+    const float* src[E];  // segment i of count[e] is `delta` further than i - 1; where `late` has bit e, the first is one slot further
+    int count[E];         // 0: finished
+    unsigned late = 0;
+    int most = 0;
+    long long delta, slot;
+    __device__ __forceinline__ void find(const PairLeft& L, int m, const int (&tile0)[E], const int (&n)[E]) {
+        slot = static_cast<long long>(L.part_rows) * 256;
+        delta = L.by_tile ? slot : 2 * slot;
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const int tile = tile0[e] + (n[e] >> 8), first = tile * L.SB / L.U;
+            count[e] = ((tile + 1) * L.SB - 1) / L.U - first + 1;
+            if (count[e] == 1 && !L.by_tile) count[e] = 0;
+            most = max(most, count[e]);
+            src[e] = L.partial + static_cast<long long>(L.by_tile ? first + tile : 2 * first) * slot + static_cast<long long>(m) * 256 + (n[e] & 255);
+            if (!L.by_tile && first * L.U < tile * L.SB) late |= 1u << e;
+        }
+    }
+    template <class F> __device__ __forceinline__ void sum(const uint16_t* const (&y)[E], uint16_t (&out)[E], F behind) {
+        constexpr int kFly = 8;
+        float total[E];
+        for (int c0 = 0; c0 == 0 || c0 < most; c0 += kFly) {
+            float v[kFly][E];
+#pragma unroll
+            for (int i = 0; i < kFly; i++)
+#pragma unroll
+                for (int e = 0; e < E; e++)
+                    if (c0 + i < count[e]) v[i][e] = __ldcg(src[e] + (c0 + i) * delta + (i == 0 && c0 == 0 && (late >> e & 1) ? slot : 0));
+            if (c0 == 0) {
+#pragma unroll
+                for (int e = 0; e < E; e++)
+                    if (count[e] == 0) out[e] = *y[e];
+                behind();
+            }
+#pragma unroll
+            for (int i = 0; i < kFly; i++)
+#pragma unroll
+                for (int e = 0; e < E; e++)
+                    if (c0 + i < count[e]) total[e] = c0 + i == 0 ? v[i][e] : __fadd_rn(total[e], v[i][e]);
+        }
+#pragma unroll
+        for (int e = 0; e < E; e++)
+            if (count[e] > 0) out[e] = Act16<NVE_DT_F16>::from_f32(total[e]);
+    }
+};
+#endif
 int gemm_pair_error(bool reset);
 
 }  // namespace nve

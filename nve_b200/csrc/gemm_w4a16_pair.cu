@@ -1008,6 +1008,16 @@ PairPlan pair_plan(const int* Ns, int num_mats, int M, int K, bool have_scratch,
 
 // What a GEMM kernel left to be finished: tiles in several segments, a row that goes through a norm, q, k and v on their way to the cache.
 template <int ODT, int MODE> static int launch_finish(const PairParams& p, unsigned tiles, const PairFinish& fin, cudaStream_t st) {
+    if (fin.left != nullptr && p.XT == 1) {
+        *fin.left = PairLeft();
+        fin.left->partial = p.by_tile || p.U % p.SB != 0 ? p.partial : nullptr;
+        fin.left->part_rows = p.part_rows;
+        fin.left->SB = p.SB;
+        fin.left->U = p.U;
+        fin.left->by_tile = p.by_tile;
+        for (int i = 1; i < 3; i++) fin.left->tile0[i] = p.wt_end[i - 1];
+        return set_status(NVE_OK);
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.stream = st;
     cudaLaunchAttribute attr[1];

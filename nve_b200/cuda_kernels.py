@@ -619,6 +619,23 @@ def attn_decode_fused_batch(q: Tensor, k_new: Tensor, v_new: Tensor, k_cache: Te
     return out
 
 
+def qkv_attn_decode_batch(x: Tensor, weights: Sequence, k_dim: int, outs: Sequence[Tensor], scratch: Tensor, k_cache: Tensor, v_cache: Tensor,
+                          cos_tab: Tensor, sin_tab: Tensor, d_pos: Tensor, d_seq_len: Tensor, num_heads: int, num_kv_heads: int,
+                          head_dim: int, max_seq_len: int, scale: float, out: Tensor) -> Tensor:
+    """gemm_w4a16_wide over q, k, v of x [B, K] and attn_decode_fused_batch, without the launch between them that finishes the
+    product; `outs` (q, k, v) are scratch, written or not."""
+    b = x.shape[0]
+    if k_cache.shape[0] != b or d_pos.numel() != b or d_seq_len.numel() != b:
+        raise ValueError("one cache, position and length per row of x")
+    arr = _mats(weights, outs, None, _F16)
+    _ffi.check("nve_b200_qkv_attn_decode_batch",
+               _lib().nve_b200_qkv_attn_decode_batch(
+                   _ptr(x, _F16, "x"), arr, k_dim, _ptr(scratch), scratch.numel() * scratch.element_size(), _ptr(k_cache, _F16), _ptr(v_cache, _F16),
+                   _ptr(cos_tab, _F16), _ptr(sin_tab, _F16), _ptr(d_pos, torch.int32, "d_pos"), _ptr(d_seq_len, torch.int32, "d_seq_len"),
+                   _ptr(out, _F16, "out"), b, num_heads, num_kv_heads, head_dim, max_seq_len, float(scale), stream()))
+    return out
+
+
 # --------------------------------------------------------------------------- whole step in one kernel
 def decode_step_workspace_bytes(model: "_ffi.DecodeModel") -> int:
     n = int(_lib().nve_b200_decode_step_workspace_bytes(C.byref(model)))

@@ -544,9 +544,17 @@ def gpu_layer_forward_decode_batch(hidden: Tensor, layer_idx: int, state: GpuInf
         normed = ck.add_rms_norm_rows(hidden, residual, w.input_norm, eps, out=None if s is None else s.normed)
     else:
         normed = ck.rms_norm_rows(hidden, w.input_norm, eps, out=None if s is None else s.normed)
-    q, k, v = matmul_x_multi(normed, [w.q_proj, w.k_proj, w.v_proj], ws, None if s is None else [s.q, s.k, s.v])
-    attn = ck.attn_decode_fused_batch(q, k, v, kv.k[layer_idx], kv.v[layer_idx], state.rope_cos, state.rope_sin, d_pos,
-                                      d_seqlen, nh, nkv, hd, kv.max_seq, scale, out=None if s is None else s.attn)
+    qkv = [w.q_proj, w.k_proj, w.v_proj]
+    if s is not None and normed.dtype == torch.float16 and normed.shape[0] > 1 and hd in (64, 128) and \
+            all(p.awq_scales is None and p.k == normed.shape[1] and p.k % 64 == 0 for p in qkv) and \
+            _workspace_holds(ws, normed.shape[0], [p.n for p in qkv], w.q_proj.k):
+        # the attention sums the segments of the product itself
+        attn = ck.qkv_attn_decode_batch(normed, [p.triple() for p in qkv], w.q_proj.k, [s.q, s.k, s.v], ws, kv.k[layer_idx], kv.v[layer_idx],
+                                        state.rope_cos, state.rope_sin, d_pos, d_seqlen, nh, nkv, hd, kv.max_seq, scale, s.attn)
+    else:
+        q, k, v = matmul_x_multi(normed, qkv, ws, None if s is None else [s.q, s.k, s.v])
+        attn = ck.attn_decode_fused_batch(q, k, v, kv.k[layer_idx], kv.v[layer_idx], state.rope_cos, state.rope_sin, d_pos,
+                                          d_seqlen, nh, nkv, hd, kv.max_seq, scale, out=None if s is None else s.attn)
     plain = hidden.dtype == torch.float16 and all(p.awq_scales is None for p in (w.o_proj, w.gate_proj, w.up_proj))
     h1 = torch.empty_like(hidden) if s is None else s.h1
     if plain and hidden.shape[0] > 1 and hidden.shape[1] % 8 == 0 and hidden.shape[1] <= 8192:
