@@ -74,7 +74,6 @@ struct PairParams {
     int sc16;        // 1: rows of scales are 16-byte aligned
     int y2;          // 1: an output is not 4-byte aligned
     int y8;          // 1: the 16-bit outputs, what is added to them, and their rows are 8-byte aligned
-    int by_cut;      // 1: a finishing block per boundary of two runs (no tile has more than one), else per tile
     int by_tile;     // 1: every segment is in the workspace, that of (run, tile) in slot run + tile (the kernel for few rows)
     const uint16_t* res;  // kPairAdd: [M, N] f16, added to the rounded product
 };
@@ -688,10 +687,11 @@ __device__ __forceinline__ float4 pair_sum4(const PairParams& p, int tile, int f
 // the tile that it cuts: most tiles of a wide call are whole (8B gate/up, 1777 rows: 73 of 784), and blocks that found that out and left
 // took most of the launch; 16-bit values move four at a time (8B layer, 1777 rows, the two finishes of the FFN: 53 us less; four rows a
 // thread instead of one: 128 rows 92.5 -> 100, 1777 rows no change).
-template <int ODT, int MODE> __global__ void __launch_bounds__(256) gemm_pair_reduce_kernel(const PairParams p) {
+// CUT: a block per boundary (a branch instead costs a call of a few rows another division).
+template <int ODT, int MODE, bool CUT> __global__ void __launch_bounds__(256) gemm_pair_reduce_kernel(const PairParams p) {
     pdl_wait();
     pdl_launch_dependents();
-    const int tile = p.by_cut ? (static_cast<int>(blockIdx.x) + 1) * p.U / p.SB : static_cast<int>(blockIdx.x);
+    const int tile = CUT ? (static_cast<int>(blockIdx.x) + 1) * p.U / p.SB : static_cast<int>(blockIdx.x);
     const int first = (tile * p.SB) / p.U, last = ((tile + 1) * p.SB - 1) / p.U;
     if (first == last && !p.by_tile) return;
     const PairTile tl = pair_locate<MODE>(p, tile);
@@ -1040,13 +1040,12 @@ template <int ODT, int MODE> static int launch_finish(const PairParams& p, unsig
         e = cudaLaunchKernelEx(&cfg, wide ? gemm_pair_reduce_norm_kernel : gemm_pair_reduce_norm_rows_kernel, p, fin.norm_w, fin.normed, fin.eps);
         count_launch();
     } else if (p.by_tile || p.U % p.SB != 0) {
-        PairParams pc = p;
-        const unsigned cuts = static_cast<unsigned>((p.total - 1) / p.U);  // boundaries of two runs
-        pc.by_cut = !p.by_tile && p.U >= p.SB && cuts > 0;
-        cfg.gridDim = dim3(pc.by_cut ? cuts : tiles, static_cast<unsigned>((p.part_rows + 3) / 4));
+        const unsigned cuts = static_cast<unsigned>((p.total - 1) / p.U);  // boundaries of two runs; no tile has more than one
+        const bool cut = !p.by_tile && p.U >= p.SB && cuts > 0;
+        cfg.gridDim = dim3(cut ? cuts : tiles, static_cast<unsigned>((p.part_rows + 3) / 4));
         cfg.blockDim = dim3(MODE == kPairSilu ? kPairTile / 8 : kPairTile / 4, MODE == kPairSilu ? 8 : 4);
         if (MODE == kPairSilu) cfg.gridDim.y = static_cast<unsigned>((p.part_rows + 7) / 8);
-        e = cudaLaunchKernelEx(&cfg, gemm_pair_reduce_kernel<ODT, MODE>, pc);
+        e = cudaLaunchKernelEx(&cfg, cut ? gemm_pair_reduce_kernel<ODT, MODE, true> : gemm_pair_reduce_kernel<ODT, MODE, false>, p);
         count_launch();
     }
     return set_cuda_status(e);
