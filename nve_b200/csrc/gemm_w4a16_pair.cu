@@ -654,32 +654,42 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     }
 }
 
-// Sum of four consecutive columns of row mm of a tile over the pairs that worked on it, in ascending K order.
-__device__ __forceinline__ float4 pair_sum4(const PairParams& p, int tile, int first, int last, int mm, int col) {
-    auto part = [&](int c) {
+// Sums of four consecutive columns of row mm of a tile, from col, col + step, ..., over the pairs that worked on it, in ascending K order.
+// Eight loads on their way at a time: one after the other each cost an L2 round trip, and that was most of the call for a row or two of
+// tiles cut into a dozen segments.  So did a second group of columns behind the first (layers, us, one group after the other / together: 8B
+// 20 rows 70.7 / 69.4, 61 rows 76.4 / 74.9, 300 rows 155.6 / 152.4, 3B 300 rows at 700 116.9 / 113.6).
+template <int C> __device__ __forceinline__ void pair_sums4(const PairParams& p, int tile, int first, int last, int mm, int col, int step, float4 (&y)[C]) {
+    auto part = [&](int c, int g) {
         // by pair: its first segment when its run starts inside this tile
         const int slot = p.by_tile ? c + tile : 2 * c + (c * p.U >= tile * p.SB ? 0 : 1);
-        return __ldcg(reinterpret_cast<const float4*>(p.partial + (static_cast<long long>(slot) * p.part_rows + mm) * kPairTile + col));
+        return __ldcg(reinterpret_cast<const float4*>(p.partial + (static_cast<long long>(slot) * p.part_rows + mm) * kPairTile + col + g * step));
     };
-    // Eight loads on their way at a time: one after the other each cost an L2 round trip, and that was most of the call for a row
-    // or two of tiles cut into a dozen segments.
-    constexpr int kFly = 8;
-    float4 y = part(first);
+    constexpr int kFly = 8 / C;
+#pragma unroll
+    for (int g = 0; g < C; g++) y[g] = part(first, g);
     for (int c = first + 1; c <= last; c += kFly) {
-        float4 v[kFly];
+        float4 v[kFly][C];
 #pragma unroll
         for (int i = 0; i < kFly; i++)
-            if (c + i <= last) v[i] = part(c + i);
+            if (c + i <= last)
+#pragma unroll
+                for (int g = 0; g < C; g++) v[i][g] = part(c + i, g);
 #pragma unroll
         for (int i = 0; i < kFly; i++)
-            if (c + i <= last) {
-                y.x = __fadd_rn(y.x, v[i].x);
-                y.y = __fadd_rn(y.y, v[i].y);
-                y.z = __fadd_rn(y.z, v[i].z);
-                y.w = __fadd_rn(y.w, v[i].w);
-            }
+            if (c + i <= last)
+#pragma unroll
+                for (int g = 0; g < C; g++) {
+                    y[g].x = __fadd_rn(y[g].x, v[i][g].x);
+                    y[g].y = __fadd_rn(y[g].y, v[i][g].y);
+                    y[g].z = __fadd_rn(y[g].z, v[i][g].z);
+                    y[g].w = __fadd_rn(y[g].w, v[i][g].w);
+                }
     }
-    return y;
+}
+__device__ __forceinline__ float4 pair_sum4(const PairParams& p, int tile, int first, int last, int mm, int col) {
+    float4 y[1];
+    pair_sums4<1>(p, tile, first, last, mm, col, 0, y);
+    return y[0];
 }
 
 // Tiles that more than one pair worked on: sum their partial tiles, finish as the epilogue would and store.  One block
@@ -705,11 +715,12 @@ template <int ODT, int MODE, bool CUT> __global__ void __launch_bounds__(256) ge
     const bool four = p.y8 && n + 4 <= Nloc;
     uint2 res = make_uint2(0, 0);
     if (MODE == kPairAdd && four) res = *reinterpret_cast<const uint2*>(p.res + o);
-    const float4 y = pair_sum4(p, tile, first, last, mm, col);
-    float yy[4] = {y.x, y.y, y.z, y.w};
+    float4 sums[MODE == kPairSilu ? 2 : 1];
+    pair_sums4(p, tile, first, last, mm, col, 64, sums);
+    float yy[4] = {sums[0].x, sums[0].y, sums[0].z, sums[0].w};
     using A = Act16<NVE_DT_F16>;
     if constexpr (MODE == kPairSilu) {
-        const float4 u = pair_sum4(p, tile, first, last, mm, col + 64);
+        const float4 u = sums[1];
         const float uu[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
         for (int e = 0; e < 4; e++) yy[e] = silu_mul_f32(A::to_f32(A::from_f32(yy[e])), A::to_f32(A::from_f32(uu[e])));
@@ -736,26 +747,32 @@ template <int ODT, int MODE, bool CUT> __global__ void __launch_bounds__(256) ge
 // takes four element pairs (i, i + hd / 2) of a head, 32 threads a row of the tile.  As launches of their own the finish and the embedding
 // cost two grid dependencies (1.85 us each) and read q, k and v once more.
 __global__ void __launch_bounds__(256) gemm_pair_reduce_rope_kernel(const PairParams p, const PairRope ro) {
-    pdl_wait();
-    pdl_launch_dependents();
     const int tile = blockIdx.x;
     const int first = (tile * p.SB) / p.U, last = ((tile + 1) * p.SB - 1) / p.U;
     const PairTile tl = pair_locate<kPairPlain>(p, tile);
     const int Nloc = p.Nm[tl.mi], half = ro.hd / 2, per = half / 4;
     const int head = static_cast<int>(threadIdx.x) / per, i = (static_cast<int>(threadIdx.x) - head * per) * 4, col = head * ro.hd + i;
     const int mm = static_cast<int>(blockIdx.y * blockDim.y + threadIdx.y), m = tl.xt * p.NB + mm, n = tl.n0 + col;
-    if (n >= Nloc || mm >= p.NB || m >= p.M) return;
+    const bool have = n < Nloc && mm < p.NB && m < p.M;
     using A = Act16<NVE_DT_F16>;
     uint16_t* y = static_cast<uint16_t*>(p.Y[tl.mi]) + static_cast<long long>(m) * Nloc + n;
     const int pos = ro.start_pos + m;
-    const uint2 cw = *reinterpret_cast<const uint2*>(ro.cos_t + static_cast<long long>(pos) * half + i);
-    const uint2 sw = *reinterpret_cast<const uint2*>(ro.sin_t + static_cast<long long>(pos) * half + i);
+    uint2 cw = make_uint2(0, 0), sw = cw;  // static, like all up to here: 61 rows 74.7 -> 74.1 us a layer (the other finishes: few rows slower)
+    if (have && tl.mi < 2) {
+        cw = *reinterpret_cast<const uint2*>(ro.cos_t + static_cast<long long>(pos) * half + i);
+        sw = *reinterpret_cast<const uint2*>(ro.sin_t + static_cast<long long>(pos) * half + i);
+    }
+    pdl_wait();
+    pdl_launch_dependents();
+    if (!have) return;
     uint2 a, b;
     if (first == last && !p.by_tile) {
         a = __ldcg(reinterpret_cast<const uint2*>(y));
         b = __ldcg(reinterpret_cast<const uint2*>(y + half));
     } else {
-        const float4 f = pair_sum4(p, tile, first, last, mm, col), g = pair_sum4(p, tile, first, last, mm, col + half);
+        float4 fg[2];
+        pair_sums4<2>(p, tile, first, last, mm, col, half, fg);
+        const float4 f = fg[0], g = fg[1];
         auto two = [](float u, float v) { return static_cast<uint32_t>(A::from_f32(u)) | (static_cast<uint32_t>(A::from_f32(v)) << 16); };
         a = make_uint2(two(f.x, f.y), two(f.z, f.w));
         b = make_uint2(two(g.x, g.y), two(g.z, g.w));
@@ -903,8 +920,9 @@ __global__ void __launch_bounds__(256) gemm_pair_reduce_norm_rows_kernel(const P
             if (first == last && !p.by_tile) {
                 unpack8(__ldcg(reinterpret_cast<const uint4*>(y16 + row) + c), a);
             } else {
-                const float4 lo = pair_sum4(p, tile, first, last, mm, col), hi = pair_sum4(p, tile, first, last, mm, col + 4);
-                const float f[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+                float4 eight[2];
+                pair_sums4<2>(p, tile, first, last, mm, col, 4, eight);
+                const float f[8] = {eight[0].x, eight[0].y, eight[0].z, eight[0].w, eight[1].x, eight[1].y, eight[1].z, eight[1].w};
 #pragma unroll
                 for (int e = 0; e < 8; e++) a[e] = Act16<NVE_DT_F16>::from_f32(f[e]);
             }
