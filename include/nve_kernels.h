@@ -220,7 +220,7 @@ NVE_API int nve_b200_silu_mul(void* gate, const void* up, int n, int dtype, nve_
  *   caches (which already hold the block); out has q's layout.  Replaces the unfused masked SDPA of
  *   src/gpu_layer.rs:846-885.  Blocks of fewer than 64 (row, KV head) pairs, and of up to two such pairs per SM behind
  *   a short prefix, run the streaming decode kernel with the row as second grid dimension, others a tiled tensor-core kernel
- *   (64 query rows share the K/V they read).  A row equals a nve_flash_decode_f16 call of length start_pos + r + 1 within
+ *   (64 query rows share the K/V they read; 128 in blocks that fill the GPU with such tiles).  A row equals a nve_flash_decode_f16 call of length start_pos + r + 1 within
  *   5e-3 of the largest output (the order of the sums follows kernel and split), and bit for bit with fewer than 64 pairs and
  *   max_seq_len up to 128.  head_dim 64 or 128; q and caches 16-byte aligned. */
 NVE_API int nve_b200_rms_norm_rows(const void* x, const void* weight, void* out, int rows, int n, float eps, int dtype,

@@ -291,8 +291,8 @@ extern "C" int nve_b200_set_attn_decode_kernel(int mode) {
 
 /* Causal attention of a block of S new positions against the cache (which already holds them): row r of q
  * [S, num_heads * head_dim] attends to positions [0, start_pos + r]; out has q's layout.  One launch.  Small blocks
- * run the streaming decode kernel with the row as second grid dimension, larger ones the tiled kernel of attn_prefill_mma.cu (64
- * query rows share the K/V they read).  A row equals a nve_flash_decode_f16 call of that length within rounding, bit for bit
+ * run the streaming decode kernel with the row as second grid dimension, larger ones a tiled kernel: 64
+ * query rows that share the K/V they read (attn_prefill_mma.cu), or 128 where such tiles fill the SMs (attn_prefill_tc.cu).  A row equals a nve_flash_decode_f16 call of that length within rounding, bit for bit
  * where both run the same kernel with the same split (fewer than 64 (row, KV head) pairs, caches of up to 128 positions). */
 extern "C" int nve_b200_attn_prefill_causal(const uint16_t* q, const uint16_t* k_cache, const uint16_t* v_cache, uint16_t* out,
                                             int rows, int start_pos, int num_heads, int num_kv_heads, int head_dim,

@@ -1,4 +1,4 @@
-// Launch parameters of the decode attention kernels (attn_decode.cu, attn_decode_mma.cu, attn_stream_mma.cu, attn_prefill_mma.cu).
+// Launch parameters of the decode attention kernels (attn_decode.cu, attn_decode_mma.cu, attn_stream_mma.cu, attn_prefill_mma.cu, attn_prefill_tc.cu).
 #pragma once
 #include "common.cuh"
 #include "gemm_w4a16.cuh"
@@ -37,7 +37,7 @@ bool attn_stream_mma_try(const AttnParams& p, int head_dim, cudaStream_t st, cud
 // attn_prefill_mma.cu: the causal block described above, in tiles of query rows; false when the shape is not covered.
 bool attn_prefill_mma_try(const AttnParams& p, int head_dim, cudaStream_t st, cudaError_t& err);
 
-// attn_prefill_tc.cu: the same in tiles of 256 query rows on tcgen05; false: not its shapes, or too few of them.
+// attn_prefill_tc.cu: the same in tiles of 128 query rows on tcgen05; false: not its shapes, or too few of them.
 bool attn_prefill_tc_try(const AttnParams& p, int head_dim, cudaStream_t st, cudaError_t& err);
 
 // attn_decode_mma.cu: decode attention of one sequence (or query row) on the tensor cores, built for latency; false when the

@@ -14,14 +14,16 @@
 // A commit behind S of step j covers every product issued before it, that of P of step j - 1 among them: whoever sees that S may
 // overwrite it and may rescale O.
 //
-// What bounds it: the chain of a step.  8B, 1777 rows: 1.7 operations per probability and cycle (0.33 of the tensor pipe); from S to P 2900
+// What bounds it: the chain of a step.  8B, 1777 rows: 0.26 of the tensor pipe's cycles; from S to P 2900
 // cycles (exponentials 2000: both tiles compute them at the same time), the two products with their waits 2000, start and end of a CTA
 // 6000.  Against tiles of 64 rows on mma.sync (us): 1777 rows 107 -> 46, 600 rows 21.7 -> 14.4, 300 rows 11.9 -> 10.0, behind 1000 positions
 // 40.1 -> 25.9; 24 heads over 8, 300 rows at 700 26.3 -> 23.5.  Tried: one thread per row (54.8 with 1777 rows: its chain is twice as long), one
 // warp issuing for both tiles (50.9), the second tile half a step behind the first (41.5 against 40.5), positions split over a cluster of two
 // or four (300 rows at 700 21 to 22, but the merge through distributed shared memory makes everything shorter slower, and its code all).
-// Error against 64 bits (2-norm, tiles of 64 / this): 128 rows 2.364e-4 / 2.341e-4, 300 2.428e-4 / 2.415e-4, 1777 2.532e-4 / 2.524e-4, heads of 64
-// 1000 rows 2.504e-4 / 2.491e-4, 300 rows at 100 2.669e-4 / 2.682e-4.
+// Error against 64 bits (2-norm over six random inputs, tiles of 64 / this): 300 rows 2.433e-4 / 2.418e-4, 600 2.474e-4 / 2.462e-4, 1777 2.532e-4 /
+// 2.523e-4, 1000 at 500 2.776e-4 / 2.781e-4; 24 over 8 heads, 300 at 700 2.073e-4 both; heads of 64, 700 rows 2.478e-4 / 2.467e-4, 300 at 400 2.751e-4 /
+// 2.759e-4.  Both round p to f16 once (3, 5, 6 and 7 heads: two numbers); which p the running maximum makes exact differs with the length of a
+// step.  With queries a quarter as large -1.2 to +0.1 %, four times as large -0.15 to +0.03 %; 0.26 % less on average.
 #include <cuda.h>
 
 #include "attn_mma.cuh"

@@ -525,7 +525,7 @@ def gpu_layer_forward_decode_batch(hidden: Tensor, layer_idx: int, state: GpuInf
 
     The projections are the tensor-core GEMM on the packed weights (q/k/v and gate/up one launch each; the residual add and
     the second RMSNorm ride on the o projection, SiLU*up on gate/up), RoPE + K/V write + attention of all sequences is one
-    launch of the fused decode kernel.  16-bit activations on every layer, as in prefill.  Row b equals the single-sequence decode of that
+    launch of the fused decode kernel, which with `scratch` also sums the segments of the q/k/v product.  16-bit activations on every layer, as in prefill.  Row b equals the single-sequence decode of that
     sequence within the tolerance that separates the tensor-core GEMM from the integer GEMV.  With `scratch` nothing is
     allocated and the result is one of scratch.out (alternating with the layer index).
 
