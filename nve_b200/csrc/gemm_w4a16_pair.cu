@@ -72,8 +72,8 @@ struct PairParams {
     int U;           // units per pair
     int total;       // units
     int sc16;        // 1: rows of scales are 16-byte aligned
-    int y2;          // 1: an output is not 4-byte aligned
-    int y8;          // 1: the 16-bit outputs, what is added to them, and their rows are 8-byte aligned
+    short y2;        // 1: an output is not 4-byte aligned
+    short y8;        // 1: the 16-bit outputs, what is added to them, and their rows are 8-byte aligned
     int by_tile;     // 1: every segment is in the workspace, that of (run, tile) in slot run + tile (the kernel for few rows)
     const uint16_t* res;  // kPairAdd: [M, N] f16, added to the rounded product
 };
