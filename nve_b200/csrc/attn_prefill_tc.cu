@@ -20,10 +20,10 @@
 // 40.1 -> 25.9; 24 heads over 8, 300 rows at 700 26.3 -> 23.5.  Tried: one thread per row (54.8 with 1777 rows: its chain is twice as long), one
 // warp issuing for both tiles (50.9), the second tile half a step behind the first (41.5 against 40.5), positions split over a cluster of two
 // or four (300 rows at 700 21 to 22, but the merge through distributed shared memory makes everything shorter slower, and its code all).
-// Error against 64 bits (2-norm over six random inputs, tiles of 64 / this): 300 rows 2.433e-4 / 2.418e-4, 600 2.474e-4 / 2.462e-4, 1777 2.532e-4 /
-// 2.523e-4, 1000 at 500 2.776e-4 / 2.781e-4; 24 over 8 heads, 300 at 700 2.073e-4 both; heads of 64, 700 rows 2.478e-4 / 2.467e-4, 300 at 400 2.751e-4 /
-// 2.759e-4.  Both round p to f16 once (3, 5, 6 and 7 heads: two numbers); which p the running maximum makes exact differs with the length of a
-// step.  With queries a quarter as large -1.2 to +0.1 %, four times as large -0.15 to +0.03 %; 0.26 % less on average.
+// Error against 64 bits (2-norm over six random inputs, tiles of 64 / this): 300 rows 2.433e-4 / 2.442e-4, 600 2.474e-4 / 2.484e-4, 1777 2.532e-4 /
+// 2.542e-4, 1000 at 500 2.776e-4 / 2.785e-4; 24 over 8 heads, 300 at 700 2.073e-4 both; heads of 64, 700 rows 2.478e-4 / 2.488e-4, 300 at 400 2.751e-4 /
+// 2.765e-4.  Both round p to f16 for the product (3, 5, 6 and 7 heads: two numbers) and sum it in f32; which p the running maximum makes exact
+// differs with the length of a step.  A sum of the rounded p has 0.45 % less here and up to ten times as much where one key dominates thousands of equal ones.
 #include <cuda.h>
 
 #include "attn_mma.cuh"
@@ -248,8 +248,7 @@ __device__ __forceinline__ void tc_block(const AttnParams& p, const TcMaps& maps
                     e.x = tc_exp2(e.x);
                     e.y = tc_exp2(e.y);
                     hi[i] = pack_f16x2(e.x, e.y);
-                    // the sum of the probabilities as they are multiplied: the rounding of a large one cancels
-                    sum[i & 1] = tc_add2(sum[i & 1], SPLIT ? e : __half22float2(*reinterpret_cast<const __half2*>(&hi[i])));
+                    sum[i & 1] = tc_add2(sum[i & 1], e);  // as they are, not as they are multiplied: f16 ends at 2^-24, and many equal small ones round the same way
                     if (SPLIT || CAREFUL) {
                         v[2 * i] = e.x;
                         v[2 * i + 1] = e.y;

@@ -81,3 +81,21 @@ def test_infinities_do_not_reach_earlier_rows(cuda, orc, nh, nkv, hd, S, start):
     assert torch.equal(got[inf:key, ..., 4:hd - 1], clean[inf:key, ..., 4:hd - 1]) and torch.equal(got[inf:nan, ..., hd - 1], clean[inf:nan, ..., hd - 1])
     assert not torch.isfinite(got[inf:key, ..., 3]).any() and not torch.isfinite(got[nan:key, ..., hd - 1]).any()
     assert torch.equal(run().view(torch.int16), got.view(torch.int16))
+
+
+@pytest.mark.parametrize("nh,nkv,hd,L,score", [(32, 8, 128, 65536, 17.3), (32, 8, 64, 131072, 18.0), (16, 16, 128, 65536, 17.3), (24, 8, 128, 65536, 17.3)])
+def test_one_dominating_key(cuda, orc, nh, nkv, hd, L, score):
+    """One position far above all others, whose equal probabilities (2^-25 of the largest, where f16 has one bit or none) count together in the sum."""
+    from nve_b200 import cuda_kernels as ck
+
+    torch = cuda
+    S = 640
+    q = torch.full((S, nh * hd), 0.5, dtype=torch.float16, device="cuda")
+    kc, vc = (torch.zeros((nkv, L, hd), dtype=torch.float16, device="cuda") for _ in range(2))
+    kc[:, 0, :16] = score * hd ** 0.5 / 8
+    vc[:, 0] = dev(orc.to_act16(orc.fill_normal(nkv * hd, 897, 1)), torch.float16).view(nkv, hd)
+    got = ck.attn_prefill_causal(q, kc, vc, L - S, nh, nkv, hd, L, hd ** -0.5).double().view(S, nkv, nh // nkv, hd)
+    others = torch.arange(L - S, L, dtype=torch.float64, device="cuda")[:, None, None, None]  # positions that a row sees behind the first
+    want = vc[None, :, None, 0].double() / (1 + others * torch.exp(-8 * hd ** -0.5 * kc[0, 0, 0].double()))
+    # one f16 rounding of the result, the f32 exponentials, the roundings of the f32 sums of up to 1024 steps
+    assert ((got - want).abs() <= (2.0 ** -11 + 2.0 ** -14) * want.abs() + 2.0 ** -25).all()
