@@ -547,6 +547,7 @@ def gpu_layer_forward_decode_batch(hidden: Tensor, layer_idx: int, state: GpuInf
     qkv = [w.q_proj, w.k_proj, w.v_proj]
     if s is not None and normed.dtype == torch.float16 and normed.shape[0] > 1 and hd in (64, 128) and \
             all(p.awq_scales is None and p.k == normed.shape[1] and p.k % 64 == 0 for p in qkv) and \
+            (normed.shape[0] <= DENSE_ROWS or all(_gemm_takes(normed, p, o) for p, o in zip(qkv, (s.q, s.k, s.v)))) and \
             _workspace_holds(ws, normed.shape[0], [p.n for p in qkv], w.q_proj.k):
         # the attention sums the segments of the product itself
         attn = ck.qkv_attn_decode_batch(normed, [p.triple() for p in qkv], w.q_proj.k, [s.q, s.k, s.v], ws, kv.k[layer_idx], kv.v[layer_idx],

@@ -2,7 +2,7 @@
 calls, bit for bit."""
 import pytest
 
-from helpers import dev
+from helpers import dev, rel_rms_err
 from test_gpu_gemm_finish import _weights, _x
 
 pytestmark = pytest.mark.gpu
@@ -65,3 +65,33 @@ def test_refuses_what_does_not_fit(cuda, orc):
             run(*args)
     with pytest.raises(ValueError):
         run(8, 2, 64, B=3)
+
+
+@pytest.mark.parametrize("what", ["nibbles", "scales"])
+def test_many_rows_of_what_the_gemm_does_not_take(cuda, orc, what):
+    """Above 128 sequences q, k and v weights off their boundaries go the dense way, as they do in matmul_x_multi."""
+    from nve_b200.gpu_layer import BatchedDecodeScratch, BatchedKvCache, gpu_layer_forward_decode_batch
+    from test_gpu_glue import _make_state
+
+    torch = cuda
+    B, hidden, ffn, nh, nkv, hd, max_seq = 130, 512, 768, 8, 2, 64, 40
+    st = _make_state(torch, orc, hidden, ffn, nh, nkv, hd, 1, max_seq, 1220, True)
+    x = _x(torch, orc, B, hidden, 1221)
+    d_pos = torch.tensor([(7 * b + 1) % max_seq for b in range(B)], dtype=torch.int32, device="cuda")
+    rows = dev(orc.to_act16(orc.fill_normal(2 * B * nkv * max_seq * hd, 1222, 1)), torch.float16).view(2, B, nkv, max_seq, hd)
+    results = []
+    for shifted in (False, True):
+        if shifted:
+            for p in (st.layer_weights[0].q_proj, st.layer_weights[0].v_proj):
+                t = getattr(p, what)
+                room = torch.empty(t.numel() + 8, dtype=t.dtype, device="cuda")
+                off = 8 if what == "nibbles" else 1
+                setattr(p, what, room[off:off + t.numel()].view(t.shape).copy_(t))
+                assert getattr(p, what).data_ptr() % (16 if what == "nibbles" else 8) != 0
+        kv = BatchedKvCache([rows[0].clone()], [rows[1].clone()], B, max_seq)
+        scratch = BatchedDecodeScratch.make(st, B, hidden, ffn)
+        out = gpu_layer_forward_decode_batch(x.clone(), 0, st, kv, d_pos, d_pos + 1, scratch)
+        results.append((out.clone(), kv.k[0], kv.v[0]))
+    for a, b in zip(*results):
+        # the same f16 weights in another product: roundings (half an f16 ulp, 2.4e-4) of q, k, v and of the launches behind that may fall the other way
+        assert rel_rms_err(b.float().cpu().numpy(), a.float().cpu().numpy()) < 2e-3
