@@ -624,9 +624,15 @@ def qkv_attn_decode_batch(x: Tensor, weights: Sequence, k_dim: int, outs: Sequen
                           head_dim: int, max_seq_len: int, scale: float, out: Tensor) -> Tensor:
     """gemm_w4a16_wide over q, k, v of x [B, K] and attn_decode_fused_batch, without the launch between them that finishes the
     product; `outs` (q, k, v) are scratch, written or not."""
+    if x.dim() != 2 or x.shape[1] != k_dim:
+        raise ValueError("qkv_attn_decode_batch: x must be [B, k]")
     b = x.shape[0]
-    if k_cache.shape[0] != b or d_pos.numel() != b or d_seq_len.numel() != b:
+    if len(weights) != 3 or len(outs) != 3 or any(o.numel() != b * w[2] for w, o in zip(weights, outs)):
+        raise ValueError("qkv_attn_decode_batch: three matrices, an output [B, n] each")
+    if k_cache.shape[0] != b or v_cache.shape != k_cache.shape or d_pos.numel() != b or d_seq_len.numel() != b:
         raise ValueError("one cache, position and length per row of x")
+    if out.numel() != b * num_heads * head_dim:
+        raise ValueError("qkv_attn_decode_batch: out must be [B, nh * hd]")
     arr = _mats(weights, outs, None, _F16)
     _ffi.check("nve_b200_qkv_attn_decode_batch",
                _lib().nve_b200_qkv_attn_decode_batch(

@@ -3,6 +3,7 @@ import os
 import re
 
 import numpy as np
+import pytest
 
 from nve_b200.gpu_layer import RoutingConfig, normalize_importance
 
@@ -55,3 +56,25 @@ def test_pair_gemm_roles_wait_on_bounded_barriers_only():
     for part in (loaders, roles):
         assert "pg_wait(" in part  # the split above still finds the roles
         assert not re.search(r"\bbar(rier)?\.(cta\.)?(sync|arrive|red)|__syncthreads|__barrier", part)
+
+
+@pytest.mark.parametrize("wrong,words", [
+    (dict(x=(4, 256)), "x must be"), (dict(x=(4, 1, 512)), "x must be"), (dict(k_dim=1024), "x must be"),
+    (dict(drop=True), "three matrices"), (dict(outs=((4, 512), (4, 128))), "three matrices"), (dict(outs=((4, 512), (4, 128), (3, 128))), "three matrices"),
+    (dict(k=(3, 2, 8, 64)), "one cache"), (dict(v=(4, 2, 7, 64)), "one cache"), (dict(pos=3), "one cache"), (dict(out=(4, 256)), "out must be"),
+    (dict(), "CUDA tensor"),  # nothing wrong but that there is no GPU
+])
+def test_qkv_attn_decode_batch_refuses_shapes_that_do_not_fit(wrong, words):
+    """Before any address is taken: a matrix too few or a row too short would be read past its end."""
+    import torch
+
+    from nve_b200 import cuda_kernels as ck
+
+    z = lambda *s: torch.zeros(s, dtype=torch.float16)
+    ws = [(torch.zeros((n, 256), dtype=torch.uint8), torch.zeros((n, 16)), n) for n in (512, 128, 128)]
+    d = torch.zeros(wrong.get("pos", 4), dtype=torch.int32)
+    with pytest.raises(ValueError, match=words):
+        ck.qkv_attn_decode_batch(z(*wrong.get("x", (4, 512))), ws[:2] if wrong.get("drop") else ws, wrong.get("k_dim", 512),
+                                 [z(*s) for s in wrong.get("outs", ((4, 512), (4, 128), (4, 128)))], torch.empty(64, dtype=torch.uint8),
+                                 z(*wrong.get("k", (4, 2, 8, 64))), z(*wrong.get("v", (4, 2, 8, 64))), z(8, 32), z(8, 32), d, d, 8, 2, 64, 8, 0.125,
+                                 z(*wrong.get("out", (4, 512))))
