@@ -307,8 +307,8 @@ __device__ __forceinline__ void tc_block(const AttnParams& p, const TcMaps& maps
             __syncwarp();
             if (lane == 0) tc_arrive(&sh.bars.p[t]);
         }
-        // ---- epilogue: the commit behind the last product of the tile is one more phase of its S barrier.  The rows leave through the
-        // tile's Q, which nobody needs any more, by TMA: sixteen bytes per lane straight to 32 different rows took 4000 cycles.
+        // ---- epilogue: the commit behind the last product of the tile is one more phase of its S barrier.  The rows go to the
+        // tile's Q, which nobody needs any more.
         if (steps > 0) {
             if (ok && !tc_wait(&sh.bars.s[t], steps & 1, abort)) ok = false;
             tc_fence_after();
@@ -351,16 +351,7 @@ __device__ __forceinline__ void tc_block(const AttnParams& p, const TcMaps& maps
                 }
             }
             if (!CAREFUL && valid && !(fabsf((probe[0] + probe[1]) + (probe[2] + probe[3])) <= 3.0e38f)) sh.bad = 1;
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            tc_tile_barrier(t);
-            if ((tid & 255) == 0 && (t == 0 ? tl.npos[0] : tl.npos[1]) > 0) {  // rows behind the block's last are outside the map
-                for (int c = 0; c < HD / 64; c++)
-                    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(&maps.out),
-                                 "r"(sq + t * kTile + c * kHalf), "r"(64 * c), "r"(tl.kvh * tl.groups), "r"(pos0)
-                                 : "memory");
-                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // for the store behind the CTA's next barrier
         }
     } else if (warp < kTcLoadWarp) {
         // -------------------------------------------------------------- MMA issue: the whole warp runs the loop, one lane issues
@@ -486,9 +477,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     pdl_launch_dependents();
     tc_block<HD, SPLIT, false>(p, maps, tl, sh, base);
     __syncthreads();
-    if (sh.bad && !sh.abort) {  // every product and every load has been waited for
-        if (warp < kTcMmaWarp && (tid & 255) == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // what was stored is written again
-        __syncthreads();
+    if (sh.bad && !sh.abort) {  // every product and every load has been waited for; nothing has been stored, so that q is as it was if out is the same memory
         TcTiles all = tl;
         all.steps[0] = all.steps[1] = max(tl.steps[0], tl.steps[1]);  // (a step that no row of a tile sees adds zeros)
         if (tid == 0) {
@@ -499,6 +488,17 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         __syncthreads();
         tc_block_careful<HD, SPLIT>(p, maps, all, sh, base);
         __syncthreads();
+    }
+    // By TMA: sixteen bytes per lane straight to 32 different rows took 4000 cycles.  Rows behind the block's last are outside the map.
+    const int t = warp >> 3;
+    if (warp < kTcMmaWarp && (tid & 255) == 0 && (t == 0 ? tl.npos[0] : tl.npos[1]) > 0) {
+        constexpr uint32_t kHalf = 128 * 128;
+        for (int c = 0; c < HD / 64; c++)
+            asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(&maps.out),
+                         "r"(base + t * (kHalf * (HD / 64)) + c * kHalf), "r"(64 * c), "r"(tl.kvh * groups), "r"(t == 0 ? tl.pos0[0] : tl.pos0[1])
+                         : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     }
     if (*static_cast<volatile int*>(&sh.abort)) {  // copies and products may still be under way: give them time
         for (int i = 0; i < 100; i++) __nanosleep(10000);

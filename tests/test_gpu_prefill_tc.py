@@ -81,6 +81,9 @@ def test_infinities_do_not_reach_earlier_rows(cuda, orc, nh, nkv, hd, S, start):
     assert torch.equal(got[inf:key, ..., 4:hd - 1], clean[inf:key, ..., 4:hd - 1]) and torch.equal(got[inf:nan, ..., hd - 1], clean[inf:nan, ..., hd - 1])
     assert not torch.isfinite(got[inf:key, ..., 3]).any() and not torch.isfinite(got[nan:key, ..., hd - 1]).any()
     assert torch.equal(run().view(torch.int16), got.view(torch.int16))
+    out = q.clone()  # in place: a tile that is computed once more still finds its queries
+    ck.attn_prefill_causal(out, kc, vc, start, nh, nkv, hd, start + S + 3, hd ** -0.5, out=out)
+    assert torch.equal(out.view(torch.int16).view_as(got), got.view(torch.int16))
 
 
 @pytest.mark.parametrize("nh,nkv,hd,L,score", [(32, 8, 128, 65536, 17.3), (32, 8, 64, 131072, 18.0), (16, 16, 128, 65536, 17.3), (24, 8, 128, 65536, 17.3)])
