@@ -569,15 +569,23 @@ bool attn_prefill_tc_try(const AttnParams& p, int head_dim, cudaStream_t st, cud
     if (groups > 64 || (head_dim != 64 && head_dim != 128)) return false;
     if (!aligned(p.q, 16) || !aligned(p.k_cache, 16) || !aligned(p.v_cache, 16) || !aligned(p.out, 16) || (p.row_stride & 7) != 0) return false;
     const bool split = am_split(groups);
-    // Tiles of 128 rows over all KV heads, and steps of the longest.  Below these numbers the form with tiles of 64 rows, which also cuts the
-    // positions of a tile into pieces, fills the SMs better (us, that form / this one, 32 over 8 heads of 128: 128 rows 5.9 / 5.9 and at
-    // 1000 16.1 / 21.7; 180 rows 7.1 / 7.9, at 300 13.8 / 12.1; 256 rows at 2500 45.8 / 47.1; 300 rows 11.9 / 10.0, at 1000 40.1 / 25.9;
-    // heads of 64: 300 rows 7.0 / 7.8, at 100 8.7 / 9.6, at 300 11.9 / 11.1; 400 rows 10.3 / 9.2).
+    // Where tiles of 128 rows take seven tenths of the SMs they are always the faster ones (us, tiles of 64 / this, 32 over 8 heads of 128 where nothing else
+    // is said: 385 rows 14.9 / 10.6, heads of 64 9.6 / 8.5).  With fewer it depends on whether the other form has more tiles than SMs
+    // (tiles64 > sm): if not, it gives each to two CTAs from 449 positions on.
+    //  - It has: this form from 257 positions on (289 rows 11.8 / 9.4).  Heads of 64: from 513 on (310 rows at 203 11.6 / 10.5) and where its tiles share most
+    //    SMs or are of similar length (16 over 4 heads, 152 tiles, 608 rows at 0 9.9 / 10.6, at 192 12.8 / 13.4, at 592 19.3 / 17.9).
+    //  - It has not: while dealing the positions out saves it little and this form has three eighths of the SMs, heads of 64 three sevenths
+    //    (224 rows at 216 11.2 / 11.6, at 225 13.5 / 11.4, at 976 24.1 / 22.7, at 2276 41.9 / 41.1, at 4108 66.8 / 67.1; heads of 64, 193 rows at 1007
+    //    15.1 / 18.0, 225 rows at 215 7.7 / 9.4, at 375 12.2 / 10.8, at 975 19.0 / 18.0).
     const long long PT = 2 * (64 / groups), ctas = (p.rows + PT - 1) / PT * p.num_kv_heads, sm = sm_count();
-    const int steps = (p.seq_len - 1 + p.rows + kTcKeys - 1) / kTcKeys;
-    if (ctas * 10 < sm * 7 && !(ctas * 20 >= sm * 10 + 40 && steps >= (head_dim == 128 ? 3 : 5)) &&
-        !(ctas * 8 >= sm * 3 && steps >= (head_dim == 128 ? 4 : 5) && steps <= 20))
-        return false;
+    const long long tiles64 = (p.rows + PT / 2 - 1) / (PT / 2) * p.num_kv_heads;
+    const int positions = p.seq_len - 1 + p.rows, steps = (positions + kTcKeys - 1) / kTcKeys;
+    if (ctas * 10 < sm * 7) {
+        if (head_dim == 128 ? (tiles64 > sm ? positions <= 256 : ctas * 8 < sm * 3 || positions <= 448 || positions > 2560)
+                            : positions <= 512 || (tiles64 * 25 < sm * 27 &&
+                                                   (tiles64 > sm ? 2 * p.rows > positions : ctas * 7 < sm * 3 || positions > 2560)))
+            return false;
+    }
     // Two tiles in a CTA take 1.4 to 1.5 times as long as one: from two waves of single tiles on, or where a second wave would be as long as
     // the first (us, one / two: 1000 rows 24.4 / 30.0, at 1000 55.9 / 51.0; 1300 rows 37.3 / 36.0; 1777 rows 59.7 / 46.2; 24 over 8 heads,
     // whose steps are longer, 1000 rows at 1000 58.4 / 59.8, 1777 rows 56.5 / 53.3).

@@ -35,6 +35,9 @@ def reference(torch, q, kc, vc, nh, nkv, hd, S, start):
     (20, 20, 128, 900, 10),  # one head per KV head: tiles of 128 positions, whose steps differ by one
     (40, 40, 64, 1100, 0),   # the same in pairs
     (64, 1, 64, 230, 300),   # 64 heads: two positions per tile
+    # on both sides of the lines to the form with tiles of 64 rows: 448 / 449 positions, 512 / 513, and 56 / 64 tiles with heads of 64
+    (32, 8, 128, 224, 224), (32, 8, 128, 224, 225), (32, 8, 128, 256, 2304), (32, 8, 128, 289, 0),
+    (32, 8, 64, 310, 202), (32, 8, 64, 310, 203), (32, 8, 64, 224, 900), (32, 8, 64, 225, 900), (16, 4, 64, 608, 600), (16, 4, 64, 608, 0),
 ])
 def test_against_f64(cuda, orc, nh, nkv, hd, S, start):
     from nve_b200 import cuda_kernels as ck
