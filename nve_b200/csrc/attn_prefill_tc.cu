@@ -41,7 +41,7 @@ struct TcBars {
     uint64_t qfull[2], kfull[2], kempty[2], vfull[2], vempty[2], s[2], p[2], o[2];
 };
 struct TcShared {
-    TcBars bars;
+    TcBars bars[2];  // of the first pass and of a second one: the last commits to kempty and vempty, which nobody waits for, may arrive late
     float pass[2][2][128];  // between the two threads of a row: [tile][half][row]
     uint32_t tmem;
     int abort, bad;
@@ -186,6 +186,7 @@ __device__ __forceinline__ void tc_block(const AttnParams& p, const TcMaps& maps
     const uint32_t sq = base, sk = sq + 2 * kTile, sv = sk + 2 * kTile;
     const int n = max(tl.steps[0], tl.steps[1]);
     volatile int* abort = &sh.abort;
+    TcBars& bars = sh.bars[CAREFUL ? 1 : 0];
     const uint32_t tmem = sh.tmem;
 
     if (warp < kTcMmaWarp) {
@@ -207,7 +208,7 @@ __device__ __forceinline__ void tc_block(const AttnParams& p, const TcMaps& maps
             for (int d = 0; d < HD; d++) extra[d] = 0.0f;
         bool ok = true;
         for (int j = 0; j < steps; j++) {
-            if (ok && !tc_wait(&sh.bars.s[t], j & 1, abort)) ok = false;  // (the steps go on: the warps of a row meet at barriers)
+            if (ok && !tc_wait(&bars.s[t], j & 1, abort)) ok = false;  // (the steps go on: the warps of a row meet at barriers)
             tc_fence_after();
             float s[64];
             tc_ld32(ts + half * 64, s);
@@ -275,7 +276,7 @@ __device__ __forceinline__ void tc_block(const AttnParams& p, const TcMaps& maps
             }
             l += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
             if (CAREFUL && (j + 1) * kTcKeys > cut_from) {  // the same for both tiles
-                if (ok && !tc_wait(&sh.bars.vfull[j & 1], (j >> 1) & 1, abort)) ok = false;
+                if (ok && !tc_wait(&bars.vfull[j & 1], (j >> 1) & 1, abort)) ok = false;
                 const uint32_t vb = sv + static_cast<uint32_t>(j & 1) * kTile;
                 float ps[64];
                 for (int i = 0; i < 64; i++) ps[i] = s[i];
@@ -305,12 +306,12 @@ __device__ __forceinline__ void tc_block(const AttnParams& p, const TcMaps& maps
             tc_st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) tc_arrive(&sh.bars.p[t]);
+            if (lane == 0) tc_arrive(&bars.p[t]);
         }
         // ---- epilogue: the commit behind the last product of the tile is one more phase of its S barrier.  The rows go to the
         // tile's Q, which nobody needs any more.
         if (steps > 0) {
-            if (ok && !tc_wait(&sh.bars.s[t], steps & 1, abort)) ok = false;
+            if (ok && !tc_wait(&bars.s[t], steps & 1, abort)) ok = false;
             tc_fence_after();
             tc_rows_barrier(rows_id);  // the last maxima have been read
             *mine = l;
@@ -367,15 +368,15 @@ __device__ __forceinline__ void tc_block(const AttnParams& p, const TcMaps& maps
                 const uint32_t o = (kk >> 2) * kHalf + (kk & 3) * 32;
                 tc_mma_ss(issuer, ds, tc_desc(a + o, 16, 1024), tc_desc(b + o, 16, 1024), kIdescS, kk > 0);
             }
-            tc_commit(issuer, &sh.bars.s[t]);
-            tc_commit(issuer, &sh.bars.kempty[j & 1]);
+            tc_commit(issuer, &bars.s[t]);
+            tc_commit(issuer, &bars.kempty[j & 1]);
             __syncwarp();
         };
-        if (steps > 0 && tc_wait(&sh.bars.qfull[t], 0, abort) && tc_wait(&sh.bars.kfull[0], 0, abort)) {
+        if (steps > 0 && tc_wait(&bars.qfull[t], 0, abort) && tc_wait(&bars.kfull[0], 0, abort)) {
             tc_fence_after();
             product_s(0);
             for (int j = 0; j < steps; j++) {
-                if (!tc_wait(&sh.bars.vfull[j & 1], (j >> 1) & 1, abort) || !tc_wait(&sh.bars.p[t], j & 1, abort)) break;
+                if (!tc_wait(&bars.vfull[j & 1], (j >> 1) & 1, abort) || !tc_wait(&bars.p[t], j & 1, abort)) break;
                 tc_fence_after();
                 const uint32_t b = sv + static_cast<uint32_t>(j & 1) * kTile;
 #pragma unroll
@@ -384,12 +385,12 @@ __device__ __forceinline__ void tc_block(const AttnParams& p, const TcMaps& maps
                     for (int kk = 0; kk < 8; kk++)  // 16 positions: two groups of eight rows
                         tc_mma_ts(issuer, dst, ds + (SPLIT ? 32 * (kk >> 1) + 8 * (kk & 1) + 16 * part : 8 * kk), tc_desc(b + kk * 2048, kHalf, 1024), kIdescO,
                                   j > 0 || kk > 0 || part > 0);
-                tc_commit(issuer, j + 1 == steps ? &sh.bars.s[t] : &sh.bars.o[t]);
-                tc_commit(issuer, &sh.bars.vempty[j & 1]);
+                tc_commit(issuer, j + 1 == steps ? &bars.s[t] : &bars.o[t]);
+                tc_commit(issuer, &bars.vempty[j & 1]);
                 __syncwarp();
                 if (j + 1 == steps) break;
                 // S of the next step comes over P: not before the product above is complete
-                if (!tc_wait(&sh.bars.kfull[(j + 1) & 1], ((j + 1) >> 1) & 1, abort) || !tc_wait(&sh.bars.o[t], j & 1, abort)) break;
+                if (!tc_wait(&bars.kfull[(j + 1) & 1], ((j + 1) >> 1) & 1, abort) || !tc_wait(&bars.o[t], j & 1, abort)) break;
                 tc_fence_after();
                 product_s(j + 1);
             }
@@ -401,8 +402,8 @@ __device__ __forceinline__ void tc_block(const AttnParams& p, const TcMaps& maps
         for (int j = 0; ok && j < n; j++) {
             const int b = j & 1;
             for (int kv = 0; ok && kv < 2; kv++) {
-                uint64_t* full = kv == 0 ? &sh.bars.kfull[b] : &sh.bars.vfull[b];
-                if (j >= 2) ok = tc_wait(kv == 0 ? &sh.bars.kempty[b] : &sh.bars.vempty[b], ((j >> 1) - 1) & 1, abort);
+                uint64_t* full = kv == 0 ? &bars.kfull[b] : &bars.vfull[b];
+                if (j >= 2) ok = tc_wait(kv == 0 ? &bars.kempty[b] : &bars.vempty[b], ((j >> 1) - 1) & 1, abort);
                 if (ok && issuer) {
                     tc_expect(full, kTile);
                     for (int c = 0; c < HD / 64; c++)
@@ -410,11 +411,11 @@ __device__ __forceinline__ void tc_block(const AttnParams& p, const TcMaps& maps
                     if (j == 0 && kv == 0)
                         for (int t = 0; t < 2; t++)
                             if (tl.npos[t] > 0) {
-                                tc_expect(&sh.bars.qfull[t], tl.PT * tl.groups * 128 * (HD / 64));  // (a box counts whole, also past the end of the block)
+                                tc_expect(&bars.qfull[t], tl.PT * tl.groups * 128 * (HD / 64));  // (a box counts whole, also past the end of the block)
                                 for (int c = 0; c < HD / 64; c++)
-                                    tc_load3(sq + t * kTile + c * kHalf, &maps.q, 64 * c, tl.kvh * tl.groups, tl.pos0[t], &sh.bars.qfull[t]);
+                                    tc_load3(sq + t * kTile + c * kHalf, &maps.q, 64 * c, tl.kvh * tl.groups, tl.pos0[t], &bars.qfull[t]);
                             } else if (CAREFUL) {
-                                tc_arrive(&sh.bars.qfull[t]);
+                                tc_arrive(&bars.qfull[t]);
                             }
                 }
                 __syncwarp();
@@ -447,21 +448,21 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         tl.npos[i] = i < per_cta ? max(0, min(PT, p.rows - tl.pos0[i])) : 0;
         tl.steps[i] = tl.npos[i] > 0 ? (tl.start + tl.pos0[i] + tl.npos[i] + kTcKeys - 1) / kTcKeys : 0;
     }
-    auto init = [&](int both) {  // tiles with steps; one may have one step less than the other, but the last ones are not waited for
+    auto init = [&](TcBars& bars, int both) {  // tiles with steps; one may have one step less than the other, but the last ones are not waited for
         for (int i = 0; i < 2; i++) {
-            tc_init(&sh.bars.qfull[i], 1);
-            tc_init(&sh.bars.kfull[i], 1);
-            tc_init(&sh.bars.kempty[i], both);
-            tc_init(&sh.bars.vfull[i], 1);
-            tc_init(&sh.bars.vempty[i], both);
-            tc_init(&sh.bars.s[i], 1);
-            tc_init(&sh.bars.p[i], 8);  // the tile's warps
-            tc_init(&sh.bars.o[i], 1);
+            tc_init(&bars.qfull[i], 1);
+            tc_init(&bars.kfull[i], 1);
+            tc_init(&bars.kempty[i], both);
+            tc_init(&bars.vfull[i], 1);
+            tc_init(&bars.vempty[i], both);
+            tc_init(&bars.s[i], 1);
+            tc_init(&bars.p[i], 8);  // the tile's warps
+            tc_init(&bars.o[i], 1);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     };
     if (tid == 0) {
-        init(tl.steps[1] > 0 ? 2 : 1);
+        init(sh.bars[0], tl.steps[1] > 0 ? 2 : 1);
         sh.abort = sh.bad = 0;
     }
     if (warp == kTcMmaWarp) {
@@ -477,14 +478,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     pdl_launch_dependents();
     tc_block<HD, SPLIT, false>(p, maps, tl, sh, base);
     __syncthreads();
-    if (sh.bad && !sh.abort) {  // every product and every load has been waited for; nothing has been stored, so that q is as it was if out is the same memory
+    if (sh.bad && !sh.abort) {  // every product and every load has been waited for, nothing has been stored: q is as it was, also where out is the same memory
         TcTiles all = tl;
         all.steps[0] = all.steps[1] = max(tl.steps[0], tl.steps[1]);  // (a step that no row of a tile sees adds zeros)
-        if (tid == 0) {
-            uint64_t* bar = reinterpret_cast<uint64_t*>(&sh.bars);
-            for (unsigned i = 0; i < sizeof(TcBars) / 8; i++) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(tc_addr(bar + i)) : "memory");
-            init(2);
-        }
+        if (tid == 0) init(sh.bars[1], 2);
         __syncthreads();
         tc_block_careful<HD, SPLIT>(p, maps, all, sh, base);
         __syncthreads();

@@ -65,7 +65,7 @@ def test_growing_scores(cuda, orc):
     assert (got.double() - reference(torch, q, kc, vc, nh, nkv, hd, S, start)).abs().max().item() < bound
 
 
-@pytest.mark.parametrize("nh,nkv,hd,S,start", [(32, 8, 128, 420, 21), (24, 8, 128, 600, 0), (32, 8, 64, 1250, 64), (32, 8, 128, 1301, 0)])
+@pytest.mark.parametrize("nh,nkv,hd,S,start", [(32, 8, 128, 420, 21), (24, 8, 128, 600, 0), (32, 8, 64, 1250, 64), (32, 8, 128, 1301, 0), (64, 8, 128, 208, 0), (64, 8, 128, 360, 0)])
 def test_infinities_do_not_reach_earlier_rows(cuda, orc, nh, nkv, hd, S, start):
     """An infinity and a NaN in v, and a NaN in k, at positions inside the block: rows that do not see them keep their bits, rows that
     do are not finite where they have to be."""
