@@ -507,12 +507,13 @@ template <int HD, int G, int NW, int NS, bool FUSED, bool LEFT> struct AsLaunch 
 template <int HD, int G, bool FUSED, bool LEFT> static cudaError_t launch_as_with(const AttnParams& p, cudaStream_t st) {
     using Wide = AsLaunch<HD, G, 8, as_wide_stages<HD, G>(), FUSED, LEFT>;
     using Narrow = AsLaunch<HD, G, 4, 3, FUSED, LEFT>;
+    using Split = AsLaunch<HD, G, 8, as_wide_stages<HD, G>(), FUSED, false>;  // the same split, and so the same values, whatever registers LEFT takes
     const int rows = p.rows > 1 ? p.rows : 1;
     const long long units = static_cast<long long>(p.num_kv_heads) * rows;
-    if (Wide::prepare() != NVE_OK || Narrow::prepare() != NVE_OK) return cudaErrorInvalidValue;
-    if (2 * units > 3ll * Wide::active(p, 1)) return Narrow::launch(p, rows, 1, st);
+    if (Split::prepare() != NVE_OK || Wide::prepare() != NVE_OK || Narrow::prepare() != NVE_OK) return cudaErrorInvalidValue;
+    if (2 * units > 3ll * Split::active(p, 1)) return Narrow::launch(p, rows, 1, st);
     int csize = kAsMaxCluster;
-    while (csize > 1 && (units > Wide::active(p, csize) || p.kv_stride <= 128 * (csize - 1))) csize--;
+    while (csize > 1 && (units > Split::active(p, csize) || p.kv_stride <= 128 * (csize - 1))) csize--;
     return Wide::launch(p, rows, csize, st);
 }
 template <int HD, int G, bool FUSED> static cudaError_t launch_as(const AttnParams& p, cudaStream_t st) {

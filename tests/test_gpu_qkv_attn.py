@@ -23,16 +23,33 @@ pytestmark = pytest.mark.gpu
     (1, 8, 2, 64, 768, True),
 ])
 def test_equals_the_two_calls(cuda, orc, B, nh, nkv, hd, K, scratch, cuda_core):
+    equals_the_two_calls(cuda, orc, B, nh, nkv, hd, K, scratch, cuda_core, 150, [(37 * b + 3) % 150 for b in range(B)])
+
+
+@pytest.mark.parametrize("B,nh,nkv,hd,K,max_seq", [
+    (2, 24, 8, 128, 1024, 2000),   # clusters of seven or eight CTAs
+    (5, 32, 8, 64, 1024, 2000),    # of several, two CTAs per SM
+    (9, 24, 8, 64, 512, 900),
+    (13, 40, 8, 128, 512, 700),    # five heads per KV head
+    (5, 64, 8, 64, 512, 1500),     # eight
+    (2, 32, 8, 64, 1024, 600),     # finished first: few units of small heads in a large cache
+    (70, 32, 8, 64, 512, 300),     # four warps per unit
+    (60, 64, 8, 128, 512, 200),
+])
+def test_equals_the_two_calls_in_large_caches(cuda, orc, B, nh, nkv, hd, K, max_seq):
+    equals_the_two_calls(cuda, orc, B, nh, nkv, hd, K, True, False, max_seq, [max_seq - 1 - 173 * b % max_seq for b in range(B)])  # the first to its end
+
+
+def equals_the_two_calls(cuda, orc, B, nh, nkv, hd, K, scratch, cuda_core, max_seq, positions):
     from nve_b200 import cuda_kernels as ck
 
     torch = cuda
-    max_seq = 150
     x = _x(torch, orc, B, K, 1201)
     Ns = [nh * hd, nkv * hd, nkv * hd]
     ws = [_weights(torch, orc, n, K, 1202 + i)[0] for i, n in enumerate(Ns)]
     kc, vc = (dev(orc.to_act16(orc.fill_normal(B * nkv * max_seq * hd, 1206, i)), torch.float16).view(B, nkv, max_seq, hd) for i in range(2))
     cos, sin = (dev(orc.to_act16(t), torch.float16) for t in orc.rope_tables_f32(hd, max_seq, 10000.0))
-    d_pos = torch.tensor([(37 * b + 3) % max_seq for b in range(B)], dtype=torch.int32, device="cuda")
+    d_pos = torch.tensor(positions, dtype=torch.int32, device="cuda")
     d_len = d_pos + 1
     nbytes = ck.gemm_w4a16_multi_scratch_bytes(B, Ns, K) if scratch else 16
     buf = lambda: [torch.full((B, n), float("nan"), dtype=torch.float16, device="cuda") for n in Ns]
