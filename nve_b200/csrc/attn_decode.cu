@@ -408,11 +408,17 @@ extern "C" int nve_b200_qkv_attn_decode_batch(const uint16_t* X, const nve_b200_
     if (mats[0].N != num_heads * head_dim || mats[1].N != num_kv_heads * head_dim || mats[2].N != mats[1].N) return set_status(NVE_ERR_BAD_SHAPE);
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
     const bool streams = batch_streams(batch, num_heads, num_kv_heads);
-    // Unfinished, but for a few units of small heads whose positions are split over large clusters: there every CTA of a cluster sums the
-    // same segments while the launch that finishes them is at its shortest (us per layer, 1B, finished / unfinished: 2 sequences of 2000
-    // 33.7 / 34.0, of 8000 36.7 / 37.9, of 100 32.5 / 31.2; 4 of 4000 37.0 / 37.7; 5 of 8000 43.2 / 42.2, 24 of 1000 49.7 / 48.1; 3B, 2 of
-    // 8000 49.3 / 48.1).
-    const bool leave = streams && batch > 1 && !(head_dim == 64 && batch * num_kv_heads < 40 && max_seq_len > 512);
+    // Unfinished, but with heads of 64 for
+    //  - few units whose positions are split over large clusters: there every CTA of a cluster sums the same segments while the launch that finishes
+    //    them is at its shortest.  The lengths are on the device, so the capacity of the caches stands for them (us per layer, 1B, finished / unfinished: 2 sequences
+    //    of 2000 33.7 / 34.0, of 8000 36.7 / 37.9, of 100 32.5 / 31.2; 4 of 4000 37.0 / 37.7; 5 of 8000 43.2 / 42.2, 24 of 1000 49.7 / 48.1; 3B, 2 of 8000
+    //    49.3 / 48.1).
+    //  - five heads and more per KV head where four warps take a unit (more than 3 per SM): a thread sums seven features and more, on 250 registers, two CTAs per
+    //    SM instead of four (us per layer, hidden 2048, finished / unfinished: 100 sequences of 300, 6 heads 63.6 / 66.3, 8 heads 66.6 / 69.6, 4 heads
+    //    62.6 / 61.2).
+    const bool leave64 = static_cast<long long>(batch) * num_kv_heads <= 3ll * sm_count() ? batch * num_kv_heads >= 40 || max_seq_len <= 512
+                                                                                          : num_heads / num_kv_heads <= 4;
+    const bool leave = streams && batch > 1 && (head_dim == 128 || leave64);
     PairLeft left;
     if (int s = gemm_qkv(X, mats, batch, K, scratch, scratch_bytes, leave ? &left : nullptr, cs); s != NVE_OK) return s;
     return attn_batch(y[0], y[1], y[2], left, k_cache, v_cache, cos_tab, sin_tab, d_pos, d_seq_len, out, batch, num_heads, num_kv_heads, head_dim, max_seq_len,

@@ -67,9 +67,11 @@ template <int HD, int G, int NW, int NS> struct AsSmem {
 
 // Fused: blockIdx.y is one of `rows` independent sequences (one sequence: rows <= 1).  Else: one of `rows` query rows over one
 // cache, row r attends to seq_len + r positions.  blockIdx.x = KV head * csize + rank.
-// LEFT (fused): q, k and v are a product whose segments are not summed yet; with heads of 64 two CTAs of eight warps still fit an SM.
+// LEFT (fused): q, k and v are a product whose segments are not summed yet; with heads of 64 as many CTAs as otherwise still fit an SM (us a layer, hidden
+// 2048, 64 sequences of 300, finished / LEFT with three CTAs of four warps / with four: one head per KV head 49.3 / 50.1 / 47.9, four 51.7 / 51.3 / 49.7; of
+// 1000 59.9 / 58.0 / 57.9 and 61.7 / 59.2 / 59.8).
 template <int HD, int G, int NW, int NS, bool FUSED, bool LEFT>
-__global__ void __launch_bounds__(32 * NW, LEFT && HD == 64 && NW == 8 ? 2 : 8 / NW) attn_stream_mma_kernel(const AttnParams pin, int csize) {
+__global__ void __launch_bounds__(32 * NW, LEFT && HD == 64 ? 16 / NW : 8 / NW) attn_stream_mma_kernel(const AttnParams pin, int csize) {
     AttnParams p = pin;
     int seq_len_row = p.seq_len;
     const long long b = blockIdx.y;

@@ -147,7 +147,7 @@ template <int E> struct PairFeatures {
         }
     }
     template <class F> __device__ __forceinline__ void sum(const uint16_t* const (&y)[E], uint16_t (&out)[E], F behind) {
-        constexpr int kFly = 8;
+        constexpr int kFly = E > 8 ? 4 : 8;  // registers (64 sequences of 300, 56 over 8 heads of 128: 75.2 -> 73.7 us a layer)
         float total[E];
         for (int c0 = 0; c0 == 0 || c0 < most; c0 += kFly) {
             float v[kFly][E];

@@ -35,6 +35,8 @@ def test_equals_the_two_calls(cuda, orc, B, nh, nkv, hd, K, scratch, cuda_core):
     (2, 32, 8, 64, 1024, 600),     # finished first: few units of small heads in a large cache
     (70, 32, 8, 64, 512, 300),     # four warps per unit
     (60, 64, 8, 128, 512, 200),
+    (57, 8, 8, 64, 512, 100),      # the same with heads of 64: one and four heads per KV head are left to the attention, five are finished
+    (57, 40, 8, 64, 512, 100),
 ])
 def test_equals_the_two_calls_in_large_caches(cuda, orc, B, nh, nkv, hd, K, max_seq):
     equals_the_two_calls(cuda, orc, B, nh, nkv, hd, K, True, False, max_seq, [max_seq - 1 - 173 * b % max_seq for b in range(B)])  # the first to its end
