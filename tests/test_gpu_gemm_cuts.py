@@ -29,10 +29,13 @@ def test_cut_tiles(cuda, orc, M, Ns, K, dtype, shift):
     ws = [_weights(torch, orc, n, K, 1101 + i)[0] for i, n in enumerate(Ns)]
     outs = [torch.full((M * n + 2,), float("nan"), dtype=dt, device="cuda") for n in Ns]
     views = [o[shift:shift + M * n].view(M, n) for o, n in zip(outs, Ns)]  # shift 1: rows that are not aligned to four values
+    scratch = torch.empty(ck.gemm_w4a16_multi_scratch_bytes(M, list(Ns), K), dtype=torch.uint8, device="cuda")
+    before = ck.launch_count()
     if M <= 64:
-        ck.gemm_w4a16_multi(x, ws, K, out_dtype=dt, outs=views)
+        ck.gemm_w4a16_multi(x, ws, K, out_dtype=dt, outs=views, scratch=scratch)
     else:
-        ck.gemm_w4a16_wide(x, ws, K, views)
+        ck.gemm_w4a16_wide(x, ws, K, views, scratch)
+    assert ck.launch_count() - before == (3 if dtype == "bfloat16" else 2)  # tiles are cut: a finishing launch (and the conversion of bf16)
     torch.cuda.synchronize()
     assert ck.gemm_error() == 0
     for o, v, w in zip(outs, views, ws):
@@ -50,7 +53,9 @@ def test_cut_tiles_silu(cuda, orc, M, N, K):
     torch = cuda
     x, g, u = _x(torch, orc, M, K, 1110), _weights(torch, orc, N, K, 1111)[0], _weights(torch, orc, N, K, 1112)[0]
     mid, gate, up = (torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda") for _ in range(3))
+    before = ck.launch_count()
     ck.gemm_w4a16_gateup_silu(x, g, u, K, mid)
+    assert ck.launch_count() - before == 2
     gd, ud = ((x.double() @ _f16_weights(w).t()) for w in (g, u))
     torch.cuda.synchronize()
     assert ck.gemm_error() == 0
