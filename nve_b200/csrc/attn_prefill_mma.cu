@@ -1,6 +1,6 @@
 // Causal attention of a block of new positions (prefill) on the tensor cores: tiles of 64 query rows against tiles
 // of 64 cached positions, online softmax, K/V staged in shared memory once per tile and used by all its rows.  Blocks that fill the
-// SMs with tiles of 128 rows go to attn_prefill_tc.cu (1777 rows 107 -> 46 us); this form is the one for shorter ones.
+// SMs with tiles of 128 rows go to attn_prefill_tc.cu (1777 rows 107 -> 41 us); this form is the one for shorter ones.
 //
 // What bounds it: with one CTA per (row, KV head) every row read the whole K/V prefix through L2 by itself (1777 rows
 // of an 8B model: 1.58 M (row, position) pairs x 512 bytes x 8 KV heads = 6.5 GB per layer); a tile of 64 rows reads

@@ -14,11 +14,12 @@
 // A commit behind S of step j covers every product issued before it, that of P of step j - 1 among them: whoever sees that S may
 // overwrite it and may rescale O.
 //
-// What bounds it: the chain of a step.  8B, 1777 rows: 0.26 of the tensor pipe's cycles; from S to P 2900
+// What bounds it: the chain of a step.  8B, 1777 rows: 0.28 of the tensor pipe's cycles; from S to P 2900
 // cycles (exponentials 2000: both tiles compute them at the same time), the two products with their waits 2000, start and end of a CTA
-// 6000.  Against tiles of 64 rows on mma.sync (us): 1777 rows 107 -> 46, 600 rows 21.7 -> 14.4, 300 rows 11.9 -> 10.0, behind 1000 positions
-// 40.1 -> 25.9; 24 heads over 8, 300 rows at 700 26.3 -> 23.5.  Tried: one thread per row (54.8 with 1777 rows: its chain is twice as long), one
-// warp issuing for both tiles (50.9), the second tile half a step behind the first (41.5 against 40.5), positions split over a cluster of two
+// 6000.  Against tiles of 64 rows on mma.sync (us): 1777 rows 107 -> 41, 600 rows 21.4 -> 13.8, 300 rows 11.9 -> 9.4, behind 1000 positions
+// 39.5 -> 24.7; 24 heads over 8, 300 rows at 700 26.2 -> 23.2.  Tried, where this form took 46 with 1777 rows (a row sum that had to convert P
+// back): one thread per row (54.8: its chain is twice as long), one warp issuing for both tiles (50.9), the second tile half a step behind the first
+// (41.5 against 40.5), positions split over a cluster of two
 // or four (300 rows at 700 21 to 22, but the merge through distributed shared memory makes everything shorter slower, and its code all).
 // Error against 64 bits (2-norm over six random inputs, tiles of 64 / this): 300 rows 2.433e-4 / 2.442e-4, 600 2.474e-4 / 2.484e-4, 1777 2.532e-4 /
 // 2.542e-4, 1000 at 500 2.776e-4 / 2.785e-4; 24 over 8 heads, 300 at 700 2.073e-4 both; heads of 64, 700 rows 2.478e-4 / 2.488e-4, 300 at 400 2.751e-4 /
@@ -127,12 +128,6 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, float* v) {
           "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15]), "=r"(u[16]), "=r"(u[17]), "=r"(u[18]), "=r"(u[19]), "=r"(u[20]),
           "=r"(u[21]), "=r"(u[22]), "=r"(u[23]), "=r"(u[24]), "=r"(u[25]), "=r"(u[26]), "=r"(u[27]), "=r"(u[28]), "=r"(u[29]), "=r"(u[30]), "=r"(u[31])
         : "r"(taddr));
-}
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t* u) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]), "=r"(u[9]), "=r"(u[10]),
-                   "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
-                 : "r"(taddr));
 }
 __device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t* u) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(u[0]),
@@ -583,9 +578,9 @@ bool attn_prefill_tc_try(const AttnParams& p, int head_dim, cudaStream_t st, cud
                                                    (tiles64 > sm ? 2 * p.rows > positions : ctas * 7 < sm * 3 || positions > 2560)))
             return false;
     }
-    // Two tiles in a CTA take 1.4 to 1.5 times as long as one: from two waves of single tiles on, or where a second wave would be as long as
-    // the first (us, one / two: 1000 rows 24.4 / 30.0, at 1000 55.9 / 51.0; 1300 rows 37.3 / 36.0; 1777 rows 59.7 / 46.2; 24 over 8 heads,
-    // whose steps are longer, 1000 rows at 1000 58.4 / 59.8, 1777 rows 56.5 / 53.3).
+    // Two tiles in a CTA take 1.3 to 1.45 times as long as one: from two waves of single tiles on, or where a second wave would be as long as
+    // the first (us, one / two: 1000 rows 23.1 / 25.4, at 500 38.2 / 36.4, at 1000 53.0 / 46.1; 1300 rows 35.8 / 31.0; 1777 rows 56.5 / 40.9; 24 over 8 heads,
+    // whose steps are longer, 1000 rows at 1000 58.0 / 58.3, 1300 rows 32.0 / 39.0, 1777 rows 56.5 / 51.8).
     const int per_cta = ctas > 2 * sm || (ctas > sm && steps >= 12 && !split) ? 2 : 1;
     if (head_dim == 128) return split ? launch_tc<128, true>(p, per_cta, st, err) : launch_tc<128, false>(p, per_cta, st, err);
     return split ? launch_tc<64, true>(p, per_cta, st, err) : launch_tc<64, false>(p, per_cta, st, err);
